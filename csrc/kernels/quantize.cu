@@ -9,87 +9,110 @@
 //          rows are routed one by one (MoE dispatch); the consumer builds the atoms of its tiles from it.
 // The reference has no quantised path; this plays the role of the activation cast in front of its
 // 16-bit GEMMs (iris/ops/matmul_all_reduce.py:95-105 consumes 16-bit tiles directly).
-// One warp per (row, K block): four elements per lane, amax by shuffles, scale = 2^ceil(log2(amax / 448)).
+//
+// Bound by memory (2 bytes in, 1 byte out per 16-bit element). Half a warp takes one (row, K block): eight
+// elements per lane, so a lane's load is 16 bytes (two for fp32) and its store 8, and a warp keeps kUnroll pairs
+// of blocks in flight before it reduces the first: with one block per warp and 8-byte loads the kernel waited on
+// latency (4096 x 8192 bf16: 61 us, now 33). amax by shuffles, scale = 2^ceil(log2(amax / 448)).
 #include <cuda.h>
 #include <cuda_runtime.h>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_fp8.h>
 #include <stdint.h>
+#include <type_traits>
 
 #include "iris/host_api.h"
 
 namespace {
 
+constexpr int kUnroll = 4;      // pairs of blocks a warp has in flight
+
+template <typename T> __device__ __forceinline__ float to_f32(T v);
+template <> __device__ __forceinline__ float to_f32<float>(float v) { return v; }
+template <> __device__ __forceinline__ float to_f32<__nv_bfloat16>(__nv_bfloat16 v) { return __bfloat162float(v); }
+template <> __device__ __forceinline__ float to_f32<__half>(__half v) { return __half2float(v); }
+
+// Eight elements as they lie in memory. vec: 2 the rows are 16-byte aligned, 1 they are aligned to four elements
+// (8 bytes of a 16-bit type), 0 element-wise, as a row's ragged tail always is.
 template <typename T>
-__device__ __forceinline__ void load4(const T* p, int n_valid, bool vec, float (&v)[4]);
-template <>
-__device__ __forceinline__ void load4<float>(const float* p, int n_valid, bool vec, float (&v)[4]) {
-  if (vec && n_valid >= 4) {
-    const float4 f = *(const float4*)p;
-    v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w;
-  } else {
-    for (int i = 0; i < 4; ++i) v[i] = i < n_valid ? p[i] : 0.f;
+struct Raw8 {
+  static constexpr int kWords = (int)sizeof(T) * 8 / 16;
+  uint4 w[kWords];
+  __device__ __forceinline__ void load(const T* p, int n_valid, int vec) {
+    if (vec == 2 && n_valid >= 8) {
+#pragma unroll
+      for (int i = 0; i < kWords; ++i) w[i] = ((const uint4*)p)[i];
+    } else if (vec == 1 && n_valid >= 8) {
+#pragma unroll
+      for (int i = 0; i < 2 * kWords; ++i) ((uint2*)w)[i] = ((const uint2*)p)[i];
+    } else {
+      T* e = (T*)w;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) e[i] = i < n_valid ? p[i] : T(0.f);
+    }
   }
-}
-template <>
-__device__ __forceinline__ void load4<__nv_bfloat16>(const __nv_bfloat16* p, int n_valid, bool vec, float (&v)[4]) {
-  if (vec && n_valid >= 4) {
-    const uint2 u = *(const uint2*)p;
-    const float2 a = __bfloat1622float2(*(const __nv_bfloat162*)&u.x), b = __bfloat1622float2(*(const __nv_bfloat162*)&u.y);
-    v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
-  } else {
-    for (int i = 0; i < 4; ++i) v[i] = i < n_valid ? __bfloat162float(p[i]) : 0.f;
-  }
-}
-template <>
-__device__ __forceinline__ void load4<__half>(const __half* p, int n_valid, bool vec, float (&v)[4]) {
-  if (vec && n_valid >= 4) {
-    const uint2 u = *(const uint2*)p;
-    const float2 a = __half22float2(*(const __half2*)&u.x), b = __half22float2(*(const __half2*)&u.y);
-    v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
-  } else {
-    for (int i = 0; i < 4; ++i) v[i] = i < n_valid ? __half2float(p[i]) : 0.f;
-  }
-}
+  __device__ __forceinline__ float get(int i) const { return to_f32<T>(((const T*)w)[i]); }
+};
 
 template <typename T>
 __global__ void __launch_bounds__(256) quantize_1x128_pow2_kernel(const T* __restrict__ x, int64_t ldx, uint8_t* __restrict__ q, int64_t ldq,
                                                                    float* __restrict__ scale, uint8_t* __restrict__ atoms,
-                                                                   uint8_t* __restrict__ rows, int64_t ld_rows, int M, int K, int KB,
-                                                                   int aligned) {
+                                                                   uint8_t* __restrict__ rows, int64_t ld_rows, int M, int M_pad, int K, int KB,
+                                                                   int x_aligned, int q_aligned) {
   const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (warp >= (int64_t)M * KB) return;
-  const int row = (int)(warp / KB), kb = (int)(warp - (int64_t)row * KB);
-  const int k0 = kb * 128 + lane * 4;
-  const int n_valid = max(0, min(4, K - k0));
-  float v[4];
-  load4<T>(x + (int64_t)row * ldx + k0, n_valid, aligned != 0, v);   // unaligned rows take the element-wise path
-  float amax = fmaxf(fmaxf(fabsf(v[0]), fabsf(v[1])), fmaxf(fabsf(v[2]), fabsf(v[3])));
+  const int lane = threadIdx.x & 31, half = lane >> 4, sub = lane & 15;
+  const int64_t units = (int64_t)M_pad * KB, u0 = warp * (2 * kUnroll);
+  if (u0 >= units) return;
+  const int64_t first = u0 + half;
+  int row = (int)(first / KB), kb = (int)(first - (int64_t)row * KB);
+  int rows_u[kUnroll], kbs_u[kUnroll];
+  Raw8<T> raw[kUnroll];
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-  amax = fmaxf(amax, 1e-12f);
-  // smallest power of two >= amax / 448, as an exponent
-  int e = (int)ceilf(log2f(amax * (1.0f / 448.0f)));
-  e = max(-127, min(127, e));
-  const float s = exp2f((float)e), inv = exp2f((float)-e);
-  uint32_t packed = 0;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const __nv_fp8_e4m3 f(fminf(fmaxf(v[i] * inv, -448.f), 448.f));
-    packed |= (uint32_t)f.__x << (8 * i);
+  for (int i = 0; i < kUnroll; ++i) {
+    rows_u[i] = row; kbs_u[i] = kb;
+    const int k0 = kb * 128 + sub * 8;
+    const int n_valid = row < M ? max(0, min(8, K - k0)) : 0;
+    raw[i].load(x + (int64_t)row * ldx + k0, n_valid, x_aligned);
+    for (kb += 2; kb >= KB; kb -= KB) ++row;
   }
-  uint8_t* dst = q + (int64_t)row * ldq + k0;
-  if (n_valid == 4 && (ldq & 3) == 0) *(uint32_t*)dst = packed;
-  else for (int i = 0; i < n_valid; ++i) dst[i] = (uint8_t)(packed >> (8 * i));
-  if (lane == 0) {
-    if (scale) scale[(int64_t)row * KB + kb] = s;
-    if (rows) rows[(int64_t)row * ld_rows + kb] = (uint8_t)(e + 127);
-    if (atoms) {
-      const uint32_t b = (uint32_t)(e + 127);
-      const int tile = row >> 7, r = row & 127;
-      *(uint32_t*)(atoms + ((int64_t)tile * KB + kb) * 512 + (r & 31) * 16 + (r >> 5) * 4) = b * 0x01010101u;
+#pragma unroll
+  for (int i = 0; i < kUnroll; ++i) {
+    const int r = rows_u[i], b = kbs_u[i];
+    float amax = 0.f;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) amax = fmaxf(amax, fabsf(raw[i].get(j)));
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+    amax = fmaxf(amax, 1e-12f);
+    // smallest power of two >= amax / 448, as an exponent
+    int e = (int)ceilf(log2f(amax * (1.0f / 448.0f)));
+    e = max(-127, min(127, e));
+    const float s = exp2f((float)e), inv = exp2f((float)-e);
+    if (r < M) {
+      uint32_t packed[2] = {0u, 0u};
+#pragma unroll
+      for (int j = 0; j < 8; j += 2) {
+        const float2 v = make_float2(fminf(fmaxf(raw[i].get(j) * inv, -448.f), 448.f), fminf(fmaxf(raw[i].get(j + 1) * inv, -448.f), 448.f));
+        packed[j >> 2] |= (uint32_t)__nv_cvt_float2_to_fp8x2(v, __NV_SATFINITE, __NV_E4M3) << (8 * (j & 3));
+      }
+      const int k0 = b * 128 + sub * 8, n_valid = max(0, min(8, K - k0));
+      uint8_t* dst = q + (int64_t)r * ldq + k0;
+      if (n_valid == 8 && q_aligned == 2) {
+        *(uint2*)dst = make_uint2(packed[0], packed[1]);
+      } else if (n_valid == 8 && q_aligned == 1) {
+        ((uint32_t*)dst)[0] = packed[0]; ((uint32_t*)dst)[1] = packed[1];
+      } else
+        for (int j = 0; j < n_valid; ++j) dst[j] = (uint8_t)(packed[j >> 2] >> (8 * (j & 3)));
+      if (sub == 0) {
+        if (scale) scale[(int64_t)r * KB + b] = s;
+        if (rows) rows[(int64_t)r * ld_rows + b] = (uint8_t)(e + 127);
+      }
+    }
+    if (sub == 0 && atoms && r < M_pad) {
+      const uint32_t byte = r < M ? (uint32_t)(e + 127) : 127u;      // rows past M: scale 1
+      const int tile = r >> 7, rr = r & 127;
+      *(uint32_t*)(atoms + ((int64_t)tile * KB + b) * 512 + (rr & 31) * 16 + (rr >> 5) * 4) = byte * 0x01010101u;
     }
   }
 }
@@ -98,23 +121,30 @@ __global__ void __launch_bounds__(256) quantize_1x128_pow2_kernel(const T* __res
 
 // x: [M, K] of `dtype` (IRIS_F32 / IRIS_BF16 / IRIS_F16), row pitch ldx elements. q: [M, K] bytes, pitch ldq.
 // scale (may be null): [M, ceil(K / 128)] fp32. atoms (may be null): [ceil(M / 128), ceil(K / 128), 512] bytes;
-// rows past M inside the last 128-row tile are NOT written (pre-fill the buffer with 127 = scale 1 if M is ragged).
+// rows past M inside the last 128-row tile are written as 127 (scale 1).
 static int quantize_launch(const void* x, int64_t ldx, int32_t dtype, void* q, int64_t ldq, float* scale, void* atoms, void* rows,
                            int64_t ld_rows, int32_t M, int32_t K, void* stream) {
   if (M <= 0 || K <= 0) return 0;
   const int KB = (K + 127) / 128;
-  const int64_t warps = (int64_t)M * KB;
+  const int M_pad = atoms ? (int)(((int64_t)M + 127) / 128 * 128) : M;
+  const int64_t warps = ((int64_t)M_pad * KB + 2 * kUnroll - 1) / (2 * kUnroll);
   const int64_t blocks = (warps * 32 + 255) / 256;
   if (blocks > 0x7fffffffll) return -3;
   cudaStream_t s = (cudaStream_t)stream;
   const int esz = dtype == IRIS_F32 ? 4 : 2;
-  const int aligned = (((uintptr_t)x % (4 * esz)) == 0 && (ldx * esz) % (4 * esz) == 0) ? 1 : 0;
-  if (dtype == IRIS_F32)
-    quantize_1x128_pow2_kernel<float><<<(unsigned)blocks, 256, 0, s>>>((const float*)x, ldx, (uint8_t*)q, ldq, scale, (uint8_t*)atoms, (uint8_t*)rows, ld_rows, M, K, KB, aligned);
-  else if (dtype == IRIS_BF16)
-    quantize_1x128_pow2_kernel<__nv_bfloat16><<<(unsigned)blocks, 256, 0, s>>>((const __nv_bfloat16*)x, ldx, (uint8_t*)q, ldq, scale, (uint8_t*)atoms, (uint8_t*)rows, ld_rows, M, K, KB, aligned);
-  else if (dtype == IRIS_F16)
-    quantize_1x128_pow2_kernel<__half><<<(unsigned)blocks, 256, 0, s>>>((const __half*)x, ldx, (uint8_t*)q, ldq, scale, (uint8_t*)atoms, (uint8_t*)rows, ld_rows, M, K, KB, aligned);
+  auto level = [](const void* p, int64_t pitch, int big, int small) {     // alignment of every row start
+    const uint64_t bits = (uint64_t)(uintptr_t)p | (uint64_t)pitch;
+    return bits % big == 0 ? 2 : (bits % small == 0 ? 1 : 0);
+  };
+  const int xa = level(x, ldx * esz, 16, 8), qa = level(q, ldq, 8, 4);
+  auto run = [&](auto* typed) {
+    using T = std::remove_cv_t<std::remove_pointer_t<decltype(typed)>>;
+    quantize_1x128_pow2_kernel<T><<<(unsigned)blocks, 256, 0, s>>>(typed, ldx, (uint8_t*)q, ldq, scale, (uint8_t*)atoms, (uint8_t*)rows,
+                                                                   ld_rows, M, M_pad, K, KB, xa, qa);
+  };
+  if (dtype == IRIS_F32) run((const float*)x);
+  else if (dtype == IRIS_BF16) run((const __nv_bfloat16*)x);
+  else if (dtype == IRIS_F16) run((const __half*)x);
   else
     return -2;
   return cudaGetLastError() == cudaSuccess ? 0 : -21;

@@ -269,7 +269,7 @@ def quantize_activation(x: torch.Tensor, out: BlockScaled | None = None) -> Bloc
     else:
         q = torch.empty((M, K), dtype=FP8, device=x.device)
         scale = torch.empty((M, kb), dtype=torch.float32, device=x.device)
-        atoms = torch.full((mt, kb, 512), 127, dtype=torch.uint8, device=x.device)   # rows past M: scale 1
+        atoms = torch.empty((mt, kb, 512), dtype=torch.uint8, device=x.device)       # the kernel writes rows past M too (scale 1)
         out = BlockScaled(q, scale, "activation").set_sf(atoms)
     lib = _lib.kernels()
     if not getattr(lib, "_iris_quant_typed", False):
