@@ -17,7 +17,11 @@ unfused path of ``iris_b200.ops`` automatically.
 """
 from __future__ import annotations
 
+import ctypes as C
+
 import torch
+
+from .. import _lib
 
 _ACTS = {
     None: (lambda x: x, lambda x: torch.ones_like(x)),
@@ -36,6 +40,42 @@ def _act_grad(name, x):
     return _ACTS[name][1](x.float()).to(x.dtype)
 
 
+_ACT_CODE = {"silu": 1, "gelu": 2}
+
+
+def _native(*tensors) -> bool:
+    """16-bit contiguous CUDA tensors on 16-byte boundaries: what ``csrc/kernels/activation.cu`` takes."""
+    return all(t.is_cuda and t.dtype in (torch.bfloat16, torch.float16) and t.dtype == tensors[0].dtype and t.is_contiguous()
+               and t.data_ptr() % 16 == 0 for t in tensors)
+
+
+def _activation_launch(name, pre, dh, h, dpre) -> None:
+    lib = _lib.kernels()
+    if not getattr(lib, "_iris_act_typed", False):
+        lib.iris_activation.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64, C.c_int32, C.c_int32, C.c_void_p]
+        lib.iris_activation.restype = C.c_int
+        lib._iris_act_typed = True
+    _lib.check(lib.iris_activation(pre.data_ptr(), None if dh is None else dh.data_ptr(), h.data_ptr(), None if dpre is None else dpre.data_ptr(),
+                                   pre.numel(), _ACT_CODE[name], _lib.DTYPE_CODE[pre.dtype], _lib.current_stream_ptr()), "activation launch", kernels=1)
+
+
+def _act_forward(name, pre):
+    if not _native(pre):
+        return _ACTS[name][0](pre)
+    h = torch.empty_like(pre)
+    _activation_launch(name, pre, None, h, None)
+    return h
+
+
+def _act_backward(name, dh, pre):
+    """``(dh * act'(pre), act(pre))``: the gradient in front of the activation and the activation itself."""
+    if not _native(pre, dh):
+        return dh * _act_grad(name, pre), _ACTS[name][0](pre)
+    h, dpre = torch.empty_like(pre), torch.empty_like(dh)
+    _activation_launch(name, pre, dh, h, dpre)
+    return dpre, h
+
+
 class _TPMLPFunction(torch.autograd.Function):
     @staticmethod
     def forward(fctx, x, w1, w2, layer):
@@ -45,7 +85,7 @@ class _TPMLPFunction(torch.autograd.Function):
         xd, w1d, w2d = x.detach(), w1.detach(), w2.detach()
         h_pre = torch.empty(W * M_local, F, dtype=x.dtype, device=x.device)
         layer._ws["ag1"] = ctx.ops.all_gather_matmul(h_pre, xd, w1d, shard_dim=0, workspace=layer._ws.get("ag1"), async_op=True)
-        h = _ACTS[layer.activation][0](h_pre) if layer.activation else h_pre
+        h = _act_forward(layer.activation, h_pre) if layer.activation else h_pre
         y = torch.empty(M_local, K, dtype=x.dtype, device=x.device)
         layer._ws["rs1"] = ctx.ops.matmul_reduce_scatter(y, h, w2d, scatter_rows=True, workspace=layer._ws.get("rs1"), async_op=True)
         fctx.layer = layer
@@ -63,8 +103,9 @@ class _TPMLPFunction(torch.autograd.Function):
         # dH = all_gather(dY) @ W2^T (W2^T is the K-major view the kernel takes without a copy)
         dh = torch.empty(W * M_local, F, dtype=x.dtype, device=x.device)
         layer._ws["ag2"] = ctx.ops.all_gather_matmul(dh, dy, w2.t(), shard_dim=0, workspace=layer._ws.get("ag2"), async_op=True)
+        h = h_pre
         if layer.activation:
-            dh = dh * _act_grad(layer.activation, h_pre)
+            dh, h = _act_backward(layer.activation, dh, h_pre)
         # dX = reduce_scatter(dH @ W1^T)
         dx = torch.empty(M_local, K, dtype=x.dtype, device=x.device)
         layer._ws["rs2"] = ctx.ops.matmul_reduce_scatter(dx, dh, w1.t(), scatter_rows=True, workspace=layer._ws.get("rs2"), async_op=True)
@@ -77,7 +118,6 @@ class _TPMLPFunction(torch.autograd.Function):
             ctx.ccl.all_gather(dy_all, dy_loc, async_op=True)
         else:
             x_all, dy_all = x, dy
-        h = _ACTS[layer.activation][0](h_pre) if layer.activation else h_pre
         dw1 = x_all.t() @ dh
         dw2 = h.t() @ dy_all
         return dx, dw1, dw2, None
