@@ -14,7 +14,8 @@
 //                count to the owner's arrival counter for that expert; GEMM CTAs (tcgen05 main
 //                loop) wait for an expert's arrivals, then multiply its rows by the expert's fused
 //                gate|up weight and write silu(gate) * up
-//                (the fusion the reference leaves as NotImplementedError, moe.py:285-286)
+//                (the fusion the reference leaves as NotImplementedError, moe.py:285-286).
+//                One rank: a gather kernel copies the rows into expert order first, and all CTAs are GEMM CTAs
 //   5 grouped GEMM 2 + combine, ONE kernel: down projection whose epilogue stores every output row
 //                straight into the (token, k) slot of the token's home rank; cross-rank round at exit
 //   6 reduce     out[t] = sum_k weight[t, k] * slot[t, k]   (the reference's sum is unweighted)
@@ -53,23 +54,30 @@ struct MoeMeta {
 };
 
 // ------------------------------------------------------------------------------------ 1 router
-__global__ void router_topk_kernel(const float* __restrict__ logits, MoeDims dm, MoeMeta m) {
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  if (warp >= dm.T) return;
-  const float* row = logits + (size_t)warp * dm.E;
-  constexpr int kPer = 32;   // up to 1024 experts
+// One warp, one token: top-k of its E logits (kPer per lane), softmax over the k selected. Lane k < K returns with
+// the k-th choice and its weight. A logit of -inf (a masked expert) or NaN ranks last but is an expert all the same:
+// with fewer than K others it is chosen, lowest index first, so an index is always in range.
+template <int kPer>
+__device__ __forceinline__ void route_token(const float* __restrict__ row, int E, int K, int lane, int& my_i, float& my_w) {
   float v[kPer];
-  const int per = (dm.E + 31) / 32;
+  unsigned avail = 0;
 #pragma unroll
-  for (int i = 0; i < kPer; ++i) v[i] = (i < per && lane + i * 32 < dm.E) ? row[lane + i * 32] : -INFINITY;
-  float sel_v[kMaxTopK];
-  int sel_i[kMaxTopK];
-  for (int k = 0; k < dm.K; ++k) {
+  for (int i = 0; i < kPer; ++i) {
+    const bool in = lane + i * 32 < E;
+    const float x = in ? row[lane + i * 32] : -INFINITY;
+    v[i] = x == x ? x : -INFINITY;
+    avail |= (in ? 1u : 0u) << i;
+  }
+  float my_v = -INFINITY;
+  my_i = 0;
+  for (int k = 0; k < K; ++k) {
     float best = -INFINITY;
     int bi = 0x7fffffff;
 #pragma unroll
-    for (int i = 0; i < kPer; ++i)
-      if (i < per && v[i] > best) { best = v[i]; bi = lane + i * 32; }
+    for (int i = 0; i < kPer; ++i) {
+      const int e = lane + i * 32;
+      if (((avail >> i) & 1u) && (v[i] > best || (v[i] == best && e < bi))) { best = v[i]; bi = e; }
+    }
     // warp arg-max, ties to the lower expert index
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -77,22 +85,37 @@ __global__ void router_topk_kernel(const float* __restrict__ logits, MoeDims dm,
       const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
       if (ob > best || (ob == best && oi < bi)) { best = ob; bi = oi; }
     }
-    sel_v[k] = best; sel_i[k] = bi;
-    if ((bi & 31) == lane) {
-#pragma unroll
-      for (int i = 0; i < kPer; ++i)
-        if (i == (bi >> 5)) v[i] = -INFINITY;
+    if (lane == k) { my_v = best; my_i = bi; }
+    if ((bi & 31) == lane) avail &= ~(1u << (bi >> 5));
+  }
+  const float ex = __expf(my_v - __shfl_sync(0xffffffffu, my_v, 0));
+  float sum = 0.f;
+  for (int k = 0; k < K; ++k) sum += __shfl_sync(0xffffffffu, ex, k);
+  my_w = ex / sum;
+}
+
+// Blocks walk the tokens and count their choices in shared memory; a block adds its histogram to the global one
+// once per expert. With one global atomic per (token, k) the counters were the bottleneck: 4096 tokens, 32 experts,
+// top-8: 36 us, now 11.
+template <int kPer>
+__global__ void __launch_bounds__(512) router_topk_kernel(const float* __restrict__ logits, MoeDims dm, MoeMeta m) {
+  __shared__ int32_t hist[1024];
+  const int lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
+  for (int e = threadIdx.x; e < dm.E; e += blockDim.x) hist[e] = 0;
+  __syncthreads();
+  for (int t = blockIdx.x * wpb + (threadIdx.x >> 5); t < dm.T; t += gridDim.x * wpb) {
+    int my_i;
+    float my_w;
+    route_token<kPer>(logits + (size_t)t * dm.E, dm.E, dm.K, lane, my_i, my_w);
+    if (lane < dm.K) {
+      m.topk_idx[(size_t)t * dm.K + lane] = my_i;
+      m.topk_w[(size_t)t * dm.K + lane] = my_w;
+      atomicAdd(&hist[my_i], 1);
     }
   }
-  if (lane == 0) {
-    float mx = sel_v[0], sum = 0.f;
-    for (int k = 0; k < dm.K; ++k) sum += __expf(sel_v[k] - mx);
-    for (int k = 0; k < dm.K; ++k) {
-      m.topk_idx[(size_t)warp * dm.K + k] = sel_i[k];
-      m.topk_w[(size_t)warp * dm.K + k] = __expf(sel_v[k] - mx) / sum;
-      atomicAdd(&m.counts_local[sel_i[k]], 1);
-    }
-  }
+  __syncthreads();
+  for (int e = threadIdx.x; e < dm.E; e += blockDim.x)
+    if (hist[e]) atomicAdd(&m.counts_local[e], hist[e]);
 }
 
 // ------------------------------------------------------------------------------------ 2 meta
@@ -156,16 +179,60 @@ __global__ void __launch_bounds__(1024) moe_meta_kernel(const __grid_constant__ 
 }
 
 // ------------------------------------------------------------------------------------ 3 sort
-__global__ void moe_sort_kernel(MoeDims dm, MoeMeta m) {
+// A block counts its pairs per expert in shared memory, reserves that many places of each bucket with one global
+// atomic per expert, and places its pairs behind them (32768 pairs, 32 experts: 11 us with an atomic per pair, now 4).
+// With one rank the bucket position is also the pair's inbox row: it is kept in `pos_of` for the gather.
+__global__ void __launch_bounds__(256) moe_sort_kernel(MoeDims dm, MoeMeta m, int32_t* pos_of) {
+  __shared__ int32_t cnt[1024], base[1024];
+  for (int e = threadIdx.x; e < dm.E; e += blockDim.x) cnt[e] = 0;
+  __syncthreads();
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= dm.T * dm.K) return;
-  const int e = m.topk_idx[p];
-  const int pos = atomicAdd(&m.cursor[e], 1);
-  m.sorted_pairs[m.list_off[e] + pos] = p;
+  int e = 0, local = 0;
+  if (p < dm.T * dm.K) {
+    e = m.topk_idx[p];
+    local = atomicAdd(&cnt[e], 1);
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < dm.E; i += blockDim.x)
+    if (cnt[i]) base[i] = m.list_off[i] + atomicAdd(&m.cursor[i], cnt[i]);
+  __syncthreads();
+  if (p < dm.T * dm.K) {
+    const int pos = base[e] + local;
+    m.sorted_pairs[pos] = p;
+    if (pos_of) pos_of[p] = pos;
+  }
 }
 __global__ void moe_clear_kernel(MoeDims dm, MoeMeta m) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < dm.E) m.counts_local[i] = 0;
+}
+
+// ------------------------------------------------------------------------------------ 4' gather (one rank)
+// With one rank every pair's row stays here, so nothing is sent: the token rows are copied into expert order by a
+// kernel of their own and the grouped GEMM runs on every SM. The communication CTAs of the multi-rank form cost the
+// GEMM 16 of 148 SMs for its whole run, and with few tokens their chain of one release per expert was what it waited
+// for (64 tokens, 32 experts, e4m3: stage 1 306 us, now 199; 4096 tokens bf16: 1808 us, now 1538 plus 89 for
+// this copy, which is bound by the 470 MB it writes). A block reads a piece of one token's row once and stores it to the
+// token's K rows.
+__global__ void __launch_bounds__(256) moe_gather_kernel(const uint8_t* __restrict__ x, uint8_t* __restrict__ inbox, int row16,
+                                                         const uint8_t* __restrict__ x_sf, uint8_t* __restrict__ inbox_sf, int sf16,
+                                                         const int32_t* __restrict__ pos_of, int K, int capacity) {
+  __shared__ int32_t dst[kMaxTopK];
+  const int t = blockIdx.x;
+  if (threadIdx.x < K) dst[threadIdx.x] = pos_of[(size_t)t * K + threadIdx.x];
+  __syncthreads();
+  const uint4* src = (const uint4*)x + (size_t)t * row16;
+  for (int c = blockIdx.y * blockDim.x + threadIdx.x; c < row16; c += gridDim.y * blockDim.x) {
+    const uint4 v = __ldg(src + c);
+    for (int k = 0; k < K; ++k)
+      if (dst[k] < capacity) ((uint4*)inbox)[(size_t)dst[k] * row16 + c] = v;
+  }
+  if (sf16 && blockIdx.y == 0) {
+    for (int u = threadIdx.x; u < sf16 * K; u += blockDim.x) {
+      const int k = u / sf16, c = u - k * sf16;
+      if (dst[k] < capacity) ((uint4*)inbox_sf)[(size_t)dst[k] * sf16 + c] = ((const uint4*)x_sf)[(size_t)t * sf16 + c];
+    }
+  }
 }
 
 // ------------------------------------------------------------------ 4/5 grouped GEMM policies
@@ -226,7 +293,7 @@ struct GroupedGemm : Common {
     if (kb == 0) {
       st.j = expert_of(tm);
       st.row0 = meta.expert_row0[st.j] + (tm - meta.tile_prefix[st.j]) * kBM;
-      if (kStage == 1 && st.key != st.j) {
+      if (kStage == 1 && ctx.world > 1 && st.key != st.j) {     // one rank: the gather kernel ran before
         if (!wait_flag_ge(ctx, meta.arrived + st.j, meta.expected_cum[st.j])) return false;
         st.key = st.j;
         ptx::fence_proxy_async();
@@ -282,7 +349,7 @@ struct GroupedGemm : Common {
       const int row = st.row0 + quarter * 32 + lane;
       unsigned long long ptr = 0;
       if (row < st.rows_end) {
-        const long long mt = meta.inbox_meta[row];
+        const long long mt = ctx.world > 1 ? meta.inbox_meta[row] : (long long)meta.sorted_pairs[row];
         const int src = (int)(mt >> 32), pair = (int)(mt & 0xffffffffll);
         ptr = (unsigned long long)ctx.remote(comb + (size_t)pair * dm.D * 2, src);      // the combine buffer stays 16-bit
       }
@@ -404,15 +471,29 @@ struct GroupedGemm : Common {
 };
 
 // ------------------------------------------------------------------------------------ 6 reduce
-__global__ void moe_reduce_kernel(const __nv_bfloat16* __restrict__ comb, const float* __restrict__ w, __nv_bfloat16* out,
-                                  int T, int K, int D) {
+// Bound by the K rows it reads per token. One thread per eight columns of a token, the loads of all K rows issued
+// before the first is used (64 tokens of 7168, top-8: 12 us with one block per token, now 5; 4096 tokens: 80 us, the time
+// its 530 MB take).
+__global__ void __launch_bounds__(128) moe_reduce_kernel(const __nv_bfloat16* __restrict__ comb, const float* __restrict__ w, __nv_bfloat16* out,
+                                                         int T, int K, int D) {
+  __shared__ float s_w[kMaxTopK];
   const int t = blockIdx.x;
-  for (int c = threadIdx.x * 8; c < D; c += blockDim.x * 8) {
-    float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    for (int k = 0; k < K; ++k) {
-      const float wk = w[(size_t)t * K + k];
-      const uint4 v = __ldcg((const uint4*)(comb + ((size_t)t * K + k) * D + c));
-      const __nv_bfloat162* h = (const __nv_bfloat162*)&v;
+  if (threadIdx.x < K) s_w[threadIdx.x] = w[(size_t)t * K + threadIdx.x];
+  __syncthreads();
+  const int c = (blockIdx.y * blockDim.x + threadIdx.x) * 8;
+  if (c >= D) return;
+  const __nv_bfloat16* rows = comb + (size_t)t * K * D + c;
+  float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+  for (int k0 = 0; k0 < K; k0 += 8) {
+    uint4 v[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      if (k0 + i < K) v[i] = __ldcg((const uint4*)(rows + (size_t)(k0 + i) * D));
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      if (k0 + i >= K) break;
+      const float wk = s_w[k0 + i];
+      const __nv_bfloat162* h = (const __nv_bfloat162*)&v[i];
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
         const float2 f = __bfloat1622float2(h[q]);
@@ -420,12 +501,12 @@ __global__ void moe_reduce_kernel(const __nv_bfloat16* __restrict__ comb, const 
         acc[2 * q + 1] += wk * f.y;
       }
     }
-    uint4 o;
-    __nv_bfloat162* oh = (__nv_bfloat162*)&o;
-#pragma unroll
-    for (int q = 0; q < 4; ++q) oh[q] = __floats2bfloat162_rn(acc[2 * q], acc[2 * q + 1]);
-    *(uint4*)(out + (size_t)t * D + c) = o;
   }
+  uint4 o;
+  __nv_bfloat162* oh = (__nv_bfloat162*)&o;
+#pragma unroll
+  for (int q = 0; q < 4; ++q) oh[q] = __floats2bfloat162_rn(acc[2 * q], acc[2 * q + 1]);
+  *(uint4*)(out + (size_t)t * D + c) = o;
 }
 
 }  // namespace
@@ -457,24 +538,42 @@ typedef struct IrisMoeDesc {
   void* H_sf;               // [capacity, sf_ld2]
   const void* w13_sf;       // scale atoms of w13: [El][2F / 256][D / 128][2][512]
   const void* w2_sf;        // scale atoms of w2:  [El][ceil(D / 224)][F / 128][2][512]
+  int32_t* pos_of;          // [T * K] one rank only: inbox row of each (token, k) pair
 } IrisMoeDesc;
 
 int iris_moe_forward(const IrisMoeDesc* d, void* stream_) {
   cudaStream_t s = (cudaStream_t)stream_;
-  if (d->K > kMaxTopK || d->E > 1024 || d->E % d->ctx.world || d->D % 64 || d->F % 128 || d->D % 256) return -3;
+  if (d->K > kMaxTopK || d->E > 1024 || d->E % d->ctx.world || d->D % 64 || d->F % 128 || d->D % 256 || d->K > d->E || d->K < 1) return -3;
+  if (d->T <= 0) return -21;
   DeviceContext ctx;
   memcpy(&ctx, &d->ctx, sizeof(ctx));
   MoeDims dm{d->T, d->K, d->E, d->El, d->D, d->F, d->capacity};
   MoeMeta m{d->topk_idx, d->topk_w, d->counts_local, d->counts_all, d->cursor, d->list_off, d->sorted_pairs, d->my_off,
             d->expert_rows, d->expert_row0, d->tile_prefix, d->expected_cum, d->arrived, (long long*)d->inbox_meta};
   moe_clear_kernel<<<(d->E + 255) / 256, 256, 0, s>>>(dm, m);
-  router_topk_kernel<<<(d->T * 32 + 255) / 256, 256, 0, s>>>(d->logits, dm, m);
+  const int sms = sm_count();
+  {
+    const int warps = d->T > 16 * sms ? 16 : 4;      // warps per block: few tokens spread over more SMs
+    const int blocks = ceil_div(d->T, warps) < sms ? ceil_div(d->T, warps) : sms;
+    auto* router = d->E <= 32 ? router_topk_kernel<1> : d->E <= 64 ? router_topk_kernel<2> : d->E <= 128 ? router_topk_kernel<4>
+                   : d->E <= 256 ? router_topk_kernel<8> : router_topk_kernel<32>;
+    router<<<blocks, warps * 32, 0, s>>>(d->logits, dm, m);
+  }
   moe_meta_kernel<<<1, 1024, 0, s>>>(ctx, (SyncBlock*)d->sync_meta, dm, m);
-  moe_sort_kernel<<<(d->T * d->K + 255) / 256, 256, 0, s>>>(dm, m);
+  const bool one_rank = ctx.world <= 1;
+  int32_t* pos_of = one_rank ? d->pos_of : nullptr;
+  if (one_rank && (!pos_of || ((uintptr_t)d->x & 15))) return -11;
+  moe_sort_kernel<<<ceil_div(d->T * d->K, 256), 256, 0, s>>>(dm, m, pos_of);
+  if (one_rank) {
+    const int row16 = d->D * (d->fp8 ? 1 : 2) / 16;
+    int split = ceil_div(4 * sms, d->T);
+    if (split > ceil_div(row16, 256)) split = ceil_div(row16, 256);
+    moe_gather_kernel<<<dim3(d->T, split), 256, 0, s>>>((const uint8_t*)d->x, (uint8_t*)d->inbox, row16, (const uint8_t*)d->x_sf,
+                                                        (uint8_t*)d->inbox_sf, d->fp8 ? d->sf_ld1 / 16 : 0, pos_of, d->K, d->capacity);
+  }
   if (cudaGetLastError() != cudaSuccess) return -21;
 
-  const int sms = sm_count();
-  const int comm = ctx.world > 0 ? (d->comm_ctas > 0 ? d->comm_ctas : 16) : 0;
+  const int comm = one_rank ? 0 : (d->comm_ctas > 0 ? d->comm_ctas : 16);
   const bool km = d->weights_kmajor != 0;
   auto common = [&](auto& pol, int bn, int N, int Kdim, bool f8) {
     pol.sh = Shape{d->capacity, N, Kdim};
@@ -551,7 +650,7 @@ int iris_moe_forward(const IrisMoeDesc* d, void* stream_) {
     if (r) return r;
   }
   }
-  moe_reduce_kernel<<<d->T, 256, 0, s>>>((const __nv_bfloat16*)d->comb, d->topk_w, (__nv_bfloat16*)d->out, d->T, d->K, d->D);
+  moe_reduce_kernel<<<dim3(d->T, ceil_div(d->D, 1024)), 128, 0, s>>>((const __nv_bfloat16*)d->comb, d->topk_w, (__nv_bfloat16*)d->out, d->T, d->K, d->D);
   return cudaGetLastError() == cudaSuccess ? 0 : -21;
 }
 

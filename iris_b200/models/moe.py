@@ -5,8 +5,8 @@ Every rank holds ``num_experts / W`` experts (SwiGLU FFN: gate/up ``[hidden, ffn
 experts (softmax over the selected k logits), moves the token rows to the experts' owners, runs
 the expert FFNs as grouped GEMMs and returns the weighted sum of the k expert outputs in token
 order. On a GPU the whole pass is the launch sequence of ``csrc/kernels/moe.cu`` on the current
-stream, with the dispatch fused into the first grouped GEMM and the combine fused into the second
-one's epilogue; the reference pipeline with its host barriers and Python-side metadata is
+stream, with the dispatch fused into the first grouped GEMM (on one rank: a gather in front of it) and the
+combine fused into the second one's epilogue; the reference pipeline with its host barriers and Python-side metadata is
 examples/31_expert_sharded_moe/moe.py:195-328. Weights are bf16, or (``fp8=True``) e4m3 with
 128 x 128 power-of-two block scales: then the tokens are quantised to e4m3 with 1 x 128 scales before
 the dispatch (half the bytes on the wire), both grouped GEMMs run on the tensor core's block-scaled
@@ -38,6 +38,7 @@ class IrisMoeDesc(C.Structure):
         ("weights_kmajor", C.c_int32),
         ("fp8", C.c_int32), ("sf_ld1", C.c_int32), ("sf_ld2", C.c_int32),
         ("x_sf", C.c_void_p), ("inbox_sf", C.c_void_p), ("H_sf", C.c_void_p), ("w13_sf", C.c_void_p), ("w2_sf", C.c_void_p),
+        ("pos_of", C.c_void_p),
     ]
 
 
@@ -115,6 +116,7 @@ class MoELayer:
         z = lambda n: torch.zeros(n, dtype=i32, device=dev)  # noqa: E731
         self.counts_local, self.cursor, self.list_off, self.my_off = z(num_experts), z(num_experts), z(num_experts + 1), z(num_experts)
         self.sorted_pairs = z(pairs)
+        self.pos_of = z(pairs) if W == 1 else None
         self.expert_rows, self.expert_row0, self.tile_prefix, self.expected_cum = z(El), z(El + 1), z(El + 1), z(El)
         ctx.barrier()
 
@@ -198,7 +200,8 @@ class MoELayer:
                      "expert_rows", "expert_row0", "tile_prefix", "expected_cum", "arrived", "inbox_meta"):
             setattr(d, name, getattr(self, name).data_ptr())
         d.weights_kmajor = 1
-        _lib.check(self._lib().iris_moe_forward(C.byref(d), C.c_void_p(_lib.current_stream_ptr())), "MoE forward launch", kernels=7)
+        d.pos_of = self.pos_of.data_ptr() if self.pos_of is not None else None
+        _lib.check(self._lib().iris_moe_forward(C.byref(d), C.c_void_p(_lib.current_stream_ptr())), "MoE forward launch", kernels=7 if self.pos_of is None else 8)
         self._keep = logits
         return out
 
