@@ -1,30 +1,36 @@
 // Ring attention with tcgen05 attention CTAs (the communication CTAs are those of
-// ring_attention_common.cuh). One attention CTA works on items of 128 queries x one head and walks
-// the key blocks in arrival order in tiles of 128 keys:
+// ring_attention_common.cuh). One attention CTA works on items of TWO tiles of 128 queries that share their
+// K/V head and walks the key blocks in arrival order in tiles of 128 keys:
 //
-//   warp 0      TMA producer: K and V tiles (three stages each) from this rank's own K/V or from
-//               the ring-buffer slot of the block's origin, after the slot's arrival counter has
+//   warp 0      TMA producer: the item's two Q tiles, then K and V tiles (two stages each) from this rank's own
+//               K/V or from the ring-buffer slot of the block's origin, after the slot's arrival counter has
 //               been seen (acquire, bounded)
-//   warp 1      MMA issuer: S = Q K^T (tcgen05.mma, M 128, N 128, K 128) into one of two TMEM
-//               buffers, and O += P V (M 128, N 128 = head_dim, K 128 keys) into a third. Q and P
-//               are read from TMEM (the A operand of both MMAs), only K and V come from shared
-//               memory, whose bandwidth is what bounds this kernel. S of tile j+1 is issued before
-//               P V of tile j, so the tensor pipe works while the softmax of tile j runs
-//   warps 2..9  softmax, two threads per query row (warp w: TMEM lanes 32 * (w % 4) .. +32, keys
-//               64 * ((w - 2) / 4) .. +64 of the tile). At the start of an item they copy their
-//               part of the Q row from global memory into TMEM (tcgen05.st). Per tile:
-//               tcgen05.ld of the 64 scores, the row maximum agreed between the two threads
-//               through shared memory, P = exp2(s - max) (one packed FMA per two scores, one
-//               ex2.approx each) written as packed 16-bit pairs over the first 64 columns of the
-//               SAME S buffer (both threads have read their scores by then; the tensor pipe runs
-//               its MMAs in issue order, so the buffer is not overwritten before P V has read it);
-//               running sum kept per thread; when a row's maximum moved, its O row in TMEM is
-//               rescaled (tcgen05.ld / st, each thread its 64 columns), which after the first tiles
-//               is rare; at the end of an item O / sum is stored
+//   warp 1      MMA issuer: per query tile i, S_i = Q_i K^T (tcgen05.mma, M 128, N 128, K 128) and
+//               O_i += P_i V (P from TMEM). Issue order PV_0(j), S_0(j+1), PV_1(j), S_1(j+1): the tensor pipe
+//               works for one query tile while the softmax of the other runs
+//   warps 4..7  softmax of query tile 0, warps 8..11 of tile 1, one thread per query row (224 registers each, the
+//               issuers give theirs up). Per tile: tcgen05.ld of
+//               the 128 scores, row maximum, P = exp2(s - max) (one packed FMA and one packed add per two scores,
+//               one ex2.approx each) written as packed 16-bit pairs over the first 64 columns of the SAME S
+//               buffer (the tensor pipe runs its MMAs in issue order, so S(j+1) does not overwrite P(j) before
+//               P V has read it). The maximum that P is taken against moves only when a row's new maximum exceeds
+//               it by more than 2^8: then the O row in TMEM is rescaled (tcgen05.ld / st). P and the row sums stay
+//               below 2^8 times their usual range, the fp32 sums and the final division are exact in that factor.
 //
-// TMEM: S0 / P0 columns [0, 128), S1 / P1 [128, 256), O [256, 384), Q [384, 448) (128 values as 64
-// columns of 16-bit pairs). Shared memory: K 3 x 32 KB, V 3 x 32 KB. Every wait (mbarriers, arrival
-// counters) is bounded.
+// What bounds it: per tile of 128 x 128 the two MMAs take 1024 cycles of the tensor pipe and the 16384 exponentials
+// 1024 cycles of the MUFU. With one query tile per CTA and two threads per row (the previous split) the softmax of a tile
+// lay open next to its MMAs and the two threads of a row met in shared memory twice: about 3000 cycles per tile
+// (8192 tokens, 32 / 8 heads, causal, bf16: 736 us). Two tiles in turn, one thread per row: 549 us; 3000 tokens, full attention, fp16, which the mma.sync
+// kernel took before: 603 -> 187 us.
+// The two tiles are two query heads of one K/V head group where the group is even (same keys, no work done twice or
+// for padding), else two neighbouring tiles of 128 queries of one head. Items are handed out longest first, in
+// alternating direction, so that a causal mask leaves no CTA with the long items at the end.
+//
+// Sequences that are not a multiple of 128: the last tile's rows and keys past the end come back as zeros from TMA
+// (the ring buffer is mapped block by block for that), its scores are masked and its rows are not stored.
+//
+// TMEM: S0 / P0 columns [0, 128), S1 / P1 [128, 256), O0 [256, 384), O1 [384, 512). Shared memory: Q 2 x 32 KB,
+// K 2 x 32 KB, V 2 x 32 KB. Every wait (mbarriers, arrival counters) is bounded.
 #include "ring_attention_common.cuh"
 
 #include "iris/gemm/sm100_mainloop.cuh"
@@ -39,20 +45,22 @@ namespace {
 
 constexpr int kTQ = 128;                 // queries per item = TMEM lanes
 constexpr int kTK = 128;                 // keys per tile
-constexpr int kTcThreads = 320;
+constexpr int kTcThreads = 384;          // three warpgroups: issuers (two of four warps work), softmax of query tile 0, of tile 1
 constexpr int kHalf = 128 * 128;         // bytes of a [128 rows][64 columns] 16-bit half tile
 constexpr int kTile = 2 * kHalf;         // 32 KB
-constexpr int kKvStages = 3;
-constexpr int kTcSmem = 1024 + kTile * 2 * kKvStages + 256 + 3072;    // K and V stages, barriers, row exchange
+constexpr int kKvStages = 2;
+constexpr int kTcSmem = 1024 + kTile * 2 + kTile * 2 * kKvStages + 256;    // Q tiles, K and V stages, barriers
+constexpr float kRescaleAt = 8.f;        // log2 of how far a row's maximum may run ahead of the one P is taken against
 constexpr uint64_t kWaitNs = 4000000000ull;
 static_assert(kTcSmem <= 227 * 1024, "shared memory budget");
 
 struct TcArgs {
   RingArgs a;
-  CUtensorMap tmKown;    // [S, Hkv * D], box 64 x 128
-  CUtensorMap tmVown;    // [S, Hkv * D], box 64 x 64
-  CUtensorMap tmKbuf;    // ring buffer seen as [2 * W * 2 * S, Hkv * D], box 64 x 128
-  CUtensorMap tmVbuf;    // same, box 64 x 64
+  CUtensorMap tmQ;       // [S, Hq * D], box 64 x 128
+  CUtensorMap tmKown;    // [1][S, Hkv * D], box 64 x 128 x 1
+  CUtensorMap tmVown;    // [1][S, Hkv * D], box 64 x 64 x 1
+  CUtensorMap tmKbuf;    // ring buffer seen as [2 * W * 2][S, Hkv * D], box 64 x 128 x 1
+  CUtensorMap tmVbuf;    // same, box 64 x 64 x 1
 };
 
 __device__ __forceinline__ void tmem_st_32x32(uint32_t taddr, const uint32_t (&r)[32]) {
@@ -67,15 +75,8 @@ __device__ __forceinline__ void tmem_st_32x32(uint32_t taddr, const uint32_t (&r
       : "memory");
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-// D[tmem] (+)= A[tmem] * B[smem desc]: A is read from TMEM (lane = row, 16-bit pairs along K per column).
-__device__ __forceinline__ void mma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(tmem_d),
-      "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// The same for a converged warp: every lane executes it with warp-uniform operands and one elected lane issues.
+// D[tmem] (+)= A[tmem] * B[smem desc]: A is read from TMEM (lane = row, 16-bit pairs along K per column). For a
+// converged warp: every lane executes it with warp-uniform operands and one elected lane issues.
 __device__ __forceinline__ void mma_f16_ts_elect(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
       "{\n\t.reg .pred p, q;\n\telect.sync _|q, 0xffffffff;\n\tsetp.ne.b32 p, %4, 0;\n\t"
@@ -89,8 +90,61 @@ __device__ __forceinline__ float ex2_approx(float x) {
   return y;
 }
 
+// 3-D tiled load by one elected lane of a converged warp (see the *_elect forms of ptx.cuh).
+__device__ __forceinline__ void tma_load_3d_elect(uint32_t smem_dst, const CUtensorMap* m, uint64_t* bar, int x, int y, int z) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t"
+      "@q cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];\n\t}" ::"r"(smem_dst),
+      "l"(m), "r"(ptx::smem_u32(bar)), "r"(x), "r"(y), "r"(z)
+      : "memory");
+}
+__device__ __forceinline__ unsigned long long pack_f32x2(float lo, float hi) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+
+// One item: two query tiles (qt[i], head h[i]) of one K/V head. n_q: how many of them exist (an odd number of
+// query tiles leaves the last item with one).
+struct Item {
+  int qt[2], h[2], kvh, n_q;
+};
+struct ItemOrder {
+  int items, rounds, stride, c, per_q, q_tiles, Hq, group;
+  bool by_head;
+  __device__ ItemOrder(const RingArgs& a) {
+    q_tiles = (a.S + kTQ - 1) / kTQ;
+    Hq = a.Hq;
+    group = a.Hq / a.Hkv;
+    by_head = group % 2 == 0;
+    per_q = by_head ? Hq / 2 : Hq;
+    items = (by_head ? q_tiles : (q_tiles + 1) / 2) * per_q;
+    stride = gridDim.x - a.n_comm;
+    c = blockIdx.x - a.n_comm;
+    rounds = (items + stride - 1) / stride;
+  }
+  // the CTA's item of a round; false when the last round has none for it. Longest items (late queries) first.
+  __device__ bool get(int round, Item& it) const {
+    const int idx = round * stride + ((round & 1) ? stride - 1 - c : c);
+    if (idx >= items) return false;
+    const int q = items / per_q - 1 - idx / per_q, hh = idx % per_q;
+    if (by_head) {
+      it.qt[0] = it.qt[1] = q;
+      it.h[0] = 2 * hh; it.h[1] = 2 * hh + 1;
+      it.n_q = 2;
+    } else {
+      it.qt[0] = 2 * q; it.qt[1] = 2 * q + 1;
+      it.h[0] = it.h[1] = hh;
+      it.n_q = it.qt[1] < q_tiles ? 2 : 1;
+    }
+    it.kvh = it.h[0] / group;
+    return true;
+  }
+};
+
 // The key tiles of one item, in the order every role walks them: blocks in arrival order (own,
-// r-1, r-2, ...), tiles inside a block in order; causal items skip what lies after their queries.
+// r-1, r-2, ...), tiles inside a block in order; causal items skip what lies after their queries. A tile is
+// visited when one of the item's query tiles needs it; needs(i) says which.
 //
 // Contiguous layout: rank r holds tokens [r*S, (r+1)*S). A causal item of query tile qt takes all
 // tiles of earlier blocks, tiles 0..qt of its own block (the last one masked on the diagonal) and
@@ -100,53 +154,58 @@ __device__ __forceinline__ float ex2_approx(float x) {
 // chunks 0..r, a query of chunk 2W-1-r sees every first-half chunk and the second-half chunks
 // of origins >= r: every rank does the same amount of work.
 struct TileWalk {
-  int W, r, T, causal, zigzag, qt;
+  int W, r, T, causal, zigzag;
+  int qt[2], n_q;
   int step = 0, t = -1, origin = 0;
-  int a0 = 0, a1 = 0, b0 = 0, b1 = 0;      // tile ranges [a0, a1) and [b0, b1) of the current block (b0 >= a1)
-  int diag = -1;                           // tile of the block that needs the diagonal mask
+  int b0 = 0;                              // second range of a block starts here (first range ends at or before it)
+  int a1[2], b1[2];                        // query tile i takes [0, a1[i]) and [b0, b1[i]) of the current block
+  int ua1 = 0, ub1 = 0;                    // their union
   bool first = false;                      // the current tile is the first one taken from its block
-  __device__ TileWalk(const RingArgs& a, int qt_)
-      : W(a.ctx.world), r(a.ctx.rank), T(a.S / kTK), causal(a.causal), zigzag(a.zigzag), qt(qt_) { open_block(); }
+  __device__ TileWalk(const RingArgs& a, const Item& it)
+      : W(a.ctx.world), r(a.ctx.rank), T((a.S + kTK - 1) / kTK), causal(a.causal), zigzag(a.zigzag), n_q(it.n_q) {
+    qt[0] = it.qt[0]; qt[1] = it.qt[1];
+    open_block();
+  }
   __device__ void ranges() {
-    a0 = 0; a1 = T; b0 = b1 = T; diag = -1;
-    if (!causal) return;
-    if (!zigzag) {
-      if (origin > r) a1 = 0;
-      else if (origin == r) { a1 = qt + 1; diag = qt; }
-      return;
-    }
     const int Th = T / 2;
-    if (qt < Th) {                  // query chunk r: first halves of origins <= r
-      if (origin > r) a1 = 0;
-      else if (origin == r) { a1 = qt + 1; diag = qt; }
-      else a1 = Th;
-    } else {                        // query chunk 2W-1-r: every first half, second halves of origins >= r
-      a1 = Th;
-      if (origin > r) { b0 = Th; b1 = T; }
-      else if (origin == r) { b0 = Th; b1 = qt + 1; diag = qt; }
+    b0 = causal && zigzag ? Th : T;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      a1[i] = T; b1[i] = b0;
+      if (i >= n_q) { a1[i] = 0; continue; }
+      if (!causal) continue;
+      if (!zigzag) a1[i] = origin > r ? 0 : origin == r ? qt[i] + 1 : T;
+      else if (qt[i] < Th) a1[i] = origin > r ? 0 : origin == r ? qt[i] + 1 : Th;   // query chunk r: first halves of origins <= r
+      else {                                                                        // query chunk 2W-1-r: every first half, second halves of origins >= r
+        a1[i] = Th;
+        b1[i] = origin > r ? T : origin == r ? qt[i] + 1 : b0;
+      }
     }
+    ua1 = max(a1[0], a1[1]); ub1 = max(b1[0], b1[1]);
   }
   __device__ void open_block() {
     for (; step < W; ++step) {
       origin = r - step;
       if (origin < 0) origin += W;
       ranges();
-      if (a1 > a0 || b1 > b0) { t = -1; return; }
+      if (ua1 > 0 || ub1 > b0) { t = -1; return; }
     }
   }
   // advances to the next tile; false when the item is finished
   __device__ bool next() {
     while (step < W) {
       first = t < 0;
-      if (t < 0) t = a1 > a0 ? a0 : b0;
-      else if (++t == a1 && b1 > b0) t = b0;
-      if ((t >= a0 && t < a1) || (t >= b0 && t < b1)) return true;
+      if (t < 0) t = ua1 > 0 ? 0 : b0;
+      else if (++t == ua1 && ub1 > b0) t = b0;
+      if (t < ua1 || (t >= b0 && t < ub1)) return true;
       ++step;
       open_block();
     }
     return false;
   }
-  __device__ bool diagonal() const { return t == diag; }
+  // (selected, not indexed: an index that is not a constant would put the arrays in local memory)
+  __device__ bool needs(int i) const { return t < (i ? a1[1] : a1[0]) || (t >= b0 && t < (i ? b1[1] : b1[0])); }
+  __device__ bool diagonal(int i) const { return causal && origin == r && t == (i ? qt[1] : qt[0]); }
 };
 
 template <bool kFp16>
@@ -157,48 +216,37 @@ __device__ void attn_main_tc(const TcArgs& g, uint8_t* smem_raw, int call) {
   const int par = call & 1;
   const int32_t target = ((call >> 1) + 1) * a.n_comm;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int q_tiles = a.S / kTQ;
-  const int items = q_tiles * a.Hq;
-  const int group = a.Hq / a.Hkv;
 
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  uint8_t* k_s = smem;                                   // [stages][kTile]
+  uint8_t* q_s = smem;                                   // [2][kTile]
+  uint8_t* k_s = q_s + 2 * kTile;                        // [stages][kTile]
   uint8_t* v_s = k_s + kKvStages * kTile;
   uint64_t* bars = (uint64_t*)(v_s + kKvStages * kTile);
-  uint64_t* q_full = bars;              // 8 softmax warps: the item's Q is in TMEM
-  uint64_t* q_free = bars + 1;          // 1: every S MMA of the item has read Q
-  uint64_t* k_full = bars + 2;          // [3]
-  uint64_t* k_empty = bars + 5;         // [3]
-  uint64_t* v_full = bars + 8;          // [3]
-  uint64_t* v_empty = bars + 11;        // [3]
-  uint64_t* s_full = bars + 14;         // [2]
-  uint64_t* p_full = bars + 16;         // [2] 8 softmax warps
-  uint64_t* o_ready = bars + 18;        // [2] by tile parity: O holds every tile up to that one
-  uint64_t* o_free = bars + 20;         // 8 softmax warps: the item's O has been read out
-  uint32_t* tmem_slot = (uint32_t*)(bars + 21);
-  // exchange between the two threads of a row (bounded waits, no bar.sync: a thread that gave up
-  // must not leave its partner blocked): values [2 parities][2 halves][128 rows], then the number
-  // of the last exchange each (half, row) published
-  float* xchg = (float*)(bars + 22);
-  uint32_t* xseq = (uint32_t*)(xchg + 512);
+  uint64_t* q_full = bars;              // [2] the item's Q tile i has landed
+  uint64_t* q_free = bars + 2;          // [2] every S MMA of the item has read Q tile i
+  uint64_t* k_full = bars + 4;          // [2]
+  uint64_t* k_empty = bars + 6;         // [2]
+  uint64_t* v_full = bars + 8;          // [2]
+  uint64_t* v_empty = bars + 10;        // [2]
+  uint64_t* s_full = bars + 12;         // [2] by query tile: its S is complete (and its P V of the tile before)
+  uint64_t* p_full = bars + 14;         // [2] by query tile: 4 softmax warps wrote P (and rescaled O)
+  uint64_t* o_full = bars + 16;         // [2] the item's O_i is complete
+  uint64_t* o_free = bars + 18;         // [2] 4 softmax warps have read the item's O_i
+  uint32_t* tmem_slot = (uint32_t*)(bars + 20);
 
   if (threadIdx.x == 0) {
-    ptx::mbar_init(q_full, 8);
-    ptx::mbar_init(q_free, 1);
+    for (int i = 0; i < 2; ++i) {
+      ptx::mbar_init(&q_full[i], 1); ptx::mbar_init(&q_free[i], 1);
+      ptx::mbar_init(&s_full[i], 1); ptx::mbar_init(&p_full[i], 4);
+      ptx::mbar_init(&o_full[i], 1); ptx::mbar_init(&o_free[i], 4);
+    }
     for (int i = 0; i < kKvStages; ++i) {
       ptx::mbar_init(&k_full[i], 1); ptx::mbar_init(&k_empty[i], 1);
       ptx::mbar_init(&v_full[i], 1); ptx::mbar_init(&v_empty[i], 1);
     }
-    for (int i = 0; i < 2; ++i) {
-      ptx::mbar_init(&s_full[i], 1);
-      ptx::mbar_init(&p_full[i], 8);
-      ptx::mbar_init(&o_ready[i], 1);
-    }
-    ptx::mbar_init(o_free, 8);
     ptx::fence_mbar_init();
     ptx::fence_proxy_async();
   }
-  for (int i = threadIdx.x; i < 256; i += blockDim.x) xseq[i] = 0;
   if (warp == 1) {
     ptx::tmem_alloc(tmem_slot, 512);
     ptx::tmem_relinquish();
@@ -207,17 +255,33 @@ __device__ void attn_main_tc(const TcArgs& g, uint8_t* smem_raw, int call) {
   __syncthreads();
   ptx::tc_fence_after();
   const uint32_t tmem_base = *(volatile uint32_t*)tmem_slot;
-  const int first = blockIdx.x - a.n_comm, stride = gridDim.x - a.n_comm;
+  const ItemOrder order(a);
 
+  // 56 + 224 + 224 = 3 x 168, what the block was launched with (the splits stand at the head of their branches:
+  // the compiler gives each branch its own budget from there)
+  if (warp < 4) {
+  asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
     unsigned arrived_mask = 1u << r;
-    uint32_t n_item = 0, n_tile = 0;        // items / tiles issued so far (barrier phases)
+    uint32_t n_tile = 0;                    // K/V tiles issued so far (barrier phases)
+    uint32_t n_q[2] = {0, 0};               // Q tiles loaded so far, per place
     bool ok = true;
-    for (int it = first; it < items && ok; it += stride, ++n_item) {
-      const int h = it % a.Hq, qt = it / a.Hq, kvh = h / group;
-      TileWalk w(a, qt);
-      while (w.next()) {
+    Item item;
+    for (int rd = 0; rd < order.rounds && ok; ++rd) {
+      if (!order.get(rd, item)) continue;
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        if (i >= item.n_q || !ok) break;
+        if (!__all_sync(0xffffffffu, ptx::mbar_wait(&q_free[i], (n_q[i] & 1) ^ 1, kWaitNs))) { ctx.fail(kTimeoutPipeline); ok = false; break; }
+        const uint32_t qd = ptx::smem_u32(q_s + i * kTile);
+        ptx::mbar_expect_tx_elect(&q_full[i], kTile);
+        ptx::tma_load_2d_elect(qd, &g.tmQ, &q_full[i], item.h[i] * kD, item.qt[i] * kTQ);
+        ptx::tma_load_2d_elect(qd + kHalf, &g.tmQ, &q_full[i], item.h[i] * kD + 64, item.qt[i] * kTQ);
+        ++n_q[i];
+      }
+      TileWalk w(a, item);
+      while (ok && w.next()) {
         if (w.first && !((arrived_mask >> w.origin) & 1u)) {
           int seen = 1;
           if (lane == 0) seen = wait_flag_ge(ctx, a.flags + (size_t)par * W + w.origin, target) ? 1 : 0;
@@ -228,29 +292,25 @@ __device__ void attn_main_tc(const TcArgs& g, uint8_t* smem_raw, int call) {
         }
         const int st = n_tile % kKvStages;
         const uint32_t ph = ((n_tile / kKvStages) & 1) ^ 1;
-        if (!__all_sync(0xffffffffu, ptx::mbar_wait(&k_empty[st], ph, kWaitNs) && ptx::mbar_wait(&v_empty[st], ph, kWaitNs))) {
-          ctx.fail(kTimeoutPipeline); ok = false; break;
-        }
-        {   // converged warp, one elected lane per instruction
-          const bool own = w.origin == r;
-          const CUtensorMap* mk = own ? &g.tmKown : &g.tmKbuf;
-          const CUtensorMap* mv = own ? &g.tmVown : &g.tmVbuf;
-          // ring buffer rows: ((parity * W + origin) * 2 + {K: 0, V: 1}) * S + position
-          const int rowk = own ? 0 : ((par * W + w.origin) * 2) * a.S;
-          const int rowv = own ? 0 : rowk + a.S;
-          const int pos0 = w.t * kTK;
-          const uint32_t kd = ptx::smem_u32(k_s + st * kTile);
-          const uint32_t vd = ptx::smem_u32(v_s + st * kTile);
-          ptx::mbar_expect_tx_elect(&k_full[st], kTile);
-          ptx::tma_load_2d_elect(kd, mk, &k_full[st], kvh * kD, rowk + pos0);
-          ptx::tma_load_2d_elect(kd + kHalf, mk, &k_full[st], kvh * kD + 64, rowk + pos0);
-          ptx::mbar_expect_tx_elect(&v_full[st], kTile);
+        const bool own = w.origin == r;
+        const CUtensorMap* mk = own ? &g.tmKown : &g.tmKbuf;
+        const CUtensorMap* mv = own ? &g.tmVown : &g.tmVbuf;
+        const int zk = own ? 0 : (par * W + w.origin) * 2;       // ring buffer blocks: (parity, origin, K | V)
+        const int zv = own ? 0 : zk + 1;
+        const int pos0 = w.t * kTK;
+        const uint32_t kd = ptx::smem_u32(k_s + st * kTile);
+        const uint32_t vd = ptx::smem_u32(v_s + st * kTile);
+        if (!__all_sync(0xffffffffu, ptx::mbar_wait(&k_empty[st], ph, kWaitNs))) { ctx.fail(kTimeoutPipeline); ok = false; break; }
+        ptx::mbar_expect_tx_elect(&k_full[st], kTile);
+        tma_load_3d_elect(kd, mk, &k_full[st], item.kvh * kD, pos0, zk);
+        tma_load_3d_elect(kd + kHalf, mk, &k_full[st], item.kvh * kD + 64, pos0, zk);
+        if (!__all_sync(0xffffffffu, ptx::mbar_wait(&v_empty[st], ph, kWaitNs))) { ctx.fail(kTimeoutPipeline); ok = false; break; }
+        ptx::mbar_expect_tx_elect(&v_full[st], kTile);
 #pragma unroll
-          for (int kh = 0; kh < 2; ++kh)
+        for (int kh = 0; kh < 2; ++kh)
 #pragma unroll
-            for (int nb = 0; nb < 2; ++nb)
-              ptx::tma_load_2d_elect(vd + kh * kHalf + nb * 8192, mv, &v_full[st], kvh * kD + nb * 64, rowv + pos0 + kh * 64);
-        }
+          for (int nb = 0; nb < 2; ++nb)
+            tma_load_3d_elect(vd + kh * kHalf + nb * 8192, mv, &v_full[st], item.kvh * kD + nb * 64, pos0 + kh * 64, zv);
         ++n_tile;
       }
     }
@@ -258,226 +318,227 @@ __device__ void attn_main_tc(const TcArgs& g, uint8_t* smem_raw, int call) {
     // ------------------------------------------------------------------ MMA issuer
     const uint32_t idesc_s = make_idesc(kTK, !kFp16, false);     // B = K tile, K-major
     const uint32_t idesc_o = make_idesc(kD, !kFp16, true);       // B = V tile, [keys, d] row-major
-    uint32_t n_item = 0, n_s = 0, n_pv = 0;     // items, S tiles and P V tiles issued so far
-    bool ok = true;
     // The warp stays converged: every lane computes the warp-uniform operands and each tensor-core instruction
     // elects its issuing lane (issued from inside `if (lane == 0)` they cost about 100 cycles apiece). Votes and
     // the warp reduction make the loop state and the TMEM base uniform for the compiler too.
     const uint32_t tmem_u = __reduce_or_sync(0xffffffffu, tmem_base);
-    // The S buffer of tile j also holds P of tile j (its first 64 columns) until the P V MMA of
-    // tile j has read it; S of tile j + 2 is issued after that MMA and the tensor pipe runs MMAs in
-    // issue order, so no barrier guards the reuse of the buffer.
-    auto issue_s = [&]() -> bool {
-      const int sb = n_s & 1, st = n_s % kKvStages;
-      if (!__all_sync(0xffffffffu, ptx::mbar_wait(&k_full[st], (n_s / kKvStages) & 1, kWaitNs))) return false;
-      ptx::tc_fence_after();
-      {
-        const uint32_t kb = ptx::smem_u32(k_s + st * kTile);
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {        // 16 of the 128 head dimensions per step: 8 columns of Q in TMEM
-          const uint32_t off = (k >> 2) * kHalf + (k & 3) * 32;
-          mma_f16_ts_elect(tmem_u + sb * 128, tmem_u + 384 + k * 8, desc_kmajor(kb + off), idesc_s, k != 0);
-        }
-        ptx::mma_commit_elect(&k_empty[st]);
-        ptx::mma_commit_elect(&s_full[sb]);
-      }
-      ++n_s;
-      return true;
+    uint32_t n_k = 0, n_v = 0;                     // K / V tiles taken so far
+    uint32_t n_qi[2] = {0, 0}, n_p[2] = {0, 0};    // items / P tiles per query tile so far
+    bool ok = true;
+    auto wait = [&](uint64_t* bar, uint32_t phase) {
+      if (!__all_sync(0xffffffffu, ptx::mbar_wait(bar, phase, kWaitNs))) { ctx.fail(kTimeoutPipeline); ok = false; }
+      return ok;
     };
-    auto issue_pv = [&](bool first_of_item) -> bool {
-      const int sb = n_pv & 1, st = n_pv % kKvStages;
-      if (!__all_sync(0xffffffffu, ptx::mbar_wait(&p_full[sb], (n_pv >> 1) & 1, kWaitNs))) return false;
-      if (!__all_sync(0xffffffffu, ptx::mbar_wait(&v_full[st], (n_pv / kKvStages) & 1, kWaitNs))) return false;
-      ptx::tc_fence_after();
+    Item item;
+    for (int rd = 0; rd < order.rounds && ok; ++rd) {
+      if (!order.get(rd, item)) continue;
+      int left_s[2] = {0, 0}, left_pv[2];          // S and P V MMAs of the item still to be issued, per query tile
       {
+        TileWalk w(a, item);
+        while (w.next()) {
+          if (w.needs(0)) ++left_s[0];
+          if (w.needs(1)) ++left_s[1];
+        }
+        left_pv[0] = left_s[0]; left_pv[1] = left_s[1];
+      }
+      const int total[2] = {left_s[0], left_s[1]};
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+        if (i < item.n_q && ok) wait(&q_full[i], n_qi[i] & 1);
+      auto issue_s = [&](int i, int st) {
+        ptx::tc_fence_after();
+        const uint32_t qb = ptx::smem_u32(q_s + i * kTile), kb = ptx::smem_u32(k_s + st * kTile);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {        // 16 of the 128 head dimensions per step
+          const uint32_t off = (k >> 2) * kHalf + (k & 3) * 32;
+          ptx::mma_f16_elect(tmem_u + i * 128, desc_kmajor(qb + off), desc_kmajor(kb + off), idesc_s, k != 0);
+        }
+        ptx::mma_commit_elect(&s_full[i]);
+        if (--left_s[i] == 0) ptx::mma_commit_elect(&q_free[i]);
+      };
+      auto issue_pv = [&](int i, int st) {
+        ptx::tc_fence_after();
         const uint32_t vb = ptx::smem_u32(v_s + st * kTile);
+        const bool clear = left_pv[i] == total[i];
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
           const uint32_t boff = (k >> 2) * kHalf + (k & 3) * 2048;        // V: 64-key halves, 16 keys = 2048 B
           // P: 16 keys = 8 columns of 16-bit pairs at the start of the tile's S buffer
-          mma_f16_ts_elect(tmem_u + 256, tmem_u + sb * 128 + k * 8, desc_mnmajor(vb + boff), idesc_o, !(first_of_item && k == 0));
+          mma_f16_ts_elect(tmem_u + 256 + i * 128, tmem_u + i * 128 + k * 8, desc_mnmajor(vb + boff), idesc_o, !(clear && k == 0));
         }
-        ptx::mma_commit_elect(&v_empty[st]);
-        ptx::mma_commit_elect(&o_ready[sb]);
+        if (--left_pv[i] == 0) ptx::mma_commit_elect(&o_full[i]);
+      };
+      TileWalk cur(a, item), nxt(a, item);
+      bool has = cur.next(), has_n = nxt.next();
+      // S of the first tile
+      if (ok && has && wait(&k_full[n_k % kKvStages], (n_k / kKvStages) & 1)) {
+        const int st = n_k % kKvStages;
+        if (cur.needs(0)) issue_s(0, st);
+        if (cur.needs(1)) issue_s(1, st);
+        ptx::mma_commit_elect(&k_empty[st]);
+        ++n_k;
       }
-      ++n_pv;
-      return true;
-    };
-    for (int it = first; it < items && ok; it += stride, ++n_item) {
-      const int qt = it / a.Hq;
-      int n = 0;
-      {
-        TileWalk w(a, qt);
-        while (w.next()) ++n;
+      while (ok && has) {
+        has_n = nxt.next();
+        const int vst = n_v % kKvStages, kst = n_k % kKvStages;
+        bool v_ready = false, k_ready = false;
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          if (cur.needs(i)) {
+            if (!wait(&p_full[i], n_p[i] & 1)) break;
+            if (!v_ready && !wait(&v_full[vst], (n_v / kKvStages) & 1)) break;
+            v_ready = true;
+            // the previous item's O must have been read out before this item's first P V overwrites it
+            if (left_pv[i] == total[i] && !wait(&o_free[i], (n_qi[i] & 1) ^ 1)) break;
+            issue_pv(i, vst);
+            ++n_p[i];
+          }
+          if (cur.needs(i) && (i == 1 || !cur.needs(1))) ptx::mma_commit_elect(&v_empty[vst]);      // the tile's last P V
+          if (has_n && nxt.needs(i)) {
+            if (!k_ready && !wait(&k_full[kst], (n_k / kKvStages) & 1)) break;
+            k_ready = true;
+            issue_s(i, kst);
+          }
+        }
+        if (!ok) break;
+        ++n_v;
+        if (has_n) { ptx::mma_commit_elect(&k_empty[kst]); ++n_k; }
+        has = has_n;
+        cur.next();
       }
-      if (!__all_sync(0xffffffffu, ptx::mbar_wait(q_full, n_item & 1, kWaitNs))) { ctx.fail(kTimeoutPipeline); break; }
-      if (!issue_s()) { ctx.fail(kTimeoutPipeline); break; }
-      for (int j = 0; j < n; ++j) {
-        if (j + 1 < n && !issue_s()) { ctx.fail(kTimeoutPipeline); ok = false; break; }
-        if (j + 1 == n) ptx::mma_commit_elect(q_free);       // every S MMA of the item is issued
-        // the previous item's O must have been read out before this item's first P V overwrites it
-        if (j == 0 && !__all_sync(0xffffffffu, ptx::mbar_wait(o_free, (n_item & 1) ^ 1, kWaitNs))) { ctx.fail(kTimeoutPipeline); ok = false; break; }
-        if (!issue_pv(j == 0)) { ctx.fail(kTimeoutPipeline); ok = false; break; }
-      }
+      ++n_qi[0];
+      if (item.n_q > 1) ++n_qi[1];
     }
+  }
   } else {
     // ------------------------------------------------------------------ softmax / correction / epilogue
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 224;");
     const int quarter = warp & 3;
-    const int half = (warp - 2) >> 2;                         // which 64 keys of a tile / 64 columns of O
+    const int i = (warp - 4) >> 2;                            // query tile of the item
     const int row = quarter * 32 + lane;                      // query row inside the tile
     const uint32_t lane_addr = tmem_base + ((uint32_t)(quarter * 32) << 16);
+    const uint32_t s_addr = lane_addr + i * 128, o_addr = lane_addr + 256 + i * 128;
     const float scale2 = a.sm_scale * kLog2e;
-    uint32_t n_item = 0, n_tile = 0, xtag = 0;
+    const unsigned long long scale_pair = pack_f32x2(scale2, scale2);
+    uint32_t n_item = 0, n_tile = 0;
     bool ok = true;
-    // publishes `v`, returns the partner's value of the same exchange (false in `ok` after 4 s)
-    auto exchange = [&](float v) -> float {
-      ++xtag;
-      volatile float* val = xchg + (xtag & 1) * 256;
-      volatile uint32_t* seq = xseq;
-      val[half * 128 + row] = v;
-      __threadfence_block();
-      seq[half * 128 + row] = xtag;
-      const int other = (half ^ 1) * 128 + row;
-      if ((int)(seq[other] - xtag) < 0) {
-        const uint64_t t0 = ptx::globaltimer();
-        uint32_t spins = 0;
-        while ((int)(seq[other] - xtag) < 0) {
-          if ((++spins & 1023u) == 0 && ptx::globaltimer() - t0 > kWaitNs) { ok = false; break; }
-        }
-      }
-      __threadfence_block();
-      return val[other];
-    };
-    for (int it = first; it < items && ok; it += stride, ++n_item) {
-      const int h = it % a.Hq, qt = it / a.Hq;
-      const int qpos = qt * kTQ + row;                        // position inside this rank's block
-      float m_run = -INFINITY, l_run = 0.f;                   // l_run: this thread's half of the row sum
-      // this thread's 64 values of the Q row -> TMEM (16-bit pairs), once every S MMA of the previous item is done
-      {
-        uint32_t qw[32];
-        const uint4* qsrc = (const uint4*)(a.q + ((size_t)(qt * kTQ + row) * a.Hq + h) * kD * 2 + half * 128);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const uint4 v = __ldg(qsrc + i);
-          qw[4 * i] = v.x; qw[4 * i + 1] = v.y; qw[4 * i + 2] = v.z; qw[4 * i + 3] = v.w;
-        }
-        if (!ptx::mbar_wait(q_free, (n_item & 1) ^ 1, kWaitNs)) { ctx.fail(kTimeoutPipeline); break; }
-        ptx::tc_fence_after();
-        tmem_st_32x32(lane_addr + 384 + half * 32, qw);
-        tmem_st_wait();
-        ptx::tc_fence_before();
-        __syncwarp();
-        if (lane == 0) ptx::mbar_arrive(q_full);
-      }
-      TileWalk w(a, qt);
+    Item item;
+    for (int rd = 0; rd < order.rounds && ok; ++rd) {
+      if (!order.get(rd, item)) continue;
+      if (i >= item.n_q) continue;
+      const int qpos = (i ? item.qt[1] : item.qt[0]) * kTQ + row;                // position inside this rank's block
+      const int head = i ? item.h[1] : item.h[0];
+      float m_run = -INFINITY;                                // what P is taken against (log2 units)
+      unsigned long long l_pair[2] = {0ull, 0ull};            // the row sum, in four parts
       int j = 0;
+      TileWalk w(a, item);
       while (w.next()) {
-        const int st = n_tile & 1;
-        if (!ptx::mbar_wait(&s_full[st], (n_tile >> 1) & 1, kWaitNs)) { ctx.fail(kTimeoutPipeline); ok = false; break; }
+        if (!w.needs(i)) continue;
+        if (!__all_sync(0xffffffffu, ptx::mbar_wait(&s_full[i], n_tile & 1, kWaitNs))) { ctx.fail(kTimeoutPipeline); ok = false; break; }
         ptx::tc_fence_after();
-        uint32_t s[64];
+        uint32_t s[128];
 #pragma unroll
-        for (int c = 0; c < 2; ++c) {
-          uint32_t (&chunk)[32] = *reinterpret_cast<uint32_t (*)[32]>(&s[c * 32]);
-          ptx::tmem_ld_32x32(lane_addr + st * 128 + half * 64 + c * 32, chunk);
-        }
+        for (int c = 0; c < 4; ++c) ptx::tmem_ld_32x32(s_addr + c * 32, *reinterpret_cast<uint32_t (*)[32]>(&s[c * 32]));
         ptx::tmem_ld_wait();
-        // causal mask on the diagonal tile, maximum of this thread's 64 raw scores
-        const bool diag = w.diagonal();
-        const int kpos0 = w.t * kTK + half * 64;
-        if (diag) {
+        // causal mask on the diagonal tile, keys past the end of the block in its last tile
+        int lim = a.S - 1 - w.t * kTK;
+        if (w.diagonal(i)) lim = min(lim, qpos - w.t * kTK);
+        if (__any_sync(0xffffffffu, lim < kTK - 1)) {
 #pragma unroll
-          for (int c = 0; c < 64; ++c)
-            if (kpos0 + c > qpos) s[c] = 0xff800000u;     // -inf
+          for (int c = 0; c < 128; ++c)
+            if (c > lim) s[c] = 0xff800000u;     // -inf
         }
         float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};      // four chains: the maximum is latency bound otherwise
 #pragma unroll
-        for (int c = 0; c < 64; c += 4) {
+        for (int c = 0; c < 128; c += 8) {
 #pragma unroll
-          for (int u = 0; u < 4; ++u) mx4[u] = fmaxf(mx4[u], __uint_as_float(s[c + u]));
+          for (int u = 0; u < 4; ++u) mx4[u] = fmaxf(mx4[u], fmaxf(__uint_as_float(s[c + u]), __uint_as_float(s[c + 4 + u])));
         }
-        float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
-        // agree on the row maximum with the thread that holds the other 64 keys
-        mx = fmaxf(mx, exchange(mx));
-        if (!__all_sync(0xffffffffu, ok)) { ctx.fail(kTimeoutPipeline); ok = false; break; }
-        const float m_new = fmaxf(m_run, mx * scale2);     // finite: the diagonal tile holds the row's own key
-        const float alpha = j == 0 ? 1.f : ex2_approx(m_run - m_new);
-        m_run = m_new;
-        // P goes over the first 64 columns of this tile's S buffer: both threads of the row have read
-        // their scores (the partner published its maximum after its loads)
-        uint32_t pw[32];        // this thread's 64 probabilities as 16-bit pairs
-        // p = exp2(s * scale - max): packed FMA for two scores at a time, one ex2.approx each, four sum chains
-        unsigned long long scale_pair, negm_pair;
-        asm("mov.b64 %0, {%1, %1};" : "=l"(scale_pair) : "f"(scale2));
-        asm("mov.b64 %0, {%1, %1};" : "=l"(negm_pair) : "f"(-m_new));
-        float rs4[4] = {0.f, 0.f, 0.f, 0.f};
+        const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * scale2;     // finite in the first tile: it holds a key the row sees
+        float alpha = 1.f;
+        if (j == 0) m_run = mx;
+        else if (mx > m_run + kRescaleAt) { alpha = ex2_approx(m_run - mx); m_run = mx; }
+        // p = exp2(s * scale - max): packed FMA for two scores at a time, one ex2.approx each, packed sums. P goes over
+        // the first 64 columns of the tile's S buffer: every thread of the row (this one) has read its scores
+        const unsigned long long negm_pair = pack_f32x2(-m_run, -m_run);
+        unsigned long long rs[2] = {0ull, 0ull};
 #pragma unroll
-        for (int c16 = 0; c16 < 8; ++c16) {       // groups of 8 keys
+        for (int hf = 0; hf < 2; ++hf) {
+          uint32_t pw[32];        // 64 probabilities as 16-bit pairs
 #pragma unroll
-          for (int e = 0; e < 4; ++e) {
+          for (int e = 0; e < 32; ++e) {
+            const int c = hf * 64 + 2 * e;
             unsigned long long sp, xp;
-            asm("mov.b64 %0, {%1, %2};" : "=l"(sp) : "r"(s[c16 * 8 + 2 * e]), "r"(s[c16 * 8 + 2 * e + 1]));
+            asm("mov.b64 %0, {%1, %2};" : "=l"(sp) : "r"(s[c]), "r"(s[c + 1]));
             asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(xp) : "l"(sp), "l"(scale_pair), "l"(negm_pair));
             float x0, x1;
             asm("mov.b64 {%0, %1}, %2;" : "=f"(x0), "=f"(x1) : "l"(xp));
             const float p0 = ex2_approx(x0), p1 = ex2_approx(x1);
-            rs4[e] += p0 + p1;
-            pw[c16 * 4 + e] = pack2<kFp16>(p0, p1);
+            asm("add.rn.f32x2 %0, %0, %1;" : "+l"(rs[e & 1]) : "l"(pack_f32x2(p0, p1)));
+            pw[e] = pack2<kFp16>(p0, p1);
           }
+          tmem_st_32x32(s_addr + hf * 32, pw);
         }
-        tmem_st_32x32(lane_addr + st * 128 + half * 32, pw);
-        l_run = l_run * alpha + ((rs4[0] + rs4[1]) + (rs4[2] + rs4[3]));
-        // rescale O when some row of this warp moved its maximum (O then holds every earlier tile)
-        if (j > 0 && __any_sync(0xffffffffu, alpha != 1.f)) {
-          // (the barrier of the previous tile's parity: this tile's S was issued after the P V of two
-          //  tiles ago and MMAs complete in issue order, so between "two tiles ago" and "the previous
-          //  tile" a phase parity is unambiguous)
-          if (!ptx::mbar_wait(&o_ready[(n_tile - 1) & 1], ((n_tile - 1) >> 1) & 1, kWaitNs)) { ctx.fail(kTimeoutPipeline); ok = false; break; }
-          ptx::tc_fence_after();
+        // rescale O when some row of this warp moved its maximum (this tile's S was issued after the previous tile's
+        // P V, and its barrier covers both: O holds every earlier tile)
+        if (__any_sync(0xffffffffu, alpha != 1.f)) {
+          const unsigned long long al = pack_f32x2(alpha, alpha);
+#pragma unroll
+          for (int u = 0; u < 2; ++u) asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(l_pair[u]) : "l"(al));
 #pragma unroll 1
-          for (int c = 0; c < 2; ++c) {
+          for (int c = 0; c < 4; ++c) {
             uint32_t o[32];
-            ptx::tmem_ld_32x32(lane_addr + 256 + half * 64 + c * 32, o);
+            ptx::tmem_ld_32x32(o_addr + c * 32, o);
             ptx::tmem_ld_wait();
 #pragma unroll
-            for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
-            tmem_st_32x32(lane_addr + 256 + half * 64 + c * 32, o);
+            for (int e = 0; e < 32; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * alpha);
+            tmem_st_32x32(o_addr + c * 32, o);
           }
         }
         tmem_st_wait();                         // P (and a rescaled O) are in TMEM before the MMA is told
         ptx::tc_fence_before();
         __syncwarp();
-        if (lane == 0) ptx::mbar_arrive(&p_full[st]);
+        if (lane == 0) ptx::mbar_arrive(&p_full[i]);
+#pragma unroll
+        for (int u = 0; u < 2; ++u) asm("add.rn.f32x2 %0, %0, %1;" : "+l"(l_pair[u]) : "l"(rs[u]));
         ++n_tile;
         ++j;
       }
       if (!ok) break;
-      // ---- item epilogue: the row sum of both halves, the last P V, O / sum -> 16-bit -> global
-      const float l_all = l_run + exchange(l_run);
-      if (!__all_sync(0xffffffffu, ok)) { ctx.fail(kTimeoutPipeline); break; }
-      if (!ptx::mbar_wait(&o_ready[(n_tile - 1) & 1], ((n_tile - 1) >> 1) & 1, kWaitNs)) { ctx.fail(kTimeoutPipeline); break; }
+      // ---- item epilogue: the row sum, the last P V, O / sum -> 16-bit -> global
+      float l_all = 0.f;
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        float x0, x1;
+        asm("mov.b64 {%0, %1}, %2;" : "=f"(x0), "=f"(x1) : "l"(l_pair[u]));
+        l_all += x0 + x1;
+      }
+      if (!__all_sync(0xffffffffu, ptx::mbar_wait(&o_full[i], n_item & 1, kWaitNs))) { ctx.fail(kTimeoutPipeline); ok = false; break; }
       ptx::tc_fence_after();
       const float inv = l_all > 0.f ? 1.f / l_all : 0.f;
-      uint8_t* orow = a.out + ((size_t)(qt * kTQ + row) * a.Hq + h) * kD * 2 + half * 128;
+      uint8_t* orow = a.out + ((size_t)qpos * a.Hq + head) * kD * 2;
 #pragma unroll 1
-      for (int c = 0; c < 2; ++c) {
+      for (int c = 0; c < 4; ++c) {
         uint32_t o[32];
-        ptx::tmem_ld_32x32(lane_addr + 256 + half * 64 + c * 32, o);
+        ptx::tmem_ld_32x32(o_addr + c * 32, o);
         ptx::tmem_ld_wait();
+        if (qpos < a.S) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          uint4 v;
-          v.x = pack2<kFp16>(__uint_as_float(o[8 * i]) * inv, __uint_as_float(o[8 * i + 1]) * inv);
-          v.y = pack2<kFp16>(__uint_as_float(o[8 * i + 2]) * inv, __uint_as_float(o[8 * i + 3]) * inv);
-          v.z = pack2<kFp16>(__uint_as_float(o[8 * i + 4]) * inv, __uint_as_float(o[8 * i + 5]) * inv);
-          v.w = pack2<kFp16>(__uint_as_float(o[8 * i + 6]) * inv, __uint_as_float(o[8 * i + 7]) * inv);
-          *(uint4*)(orow + c * 64 + i * 16) = v;
+          for (int e = 0; e < 4; ++e) {
+            uint4 v;
+            v.x = pack2<kFp16>(__uint_as_float(o[8 * e]) * inv, __uint_as_float(o[8 * e + 1]) * inv);
+            v.y = pack2<kFp16>(__uint_as_float(o[8 * e + 2]) * inv, __uint_as_float(o[8 * e + 3]) * inv);
+            v.z = pack2<kFp16>(__uint_as_float(o[8 * e + 4]) * inv, __uint_as_float(o[8 * e + 5]) * inv);
+            v.w = pack2<kFp16>(__uint_as_float(o[8 * e + 6]) * inv, __uint_as_float(o[8 * e + 7]) * inv);
+            *(uint4*)(orow + c * 64 + e * 16) = v;
+          }
         }
       }
       ptx::tc_fence_before();
       __syncwarp();
-      if (lane == 0) ptx::mbar_arrive(o_free);
-      if (a.lse && half == 0) a.lse[(size_t)(qt * kTQ + row) * a.Hq + h] = l_all > 0.f ? (m_run + log2f(l_all)) / kLog2e : -INFINITY;
+      if (lane == 0) ptx::mbar_arrive(&o_free[i]);
+      if (a.lse && qpos < a.S) a.lse[(size_t)qpos * a.Hq + head] = l_all > 0.f ? (m_run + log2f(l_all)) / kLog2e : -INFINITY;
+      ++n_item;
     }
   }
   ptx::tc_fence_before();
@@ -498,7 +559,9 @@ __global__ void __launch_bounds__(kTcThreads, 1) ring_attention_tc_kernel(const 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-bool make_map16(CUtensorMap* m, const void* base, bool fp16, uint64_t rows, uint64_t cols, uint32_t box_rows) {
+// blocks x [rows, cols] of 16-bit elements (blocks = 0: a 2-D map of one), box 64 x box_rows x 1: rows past the end of a block
+// come back as zeros.
+bool make_map16(CUtensorMap* m, const void* base, bool fp16, uint64_t blocks, uint64_t rows, uint64_t cols, uint32_t box_rows) {
   static EncodeTiledFn enc = nullptr;
   if (!enc) {
     void* p = nullptr;
@@ -507,11 +570,11 @@ bool make_map16(CUtensorMap* m, const void* base, bool fp16, uint64_t rows, uint
     enc = (EncodeTiledFn)p;
   }
   if (((uint64_t)base & 15) || ((cols * 2) & 15)) return false;
-  cuuint64_t dims[2] = {cols, rows};
-  cuuint64_t strides[1] = {cols * 2};
-  cuuint32_t box[2] = {64, box_rows};
-  cuuint32_t estr[2] = {1, 1};
-  return enc(m, fp16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (void*)base, dims, strides, box,
+  cuuint64_t dims[3] = {cols, rows, blocks};
+  cuuint64_t strides[2] = {cols * 2, rows * cols * 2};
+  cuuint32_t box[3] = {64, box_rows, 1};
+  cuuint32_t estr[3] = {1, 1, 1};
+  return enc(m, fp16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, blocks ? 3 : 2, (void*)base, dims, strides, box,
              estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
@@ -521,18 +584,19 @@ bool make_map16(CUtensorMap* m, const void* base, bool fp16, uint64_t rows, uint
 namespace iris_ring {
 
 int launch_ring_attention_tc(const RingArgs& a, cudaStream_t stream) {
-  if (a.S % kTQ || a.S <= 0) return 1;
+  if (a.S <= 0) return 1;
   const int W = a.ctx.world;
   TcArgs g;
   g.a = a;
   const bool f16 = a.is_fp16 != 0;
   const uint64_t kvc = (uint64_t)a.Hkv * kD;
-  if ((uint64_t)a.q & 15) return 1;      // Q rows are read with 16-byte loads
-  if (!make_map16(&g.tmKown, a.k, f16, a.S, kvc, kTK)) return 1;
-  if (!make_map16(&g.tmVown, a.v, f16, a.S, kvc, 64)) return 1;
+  if ((uint64_t)a.out & 15) return 1;    // output rows are written with 16-byte stores
+  if (!make_map16(&g.tmQ, a.q, f16, 0, a.S, (uint64_t)a.Hq * kD, kTQ)) return 1;
+  if (!make_map16(&g.tmKown, a.k, f16, 1, a.S, kvc, kTK)) return 1;
+  if (!make_map16(&g.tmVown, a.v, f16, 1, a.S, kvc, 64)) return 1;
   if (W > 1) {
-    if (!make_map16(&g.tmKbuf, a.kv_buf, f16, 4ull * W * a.S, kvc, kTK)) return 1;
-    if (!make_map16(&g.tmVbuf, a.kv_buf, f16, 4ull * W * a.S, kvc, 64)) return 1;
+    if (!make_map16(&g.tmKbuf, a.kv_buf, f16, 4ull * W, a.S, kvc, kTK)) return 1;
+    if (!make_map16(&g.tmVbuf, a.kv_buf, f16, 4ull * W, a.S, kvc, 64)) return 1;
   } else {
     g.tmKbuf = g.tmKown;
     g.tmVbuf = g.tmVown;
@@ -546,8 +610,9 @@ int launch_ring_attention_tc(const RingArgs& a, cudaStream_t stream) {
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const int items = (a.S / kTQ) * a.Hq;
-  int attn = sms - a.n_comm;                 // one CTA per SM (196 KB of shared memory), all resident
+  const int q_tiles = (a.S + kTQ - 1) / kTQ;
+  const int items = (a.Hq / a.Hkv) % 2 == 0 ? q_tiles * (a.Hq / 2) : (q_tiles + 1) / 2 * a.Hq;
+  int attn = sms - a.n_comm;                 // one CTA per SM (194 KB of shared memory), all resident
   if (attn > items) attn = items;
   if (attn < 1) return 1;
   const int grid = a.n_comm + attn;

@@ -98,3 +98,34 @@ def test_moe_one_rank_router_sort_gather(ctx, T, E, K):
         idx = layer.topk_idx[:T].long()
         assert (idx >= 0).all() and (idx < E).all() and all(len(set(r)) == K for r in idx.tolist())
     ctx.heap_release(mark)
+
+
+# ------------------------------------------------------------------------------------ attention on one rank
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("S,Hq,Hkv", [(1, 2, 2), (64, 4, 2), (127, 8, 2), (128, 3, 1), (129, 4, 4), (257, 6, 2), (384, 5, 5), (1000, 8, 8), (2500, 16, 2)])
+@pytest.mark.parametrize("causal", [False, True])
+def test_attention_any_length_and_group(ctx, dtype, S, Hq, Hkv, causal):
+    """Lengths on both sides of the 128-row tiles, head groups of odd size (two query tiles of one head per item, the
+    last item of an odd count with one) and of even size (two heads per item), against fp32 attention. P and the
+    output are rounded to 16 bits: |error| <= 2 u max|v| with u = 2^-8 (bf16) or 2^-11 (fp16), and max|v| < 6 here.
+    The scores are scaled up so that rows move their maximum late (the rescaling of O) as well as early."""
+    from iris_b200.models import RingAttention, reference_attention
+
+    g = _gen(S + Hq)
+    mk = lambda h, scale=1.0: (torch.randn(S, h, 128, device="cuda", generator=g) * scale).to(dtype)  # noqa: E731
+    q, k, v = mk(Hq, 3.0), mk(Hkv), mk(Hkv).clamp(-6, 6)
+    k = (k.float() * torch.linspace(0.1, 2.0, S, device="cuda")[:, None, None]).to(dtype)      # later keys score higher
+    mark = ctx.heap_mark()
+    layer = RingAttention(ctx, S, Hq, Hkv, dtype=dtype)
+    out, lse = layer(q, k, v, causal=causal, return_lse=True)
+    out2 = layer(q, k, v, causal=causal)                       # the other call parity
+    want = reference_attention(q, k, v, causal)
+    u = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+    assert (out.float() - want).abs().max().item() <= 2 * u * 6
+    assert torch.equal(out, out2)
+    kf = k.float().repeat_interleave(Hq // Hkv, dim=1)
+    s = torch.einsum("qhd,khd->qhk", q.float(), kf) * 128 ** -0.5
+    if causal:
+        s = s.masked_fill((torch.arange(S, device="cuda")[None, :] > torch.arange(S, device="cuda")[:, None])[:, None, :], float("-inf"))
+    assert (lse - torch.logsumexp(s, -1)).abs().max().item() < 1e-3
+    ctx.heap_release(mark)
