@@ -42,6 +42,8 @@ struct Common {
   CUtensorMap tmSFB;
   const float* bias_row;
   const float* bias_col;
+  int bias16 = 0;                  // 1: the biases have the output's 16-bit type
+  int bias_vec = 0;                // 1: bias_col is 16-byte aligned
   int32_t* status;
   int64_t* timeline;   // optional [tiles + chunks][4] nanosecond stamps (globaltimer)
 
@@ -56,8 +58,31 @@ struct Common {
   IRIS_D int b_sf_row(int tn, int kb) const { return (tn * kblocks + kb) * sfb_atoms; }
   IRIS_D bool is_bf16() const { return bf16 != 0; }
   IRIS_D bool has_bias() const { return bias_row != nullptr || bias_col != nullptr; }
-  IRIS_D float row_bias(int row) const { return (bias_row && row < sh.M) ? bias_row[row] : 0.f; }
-  IRIS_D float col_bias(int col) const { return (bias_col && col < sh.N) ? bias_col[col] : 0.f; }
+  IRIS_D float bias_at(const float* p, int i) const {
+    if (!bias16) return p[i];
+    return bf16 ? __bfloat162float(((const __nv_bfloat16*)p)[i]) : __half2float(((const __half*)p)[i]);
+  }
+  IRIS_D float row_bias(int row) const { return (bias_row && row < sh.M) ? bias_at(bias_row, row) : 0.f; }
+  // Biases of columns [col, col + 8), added to `v`. Every lane reads the same ones: as one or two 16-byte loads
+  // where the bias is aligned (N is a multiple of 8, so eight columns are inside together), not one load per value.
+  IRIS_D void add_col_bias8(int col, float (&v)[8]) const {
+    if (!bias_col || col >= sh.N) return;
+    if (!bias_vec) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) v[i] += bias_at(bias_col, col + i);
+    } else if (!bias16) {
+      const float4 a = __ldg((const float4*)(bias_col + col)), b = __ldg((const float4*)(bias_col + col) + 1);
+      v[0] += a.x; v[1] += a.y; v[2] += a.z; v[3] += a.w; v[4] += b.x; v[5] += b.y; v[6] += b.z; v[7] += b.w;
+    } else {
+      const uint4 u = __ldg((const uint4*)((const uint16_t*)bias_col + col));
+      const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float2 f = bf16 ? __bfloat1622float2(*(const __nv_bfloat162*)&w[i]) : __half22float2(*(const __half2*)&w[i]);
+        v[2 * i] += f.x; v[2 * i + 1] += f.y;
+      }
+    }
+  }
   IRIS_D void fail(int code) const {
     if (status) atomicCAS(status, 0, code);
   }

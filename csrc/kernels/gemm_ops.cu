@@ -24,6 +24,7 @@ using namespace iris;
 using namespace iris::gemm;
 
 #include "gemm_host.cuh"
+#include "gemm_skinny.h"
 
 namespace {
 
@@ -909,6 +910,8 @@ int fill_common(Common& c, const IrisGemmDesc* d, int bn, int pair, int gemm_cta
   }
   c.bias_row = d->bias_row;
   c.bias_col = d->bias_col;
+  c.bias16 = d->bias16;
+  c.bias_vec = ((uintptr_t)d->bias_col & 15) == 0;
   c.status = d->ctx.status;
   c.timeline = (int64_t*)d->timeline;
   return 0;
@@ -1044,7 +1047,9 @@ extern "C" int iris_gemm_launch(const IrisGemmDesc* d, void* stream_) {
   DeviceContext ctx;
   memcpy(&ctx, &d->ctx, sizeof(ctx));
 
-  if (d->op == IRIS_GEMM_LOCAL) {
+  // One rank: gathering and reducing over ranks is the identity, and every op is a local GEMM.
+  if (d->op == IRIS_GEMM_LOCAL || ctx.world <= 1) {
+    if (iris_gemm_skinny_takes(d)) return iris_gemm_skinny(d, stream);
     LocalGemm pol;
     r = fill_common(pol, d, p.bn, p.pair, p.gemm_ctas, d->A, d->M, d->K, d->lda);
     if (r) return r;

@@ -58,7 +58,7 @@ typedef struct IrisGemmDesc {
   const void* A; int64_t lda;
   const void* B; int64_t ldb;
   void* C; int64_t ldc;
-  const float* bias_row;  // [M] or null
+  const float* bias_row;  // [M] or null (see bias16)
   const float* bias_col;  // [N] or null
   IrisCtx ctx;
   void* sync_block;       // iris::SyncBlock on the heap
@@ -85,6 +85,8 @@ typedef struct IrisGemmDesc {
   // output and raise a per-tile flag, `comm_ctas` communication CTAs of the same kernel wait for the flags
   // and forward the tiles to the peers ("workgroup specialised"; flags: [2][128-row tiles x column tiles]).
   int32_t overlap;
+  // 0: bias_row / bias_col are fp32; 1: they have the output's 16-bit type (IRIS_GEMM_LOCAL)
+  int32_t bias16;
 } IrisGemmDesc;
 
 // Block-scaled fp8 (e4m3) GEMM: C = (A * scale_a) @ (B * scale_b)^T with A [M, K] and B [N, K]

@@ -69,6 +69,7 @@ class IrisGemmDesc(C.Structure):
         ("sf_b", C.c_void_p),
         ("sf_inbox", C.c_void_p),
         ("overlap", C.c_int32),
+        ("bias16", C.c_int32),
     ]
 
 

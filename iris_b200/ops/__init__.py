@@ -217,6 +217,29 @@ def _launch(ctx, d, ws) -> None:
     _lib.check(_lib.kernels().iris_gemm_launch(C.byref(d), C.c_void_p(_lib.current_stream_ptr())), f"{ws.operation} launch", kernels=1)
 
 
+def _span(t):
+    """First and one-past-last byte that ``t`` touches."""
+    return t.data_ptr(), t.data_ptr() + (sum((n - 1) * s for n, s in zip(t.shape, t.stride())) + 1) * t.element_size()
+
+
+def _one_rank_direct(ctx, out, A, B, bias) -> bool:
+    """One rank, a shape outside the fused kernels' tiles (rows not a multiple of 128): the op is a local GEMM, and it can
+    write ``out`` itself when the operands are what the kernel takes as they lie (16-byte aligned rows) and ``out``
+    overlaps neither; anything else keeps the staged path, which copies."""
+    if ctx.num_ranks != 1 or not (A.is_cuda and B.is_cuda and out.is_cuda) or not (A.dtype == B.dtype == out.dtype) or A.dtype not in _FUSED_DTYPES:
+        return False
+    if A.dim() != 2 or out.dim() != 2 or A.stride(1) != 1 or out.stride(1) != 1 or 0 in out.shape or A.shape[1] == 0:
+        return False
+    if (A.data_ptr() | out.data_ptr()) & 15 or (A.stride(0) | out.stride(0)) & 7 or out.stride(0) < out.shape[1]:
+        return False
+    lo, hi = _span(out)
+    for t in (A, B) if bias is None else (A, B, bias):
+        a, b = _span(t)
+        if a < hi and lo < b:
+            return False
+    return True
+
+
 def _local_matmul(A, B, bias=None, bias_dim=1):
     if A.is_cuda and A.dtype in _FUSED_DTYPES and A.stride(-1) == 1:
         return matmul(A, B, bias=bias, bias_dim=bias_dim)
@@ -308,8 +331,11 @@ def all_gather_matmul(shmem, output_tensor, A_sharded, B, bias=None, async_op=Fa
                              lambda: all_gather_matmul_preamble(shmem, A_sharded, B, config, shard_dim), extra=B.stride(-1) == 1)
     if ws.variant == "unfused":
         A_sharded, B = _lower_fp8(A_sharded, B, output_tensor.dtype)
-        gathered = _unfused_gather(shmem, ws, A_sharded, shard_dim)
-        output_tensor.copy_(_local_matmul(gathered, B, bias, bias_dim=0))
+        if _one_rank_direct(shmem, output_tensor, A_sharded, B, bias):
+            matmul(A_sharded, B, bias=bias, out=output_tensor, bias_dim=0)
+        else:
+            gathered = _unfused_gather(shmem, ws, A_sharded, shard_dim)
+            output_tensor.copy_(_local_matmul(gathered, B, bias, bias_dim=0))
     else:
         d, keep = _cached_desc(ws, _ptr_key(output_tensor, A_sharded, B, bias) + (id(shmem._ctx_epoch),),
                                lambda: _with_bias(bias, lambda b32: _agm_desc(shmem, output_tensor, A_sharded, B, b32, config, shard_dim)))
@@ -537,6 +563,10 @@ def matmul_reduce_scatter(shmem, output_tensor, A, B, bias=None, async_op=False,
         from ..ccl import Config
 
         A, B = _lower_fp8(A, B, output_tensor.dtype)
+        if scatter_rows and _one_rank_direct(shmem, output_tensor, A, B, b):
+            matmul(A, B, bias=b, out=output_tensor, bias_dim=0)
+            _finish(shmem, async_op)
+            return ws
         part = _on_heap(shmem, ws, "part", _local_matmul(A, B, b, bias_dim=0))
         if scatter_rows:
             dst = _scratch(shmem, ws, "out", want, A.dtype)

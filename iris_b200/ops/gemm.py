@@ -9,10 +9,13 @@ main loop the reference's fused ops are built on (iris/ops/matmul_all_reduce.py:
 from __future__ import annotations
 
 import ctypes as C
+import struct
+import threading
 
 import torch
 
 from .. import _lib
+from .gemm_fp8 import BlockScaled, blockscaled_tile_n, matmul_fp8_blockscaled
 
 
 def b_layout(B: torch.Tensor):
@@ -48,6 +51,25 @@ def fill_desc(desc: _lib.IrisGemmDesc, A: torch.Tensor, B: torch.Tensor, out: to
     return Bd
 
 
+_DTYPES = (torch.bfloat16, torch.float16)
+# The descriptor's fields up to ctx: twelve 32-bit ones (op ... two_sm), then A, lda, B, ldb, C, ldc and the two biases.
+_HEAD = struct.Struct("12i8Q")
+assert _lib.IrisGemmDesc.ctx.offset == _HEAD.size
+_tls = threading.local()
+
+
+def _local_desc():
+    """This thread's descriptor of a local GEMM and the memory under it. Setting the fields one by one cost more than
+    the launch; the launch reads the descriptor before it returns, so one per thread is enough."""
+    hit = getattr(_tls, "desc", None)
+    if hit is None:
+        buf = bytearray(C.sizeof(_lib.IrisGemmDesc))
+        desc = _lib.IrisGemmDesc.from_buffer(buf)
+        desc.ctx.world = 1
+        hit = _tls.desc = (desc, buf)
+    return hit
+
+
 def matmul(A: torch.Tensor, B: torch.Tensor, bias: torch.Tensor | None = None, out: torch.Tensor | None = None,
            bias_dim: int = 1, bn: int = 0, two_sm: bool | None = None) -> torch.Tensor:
     """``out = A @ B (+ bias)``; ``bias_dim=0`` adds ``bias[m]`` to every row m, ``1`` adds ``bias[n]``.
@@ -58,8 +80,6 @@ def matmul(A: torch.Tensor, B: torch.Tensor, bias: torch.Tensor | None = None, o
 
     Block-scaled e4m3 operands (``BlockScaled`` activation and weight, see ``gemm_fp8``) go to the
     hardware-scaled kernel; the result is bf16 unless ``out`` says otherwise."""
-    from .gemm_fp8 import BlockScaled, blockscaled_tile_n, matmul_fp8_blockscaled
-
     if isinstance(A, BlockScaled) or isinstance(B, BlockScaled):
         if not (isinstance(A, BlockScaled) and isinstance(B, BlockScaled) and A.kind == "activation" and B.kind == "weight"):
             raise TypeError("an fp8 product takes a BlockScaled activation and a BlockScaled weight")
@@ -77,13 +97,20 @@ def matmul(A: torch.Tensor, B: torch.Tensor, bias: torch.Tensor | None = None, o
         raise ValueError(f"out must be {(M, N)} on {A.device}, got {tuple(out.shape)} on {out.device}")
     if bias is not None and (bias_dim not in (0, 1) or bias.dim() != 1 or bias.numel() != (M if bias_dim == 0 else N)):
         raise ValueError(f"bias must have {M if bias_dim == 0 else N} entries for bias_dim={bias_dim}, got {tuple(bias.shape)}")
-    desc = _lib.IrisGemmDesc()
-    desc.op = _lib.GEMM_LOCAL
-    desc.M, desc.N, desc.K = M, N, K
-    b32 = bias.float().contiguous() if bias is not None else None
-    keep = fill_desc(desc, A, B, out, bias_row=b32 if bias_dim == 0 else None, bias_col=b32 if bias_dim == 1 else None, bn=bn)
-    desc.ctx.world = 1
-    desc.two_sm = 0 if two_sm is None else (2 if two_sm else 1)
+    if A.dtype not in _DTYPES or B.dtype != A.dtype or out.dtype != A.dtype:
+        raise TypeError("the sm_100a GEMM takes fp16 or bf16 operands of one dtype")
+    if A.stride(1) != 1 or out.stride(1) != 1:
+        raise ValueError("A and the output must be row-major")
+    Bd, kmajor, ldb = b_layout(B)
+    bv, bias16 = None, 0
+    if bias is not None:         # read as it is when it has the operands' type, else as fp32
+        bias16 = 1 if bias.dtype == A.dtype else 0
+        bv = (bias if bias16 else bias.float()).contiguous()
+    bp = bv.data_ptr() if bv is not None else 0
+    desc, buf = _local_desc()
+    _HEAD.pack_into(buf, 0, _lib.GEMM_LOCAL, M, N, K, _lib.DTYPE_CODE[A.dtype], kmajor, bn, 0, 0, 0, 0,
+                    0 if two_sm is None else (2 if two_sm else 1), A.data_ptr(), A.stride(0), Bd.data_ptr(), ldb, out.data_ptr(), out.stride(0),
+                    bp if bias_dim == 0 else 0, bp if bias_dim == 1 else 0)
+    desc.bias16 = bias16
     _lib.check(_lib.kernels().iris_gemm_launch(C.byref(desc), _lib.current_stream_ptr()), "gemm launch", kernels=1)
-    del keep
     return out

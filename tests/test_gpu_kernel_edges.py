@@ -129,3 +129,75 @@ def test_attention_any_length_and_group(ctx, dtype, S, Hq, Hkv, causal):
         s = s.masked_fill((torch.arange(S, device="cuda")[None, :] > torch.arange(S, device="cuda")[:, None])[:, None, :], float("-inf"))
     assert (lse - torch.logsumexp(s, -1)).abs().max().item() < 1e-3
     ctx.heap_release(mark)
+
+
+# ------------------------------------------------------------------------------------ few rows
+@pytest.mark.parametrize("kmajor", [True, False])
+@pytest.mark.parametrize("M,N,K", [(1, 8, 8), (1, 1024, 64), (16, 136, 520), (17, 1032, 2048), (32, 3584, 72), (33, 264, 4096), (64, 2000, 3000),
+                                   (65, 1024, 2048), (128, 640, 2056), (129, 256, 2816), (256, 4096, 2816), (200, 1544, 8192), (256, 128, 16384)])
+def test_few_rows_gemm(kmajor, M, N, K):
+    """Both sides of every step of the dispatch, ragged N and K, clusters of 1 to 8, biases of either kind and type, an
+    output whose rows take no 8-byte stores. fp32 sums of bf16 products: |error| <= 2^-8 |C| (the output's rounding)
+    plus a few 2^-24 sum |a||b|."""
+    from iris_b200.ops import matmul
+
+    for dtype, u in ((torch.bfloat16, 2.0 ** -8), (torch.float16, 2.0 ** -11)):
+        g = _gen(M + N + K)
+        A = torch.randn(M, K, device="cuda", generator=g).to(dtype)
+        W = (torch.randn(N, K, device="cuda", generator=g) * K ** -0.5).to(dtype)
+        B = W.t() if kmajor else W.t().contiguous()
+        ref = A.double() @ B.double()
+        slack = 32 * 2.0 ** -24 * (A.double().abs() @ B.double().abs())
+        wide = torch.empty(M, N + 3, device="cuda", dtype=dtype)
+        for bias, dim in ((None, 1), (torch.randn(N, device="cuda", generator=g).to(dtype), 1), (torch.randn(N, device="cuda", generator=g), 1),
+                          (torch.randn(M, device="cuda", generator=g).to(dtype), 0), (torch.randn(M + 1, device="cuda", generator=g)[1:], 0)):
+            want = ref if bias is None else ref + (bias.double()[:, None] if dim == 0 else bias.double()[None, :])
+            for out in (None, wide[:, 1:1 + N] if M <= 32 else None):
+                C = matmul(A, B, bias=bias, bias_dim=dim, out=out)
+                assert ((C.double() - want).abs() <= 1.01 * u * want.abs() + slack + 1e-7).all()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("offset", [0, 1, 4])
+def test_column_bias_of_the_main_loop(dtype, offset):
+    """The epilogue reads a column bias by 16-byte loads where it is aligned and one by one elsewhere, in fp32 and in
+    the operands' type; N ends inside a 32-column chunk. Same bound as the test above."""
+    from iris_b200.ops import matmul
+
+    M, N, K = 300, 1000, 256
+    g = _gen(offset)
+    A = torch.randn(M, K, device="cuda", generator=g).to(dtype)
+    B = (torch.randn(N, K, device="cuda", generator=g) * K ** -0.5).to(dtype).t()
+    u = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+    slack = 32 * 2.0 ** -24 * (A.double().abs() @ B.double().abs())
+    for bdt in (dtype, torch.float32):
+        bias = torch.randn(N + 8, device="cuda", generator=g).to(bdt)[offset:offset + N]
+        want = A.double() @ B.double() + bias.double()[None, :]
+        for kw in ({}, {"bn": 128}, {"bn": 224, "two_sm": False}, {"bn": 256, "two_sm": True}):
+            assert ((matmul(A, B, bias=bias, **kw).double() - want).abs() <= 1.01 * u * want.abs() + slack + 1e-7).all()
+
+
+@pytest.mark.parametrize("T,D,F", [(48, 1024, 512), (1, 256, 128), (130, 512, 384), (1000, 256, 512)])
+def test_one_rank_ops_take_any_row_count(ctx, T, D, F):
+    """Rows that are not a multiple of 128 on one rank: the op writes the output directly where it can, and still takes
+    outputs it cannot write (another dtype, overlapping an input, unaligned rows)."""
+    g = _gen(T)
+    x = torch.randn(T, D, device="cuda", generator=g).to(torch.bfloat16)
+    w1 = (torch.randn(F, D, device="cuda", generator=g) * D ** -0.5).to(torch.bfloat16).t()
+    w2 = (torch.randn(D, F, device="cuda", generator=g) * F ** -0.5).to(torch.bfloat16).t()
+    bias = torch.randn(T, device="cuda", generator=g).to(torch.bfloat16)
+    h_ref = x.double() @ w1.double() + bias.double()[:, None]
+    outs = [torch.empty(T, F, dtype=torch.bfloat16, device="cuda"), torch.empty(T, F + 1, dtype=torch.bfloat16, device="cuda")[:, 1:],
+            torch.empty(T, F, dtype=torch.float32, device="cuda"), torch.empty(F, T, dtype=torch.bfloat16, device="cuda").t()]
+    for h in outs:
+        ctx.ops.all_gather_matmul(h, x, w1, bias=bias, shard_dim=0, async_op=True)
+        assert ((h.double() - h_ref).norm() / h_ref.norm()).item() < 4e-3
+    h = outs[0]
+    y_ref = h.double() @ w2.double()
+    for y in (torch.empty(T, D, dtype=torch.bfloat16, device="cuda"), torch.empty(T, D, dtype=torch.float32, device="cuda")):
+        ctx.ops.matmul_reduce_scatter(y, h, w2, scatter_rows=True, async_op=True)
+        assert ((y.double() - y_ref).norm() / y_ref.norm()).item() < 4e-3
+    sq = (torch.randn(D, D, device="cuda", generator=g) * D ** -0.5).to(torch.bfloat16)
+    want = x.double() @ sq.double()
+    ctx.ops.all_gather_matmul(x, x, sq, shard_dim=0, async_op=True)          # in place
+    assert ((x.double() - want).norm() / want.norm()).item() < 4e-3
