@@ -2,13 +2,17 @@
 // over the ranks (reference: examples/13_flash_decode/decode_kernels.py:141-415 and
 // flash_decode_fused_layer.py:38-148).
 //
-//   1. splitk kernel  grid (splits, kv_heads * head_groups, batch): attention of the query heads
-//      of one KV head over one slice of the LOCAL KV shard, paged KV gathered through the block
-//      table, online softmax; writes a normalised partial output and its log-sum-exp per split.
+//   1. splitk kernel  two CTAs per SM; the query heads of one KV head attend over a run of tiles of 64 positions of
+//      the LOCAL KV shard, paged KV gathered through the block table, online softmax; writes a normalised
+//      partial output and its log-sum-exp per run. The tiles of all (sequence, KV head) pairs form one list that
+//      is cut into equal pieces, one per CTA, on the device, from the lengths: a CTA may end one pair and begin the next, a pair
+//      may be spread over many CTAs. (With the same number of splits for every sequence, the CTAs of the longest
+//      one finished last: 32 sequences of 8192 to 32768 positions, 640 us where the bytes take 404; now 450. One
+//      sequence of 32768: 512 CTAs on 296 places; 53 us, now 39.)
 //      K/V stream through a ring of swizzled shared-memory tiles; QK^T and PV run on tensor
 //      cores with the query heads of the group as the M dimension (each K/V byte is read from HBM
-//      exactly once; the kernel is bound by HBM bandwidth). Two ways of filling the ring: one
-//      thread issuing TMA box loads per page through a tensor map over the cache (page sizes 8,
+//      exactly once; the kernel is bound by HBM bandwidth). Two ways of filling the ring: a
+//      warp issuing TMA box loads per page through a tensor map over the cache (page sizes 8,
 //      16, 32 or a multiple of 64; completion on an mbarrier per stage), or all threads issuing
 //      16-byte cp.async copies (any page size).
 //   2. exchange kernel (persistent): phase A combines the local splits of every (batch, head) and
@@ -17,7 +21,8 @@
 //      bounded) for the flags of all source ranks and merges the W partials into the final output.
 //      All pushes are issued before any wait, so ranks never wait on each other in a cycle; the
 //      buffers are double-buffered by call parity and flags carry the call number, so nothing is
-//      cleared between calls (the reference zeroes its flags and runs a host barrier per call).
+//      cleared between calls (the reference zeroes its flags and runs a host barrier per call). One rank has nothing
+//      to exchange: a kernel of one block per (batch, head) folds the partials into the output.
 // lse is kept in fp32 (the reference stores it in the fp16 payload).
 #include <cuda_runtime.h>
 #include <cuda_bf16.h>
@@ -56,8 +61,9 @@ struct DecodeArgs {
   const __nv_bfloat16* v_cache;
   const int32_t* block_table;      // [B, max_blocks]
   const int32_t* kv_lens;          // [B] local lengths
-  float* partial;                  // [B, Hq, splits, D + 1]  (o normalised, lse in log2 units)
-  int B, Hq, Hkv, page, max_blocks, splits, group, head_groups;
+  float* partial;                  // [B, Hq, splits, D + 1]  (o normalised, lse in log2 units; -inf in places that no run fills)
+  int B, Hq, Hkv, page, max_blocks, group, head_groups;
+  int splits;                      // places for partial results per (sequence, head)
   float sm_scale, soft_cap;
   int is_fp16;
 };
@@ -101,31 +107,100 @@ __device__ __forceinline__ uint32_t tile_off(int row, int chunk) {
 }
 
 constexpr uint64_t kTmaWaitNs = 2000000000ull;
+constexpr int kMaxSeqs = 1024;     // sequences of one launch (the tile list's prefix sums lie in shared memory)
+constexpr int kMinRun = 4;         // tiles a CTA takes at least
+constexpr int kRingBytes = kStages * 2 * kTileBytes;
+static_assert(kWarps * 16 * kD * (int)sizeof(float) == 2 * kTileBytes, "a run's end uses one stage as scratch");
+// ring, stage barriers, the warps' row maxima and sums, prefix sums
+constexpr int kDecodeSmem = kRingBytes + 64 + kWarps * 16 * 2 * 4 + (kMaxSeqs + 2) * 4;
+constexpr int kDecodeSmemTma = kDecodeSmem + 1024;      // alignment slack
 
+// One run: tiles [t_first, t_first + n_tiles) of one (sequence, KV head, group of up to 16 query heads).
+struct Run {
+  int b, kvh, h0, heads_here, t_first, n_tiles, slot, n_slots, lo, hi;
+};
+// The CTA's runs (see the head of this file); every role walks the same list.
+struct RunList {
+  const DecodeArgs& a;
+  const int* pre;               // [B + 1] tiles in front of sequence b, then the longest sequence's
+  int heads_kv, per, flat, flat_end, whole;
+  __device__ RunList(const DecodeArgs& a_, const int* pre_) : a(a_), pre(pre_) {
+    heads_kv = a.Hkv * a.head_groups;
+    const int total = pre[a.B] * heads_kv, longest = pre[a.B + 1];
+    // tiles per CTA: an equal share, but not a handful, and no pair cut into more runs than there are places
+    per = max(kMinRun, (total + (int)gridDim.x - 1) / (int)gridDim.x);
+    if (a.splits > 1) per = max(per, (longest - 1 + a.splits - 2) / (a.splits - 1));
+    flat = min(total, (int)blockIdx.x * per);
+    flat_end = min(total, flat + per);
+    whole = blockIdx.x;         // with one place per pair whole pairs are handed out instead
+  }
+  __device__ bool next(Run& r) {
+    int x;
+    if (a.splits > 1) {
+      if (flat >= flat_end) return false;
+      const int u = flat / heads_kv;                     // lies in the sequence's [pre[b], pre[b + 1])
+      int lo_b = 0, hi_b = a.B - 1;
+      while (lo_b < hi_b) {
+        const int mid = (lo_b + hi_b + 1) >> 1;
+        if (pre[mid] <= u) lo_b = mid; else hi_b = mid - 1;
+      }
+      r.b = lo_b;
+      const int n_b = pre[r.b + 1] - pre[r.b], rem = flat - pre[r.b] * heads_kv;
+      x = rem / n_b;
+      r.t_first = rem - x * n_b;
+      r.n_tiles = min(n_b - r.t_first, flat_end - flat);
+      const int pair0 = flat - r.t_first;                // first tile of the pair in the list
+      r.slot = blockIdx.x - pair0 / per;
+      r.n_slots = (pair0 + n_b - 1) / per - pair0 / per + 1;
+      flat += r.n_tiles;
+    } else {
+      if (whole >= a.B * heads_kv) return false;
+      r.b = whole / heads_kv;
+      x = whole - r.b * heads_kv;
+      r.t_first = 0;
+      r.n_tiles = pre[r.b + 1] - pre[r.b];
+      r.slot = 0; r.n_slots = 1;
+      whole += gridDim.x;
+    }
+    r.kvh = x / a.head_groups;
+    const int hg = x - r.kvh * a.head_groups;
+    r.heads_here = min(16, a.group - hg * 16);
+    r.h0 = r.kvh * a.group + hg * 16;
+    r.lo = r.t_first * kBlockN;
+    r.hi = min(a.kv_lens[r.b], r.lo + r.n_tiles * kBlockN);
+    return true;
+  }
+};
+// One warp: the prefix sums. A sequence without positions still takes one (empty) tile: somebody has to write its result.
+__device__ __forceinline__ void prefix_tiles(const DecodeArgs& a, int* pre, int lane) {
+  int carry = 0, longest = 0;
+  for (int base = 0; base < a.B; base += 32) {
+    const int n = base + lane < a.B ? max(1, (a.kv_lens[base + lane] + kBlockN - 1) / kBlockN) : 0;
+    int incl = n;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int up = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += up;
+    }
+    if (base + lane < a.B) pre[base + lane + 1] = carry + incl;
+    carry += __shfl_sync(0xffffffffu, incl, 31);
+    longest = max(longest, __reduce_max_sync(0xffffffffu, n));
+  }
+  if (lane == 0) { pre[0] = 0; pre[a.B + 1] = longest; }
+}
+
+// Attention state of one of the four computing warps: up to 16 query heads (rows) against the warp's 16 positions of
+// each tile.
 template <bool kFp16, bool kTma>
-__global__ void __launch_bounds__(kWarps * 32, 2) decode_splitk_kernel(const __grid_constant__ DecodeArgs a) {
-  extern __shared__ __align__(128) uint8_t smem_raw[];
-  // the TMA path needs 1024-byte aligned tiles (the launch adds the slack)
-  uint8_t* smem = kTma ? (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023) : smem_raw;
-  const int split = blockIdx.x;
-  const int kvh = blockIdx.y / a.head_groups, hg = blockIdx.y % a.head_groups;
-  const int b = blockIdx.z;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int heads_here = min(16, a.group - hg * 16);   // query heads of this KV head handled by this CTA
-  const int h0 = kvh * a.group + hg * 16;
+struct Attend {
+  uint32_t qf[8][4];             // Q fragments (A operand, rows = heads, padded to 16 with zeros)
+  float o[16][4], m_run[2], l_run[2];
 
-  const int len = a.kv_lens[b];
-  const int per = ((len + a.splits - 1) / a.splits + kBlockN - 1) / kBlockN * kBlockN;   // positions per split, tile aligned
-  const int lo = min(len, split * per), hi = min(len, lo + per);
-  const int n_tiles = (hi - lo + kBlockN - 1) / kBlockN;
-
-  // ---- Q fragments (A operand, rows = heads, padded to 16 with zeros)
-  uint32_t qf[8][4];
-  {
+  __device__ __forceinline__ void begin(const DecodeArgs& a, const Run& r, int lane) {
     const int r0 = lane >> 2, c0 = (lane & 3) * 2;
-    const uint32_t* qrow0 = (const uint32_t*)(a.q + ((size_t)b * a.Hq + h0 + r0) * kD);
-    const uint32_t* qrow1 = (const uint32_t*)(a.q + ((size_t)b * a.Hq + h0 + r0 + 8) * kD);
-    const bool v0 = r0 < heads_here, v1 = r0 + 8 < heads_here;
+    const uint32_t* qrow0 = (const uint32_t*)(a.q + ((size_t)r.b * a.Hq + r.h0 + r0) * kD);
+    const uint32_t* qrow1 = (const uint32_t*)(a.q + ((size_t)r.b * a.Hq + r.h0 + r0 + 8) * kD);
+    const bool v0 = r0 < r.heads_here, v1 = r0 + 8 < r.heads_here;
 #pragma unroll
     for (int ks = 0; ks < 8; ++ks) {
       const int c = (ks * 16 + c0) >> 1;
@@ -134,104 +209,15 @@ __global__ void __launch_bounds__(kWarps * 32, 2) decode_splitk_kernel(const __g
       qf[ks][2] = v0 ? qrow0[c + 4] : 0u;
       qf[ks][3] = v1 ? qrow1[c + 4] : 0u;
     }
+#pragma unroll
+    for (int i = 0; i < 16; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
+    m_run[0] = m_run[1] = -INFINITY;
+    l_run[0] = l_run[1] = 0.f;
   }
-  float o[16][4];
-#pragma unroll
-  for (int i = 0; i < 16; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
-  float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f};
-  const float scale2 = a.sm_scale * kLog2e;
-
-  const uint32_t smem_base = (uint32_t)__cvta_generic_to_shared(smem);
-  const int32_t* bt = a.block_table + (size_t)b * a.max_blocks;
-  const size_t pos_stride = (size_t)a.Hkv * kD;   // elements between consecutive positions of a page
-
-  auto issue_tile = [&](int t) {
-    const int stage = t % kStages;
-    const uint32_t ks = smem_base + stage * 2 * kTileBytes, vs = ks + kTileBytes;
-    // 64 rows x 16 chunks for K and for V = 2048 chunks, 128 threads -> 16 each
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const int idx = threadIdx.x + i * 128;     // 0..1023
-      const int row = idx >> 4, chunk = idx & 15;
-      const int pos = lo + t * kBlockN + row;
-      if (pos < hi) {
-        const int blk = bt[pos / a.page];
-        const size_t e = ((size_t)blk * a.page + pos % a.page) * pos_stride + (size_t)kvh * kD + chunk * 8;
-        cp_async16(ks + tile_off<false>(row, chunk), a.k_cache + e);
-        cp_async16(vs + tile_off<false>(row, chunk), a.v_cache + e);
-      } else {
-        *(uint4*)(smem + stage * 2 * kTileBytes + tile_off<false>(row, chunk)) = make_uint4(0, 0, 0, 0);
-        *(uint4*)(smem + stage * 2 * kTileBytes + kTileBytes + tile_off<false>(row, chunk)) = make_uint4(0, 0, 0, 0);
-      }
-    }
-  };
-  // TMA path, one thread: one box per page piece and half of the head dimension, for K and for V.
-  // Tiles start at multiples of 64 positions, so a box never straddles a page.
-  uint64_t* full = (uint64_t*)(smem + kStages * 2 * kTileBytes);
-  auto issue_tile_tma = [&](int t) {
-    const int stage = t % kStages;
-    uint8_t* kdst = smem + stage * 2 * kTileBytes;
-    uint8_t* vdst = kdst + kTileBytes;
-    const int pos0 = lo + t * kBlockN;
-    const int rows = min(kBlockN, hi - pos0);
-    const int nbox = (rows + a.box_rows - 1) / a.box_rows;
-    ptx::mbar_expect_tx(&full[stage], (uint32_t)(nbox * a.box_rows * 128 * 4));
-    for (int j = 0; j < nbox; ++j) {
-      const int pos = pos0 + j * a.box_rows;
-      const int y = bt[pos / a.page] * a.page + pos % a.page;
-      const int off = j * a.box_rows * 128;
-#pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        ptx::tma_load_2d(kdst + half * (kBlockN * 128) + off, &a.tmK, &full[stage], kvh * kD + half * 64, y);
-        ptx::tma_load_2d(vdst + half * (kBlockN * 128) + off, &a.tmV, &full[stage], kvh * kD + half * 64, y);
-      }
-    }
-  };
-
-  if constexpr (kTma) {
-    if (threadIdx.x == 0) {
-      for (int i = 0; i < kStages; ++i) ptx::mbar_init(&full[i], 1);
-      ptx::fence_mbar_init();
-      ptx::fence_proxy_async();
-    }
-    __syncthreads();
-    if (threadIdx.x == 0)
-      for (int t = 0; t < kStages - 1 && t < n_tiles; ++t) issue_tile_tma(t);
-  } else {
-    for (int t = 0; t < kStages - 1; ++t) {
-      if (t < n_tiles) issue_tile(t);
-      cp_async_commit();
-    }
-  }
-  for (int t = 0; t < n_tiles; ++t) {
-    const int stage = t % kStages;
-    if constexpr (kTma) {
-      if (!ptx::mbar_wait(&full[stage], (uint32_t)((t / kStages) & 1), kTmaWaitNs)) {
-        if (a.status) atomicCAS(a.status, 0, (int)kTimeoutPipeline);
-        break;     // every thread of the CTA waits on the same barrier, so all of them leave here
-      }
-      __syncthreads();   // everybody is done with tile t-1: its stage can be refilled
-      if (threadIdx.x == 0 && t + kStages - 1 < n_tiles) issue_tile_tma(t + kStages - 1);
-      const int rows = hi - (lo + t * kBlockN);
-      if (rows < kBlockN) {
-        // last, partial tile: rows past the end hold whatever the page (or an older tile) held;
-        // their scores are masked below, and their V rows are cleared so that 0 * NaN cannot arise
-        uint8_t* vt = smem + stage * 2 * kTileBytes + kTileBytes;
-        for (int idx = threadIdx.x; idx < (kBlockN - rows) * 16; idx += blockDim.x) {
-          const int row = rows + (idx >> 4), chunk = idx & 15;
-          *(uint4*)(vt + tile_off<true>(row, chunk)) = make_uint4(0, 0, 0, 0);
-        }
-        __syncthreads();
-      }
-    } else {
-      cp_async_wait<kStages - 2>();
-      __syncthreads();
-      if (t + kStages - 1 < n_tiles) issue_tile(t + kStages - 1);
-      cp_async_commit();
-    }
-    const uint32_t ks = smem_base + stage * 2 * kTileBytes, vs = ks + kTileBytes;
+  // ks, vs: shared-memory addresses of the K and V tile; pos0: position of the tile's first row
+  __device__ __forceinline__ void tile(const DecodeArgs& a, uint32_t ks, uint32_t vs, int pos0, int hi, int warp, int lane) {
+    const float scale2 = a.sm_scale * kLog2e;
     const int p0 = warp * 16;   // this warp's 16 positions of the tile
-
     // ---- S = Q K^T for 16 heads x 16 positions
     float s[2][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}};
 #pragma unroll
@@ -243,7 +229,7 @@ __global__ void __launch_bounds__(kWarps * 32, 2) decode_splitk_kernel(const __g
       mma16816<kFp16>(s[1], qf[kk], kf[2], kf[3]);
     }
     // ---- online softmax (rows lane/4 and lane/4 + 8; columns: nb * 8 + (lane % 4) * 2 + {0, 1})
-    const int pos_base = lo + t * kBlockN + p0 + (lane & 3) * 2;
+    const int pos_base = pos0 + p0 + (lane & 3) * 2;
     float mx[2] = {-INFINITY, -INFINITY};
 #pragma unroll
     for (int nb = 0; nb < 2; ++nb)
@@ -300,13 +286,9 @@ __global__ void __launch_bounds__(kWarps * 32, 2) decode_splitk_kernel(const __g
       mma16816<kFp16>(o[nb2 * 2 + 1], pf, vf[2], vf[3]);
     }
   }
-  if constexpr (!kTma) cp_async_wait<0>();
-  __syncthreads();
-
-  // ---- merge the 4 warps (each saw a quarter of the positions), write the partial for this split
-  float* sm_o = (float*)smem;                         // [warps][8 rows... 16][128]
-  float* sm_ml = sm_o + kWarps * 16 * kD;             // [warps][16][2]
-  {
+  // Merges the four warps (each saw a quarter of the positions) and writes the partial of the run. `sm_o` is 32 KB that
+  // nobody else uses, `sm_ml` 512 bytes; the computing warps' threads call it together (named barrier 1).
+  __device__ __forceinline__ void finish(const DecodeArgs& a, const Run& run, float* sm_o, float* sm_ml, int warp, int lane) {
     const int r0 = lane >> 2, c0 = (lane & 3) * 2;
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
@@ -318,25 +300,208 @@ __global__ void __launch_bounds__(kWarps * 32, 2) decode_splitk_kernel(const __g
       sm_ml[(warp * 16 + r0) * 2] = m_run[0]; sm_ml[(warp * 16 + r0) * 2 + 1] = l_run[0];
       sm_ml[(warp * 16 + r0 + 8) * 2] = m_run[1]; sm_ml[(warp * 16 + r0 + 8) * 2 + 1] = l_run[1];
     }
+    ptx::named_barrier(1, kWarps * 32);
+    const int tid = warp * 32 + lane;
+    for (int idx = tid; idx < run.heads_here * kD; idx += kWarps * 32) {
+      const int h = idx / kD, d = idx - h * kD;
+      float m = -INFINITY;
+#pragma unroll
+      for (int w = 0; w < kWarps; ++w) m = fmaxf(m, sm_ml[(w * 16 + h) * 2]);
+      float l = 0.f, acc = 0.f;
+#pragma unroll
+      for (int w = 0; w < kWarps; ++w) {
+        const float mw = sm_ml[(w * 16 + h) * 2];
+        const float sc = mw == -INFINITY ? 0.f : exp2f(mw - m);
+        l += sm_ml[(w * 16 + h) * 2 + 1] * sc;
+        acc += sm_o[(w * 16 + h) * kD + d] * sc;
+      }
+      float* dst = a.partial + (((size_t)run.b * a.Hq + run.h0 + h) * a.splits + run.slot) * (kD + 1);
+      dst[d] = l > 0.f ? acc / l : 0.f;
+      if (d == 0) dst[kD] = l > 0.f ? m + log2f(l) : -INFINITY;
+    }
+    // the run that begins a pair marks the places no run fills
+    const int spare = a.splits - run.n_slots;
+    if (run.t_first == 0)
+      for (int idx = tid; idx < run.heads_here * spare; idx += kWarps * 32) {
+        const int h = idx / spare, s = run.n_slots + idx % spare;
+        a.partial[(((size_t)run.b * a.Hq + run.h0 + h) * a.splits + s) * (kD + 1) + kD] = -INFINITY;
+      }
+    ptx::named_barrier(1, kWarps * 32);       // the scratch has been read
+  }
+};
+
+// TMA fill. Warp 4 fetches: a lane per box (page piece, half of the head dimension, K or V) looks up its page and
+// issues its load, so the four computing warps never wait for block-table lookups (with them in thread 0 of a computing warp, 16
+// boxes per tile at a page size of 16 took longer than the tile's bytes). The computing warps wait for a tile and hand
+// it back one by one, no barrier of the CTA per tile.
+template <bool kFp16>
+__global__ void __launch_bounds__(kWarps * 32 + 32, 2) decode_splitk_tma_kernel(const __grid_constant__ DecodeArgs a) {
+  extern __shared__ __align__(128) uint8_t smem_raw[];
+  uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  uint64_t* full = (uint64_t*)(smem + kRingBytes);
+  uint64_t* empty = full + kStages;
+  float* sm_ml = (float*)(smem + kRingBytes + 64);
+  int* pre = (int*)(smem + kRingBytes + 64 + kWarps * 16 * 2 * 4);
+  if (warp == 0) prefix_tiles(a, pre, lane);
+  if (threadIdx.x == 32) {
+    for (int i = 0; i < kStages; ++i) { ptx::mbar_init(&full[i], 1); ptx::mbar_init(&empty[i], kWarps); }
+    ptx::fence_mbar_init();
+    ptx::fence_proxy_async();
   }
   __syncthreads();
-  for (int idx = threadIdx.x; idx < heads_here * kD; idx += blockDim.x) {
-    const int h = idx / kD, d = idx - h * kD;
-    float m = -INFINITY;
-#pragma unroll
-    for (int w = 0; w < kWarps; ++w) m = fmaxf(m, sm_ml[(w * 16 + h) * 2]);
-    float l = 0.f, acc = 0.f;
-#pragma unroll
-    for (int w = 0; w < kWarps; ++w) {
-      const float mw = sm_ml[(w * 16 + h) * 2];
-      const float sc = mw == -INFINITY ? 0.f : exp2f(mw - m);
-      l += sm_ml[(w * 16 + h) * 2 + 1] * sc;
-      acc += sm_o[(w * 16 + h) * kD + d] * sc;
+  RunList list(a, pre);
+  Run run;
+  const uint32_t base = (uint32_t)__cvta_generic_to_shared(smem);
+  uint32_t it = 0;                           // tiles so far (ring position)
+  auto fail = [&]() { if (a.status) atomicCAS(a.status, 0, (int)kTimeoutPipeline); };
+  if (warp == kWarps) {
+    while (list.next(run)) {
+      const int32_t* bt = a.block_table + (size_t)run.b * a.max_blocks;
+      const int j = lane >> 2, hf = (lane >> 1) & 1, is_v = lane & 1;
+      for (int t = 0; t < run.n_tiles; ++t, ++it) {
+        const int stage = it % kStages;
+        const int pos0 = run.lo + t * kBlockN;
+        const int rows = max(0, min(kBlockN, run.hi - pos0));
+        const int nbox = (rows + a.box_rows - 1) / a.box_rows;
+        const int pos = pos0 + j * a.box_rows;
+        int y = 0;
+        if (j < nbox) y = __ldg(bt + pos / a.page) * a.page + pos % a.page;      // looked up before the stage is waited for
+        if (!__all_sync(0xffffffffu, ptx::mbar_wait(&empty[stage], ((it / kStages) & 1) ^ 1, kTmaWaitNs))) { fail(); return; }
+        if (lane == 0) ptx::mbar_expect_tx(&full[stage], (uint32_t)(nbox * a.box_rows * 128 * 4));
+        __syncwarp();
+        if (j < nbox)
+          ptx::tma_load_2d(smem + stage * 2 * kTileBytes + is_v * kTileBytes + hf * (kBlockN * 128) + j * a.box_rows * 128,
+                           is_v ? &a.tmV : &a.tmK, &full[stage], run.kvh * kD + hf * 64, y);
+        __syncwarp();
+      }
     }
-    float* dst = a.partial + (((size_t)b * a.Hq + h0 + h) * a.splits + split) * (kD + 1);
-    dst[d] = l > 0.f ? acc / l : 0.f;
-    if (d == 0) dst[kD] = l > 0.f ? m + log2f(l) : -INFINITY;
+    return;
   }
+  Attend<kFp16, true> at;
+  bool dead = false;                         // a wait ran out (recorded): walk on without data, so that no warp waits at a barrier for this one
+  while (list.next(run)) {
+    at.begin(a, run, lane);
+    for (int t = 0; t < run.n_tiles; ++t, ++it) {
+      const int stage = it % kStages;
+      if (!dead && !__all_sync(0xffffffffu, ptx::mbar_wait(&full[stage], (it / kStages) & 1, kTmaWaitNs))) { fail(); dead = true; }
+      uint8_t* vt = smem + stage * 2 * kTileBytes + kTileBytes;
+      const int rows = max(0, run.hi - (run.lo + t * kBlockN));
+      if (rows < warp * 16 + 16) {
+        // rows past the end hold whatever the page (or an older tile) held; their scores are masked, and this warp's V
+        // rows among them are cleared so that 0 * NaN cannot arise
+        for (int idx = lane; idx < 16 * 16; idx += 32) {
+          const int row = warp * 16 + (idx >> 4), chunk = idx & 15;
+          if (row >= rows) *(uint4*)(vt + tile_off<true>(row, chunk)) = make_uint4(0, 0, 0, 0);
+        }
+        ptx::fence_proxy_async_smem();       // before TMA writes the stage again
+        __syncwarp();
+      }
+      const uint32_t ks = base + stage * 2 * kTileBytes;
+      if (!dead) at.tile(a, ks, ks + kTileBytes, run.lo + t * kBlockN, run.hi, warp, lane);
+      __syncwarp();
+      // the last tile's stage serves as scratch first
+      if (t + 1 < run.n_tiles && lane == 0) ptx::mbar_arrive(&empty[stage]);
+    }
+    const int last = (it - 1) % kStages;
+    ptx::named_barrier(1, kWarps * 32);      // every warp has read the last tile
+    at.finish(a, run, (float*)(smem + last * 2 * kTileBytes), sm_ml, warp, lane);
+    ptx::fence_proxy_async_smem();
+    __syncwarp();
+    if (lane == 0) ptx::mbar_arrive(&empty[last]);
+  }
+}
+
+// cp.async fill by the computing threads themselves: any page size.
+template <bool kFp16>
+__global__ void __launch_bounds__(kWarps * 32, 2) decode_splitk_kernel(const __grid_constant__ DecodeArgs a) {
+  extern __shared__ __align__(128) uint8_t smem[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  float* sm_ml = (float*)(smem + kRingBytes + 64);
+  int* pre = (int*)(smem + kRingBytes + 64 + kWarps * 16 * 2 * 4);
+  if (warp == 0) prefix_tiles(a, pre, lane);
+  __syncthreads();
+  RunList list(a, pre);
+  Run run;
+  const uint32_t base = (uint32_t)__cvta_generic_to_shared(smem);
+  const size_t pos_stride = (size_t)a.Hkv * kD;   // elements between consecutive positions of a page
+  Attend<kFp16, false> at;
+  while (list.next(run)) {
+    const int32_t* bt = a.block_table + (size_t)run.b * a.max_blocks;
+    auto issue_tile = [&](int t) {
+      const int stage = t % kStages;
+      const uint32_t ks = base + stage * 2 * kTileBytes, vs = ks + kTileBytes;
+      // 64 rows x 16 chunks for K and for V = 2048 chunks, 128 threads -> 16 each
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int idx = threadIdx.x + i * 128;     // 0..1023
+        const int row = idx >> 4, chunk = idx & 15;
+        const int pos = run.lo + t * kBlockN + row;
+        if (pos < run.hi) {
+          const int blk = bt[pos / a.page];
+          const size_t e = ((size_t)blk * a.page + pos % a.page) * pos_stride + (size_t)run.kvh * kD + chunk * 8;
+          cp_async16(ks + tile_off<false>(row, chunk), a.k_cache + e);
+          cp_async16(vs + tile_off<false>(row, chunk), a.v_cache + e);
+        } else {
+          *(uint4*)(smem + stage * 2 * kTileBytes + tile_off<false>(row, chunk)) = make_uint4(0, 0, 0, 0);
+          *(uint4*)(smem + stage * 2 * kTileBytes + kTileBytes + tile_off<false>(row, chunk)) = make_uint4(0, 0, 0, 0);
+        }
+      }
+    };
+    at.begin(a, run, lane);
+    for (int t = 0; t < kStages - 1; ++t) {
+      if (t < run.n_tiles) issue_tile(t);
+      cp_async_commit();
+    }
+    for (int t = 0; t < run.n_tiles; ++t) {
+      cp_async_wait<kStages - 2>();
+      __syncthreads();
+      if (t + kStages - 1 < run.n_tiles) issue_tile(t + kStages - 1);
+      cp_async_commit();
+      const uint32_t ks = base + (t % kStages) * 2 * kTileBytes;
+      at.tile(a, ks, ks + kTileBytes, run.lo + t * kBlockN, run.hi, warp, lane);
+    }
+    cp_async_wait<0>();
+    __syncthreads();
+    at.finish(a, run, (float*)smem, sm_ml, warp, lane);
+  }
+}
+
+// Folds the partial results of one (sequence, head) into (o, lse), thread d taking dimension d. All of the block's
+// threads call it; `s_w` is kD floats of shared memory. The weights are taken once, by a thread per place, and the loads
+// of eight places are in flight together (two serial passes over 64 places took most of 24 us).
+__device__ __forceinline__ void combine_splits(const float* p, int splits, float* s_w, float& o, float& lse) {
+  const int d = threadIdx.x;
+  __shared__ float s_m[kD / 32];
+  float m = -INFINITY;
+  for (int s = d; s < splits; s += kD) m = fmaxf(m, __ldcg(p + (size_t)s * (kD + 1) + kD));
+#pragma unroll
+  for (int k = 16; k > 0; k >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, k));
+  __syncthreads();
+  if ((d & 31) == 0) s_m[d >> 5] = m;
+  __syncthreads();
+#pragma unroll
+  for (int w = 0; w < kD / 32; ++w) m = fmaxf(m, s_m[w]);
+  float l = 0.f, acc = 0.f;
+  for (int s0 = 0; s0 < splits; s0 += kD) {
+    const int n = min(kD, splits - s0);
+    __syncthreads();
+    if (d < n) {
+      const float ls = __ldcg(p + (size_t)(s0 + d) * (kD + 1) + kD);
+      s_w[d] = ls == -INFINITY ? 0.f : exp2f(ls - m);
+    }
+    __syncthreads();
+    for (int s = 0; s < n; s += 8) {
+      float v[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) v[k] = s + k < n && s_w[s + k] != 0.f ? __ldcg(p + (size_t)(s0 + s + k) * (kD + 1) + d) : 0.f;
+#pragma unroll
+      for (int k = 0; k < 8; ++k)
+        if (s + k < n) { l += s_w[s + k]; acc += s_w[s + k] * v[k]; }
+    }
+  }
+  o = l > 0.f ? acc / l : 0.f;
+  lse = l > 0.f ? m + log2f(l) : -INFINITY;
 }
 
 // ------------------------------------------------------------------------------ exchange + merge
@@ -360,23 +525,13 @@ __global__ void __launch_bounds__(kD) decode_exchange_kernel(const __grid_consta
   const int32_t tag = (call >> 1) + 1;
   const int items = a.B * a.Hq;
   const int d = threadIdx.x;
-  __shared__ float s_w[64];
+  __shared__ float s_w[64], s_part[kD];
   __shared__ int s_ok;
   // phase A: combine local splits, push to every rank
   for (int it = blockIdx.x; it < items; it += gridDim.x) {
     const int b = it / a.Hq, h = it - b * a.Hq;
-    const float* p = a.partial + (size_t)it * a.splits * (kD + 1);
-    float m = -INFINITY;
-    for (int s = 0; s < a.splits; ++s) m = fmaxf(m, p[s * (kD + 1) + kD]);
-    float l = 0.f, acc = 0.f;
-    for (int s = 0; s < a.splits; ++s) {
-      const float ls = p[s * (kD + 1) + kD];
-      const float w = ls == -INFINITY ? 0.f : exp2f(ls - m);
-      l += w;
-      acc += w * p[s * (kD + 1) + d];
-    }
-    const float o = l > 0.f ? acc / l : 0.f;
-    const float lse = l > 0.f ? m + log2f(l) : -INFINITY;
+    float o, lse;
+    combine_splits(a.partial + (size_t)it * a.splits * (kD + 1), a.splits, s_part, o, lse);
     float* slot = a.gathered + ((((size_t)buf * W + ctx.rank) * a.Bmax + b) * a.Hq + h) * (kD + 1);
     int32_t* flag = a.flags + (((size_t)buf * W + ctx.rank) * a.Bmax + b) * a.Hq + h;
     for (int i = 0; i < W; ++i) {
@@ -433,26 +588,42 @@ __global__ void __launch_bounds__(kD) decode_exchange_kernel(const __grid_consta
   }
 }
 
-// Local-only finish (exchange == 2): fold this rank's splits into (o, lse) without talking to any peer.
-// What a decode over a KV shard returns when the cross-rank merge is done elsewhere, e.g. by an
+// Finish without a peer: fold this rank's partials into (o, lse). With one rank that is the whole result; with
+// exchange == 2 it is what a decode over a KV shard returns when the cross-rank merge is done elsewhere, e.g. by an
 // all-gather of the partial results as in the reference's RCCL baseline
 // (examples/benchmark/reference/flash_decode_rccl/flash_decode_layer_rccl.py:100-130).
 __global__ void __launch_bounds__(kD) decode_local_finish_kernel(const float* partial, void* out, float* out_lse, int splits, int is_fp16) {
   const int it = blockIdx.x, d = threadIdx.x;
-  const float* p = partial + (size_t)it * splits * (kD + 1);
-  float m = -INFINITY;
-  for (int s = 0; s < splits; ++s) m = fmaxf(m, p[s * (kD + 1) + kD]);
-  float l = 0.f, acc = 0.f;
-  for (int s = 0; s < splits; ++s) {
-    const float ls = p[s * (kD + 1) + kD];
-    const float w = ls == -INFINITY ? 0.f : exp2f(ls - m);
-    l += w;
-    acc += w * p[s * (kD + 1) + d];
-  }
-  const float o = l > 0.f ? acc / l : 0.f;
+  __shared__ float s_part[kD];
+  asm volatile("griddepcontrol.wait;" ::: "memory");      // launched early: the partials are complete from here on
+  float o, lse;
+  combine_splits(partial + (size_t)it * splits * (kD + 1), splits, s_part, o, lse);
   if (is_fp16) ((__half*)out)[(size_t)it * kD + d] = __float2half_rn(o);
   else ((__nv_bfloat16*)out)[(size_t)it * kD + d] = __float2bfloat16_rn(o);
-  if (out_lse && d == 0) out_lse[it] = l > 0.f ? (m + log2f(l)) / kLog2e : -INFINITY;
+  if (out_lse && d == 0) out_lse[it] = lse == -INFINITY ? -INFINITY : lse / kLog2e;
+}
+
+// Split-K pass over `a.B` sequences, in launches of up to kMaxSeqs, on two CTAs per SM.
+template <bool kTma>
+int launch_splitk(DecodeArgs a, cudaStream_t s) {
+  constexpr int smem = kTma ? kDecodeSmemTma : kDecodeSmem;
+  auto* kern = kTma ? (a.is_fp16 ? decode_splitk_tma_kernel<true> : decode_splitk_tma_kernel<false>)
+                    : (a.is_fp16 ? decode_splitk_kernel<true> : decode_splitk_kernel<false>);
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -20;
+  int dev = 0, sms = 148;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int total = a.B;
+  for (int b0 = 0; b0 < total; b0 += kMaxSeqs) {
+    DecodeArgs p = a;
+    p.B = total - b0 < kMaxSeqs ? total - b0 : kMaxSeqs;
+    p.q = a.q + (size_t)b0 * a.Hq * kD;
+    p.block_table = a.block_table + (size_t)b0 * a.max_blocks;
+    p.kv_lens = a.kv_lens + b0;
+    p.partial = a.partial + (size_t)b0 * a.Hq * a.splits * (kD + 1);
+    kern<<<2 * sms, kWarps * 32 + (kTma ? 32 : 0), smem, s>>>(p);
+  }
+  return cudaGetLastError() == cudaSuccess ? 0 : -21;
 }
 
 }  // namespace
@@ -517,30 +688,21 @@ int iris_flash_decode(const IrisDecodeDesc* d, void* stream) {
     tma = make_cache_map(&a.tmK, d->k_cache, d->dtype, positions, row, a.box_rows) &&
           make_cache_map(&a.tmV, d->v_cache, d->dtype, positions, row, a.box_rows);
   }
-  const int smem = kStages * 2 * kTileBytes > (int)((kWarps * 16 * kD + kWarps * 32) * sizeof(float))
-                       ? kStages * 2 * kTileBytes : (int)((kWarps * 16 * kD + kWarps * 32) * sizeof(float));
-  const int smem_tma = smem + 64 + 1024;     // stage barriers, alignment slack
-  static bool attr = false;
-  if (!attr) {
-    if (cudaFuncSetAttribute(decode_splitk_kernel<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -20;
-    if (cudaFuncSetAttribute(decode_splitk_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -20;
-    if (cudaFuncSetAttribute(decode_splitk_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_tma) != cudaSuccess) return -20;
-    if (cudaFuncSetAttribute(decode_splitk_kernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_tma) != cudaSuccess) return -20;
-    attr = true;
-  }
-  dim3 grid(d->splits, d->Hkv * a.head_groups, d->B);
-  if (tma) {
-    if (a.is_fp16) decode_splitk_kernel<true, true><<<grid, kWarps * 32, smem_tma, s>>>(a);
-    else decode_splitk_kernel<false, true><<<grid, kWarps * 32, smem_tma, s>>>(a);
-  } else {
-    if (a.is_fp16) decode_splitk_kernel<true, false><<<grid, kWarps * 32, smem, s>>>(a);
-    else decode_splitk_kernel<false, false><<<grid, kWarps * 32, smem, s>>>(a);
-  }
-  if (cudaGetLastError() != cudaSuccess) return -21;
+  const int r = tma ? launch_splitk<true>(a, s) : launch_splitk<false>(a, s);
+  if (r) return r;
   if (!d->exchange) return 0;
-  if (d->exchange == 2) {
-    decode_local_finish_kernel<<<d->B * d->Hq, kD, 0, s>>>(d->partial, d->out, d->out_lse, d->splits, a.is_fp16);
-    return cudaGetLastError() == cudaSuccess ? 0 : -21;
+  if (d->exchange == 2 || d->ctx.world <= 1) {
+    // programmatic launch: the blocks are placed while the split-K kernel drains and wait for it in the kernel
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(d->B * d->Hq, 1, 1);
+    cfg.blockDim = dim3(kD, 1, 1);
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at; cfg.numAttrs = 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, decode_local_finish_kernel, (const float*)d->partial, d->out, d->out_lse, (int)d->splits, a.is_fp16);
+    return e == cudaSuccess && cudaGetLastError() == cudaSuccess ? 0 : -21;
   }
   ExchangeArgs x;
   memcpy(&x.ctx, &d->ctx, sizeof(DeviceContext));
@@ -567,22 +729,13 @@ static __device__ __align__(256) unsigned char g_decode_static_scratch[IRIS_DECO
 
 constexpr int kStaticMaxDevices = 64;
 float* g_static_scratch_addr[kStaticMaxDevices] = {};
-bool g_static_attr_done[kStaticMaxDevices] = {};   // shared-memory limit raised on that device's function handles
 std::mutex g_static_setup_mutex;
 
 __global__ void __launch_bounds__(kD) decode_local_combine_kernel(const float* partial, void* out, int splits, int is_fp16) {
   const int it = blockIdx.x, d = threadIdx.x;
-  const float* p = partial + (size_t)it * splits * (kD + 1);
-  float m = -INFINITY;
-  for (int s = 0; s < splits; ++s) m = fmaxf(m, p[s * (kD + 1) + kD]);
-  float l = 0.f, acc = 0.f;
-  for (int s = 0; s < splits; ++s) {
-    const float ls = p[s * (kD + 1) + kD];
-    const float w = ls == -INFINITY ? 0.f : exp2f(ls - m);
-    l += w;
-    acc += w * p[s * (kD + 1) + d];
-  }
-  const float o = l > 0.f ? acc / l : 0.f;
+  __shared__ float s_part[kD];
+  float o, lse;
+  combine_splits(partial + (size_t)it * splits * (kD + 1), splits, s_part, o, lse);
   if (is_fp16) ((__half*)out)[(size_t)it * kD + d] = __float2half_rn(o);
   else ((__nv_bfloat16*)out)[(size_t)it * kD + d] = __float2bfloat16_rn(o);
 }
@@ -626,11 +779,8 @@ extern "C" int iris_flash_decode_static(const void* q, const void* k_cache, cons
     static_err(err, errlen, "iris_flash_decode_static: no current CUDA device");
     return -4;
   }
-  // Both tables below are per device: the array's address differs from GPU to GPU, and the raised
-  // shared-memory limit belongs to the function handle of the device that was current when it was
-  // set. One mutex covers the set-up, so that two host threads making a device's first call agree.
-  const int smem = kStages * 2 * kTileBytes > (int)((kWarps * 16 * kD + kWarps * 32) * sizeof(float))
-                       ? kStages * 2 * kTileBytes : (int)((kWarps * 16 * kD + kWarps * 32) * sizeof(float));
+  // The table below is per device: the array's address differs from GPU to GPU. One mutex covers the set-up, so
+  // that two host threads making a device's first call agree.
   {
     std::lock_guard<std::mutex> guard(g_static_setup_mutex);
     if (!g_static_scratch_addr[dev]) {
@@ -642,14 +792,6 @@ extern "C" int iris_flash_decode_static(const void* q, const void* k_cache, cons
       }
       g_static_scratch_addr[dev] = (float*)p;
     }
-    if (!g_static_attr_done[dev]) {
-      if (cudaFuncSetAttribute(decode_splitk_kernel<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess ||
-          cudaFuncSetAttribute(decode_splitk_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) {
-        static_err(err, errlen, "iris_flash_decode_static: cannot raise the kernel's shared-memory limit");
-        return -20;
-      }
-      g_static_attr_done[dev] = true;
-    }
   }
   float* scratch = g_static_scratch_addr[dev];
 
@@ -660,10 +802,7 @@ extern "C" int iris_flash_decode_static(const void* q, const void* k_cache, cons
   a.group = Hq / Hkv; a.head_groups = (a.group + 15) / 16;
   a.sm_scale = sm_scale; a.soft_cap = soft_cap; a.is_fp16 = dtype == IRIS_F16;
   a.status = nullptr; a.box_rows = 0;     // the cp.async instantiation: no tensor maps
-  dim3 grid(splits, Hkv * a.head_groups, B);
-  if (a.is_fp16) decode_splitk_kernel<true, false><<<grid, kWarps * 32, smem, s>>>(a);
-  else decode_splitk_kernel<false, false><<<grid, kWarps * 32, smem, s>>>(a);
-  if (cudaGetLastError() != cudaSuccess) {
+  if (launch_splitk<false>(a, s)) {
     static_err(err, errlen, "iris_flash_decode_static: split-K kernel launch failed");
     return -21;
   }

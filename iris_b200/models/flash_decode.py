@@ -9,7 +9,7 @@ sequence across ranks (reference: examples/13_flash_decode/flash_decode_fused_la
 * ``block_table``   ``int32 [B, max_blocks]``: page ids of this rank's shard
 
 Two kernel launches on the current stream (``csrc/kernels/flash_decode.cu``): the split-K pass
-over the local shard, then combine + exchange of the partial ``(o, lse)`` by remote stores with
+over the local shard, then (one rank: the combination of its partial results; else) combine + exchange of the partial ``(o, lse)`` by remote stores with
 per-(source, batch, head) flags + final merge. No host synchronisation, no flag reset between
 calls. ``reference_decode`` is the plain fp32 PyTorch statement of the same computation.
 """
@@ -110,10 +110,13 @@ class FlashDecodeLayer:
         return lib
 
     def num_splits(self, batch: int, max_len: int) -> int:
+        """Places for partial results per (sequence, head). The kernel cuts the tiles of all sequences into equal
+        runs, one per CTA (two CTAs per SM): the sequence with every tile is spread over 2 * SMs / heads of them, one more
+        at each end, and a run is at least 256 positions."""
         sms = max(self.ctx.get_cu_count(), 1)
         per_seq = self.Hkv * -(-(self.Hq // self.Hkv) // 16)
-        want = -(-4 * sms // max(batch * per_seq, 1))          # ~2 waves of 2 CTAs per SM
-        by_len = max(1, -(-max_len // 256))                     # at least 256 positions per split
+        want = 2 * sms // per_seq + 2
+        by_len = max(1, -(-max_len // 256))
         return max(1, min(self.max_splits, want, by_len))
 
     def forward(self, q, k_cache, v_cache, global_kv_lens, block_table, out=None, return_lse: bool = False,
@@ -152,7 +155,7 @@ class FlashDecodeLayer:
         d.num_blocks = 0 if self.use_tma is False else k_cache.shape[0]     # > 0 lets the kernel fill its tiles by TMA
         if not (q.is_contiguous() and k_cache.is_contiguous() and v_cache.is_contiguous() and block_table.is_contiguous()):
             raise ValueError("flash decode takes contiguous q, caches and block table")
-        _lib.check(self._lib().iris_flash_decode(C.byref(d), C.c_void_p(_lib.current_stream_ptr())), "flash decode launch", kernels=2)
+        _lib.check(self._lib().iris_flash_decode(C.byref(d), C.c_void_p(_lib.current_stream_ptr())), "flash decode launch", kernels=1 + -(-B // 1024))
         return (out, lse) if (return_lse or local_only) else out
 
     __call__ = forward

@@ -131,6 +131,38 @@ def test_attention_any_length_and_group(ctx, dtype, S, Hq, Hkv, causal):
     ctx.heap_release(mark)
 
 
+# ------------------------------------------------------------------------------------ decode
+@pytest.mark.parametrize("tma", [None, False])
+@pytest.mark.parametrize("B,Hq,Hkv,page,lens", [
+    (1, 8, 1, 16, (1,)), (1, 8, 8, 64, (4096,)), (3, 8, 2, 16, (0, 63, 65)), (5, 32, 2, 32, (1, 256, 257, 5000, 0)),
+    (2, 40, 1, 8, (4097, 129)), (33, 4, 4, 128, tuple(range(0, 33 * 37, 37))), (2, 64, 8, 24, (700, 2500)),
+    (1100, 2, 1, 16, tuple((i * 7) % 90 for i in range(1100)))])
+def test_decode_runs_cut_sequences_anywhere(ctx, tma, B, Hq, Hkv, page, lens):
+    """Empty sequences, one tile, lengths around tile and run boundaries, many sequences per CTA and many CTAs per
+    sequence, more sequences than one launch takes, head groups above 16 and page sizes without a TMA box. Probabilities and
+    output are rounded to bf16 (2^-8 each) and |v| < 6: within 2 * 2^-8 * 6 of the fp32 result."""
+    from iris_b200.models import FlashDecodeLayer, reference_decode
+
+    g = _gen(B + Hq + page)
+    L = max(max(lens), 1)
+    blocks = -(-L // page)
+    r = lambda *sh: torch.randn(*sh, device="cuda", generator=g).clamp(-6, 6).to(torch.bfloat16)  # noqa: E731
+    q, k, v = r(B, Hq, 128), r(B * blocks, page, Hkv, 128), r(B * blocks, page, Hkv, 128)
+    table = torch.randperm(B * blocks, device="cuda", generator=g).to(torch.int32).view(B, blocks)
+    kv = torch.tensor([lens], dtype=torch.int32, device="cuda")
+    mark = ctx.heap_mark()
+    layer = FlashDecodeLayer(ctx, Hq, Hkv, max_batch=B, use_tma=tma)
+    want, want_lse = reference_decode(q, k, v, kv[0], table)
+    for splits in (64, 2, 1):
+        layer.max_splits = splits
+        out, lse = layer(q, k, v, kv, table, return_lse=True)
+        assert (out.float() - want).abs().max().item() <= 2 * 2.0 ** -8 * 6
+        seen = kv[0] > 0
+        assert (lse[seen] - want_lse[seen]).abs().max().item() < 1e-3 if bool(seen.any()) else True
+        assert torch.isneginf(lse[~seen]).all() and (out[~seen] == 0).all()
+    ctx.heap_release(mark)
+
+
 # ------------------------------------------------------------------------------------ few rows
 @pytest.mark.parametrize("kmajor", [True, False])
 @pytest.mark.parametrize("M,N,K", [(1, 8, 8), (1, 1024, 64), (16, 136, 520), (17, 1032, 2048), (32, 3584, 72), (33, 264, 4096), (64, 2000, 3000),
