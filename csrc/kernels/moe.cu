@@ -26,6 +26,7 @@
 #include <string.h>
 
 #include "gemm_host.cuh"
+#include "quantize_common.cuh"
 
 namespace {
 
@@ -207,6 +208,59 @@ __global__ void moe_clear_kernel(MoeDims dm, MoeMeta m) {
   if (i < dm.E) m.counts_local[i] = 0;
 }
 
+// ------------------------------------------------------------------------------------ 1-3 in one block (one rank)
+// One rank and few tokens: routing, offsets and sort in one launch instead of four, whose latency is all they cost
+// (64 tokens, 32 experts: 18 us in four kernels, now 12). With more tokens the work of a single block would be the longer.
+constexpr int kPrepMaxTokens = 256;
+template <int kPer>
+__global__ void __launch_bounds__(1024) moe_prep_kernel(const float* __restrict__ logits, const __grid_constant__ DeviceContext ctx, MoeDims dm,
+                                                        MoeMeta m, int32_t* pos_of) {
+  __shared__ int32_t hist[1024], off[1024], w_rows[32], w_tiles[32];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  hist[tid] = 0;
+  __syncthreads();
+  for (int t = warp; t < dm.T; t += 32) {
+    int my_i;
+    float my_w;
+    route_token<kPer>(logits + (size_t)t * dm.E, dm.E, dm.K, lane, my_i, my_w);
+    if (lane < dm.K) {
+      const size_t p = (size_t)t * dm.K + lane;
+      m.topk_idx[p] = my_i;
+      m.topk_w[p] = my_w;
+      pos_of[p] = atomicAdd(&hist[my_i], 1);       // place inside the expert's rows
+    }
+  }
+  __syncthreads();
+  // exclusive prefix sums of rows and 128-row tiles over the experts, one expert per thread
+  const int rows = tid < dm.E ? hist[tid] : 0, tiles = (rows + kBM - 1) / kBM;
+  int pr = rows, pt = tiles;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int ur = __shfl_up_sync(0xffffffffu, pr, o), ut = __shfl_up_sync(0xffffffffu, pt, o);
+    if (lane >= o) { pr += ur; pt += ut; }
+  }
+  if (lane == 31) { w_rows[warp] = pr; w_tiles[warp] = pt; }
+  __syncthreads();
+  for (int w = 0; w < warp; ++w) { pr += w_rows[w]; pt += w_tiles[w]; }
+  if (tid < dm.E) {
+    off[tid] = pr - rows;
+    m.expert_rows[tid] = rows;
+    m.expert_row0[tid] = pr - rows;
+    m.tile_prefix[tid] = pt - tiles;
+    if (tid == dm.E - 1) {
+      m.expert_row0[dm.E] = pr;
+      m.tile_prefix[dm.E] = pt;
+      if (pr > dm.capacity) ctx.fail(kBadTranslate);     // more rows routed here than the inbox holds
+    }
+  }
+  __syncthreads();
+  for (int p = tid; p < dm.T * dm.K; p += blockDim.x) {
+    const int pos = off[m.topk_idx[p]] + pos_of[p];
+    m.sorted_pairs[pos] = p;
+    pos_of[p] = pos;
+  }
+}
+
 // ------------------------------------------------------------------------------------ 4' gather (one rank)
 // With one rank every pair's row stays here, so nothing is sent: the token rows are copied into expert order by a
 // kernel of their own and the grouped GEMM runs on every SM. The communication CTAs of the multi-rank form cost the
@@ -215,7 +269,6 @@ __global__ void moe_clear_kernel(MoeDims dm, MoeMeta m) {
 // this copy, which is bound by the 470 MB it writes). A block reads a piece of one token's row once and stores it to the
 // token's K rows.
 __global__ void __launch_bounds__(256) moe_gather_kernel(const uint8_t* __restrict__ x, uint8_t* __restrict__ inbox, int row16,
-                                                         const uint8_t* __restrict__ x_sf, uint8_t* __restrict__ inbox_sf, int sf16,
                                                          const int32_t* __restrict__ pos_of, int K, int capacity) {
   __shared__ int32_t dst[kMaxTopK];
   const int t = blockIdx.x;
@@ -227,11 +280,27 @@ __global__ void __launch_bounds__(256) moe_gather_kernel(const uint8_t* __restri
     for (int k = 0; k < K; ++k)
       if (dst[k] < capacity) ((uint4*)inbox)[(size_t)dst[k] * row16 + c] = v;
   }
-  if (sf16 && blockIdx.y == 0) {
-    for (int u = threadIdx.x; u < sf16 * K; u += blockDim.x) {
-      const int k = u / sf16, c = u - k * sf16;
-      if (dst[k] < capacity) ((uint4*)inbox_sf)[(size_t)dst[k] * sf16 + c] = ((const uint4*)x_sf)[(size_t)t * sf16 + c];
-    }
+}
+
+// The same for e4m3 rows, from the 16-bit tokens: half a warp quantises one 128-column block of a token and stores the
+// values and the scale byte to the token's K rows.
+__global__ void __launch_bounds__(256) moe_gather_quant_kernel(const __nv_bfloat16* __restrict__ x, uint8_t* __restrict__ inbox,
+                                                               uint8_t* __restrict__ inbox_sf, int sf_ld, int D,
+                                                               const int32_t* __restrict__ pos_of, int K, int capacity) {
+  __shared__ int32_t dst[kMaxTopK];
+  const int t = blockIdx.x, half = threadIdx.x >> 4, sub = threadIdx.x & 15;
+  if (threadIdx.x < K) dst[threadIdx.x] = pos_of[(size_t)t * K + threadIdx.x];
+  __syncthreads();
+  const int kb = blockIdx.y * 16 + half, c = kb * 128 + sub * 8;       // D is a multiple of 256: whole blocks
+  Raw8<__nv_bfloat16> raw;
+  raw.load(x + (size_t)t * D + c, c < D ? 8 : 0, 2);
+  const int e = block_exponent(raw);
+  if (c >= D) return;
+  const uint2 v = quantised8(raw, e);
+  for (int k = 0; k < K; ++k) {
+    if (dst[k] >= capacity) continue;
+    *(uint2*)(inbox + (size_t)dst[k] * D + c) = v;
+    if (sub == 0) inbox_sf[(size_t)dst[k] * sf_ld + kb] = (uint8_t)(e + 127);
   }
 }
 
@@ -289,9 +358,22 @@ struct GroupedGemm : Common {
     while (j + 1 < dm.El && meta.tile_prefix[j + 1] <= tm) ++j;
     return j;
   }
+  // The same asked by a whole converged warp, 32 experts per load and vote: the producer's search stands in front of
+  // every tile's loads, and one dependent load per expert lasted longer than its ring.
+  IRIS_D int expert_of_warp(int tm) const {
+    const int lane = threadIdx.x & 31;
+    int j = 0;
+    for (int base = 0; base + 1 < dm.El; base += 32) {
+      const int e = base + lane;
+      const int n = __popc(__ballot_sync(0xffffffffu, e + 1 < dm.El && meta.tile_prefix[e + 1] <= tm));
+      j += n;
+      if (n < 32) break;
+    }
+    return j;
+  }
   IRIS_D bool a_source(State& st, int tm, int kb, ASource& s) const {
     if (kb == 0) {
-      st.j = expert_of(tm);
+      st.j = expert_of_warp(tm);
       st.row0 = meta.expert_row0[st.j] + (tm - meta.tile_prefix[st.j]) * kBM;
       if (kStage == 1 && ctx.world > 1 && st.key != st.j) {     // one rank: the gather kernel ran before
         if (!wait_flag_ge(ctx, meta.arrived + st.j, meta.expected_cum[st.j])) return false;
@@ -539,6 +621,7 @@ typedef struct IrisMoeDesc {
   const void* w13_sf;       // scale atoms of w13: [El][2F / 256][D / 128][2][512]
   const void* w2_sf;        // scale atoms of w2:  [El][ceil(D / 224)][F / 128][2][512]
   int32_t* pos_of;          // [T * K] one rank only: inbox row of each (token, k) pair
+  const void* x16;          // one rank, e4m3: the bf16 tokens [T, D], quantised on the way into the inbox (x and x_sf are not read)
 } IrisMoeDesc;
 
 int iris_moe_forward(const IrisMoeDesc* d, void* stream_) {
@@ -550,26 +633,34 @@ int iris_moe_forward(const IrisMoeDesc* d, void* stream_) {
   MoeDims dm{d->T, d->K, d->E, d->El, d->D, d->F, d->capacity};
   MoeMeta m{d->topk_idx, d->topk_w, d->counts_local, d->counts_all, d->cursor, d->list_off, d->sorted_pairs, d->my_off,
             d->expert_rows, d->expert_row0, d->tile_prefix, d->expected_cum, d->arrived, (long long*)d->inbox_meta};
-  moe_clear_kernel<<<(d->E + 255) / 256, 256, 0, s>>>(dm, m);
   const int sms = sm_count();
-  {
+  const bool one_rank = ctx.world <= 1;
+  int32_t* pos_of = one_rank ? d->pos_of : nullptr;
+  if (one_rank && (!pos_of || ((uintptr_t)d->x & 15) || ((uintptr_t)d->x16 & 15) || (d->fp8 && !d->x16))) return -11;
+  if (one_rank && d->T <= kPrepMaxTokens) {
+    auto* prep = d->E <= 32 ? moe_prep_kernel<1> : d->E <= 64 ? moe_prep_kernel<2> : d->E <= 128 ? moe_prep_kernel<4>
+                 : d->E <= 256 ? moe_prep_kernel<8> : moe_prep_kernel<32>;
+    prep<<<1, 1024, 0, s>>>(d->logits, ctx, dm, m, pos_of);
+  } else {
+    moe_clear_kernel<<<(d->E + 255) / 256, 256, 0, s>>>(dm, m);
     const int warps = d->T > 16 * sms ? 16 : 4;      // warps per block: few tokens spread over more SMs
     const int blocks = ceil_div(d->T, warps) < sms ? ceil_div(d->T, warps) : sms;
     auto* router = d->E <= 32 ? router_topk_kernel<1> : d->E <= 64 ? router_topk_kernel<2> : d->E <= 128 ? router_topk_kernel<4>
                    : d->E <= 256 ? router_topk_kernel<8> : router_topk_kernel<32>;
     router<<<blocks, warps * 32, 0, s>>>(d->logits, dm, m);
+    moe_meta_kernel<<<1, 1024, 0, s>>>(ctx, (SyncBlock*)d->sync_meta, dm, m);
+    moe_sort_kernel<<<ceil_div(d->T * d->K, 256), 256, 0, s>>>(dm, m, pos_of);
   }
-  moe_meta_kernel<<<1, 1024, 0, s>>>(ctx, (SyncBlock*)d->sync_meta, dm, m);
-  const bool one_rank = ctx.world <= 1;
-  int32_t* pos_of = one_rank ? d->pos_of : nullptr;
-  if (one_rank && (!pos_of || ((uintptr_t)d->x & 15))) return -11;
-  moe_sort_kernel<<<ceil_div(d->T * d->K, 256), 256, 0, s>>>(dm, m, pos_of);
   if (one_rank) {
-    const int row16 = d->D * (d->fp8 ? 1 : 2) / 16;
-    int split = ceil_div(4 * sms, d->T);
-    if (split > ceil_div(row16, 256)) split = ceil_div(row16, 256);
-    moe_gather_kernel<<<dim3(d->T, split), 256, 0, s>>>((const uint8_t*)d->x, (uint8_t*)d->inbox, row16, (const uint8_t*)d->x_sf,
-                                                        (uint8_t*)d->inbox_sf, d->fp8 ? d->sf_ld1 / 16 : 0, pos_of, d->K, d->capacity);
+    if (d->fp8) {
+      moe_gather_quant_kernel<<<dim3(d->T, ceil_div(d->D, 2048)), 256, 0, s>>>((const __nv_bfloat16*)d->x16, (uint8_t*)d->inbox, (uint8_t*)d->inbox_sf,
+                                                                             d->sf_ld1, d->D, pos_of, d->K, d->capacity);
+    } else {
+      const int row16 = d->D * 2 / 16;
+      int split = ceil_div(4 * sms, d->T);
+      if (split > ceil_div(row16, 256)) split = ceil_div(row16, 256);
+      moe_gather_kernel<<<dim3(d->T, split), 256, 0, s>>>((const uint8_t*)d->x, (uint8_t*)d->inbox, row16, pos_of, d->K, d->capacity);
+    }
   }
   if (cudaGetLastError() != cudaSuccess) return -21;
 

@@ -23,37 +23,11 @@
 #include <type_traits>
 
 #include "iris/host_api.h"
+#include "quantize_common.cuh"
 
 namespace {
 
 constexpr int kUnroll = 4;      // pairs of blocks a warp has in flight
-
-template <typename T> __device__ __forceinline__ float to_f32(T v);
-template <> __device__ __forceinline__ float to_f32<float>(float v) { return v; }
-template <> __device__ __forceinline__ float to_f32<__nv_bfloat16>(__nv_bfloat16 v) { return __bfloat162float(v); }
-template <> __device__ __forceinline__ float to_f32<__half>(__half v) { return __half2float(v); }
-
-// Eight elements as they lie in memory. vec: 2 the rows are 16-byte aligned, 1 they are aligned to four elements
-// (8 bytes of a 16-bit type), 0 element-wise, as a row's ragged tail always is.
-template <typename T>
-struct Raw8 {
-  static constexpr int kWords = (int)sizeof(T) * 8 / 16;
-  uint4 w[kWords];
-  __device__ __forceinline__ void load(const T* p, int n_valid, int vec) {
-    if (vec == 2 && n_valid >= 8) {
-#pragma unroll
-      for (int i = 0; i < kWords; ++i) w[i] = ((const uint4*)p)[i];
-    } else if (vec == 1 && n_valid >= 8) {
-#pragma unroll
-      for (int i = 0; i < 2 * kWords; ++i) ((uint2*)w)[i] = ((const uint2*)p)[i];
-    } else {
-      T* e = (T*)w;
-#pragma unroll
-      for (int i = 0; i < 8; ++i) e[i] = i < n_valid ? p[i] : T(0.f);
-    }
-  }
-  __device__ __forceinline__ float get(int i) const { return to_f32<T>(((const T*)w)[i]); }
-};
 
 template <typename T>
 __global__ void __launch_bounds__(256) quantize_1x128_pow2_kernel(const T* __restrict__ x, int64_t ldx, uint8_t* __restrict__ q, int64_t ldq,
@@ -79,33 +53,19 @@ __global__ void __launch_bounds__(256) quantize_1x128_pow2_kernel(const T* __res
 #pragma unroll
   for (int i = 0; i < kUnroll; ++i) {
     const int r = rows_u[i], b = kbs_u[i];
-    float amax = 0.f;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) amax = fmaxf(amax, fabsf(raw[i].get(j)));
-#pragma unroll
-    for (int o = 8; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-    amax = fmaxf(amax, 1e-12f);
-    // smallest power of two >= amax / 448, as an exponent
-    int e = (int)ceilf(log2f(amax * (1.0f / 448.0f)));
-    e = max(-127, min(127, e));
-    const float s = exp2f((float)e), inv = exp2f((float)-e);
+    const int e = block_exponent(raw[i]);
     if (r < M) {
-      uint32_t packed[2] = {0u, 0u};
-#pragma unroll
-      for (int j = 0; j < 8; j += 2) {
-        const float2 v = make_float2(fminf(fmaxf(raw[i].get(j) * inv, -448.f), 448.f), fminf(fmaxf(raw[i].get(j + 1) * inv, -448.f), 448.f));
-        packed[j >> 2] |= (uint32_t)__nv_cvt_float2_to_fp8x2(v, __NV_SATFINITE, __NV_E4M3) << (8 * (j & 3));
-      }
+      const uint2 v = quantised8(raw[i], e);
       const int k0 = b * 128 + sub * 8, n_valid = max(0, min(8, K - k0));
       uint8_t* dst = q + (int64_t)r * ldq + k0;
       if (n_valid == 8 && q_aligned == 2) {
-        *(uint2*)dst = make_uint2(packed[0], packed[1]);
+        *(uint2*)dst = v;
       } else if (n_valid == 8 && q_aligned == 1) {
-        ((uint32_t*)dst)[0] = packed[0]; ((uint32_t*)dst)[1] = packed[1];
+        ((uint32_t*)dst)[0] = v.x; ((uint32_t*)dst)[1] = v.y;
       } else
-        for (int j = 0; j < n_valid; ++j) dst[j] = (uint8_t)(packed[j >> 2] >> (8 * (j & 3)));
+        for (int j = 0; j < n_valid; ++j) dst[j] = (uint8_t)((j < 4 ? v.x : v.y) >> (8 * (j & 3)));
       if (sub == 0) {
-        if (scale) scale[(int64_t)r * KB + b] = s;
+        if (scale) scale[(int64_t)r * KB + b] = exp2f((float)e);
         if (rows) rows[(int64_t)r * ld_rows + b] = (uint8_t)(e + 127);
       }
     }

@@ -1,0 +1,64 @@
+// The 1 x 128 power-of-two quantiser of one (row, K block), shared by the kernels that quantise activations
+// (quantize.cu) and those that quantise on the way somewhere (moe.cu). Half a warp takes a block, eight elements per lane.
+#pragma once
+#include <cuda_runtime.h>
+#include <cuda_bf16.h>
+#include <cuda_fp16.h>
+#include <cuda_fp8.h>
+#include <stdint.h>
+
+namespace {
+
+template <typename T> __device__ __forceinline__ float to_f32(T v);
+template <> __device__ __forceinline__ float to_f32<float>(float v) { return v; }
+template <> __device__ __forceinline__ float to_f32<__nv_bfloat16>(__nv_bfloat16 v) { return __bfloat162float(v); }
+template <> __device__ __forceinline__ float to_f32<__half>(__half v) { return __half2float(v); }
+
+// Eight elements as they lie in memory. vec: 2 the rows are 16-byte aligned, 1 they are aligned to four elements
+// (8 bytes of a 16-bit type), 0 element-wise, as a row's ragged tail always is.
+template <typename T>
+struct Raw8 {
+  static constexpr int kWords = (int)sizeof(T) * 8 / 16;
+  uint4 w[kWords];
+  __device__ __forceinline__ void load(const T* p, int n_valid, int vec) {
+    if (vec == 2 && n_valid >= 8) {
+#pragma unroll
+      for (int i = 0; i < kWords; ++i) w[i] = ((const uint4*)p)[i];
+    } else if (vec == 1 && n_valid >= 8) {
+#pragma unroll
+      for (int i = 0; i < 2 * kWords; ++i) ((uint2*)w)[i] = ((const uint2*)p)[i];
+    } else {
+      T* e = (T*)w;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) e[i] = i < n_valid ? p[i] : T(0.f);
+    }
+  }
+  __device__ __forceinline__ float get(int i) const { return to_f32<T>(((const T*)w)[i]); }
+};
+
+// Exponent of the block's scale, the smallest power of two >= amax / 448, for the 16 lanes that hold the block.
+template <typename T>
+__device__ __forceinline__ int block_exponent(const Raw8<T>& raw) {
+  float amax = 0.f;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) amax = fmaxf(amax, fabsf(raw.get(j)));
+#pragma unroll
+  for (int o = 8; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+  amax = fmaxf(amax, 1e-12f);
+  const int e = (int)ceilf(log2f(amax * (1.0f / 448.0f)));
+  return max(-127, min(127, e));
+}
+// The lane's eight values divided by 2^e, as e4m3.
+template <typename T>
+__device__ __forceinline__ uint2 quantised8(const Raw8<T>& raw, int e) {
+  const float inv = exp2f((float)-e);
+  uint32_t packed[2] = {0u, 0u};
+#pragma unroll
+  for (int j = 0; j < 8; j += 2) {
+    const float2 v = make_float2(fminf(fmaxf(raw.get(j) * inv, -448.f), 448.f), fminf(fmaxf(raw.get(j + 1) * inv, -448.f), 448.f));
+    packed[j >> 2] |= (uint32_t)__nv_cvt_float2_to_fp8x2(v, __NV_SATFINITE, __NV_E4M3) << (8 * (j & 3));
+  }
+  return make_uint2(packed[0], packed[1]);
+}
+
+}  // namespace

@@ -39,6 +39,7 @@ class IrisMoeDesc(C.Structure):
         ("fp8", C.c_int32), ("sf_ld1", C.c_int32), ("sf_ld2", C.c_int32),
         ("x_sf", C.c_void_p), ("inbox_sf", C.c_void_p), ("H_sf", C.c_void_p), ("w13_sf", C.c_void_p), ("w2_sf", C.c_void_p),
         ("pos_of", C.c_void_p),
+        ("x16", C.c_void_p),
     ]
 
 
@@ -145,7 +146,7 @@ class MoELayer:
         self.inbox_sf.fill_(127)
         self.H = torch.zeros(self.capacity, F, dtype=u8, device=dev)
         self.H_sf = torch.full((self.capacity, self.sf_ld2), 127, dtype=u8, device=dev)
-        self.xq = torch.zeros(self.T, D, dtype=u8, device=dev)
+        self.xq = torch.zeros(self.T, D, dtype=u8, device=dev)                   # the tokens as they are sent (one rank quantises in its gather)
         self.x_sf = torch.full((self.T, self.sf_ld1), 127, dtype=u8, device=dev)
         del self.w13, self.w2
 
@@ -182,11 +183,17 @@ class MoELayer:
             out = torch.empty_like(x)
         elif out.shape != x.shape or out.dtype != x.dtype or not out.is_contiguous() or out.device != x.device:
             raise ValueError("out must be a contiguous tensor of x's shape, dtype and device")
+        one_rank = self.pos_of is not None
+        if one_rank and x.data_ptr() % 16:       # the gather reads 16 bytes at a time
+            x = x.clone()
         d = IrisMoeDesc()
         d.ctx = ctx.ctx_struct()
         d.T, d.K, d.E, d.El, d.D, d.F, d.capacity, d.comm_ctas = T, self.K, self.E, self.El, self.D, self.F, self.capacity, self.comm_sms
         if self.fp8:
-            self._quantise_tokens(x)
+            if one_rank:                         # quantised by the gather
+                d.x16 = x.data_ptr()
+            else:
+                self._quantise_tokens(x)
             d.fp8, d.sf_ld1, d.sf_ld2 = 1, self.sf_ld1, self.sf_ld2
             d.x, d.w13, d.w2 = self.xq.data_ptr(), self.w13_q.data_ptr(), self.w2_q.data_ptr()
             d.x_sf, d.inbox_sf, d.H_sf = self.x_sf.data_ptr(), self.inbox_sf.data_ptr(), self.H_sf.data_ptr()
@@ -200,8 +207,9 @@ class MoELayer:
                      "expert_rows", "expert_row0", "tile_prefix", "expected_cum", "arrived", "inbox_meta"):
             setattr(d, name, getattr(self, name).data_ptr())
         d.weights_kmajor = 1
-        d.pos_of = self.pos_of.data_ptr() if self.pos_of is not None else None
-        _lib.check(self._lib().iris_moe_forward(C.byref(d), C.c_void_p(_lib.current_stream_ptr())), "MoE forward launch", kernels=7 if self.pos_of is None else 8)
+        d.pos_of = self.pos_of.data_ptr() if one_rank else None
+        _lib.check(self._lib().iris_moe_forward(C.byref(d), C.c_void_p(_lib.current_stream_ptr())), "MoE forward launch",
+                   kernels=7 if not one_rank else (5 if T <= 256 else 8))
         self._keep = logits
         return out
 
