@@ -8,7 +8,7 @@
 //   warp 1      MMA issuer: per query tile i, S_i = Q_i K^T (tcgen05.mma, M 128, N 128, K 128) and
 //               O_i += P_i V (P from TMEM). Issue order PV_0(j), S_0(j+1), PV_1(j), S_1(j+1): the tensor pipe
 //               works for one query tile while the softmax of the other runs
-//   warps 4..7  softmax of query tile 0, warps 8..11 of tile 1, one thread per query row (224 registers each, the
+//   warps 4..7  softmax of query tile 0, warps 8..11 of tile 1, one thread per query row (208 registers each, the
 //               issuers give theirs up). Per tile: tcgen05.ld of
 //               the 128 scores, row maximum, P = exp2(s - max) (one packed FMA and one packed add per two scores,
 //               one ex2.approx each) written as packed 16-bit pairs over the first 64 columns of the SAME S
@@ -20,8 +20,10 @@
 // What bounds it: per tile of 128 x 128 the two MMAs take 1024 cycles of the tensor pipe and the 16384 exponentials
 // 1024 cycles of the MUFU. With one query tile per CTA and two threads per row (the previous split) the softmax of a tile
 // lay open next to its MMAs and the two threads of a row met in shared memory twice: about 3000 cycles per tile
-// (8192 tokens, 32 / 8 heads, causal, bf16: 736 us). Two tiles in turn, one thread per row: 549 us; 3000 tokens, full attention, fp16, which the mma.sync
-// kernel took before: 603 -> 187 us.
+// (8192 tokens, 32 / 8 heads, causal, bf16: 736 us). Two tiles in turn, one thread per row: 549 us, with the MMAs issued eight
+// to a statement 511; 3000 tokens, full attention, fp16, which the mma.sync kernel took before: 603, 187, 176 us.
+// Slower were: 64-key halves with S double-buffered (more MMAs to issue: 746), P released to the MMAs in halves, part of the
+// exponentials as a polynomial on the FMA pipe (the softmax warps are short of issue slots).
 // The two tiles are two query heads of one K/V head group where the group is even (same keys, no work done twice or
 // for padding), else two neighbouring tiles of 128 queries of one head. Items are handed out longest first, in
 // alternating direction, so that a causal mask leaves no CTA with the long items at the end.
@@ -75,13 +77,54 @@ __device__ __forceinline__ void tmem_st_32x32(uint32_t taddr, const uint32_t (&r
       : "memory");
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-// D[tmem] (+)= A[tmem] * B[smem desc]: A is read from TMEM (lane = row, 16-bit pairs along K per column). For a
-// converged warp: every lane executes it with warp-uniform operands and one elected lane issues.
-__device__ __forceinline__ void mma_f16_ts_elect(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+// The eight MMAs of one 128 x 128 x 128 product, issued by one elected lane of a converged warp in one statement: K steps
+// of 16, whose descriptors lie constant distances apart (in 16-byte units). One elect, one add per operand: with the
+// descriptor of every step computed from its address and an elect each, an MMA cost the issuing warp about 100 cycles and this
+// warp, not the tensor pipe (64 cycles per MMA) or the softmax, set the pace.
+// S = Q K^T: both operands [128 rows][64 + 64 columns] in shared memory, K-major.
+__device__ __forceinline__ void mma_s_elect(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
-      "{\n\t.reg .pred p, q;\n\telect.sync _|q, 0xffffffff;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(tmem_d),
-      "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      "{\n\t.reg .pred p, q, t;\n\t.reg .b64 a;\n\t.reg .b64 b;\n\telect.sync _|q, 0xffffffff;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.eq.b32 t, 0, 0;\n\t"
+      "add.s64 a, %1, 0;\n\tadd.s64 b, %2, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, p;\n\t"
+      "add.s64 a, %1, 2;\n\tadd.s64 b, %2, 2;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, t;\n\t"
+      "add.s64 a, %1, 4;\n\tadd.s64 b, %2, 4;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, t;\n\t"
+      "add.s64 a, %1, 6;\n\tadd.s64 b, %2, 6;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, t;\n\t"
+      "add.s64 a, %1, 1024;\n\tadd.s64 b, %2, 1024;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, t;\n\t"
+      "add.s64 a, %1, 1026;\n\tadd.s64 b, %2, 1026;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, t;\n\t"
+      "add.s64 a, %1, 1028;\n\tadd.s64 b, %2, 1028;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, t;\n\t"
+      "add.s64 a, %1, 1030;\n\tadd.s64 b, %2, 1030;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, t;\n\t"
+      "}" ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+// O += P V: P from TMEM (lane = row, 16-bit pairs along K per column), V in 64-key halves, MN-major.
+__device__ __forceinline__ void mma_pv_elect(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p, q, t;\n\t.reg .b32 a;\n\t.reg .b64 b;\n\telect.sync _|q, 0xffffffff;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.eq.b32 t, 0, 0;\n\t"
+      "add.s32 a, %1, 0;\n\tadd.s64 b, %2, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [a], b, %3, p;\n\t"
+      "add.s32 a, %1, 8;\n\tadd.s64 b, %2, 128;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [a], b, %3, t;\n\t"
+      "add.s32 a, %1, 16;\n\tadd.s64 b, %2, 256;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [a], b, %3, t;\n\t"
+      "add.s32 a, %1, 24;\n\tadd.s64 b, %2, 384;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [a], b, %3, t;\n\t"
+      "add.s32 a, %1, 32;\n\tadd.s64 b, %2, 1024;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [a], b, %3, t;\n\t"
+      "add.s32 a, %1, 40;\n\tadd.s64 b, %2, 1152;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [a], b, %3, t;\n\t"
+      "add.s32 a, %1, 48;\n\tadd.s64 b, %2, 1280;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [a], b, %3, t;\n\t"
+      "add.s32 a, %1, 56;\n\tadd.s64 b, %2, 1408;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [a], b, %3, t;\n\t"
+      "}" ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
 __device__ __forceinline__ float ex2_approx(float x) {
@@ -257,10 +300,10 @@ __device__ void attn_main_tc(const TcArgs& g, uint8_t* smem_raw, int call) {
   const uint32_t tmem_base = *(volatile uint32_t*)tmem_slot;
   const ItemOrder order(a);
 
-  // 56 + 224 + 224 = 3 x 168, what the block was launched with (the splits stand at the head of their branches:
+  // 88 + 208 + 208 = 3 x 168, what the block was launched with (the splits stand at the head of their branches:
   // the compiler gives each branch its own budget from there)
   if (warp < 4) {
-  asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
+  asm volatile("setmaxnreg.dec.sync.aligned.u32 88;");
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
     unsigned arrived_mask = 1u << r;
@@ -348,11 +391,7 @@ __device__ void attn_main_tc(const TcArgs& g, uint8_t* smem_raw, int call) {
       auto issue_s = [&](int i, int st) {
         ptx::tc_fence_after();
         const uint32_t qb = ptx::smem_u32(q_s + i * kTile), kb = ptx::smem_u32(k_s + st * kTile);
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {        // 16 of the 128 head dimensions per step
-          const uint32_t off = (k >> 2) * kHalf + (k & 3) * 32;
-          ptx::mma_f16_elect(tmem_u + i * 128, desc_kmajor(qb + off), desc_kmajor(kb + off), idesc_s, k != 0);
-        }
+        mma_s_elect(tmem_u + i * 128, desc_kmajor(qb), desc_kmajor(kb), idesc_s, 0);
         ptx::mma_commit_elect(&s_full[i]);
         if (--left_s[i] == 0) ptx::mma_commit_elect(&q_free[i]);
       };
@@ -360,12 +399,8 @@ __device__ void attn_main_tc(const TcArgs& g, uint8_t* smem_raw, int call) {
         ptx::tc_fence_after();
         const uint32_t vb = ptx::smem_u32(v_s + st * kTile);
         const bool clear = left_pv[i] == total[i];
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          const uint32_t boff = (k >> 2) * kHalf + (k & 3) * 2048;        // V: 64-key halves, 16 keys = 2048 B
-          // P: 16 keys = 8 columns of 16-bit pairs at the start of the tile's S buffer
-          mma_f16_ts_elect(tmem_u + 256 + i * 128, tmem_u + i * 128 + k * 8, desc_mnmajor(vb + boff), idesc_o, !(clear && k == 0));
-        }
+        // P: 16 keys = 8 columns of 16-bit pairs at the start of the tile's S buffer
+        mma_pv_elect(tmem_u + 256 + i * 128, tmem_u + i * 128, desc_mnmajor(vb), idesc_o, !clear);
         if (--left_pv[i] == 0) ptx::mma_commit_elect(&o_full[i]);
       };
       TileWalk cur(a, item), nxt(a, item);
@@ -412,7 +447,7 @@ __device__ void attn_main_tc(const TcArgs& g, uint8_t* smem_raw, int call) {
   }
   } else {
     // ------------------------------------------------------------------ softmax / correction / epilogue
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 224;");
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 208;");
     const int quarter = warp & 3;
     const int i = (warp - 4) >> 2;                            // query tile of the item
     const int row = quarter * 32 + lane;                      // query row inside the tile
