@@ -63,23 +63,29 @@ struct Common {
     return bf16 ? __bfloat162float(((const __nv_bfloat16*)p)[i]) : __half2float(((const __half*)p)[i]);
   }
   IRIS_D float row_bias(int row) const { return (bias_row && row < sh.M) ? bias_at(bias_row, row) : 0.f; }
-  // Biases of columns [col, col + 8), added to `v`. Every lane reads the same ones: as one or two 16-byte loads
-  // where the bias is aligned (N is a multiple of 8, so eight columns are inside together), not one load per value.
-  IRIS_D void add_col_bias8(int col, float (&v)[8]) const {
-    if (!bias_col || col >= sh.N) return;
-    if (!bias_vec) {
+  // Adds a row's bias and the biases of columns [col, col + 32) to `v`. Every lane reads the same column biases: by 16-byte
+  // loads where they are aligned (N is a multiple of 8, so eight columns are inside together), not one load per value.
+  IRIS_D void add_bias32(float rb, int col, float (&v)[32]) const {
 #pragma unroll
-      for (int i = 0; i < 8; ++i) v[i] += bias_at(bias_col, col + i);
-    } else if (!bias16) {
-      const float4 a = __ldg((const float4*)(bias_col + col)), b = __ldg((const float4*)(bias_col + col) + 1);
-      v[0] += a.x; v[1] += a.y; v[2] += a.z; v[3] += a.w; v[4] += b.x; v[5] += b.y; v[6] += b.z; v[7] += b.w;
-    } else {
-      const uint4 u = __ldg((const uint4*)((const uint16_t*)bias_col + col));
-      const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+    for (int i = 0; i < 32; ++i) v[i] += rb;
+    if (!bias_col) return;
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const float2 f = bf16 ? __bfloat1622float2(*(const __nv_bfloat162*)&w[i]) : __half22float2(*(const __half2*)&w[i]);
-        v[2 * i] += f.x; v[2 * i + 1] += f.y;
+    for (int g = 0; g < 32; g += 8) {
+      if (col + g >= sh.N) break;
+      if (!bias_vec) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[g + i] += bias_at(bias_col, col + g + i);
+      } else if (!bias16) {
+        const float4 a = __ldg((const float4*)(bias_col + col + g)), b = __ldg((const float4*)(bias_col + col + g) + 1);
+        v[g] += a.x; v[g + 1] += a.y; v[g + 2] += a.z; v[g + 3] += a.w; v[g + 4] += b.x; v[g + 5] += b.y; v[g + 6] += b.z; v[g + 7] += b.w;
+      } else {
+        const uint4 u = __ldg((const uint4*)((const uint16_t*)bias_col + col + g));
+        const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const float2 f = bf16 ? __bfloat1622float2(*(const __nv_bfloat162*)&w[i]) : __half22float2(*(const __half2*)&w[i]);
+          v[g + 2 * i] += f.x; v[g + 2 * i + 1] += f.y;
+        }
       }
     }
   }

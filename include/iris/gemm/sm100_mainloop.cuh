@@ -160,7 +160,7 @@ struct Pipeline {
 //   static constexpr bool kSwiGLU;                         (row-major path: the tile's columns are
 //        [gate 128 | up 128]; emit silu(gate) * up, 128 columns per 256-wide tile)
 //   void store16(State&, int row, int col, uint4 v) const; (8 consecutive outputs of one row)
-//   float row_bias(int row) const;  void add_col_bias8(int col, float (&v)[8]) const;  bool has_bias() const;
+//   float row_bias(int row) const;  void add_bias32(float row_bias, int col, float (&v)[32]) const;  bool has_bias() const;
 //   static constexpr bool kSfaFromRows;  void sfa_fill(State&, int m_tile, int kb, uint8_t* atom, int lane) const;
 //        (fp8: the producer warp builds A's 512-byte scale atom itself, lane l writing bytes [16 l, 16 l + 16))
 //   static constexpr bool kQuantOut;  void store_q32(State&, int row, int col, uint4, uint4) const;
@@ -420,21 +420,18 @@ IRIS_D void gemm_cta_main(const Policy& pol, uint8_t* smem_raw) {
       const float rb = has_bias ? pol.row_bias(row0 + lane) : 0.f;
       // fp32 accumulators of 32 columns -> 16-bit pairs (bias added)
       auto pack32 = [&](const uint32_t (&r)[32], int col0, uint32_t (&packed)[16]) {
+        float v[32];
 #pragma unroll
-        for (int j = 0; j < 16; j += 4) {
-          float v[8];
+        for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
+        if (has_bias) pol.add_bias32(rb, col0, v);
 #pragma unroll
-          for (int e = 0; e < 8; ++e) v[e] = __uint_as_float(r[2 * j + e]) + rb;
-          if (has_bias) pol.add_col_bias8(col0 + 2 * j, v);
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            if (bf16) {
-              __nv_bfloat162 h = __floats2bfloat162_rn(v[2 * e], v[2 * e + 1]);
-              packed[j + e] = *(uint32_t*)&h;
-            } else {
-              __half2 h = __floats2half2_rn(v[2 * e], v[2 * e + 1]);
-              packed[j + e] = *(uint32_t*)&h;
-            }
+        for (int j = 0; j < 16; ++j) {
+          if (bf16) {
+            __nv_bfloat162 h = __floats2bfloat162_rn(v[2 * j], v[2 * j + 1]);
+            packed[j] = *(uint32_t*)&h;
+          } else {
+            __half2 h = __floats2half2_rn(v[2 * j], v[2 * j + 1]);
+            packed[j] = *(uint32_t*)&h;
           }
         }
       };
