@@ -10,10 +10,12 @@
 // The reference has no quantised path; this plays the role of the activation cast in front of its
 // 16-bit GEMMs (iris/ops/matmul_all_reduce.py:95-105 consumes 16-bit tiles directly).
 //
-// Bound by memory (2 bytes in, 1 byte out per 16-bit element). Half a warp takes one (row, K block): eight
-// elements per lane, so a lane's load is 16 bytes (two for fp32) and its store 8, and a warp keeps kUnroll pairs
-// of blocks in flight before it reduces the first: with one block per warp and 8-byte loads the kernel waited on
-// latency (4096 x 8192 bf16: 61 us, now 33). amax by shuffles, scale = 2^ceil(log2(amax / 448)).
+// Half a warp takes one (row, K block): eight elements per lane, so a lane's load is 16 bytes (two for fp32) and its store
+// 8, and a warp keeps kUnroll pairs of blocks in flight before it reduces the first. With one block per warp and 8-byte loads
+// the kernel waited on latency (4096 x 8192 bf16: 61 us); since then the arithmetic per element bounds it, not its bytes
+// (15 us): maxima on pairs of 16-bit values, one exponent and one scale write per block instead of one per lane and
+// block, 32-bit index arithmetic (33 us, now 23). Collecting the scale atoms in shared memory was slower (38 us).
+// amax by shuffles, scale = 2^ceil(log2(amax / 448)).
 #include <cuda.h>
 #include <cuda_runtime.h>
 #include <cuda_bf16.h>
@@ -27,10 +29,10 @@
 
 namespace {
 
-constexpr int kUnroll = 4;      // pairs of blocks a warp has in flight
+constexpr int kUnroll = 4;      // pairs of blocks a warp has in flight (the reduction below is written for four)
 
 template <typename T>
-__global__ void __launch_bounds__(256) quantize_1x128_pow2_kernel(const T* __restrict__ x, int64_t ldx, uint8_t* __restrict__ q, int64_t ldq,
+__global__ void __launch_bounds__(128) quantize_1x128_pow2_kernel(const T* __restrict__ x, int64_t ldx, uint8_t* __restrict__ q, int64_t ldq,
                                                                    float* __restrict__ scale, uint8_t* __restrict__ atoms,
                                                                    uint8_t* __restrict__ rows, int64_t ld_rows, int M, int M_pad, int K, int KB,
                                                                    int x_aligned, int q_aligned) {
@@ -39,7 +41,9 @@ __global__ void __launch_bounds__(256) quantize_1x128_pow2_kernel(const T* __res
   const int64_t units = (int64_t)M_pad * KB, u0 = warp * (2 * kUnroll);
   if (u0 >= units) return;
   const int64_t first = u0 + half;
-  int row = (int)(first / KB), kb = (int)(first - (int64_t)row * KB);
+  // (a 64-bit division costs as much as the rest of the thread's addressing: only when the count needs it)
+  int row = units <= 0x7fffffffll ? (int)((unsigned)first / (unsigned)KB) : (int)(first / KB);
+  int kb = (int)(first - (int64_t)row * KB);
   int rows_u[kUnroll], kbs_u[kUnroll];
   Raw8<T> raw[kUnroll];
 #pragma unroll
@@ -50,10 +54,36 @@ __global__ void __launch_bounds__(256) quantize_1x128_pow2_kernel(const T* __res
     raw[i].load(x + (int64_t)row * ldx + k0, n_valid, x_aligned);
     for (kb += 2; kb >= KB; kb -= KB) ++row;
   }
+  // The four blocks' maxima by halving: each exchange leaves a lane with half of its blocks, until four lanes share one
+  // block; they work its exponent out once, and everybody fetches the four exponents.
+  float amax[kUnroll];
+#pragma unroll
+  for (int i = 0; i < kUnroll; ++i) amax[i] = block_amax_lane(raw[i]);
+  const bool hi8 = sub & 8, hi4 = sub & 4;
+  float m0 = hi8 ? amax[2] : amax[0], m1 = hi8 ? amax[3] : amax[1];
+  m0 = fmaxf(m0, __shfl_xor_sync(0xffffffffu, hi8 ? amax[0] : amax[2], 8));
+  m1 = fmaxf(m1, __shfl_xor_sync(0xffffffffu, hi8 ? amax[1] : amax[3], 8));
+  float mine = fmaxf(hi4 ? m1 : m0, __shfl_xor_sync(0xffffffffu, hi4 ? m0 : m1, 4));
+  mine = fmaxf(mine, __shfl_xor_sync(0xffffffffu, mine, 2));
+  mine = fmaxf(mine, __shfl_xor_sync(0xffffffffu, mine, 1));
+  const int e_mine = scale_exponent(mine);           // of block sub / 4
+  if ((sub & 3) == 0) {                               // whose scale one of the four lanes writes
+    const int r = hi8 ? (hi4 ? rows_u[3] : rows_u[2]) : (hi4 ? rows_u[1] : rows_u[0]);
+    const int b = hi8 ? (hi4 ? kbs_u[3] : kbs_u[2]) : (hi4 ? kbs_u[1] : kbs_u[0]);
+    if (r < M) {
+      if (scale) scale[(int64_t)r * KB + b] = exp2f((float)e_mine);
+      if (rows) rows[(int64_t)r * ld_rows + b] = (uint8_t)(e_mine + 127);
+    }
+    if (atoms && r < M_pad) {
+      const uint32_t byte = r < M ? (uint32_t)(e_mine + 127) : 127u;      // rows past M: scale 1
+      const int tile = r >> 7, rr = r & 127;
+      *(uint32_t*)(atoms + ((int64_t)tile * KB + b) * 512 + (rr & 31) * 16 + (rr >> 5) * 4) = byte * 0x01010101u;
+    }
+  }
 #pragma unroll
   for (int i = 0; i < kUnroll; ++i) {
     const int r = rows_u[i], b = kbs_u[i];
-    const int e = block_exponent(raw[i]);
+    const int e = __shfl_sync(0xffffffffu, e_mine, (lane & 16) + i * 4);
     if (r < M) {
       const uint2 v = quantised8(raw[i], e);
       const int k0 = b * 128 + sub * 8, n_valid = max(0, min(8, K - k0));
@@ -64,15 +94,6 @@ __global__ void __launch_bounds__(256) quantize_1x128_pow2_kernel(const T* __res
         ((uint32_t*)dst)[0] = v.x; ((uint32_t*)dst)[1] = v.y;
       } else
         for (int j = 0; j < n_valid; ++j) dst[j] = (uint8_t)((j < 4 ? v.x : v.y) >> (8 * (j & 3)));
-      if (sub == 0) {
-        if (scale) scale[(int64_t)r * KB + b] = exp2f((float)e);
-        if (rows) rows[(int64_t)r * ld_rows + b] = (uint8_t)(e + 127);
-      }
-    }
-    if (sub == 0 && atoms && r < M_pad) {
-      const uint32_t byte = r < M ? (uint32_t)(e + 127) : 127u;      // rows past M: scale 1
-      const int tile = r >> 7, rr = r & 127;
-      *(uint32_t*)(atoms + ((int64_t)tile * KB + b) * 512 + (rr & 31) * 16 + (rr >> 5) * 4) = byte * 0x01010101u;
     }
   }
 }
@@ -88,7 +109,7 @@ static int quantize_launch(const void* x, int64_t ldx, int32_t dtype, void* q, i
   const int KB = (K + 127) / 128;
   const int M_pad = atoms ? (int)(((int64_t)M + 127) / 128 * 128) : M;
   const int64_t warps = ((int64_t)M_pad * KB + 2 * kUnroll - 1) / (2 * kUnroll);
-  const int64_t blocks = (warps * 32 + 255) / 256;
+  const int64_t blocks = (warps * 32 + 127) / 128;
   if (blocks > 0x7fffffffll) return -3;
   cudaStream_t s = (cudaStream_t)stream;
   const int esz = dtype == IRIS_F32 ? 4 : 2;
@@ -99,7 +120,7 @@ static int quantize_launch(const void* x, int64_t ldx, int32_t dtype, void* q, i
   const int xa = level(x, ldx * esz, 16, 8), qa = level(q, ldq, 8, 4);
   auto run = [&](auto* typed) {
     using T = std::remove_cv_t<std::remove_pointer_t<decltype(typed)>>;
-    quantize_1x128_pow2_kernel<T><<<(unsigned)blocks, 256, 0, s>>>(typed, ldx, (uint8_t*)q, ldq, scale, (uint8_t*)atoms, (uint8_t*)rows,
+    quantize_1x128_pow2_kernel<T><<<(unsigned)blocks, 128, 0, s>>>(typed, ldx, (uint8_t*)q, ldq, scale, (uint8_t*)atoms, (uint8_t*)rows,
                                                                    ld_rows, M, M_pad, K, KB, xa, qa);
   };
   if (dtype == IRIS_F32) run((const float*)x);

@@ -36,26 +36,51 @@ struct Raw8 {
   __device__ __forceinline__ float get(int i) const { return to_f32<T>(((const T*)w)[i]); }
 };
 
-// Exponent of the block's scale, the smallest power of two >= amax / 448, for the 16 lanes that hold the block.
+// Largest magnitude among the lane's eight values. 16-bit types: on pairs as they lie (a maximum of magnitudes is exact in
+// any format, and NaN loses against a number as in fmaxf).
 template <typename T>
-__device__ __forceinline__ int block_exponent(const Raw8<T>& raw) {
+__device__ __forceinline__ float block_amax_lane(const Raw8<T>& raw) {
   float amax = 0.f;
 #pragma unroll
   for (int j = 0; j < 8; ++j) amax = fmaxf(amax, fabsf(raw.get(j)));
+  return amax;
+}
+template <>
+__device__ __forceinline__ float block_amax_lane<__nv_bfloat16>(const Raw8<__nv_bfloat16>& raw) {
+  const __nv_bfloat162* h = (const __nv_bfloat162*)raw.w;
+  const __nv_bfloat162 m = __hmax2(__hmax2(__habs2(h[0]), __habs2(h[1])), __hmax2(__habs2(h[2]), __habs2(h[3])));
+  const float2 f = __bfloat1622float2(m);
+  return fmaxf(fmaxf(f.x, f.y), 0.f);
+}
+template <>
+__device__ __forceinline__ float block_amax_lane<__half>(const Raw8<__half>& raw) {
+  const __half2* h = (const __half2*)raw.w;
+  const __half2 m = __hmax2(__hmax2(__habs2(h[0]), __habs2(h[1])), __hmax2(__habs2(h[2]), __habs2(h[3])));
+  const float2 f = __half22float2(m);
+  return fmaxf(fmaxf(f.x, f.y), 0.f);
+}
+// Exponent of the scale of a block with this largest magnitude: the smallest power of two >= amax / 448.
+__device__ __forceinline__ int scale_exponent(float amax) {
+  const int e = (int)ceilf(log2f(fmaxf(amax, 1e-12f) * (1.0f / 448.0f)));
+  return max(-127, min(127, e));
+}
+// The same for the 16 lanes that hold one block.
+template <typename T>
+__device__ __forceinline__ int block_exponent(const Raw8<T>& raw) {
+  float amax = block_amax_lane(raw);
 #pragma unroll
   for (int o = 8; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-  amax = fmaxf(amax, 1e-12f);
-  const int e = (int)ceilf(log2f(amax * (1.0f / 448.0f)));
-  return max(-127, min(127, e));
+  return scale_exponent(amax);
 }
 // The lane's eight values divided by 2^e, as e4m3.
 template <typename T>
 __device__ __forceinline__ uint2 quantised8(const Raw8<T>& raw, int e) {
-  const float inv = exp2f((float)-e);
+  const float inv = e == 127 ? 0x1p-127f : __int_as_float((127 - e) << 23);      // 2^-e
   uint32_t packed[2] = {0u, 0u};
 #pragma unroll
   for (int j = 0; j < 8; j += 2) {
-    const float2 v = make_float2(fminf(fmaxf(raw.get(j) * inv, -448.f), 448.f), fminf(fmaxf(raw.get(j + 1) * inv, -448.f), 448.f));
+    // (the conversion saturates at 448; the maximum is for the lower end's sake of NaN, which counts as -448)
+    const float2 v = make_float2(fmaxf(raw.get(j) * inv, -448.f), fmaxf(raw.get(j + 1) * inv, -448.f));
     packed[j >> 2] |= (uint32_t)__nv_cvt_float2_to_fp8x2(v, __NV_SATFINITE, __NV_E4M3) << (8 * (j & 3));
   }
   return make_uint2(packed[0], packed[1]);

@@ -233,3 +233,19 @@ def test_one_rank_ops_take_any_row_count(ctx, T, D, F):
     want = x.double() @ sq.double()
     ctx.ops.all_gather_matmul(x, x, sq, shard_dim=0, async_op=True)          # in place
     assert ((x.double() - want).norm() / want.norm()).item() < 4e-3
+
+
+def test_quantiser_special_values():
+    """Infinities saturate, NaN counts as -448 and does not move its block's scale, zeros stay zero, in every position of
+    a lane and of a block."""
+    from iris_b200.ops.gemm_fp8 import quantize_activation
+
+    for dtype in (torch.bfloat16, torch.float16, torch.float32):
+        for pos in (0, 1, 7, 8, 63, 127):
+            x = torch.ones(3, 256, device="cuda", dtype=dtype)
+            x[0, pos], x[1, 128 + pos], x[2, :128] = float("nan"), float("inf"), 0.0
+            got = quantize_activation(x)
+            q = got.q.float()
+            assert q[0, pos].item() == -448.0 and got.scale[0, 0].item() == got.scale[0, 1].item() == 2.0 ** -8
+            assert q[1, 128 + pos].item() == 448.0 and got.scale[1, 1].item() == 2.0 ** 127
+            assert (q[2, :128] == 0).all() and (q[2, 128:] == 256).all()
