@@ -620,6 +620,11 @@ namespace iris_ring {
 
 int launch_ring_attention_tc(const RingArgs& a, cudaStream_t stream) {
   if (a.S <= 0) return 1;
+  // Short sequences of one rank are a chain of few tiles per CTA, whose latency counts (a 128 x 128 tile from scores to P V
+  // takes about 2 us here): the mma.sync CTAs with their 64 x 64 tiles are through earlier. Measured, us, here / mma.sync, 8 heads:
+  // 129 tokens 13.3 / 9.7, 300 tokens 14 to 17 / 13, 500 tokens 18 to 19 / 17 to 18, 700 tokens 21 to 23 / 22; 32 heads:
+  // 200 tokens 14 / 11, 300 tokens 15 to 17 / 15 to 18, 500 tokens 19 / 22 to 26.
+  if (a.ctx.world == 1 && !a.zigzag && (a.S <= 256 || (a.S <= 512 && a.Hq <= 8))) return 1;
   const int W = a.ctx.world;
   TcArgs g;
   g.a = a;
