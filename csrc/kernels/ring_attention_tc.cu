@@ -58,6 +58,7 @@ static_assert(kTcSmem <= 227 * 1024, "shared memory budget");
 
 struct TcArgs {
   RingArgs a;
+  int single;            // 1: items of one query tile (few items: a CTA each, nothing to share the SM with)
   CUtensorMap tmQ;       // [S, Hq * D], box 64 x 128
   CUtensorMap tmKown;    // [1][S, Hkv * D], box 64 x 128 x 1
   CUtensorMap tmVown;    // [1][S, Hkv * D], box 64 x 64 x 1
@@ -154,14 +155,15 @@ struct Item {
 };
 struct ItemOrder {
   int items, rounds, stride, c, per_q, q_tiles, Hq, group;
-  bool by_head;
-  __device__ ItemOrder(const RingArgs& a) {
+  bool by_head, single;
+  __device__ ItemOrder(const RingArgs& a, int single_) {
+    single = single_ != 0;
     q_tiles = (a.S + kTQ - 1) / kTQ;
     Hq = a.Hq;
     group = a.Hq / a.Hkv;
-    by_head = group % 2 == 0;
+    by_head = !single && group % 2 == 0;
     per_q = by_head ? Hq / 2 : Hq;
-    items = (by_head ? q_tiles : (q_tiles + 1) / 2) * per_q;
+    items = (by_head || single ? q_tiles : (q_tiles + 1) / 2) * per_q;
     stride = gridDim.x - a.n_comm;
     c = blockIdx.x - a.n_comm;
     rounds = (items + stride - 1) / stride;
@@ -175,6 +177,10 @@ struct ItemOrder {
       it.qt[0] = it.qt[1] = q;
       it.h[0] = 2 * hh; it.h[1] = 2 * hh + 1;
       it.n_q = 2;
+    } else if (single) {
+      it.qt[0] = q; it.qt[1] = q_tiles;
+      it.h[0] = it.h[1] = hh;
+      it.n_q = 1;
     } else {
       it.qt[0] = 2 * q; it.qt[1] = 2 * q + 1;
       it.h[0] = it.h[1] = hh;
@@ -298,7 +304,7 @@ __device__ void attn_main_tc(const TcArgs& g, uint8_t* smem_raw, int call) {
   __syncthreads();
   ptx::tc_fence_after();
   const uint32_t tmem_base = *(volatile uint32_t*)tmem_slot;
-  const ItemOrder order(a);
+  const ItemOrder order(a, g.single);
 
   // 88 + 208 + 208 = 3 x 168, what the block was launched with (the splits stand at the head of their branches:
   // the compiler gives each branch its own budget from there)
@@ -620,11 +626,10 @@ namespace iris_ring {
 
 int launch_ring_attention_tc(const RingArgs& a, cudaStream_t stream) {
   if (a.S <= 0) return 1;
-  // Short sequences of one rank are a chain of few tiles per CTA, whose latency counts (a 128 x 128 tile from scores to P V
-  // takes about 2 us here): the mma.sync CTAs with their 64 x 64 tiles are through earlier. Measured, us, here / mma.sync, 8 heads:
-  // 129 tokens 13.3 / 9.7, 300 tokens 14 to 17 / 13, 500 tokens 18 to 19 / 17 to 18, 700 tokens 21 to 23 / 22; 32 heads:
-  // 200 tokens 14 / 11, 300 tokens 15 to 17 / 15 to 18, 500 tokens 19 / 22 to 26.
-  if (a.ctx.world == 1 && !a.zigzag && (a.S <= 256 || (a.S <= 512 && a.Hq <= 8))) return 1;
+  // The shortest sequences of one rank are a chain of one or two tiles, whose latency counts: the mma.sync CTAs with their
+  // 64 x 64 tiles are through earlier. Measured, us, here / mma.sync: 129 tokens 13.3 / 9.7 (8 heads), 200 tokens 14 / 11
+  // (32 heads), 384 tokens 12.9 / 14.6, 512 tokens 14.5 / 17.8.
+  if (a.ctx.world == 1 && !a.zigzag && a.S <= 256) return 1;
   const int W = a.ctx.world;
   TcArgs g;
   g.a = a;
@@ -651,7 +656,10 @@ int launch_ring_attention_tc(const RingArgs& a, cudaStream_t stream) {
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const int q_tiles = (a.S + kTQ - 1) / kTQ;
-  const int items = (a.Hq / a.Hkv) % 2 == 0 ? q_tiles * (a.Hq / 2) : (q_tiles + 1) / 2 * a.Hq;
+  int items = (a.Hq / a.Hkv) % 2 == 0 ? q_tiles * (a.Hq / 2) : (q_tiles + 1) / 2 * a.Hq;
+  // one query tile per item while every tile can have an SM of its own (1000 tokens, 8 heads: 26.0 us with two, 22.4 with one)
+  g.single = q_tiles * a.Hq <= sms - a.n_comm ? 1 : 0;
+  if (g.single) items = q_tiles * a.Hq;
   int attn = sms - a.n_comm;                 // one CTA per SM (194 KB of shared memory), all resident
   if (attn > items) attn = items;
   if (attn < 1) return 1;
