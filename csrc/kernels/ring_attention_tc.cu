@@ -257,7 +257,9 @@ struct TileWalk {
   __device__ bool diagonal(int i) const { return causal && origin == r && t == (i ? qt[1] : qt[0]); }
 };
 
-template <bool kFp16>
+// kScaleFirst: a scale that is not positive is applied before the mask and the maximum (0 times a masked -inf is NaN, a negative
+// factor turns maximum and mask round); a positive one changes neither and goes into the exponentials' FMA.
+template <bool kFp16, bool kScaleFirst>
 __device__ void attn_main_tc(const TcArgs& g, uint8_t* smem_raw, int call) {
   const RingArgs& a = g.a;
   const DeviceContext& ctx = a.ctx;
@@ -459,7 +461,7 @@ __device__ void attn_main_tc(const TcArgs& g, uint8_t* smem_raw, int call) {
     const int row = quarter * 32 + lane;                      // query row inside the tile
     const uint32_t lane_addr = tmem_base + ((uint32_t)(quarter * 32) << 16);
     const uint32_t s_addr = lane_addr + i * 128, o_addr = lane_addr + 256 + i * 128;
-    const float scale2 = a.sm_scale * kLog2e;
+    const float scale2 = kScaleFirst ? 1.f : a.sm_scale * kLog2e;
     const unsigned long long scale_pair = pack_f32x2(scale2, scale2);
     uint32_t n_item = 0, n_tile = 0;
     bool ok = true;
@@ -481,6 +483,10 @@ __device__ void attn_main_tc(const TcArgs& g, uint8_t* smem_raw, int call) {
 #pragma unroll
         for (int c = 0; c < 4; ++c) ptx::tmem_ld_32x32(s_addr + c * 32, *reinterpret_cast<uint32_t (*)[32]>(&s[c * 32]));
         ptx::tmem_ld_wait();
+        if constexpr (kScaleFirst) {
+#pragma unroll
+          for (int c = 0; c < 128; ++c) s[c] = __float_as_uint(__uint_as_float(s[c]) * (a.sm_scale * kLog2e));
+        }
         // causal mask on the diagonal tile, keys past the end of the block in its last tile
         int lim = a.S - 1 - w.t * kTK;
         if (w.diagonal(i)) lim = min(lim, qpos - w.t * kTK);
@@ -495,13 +501,14 @@ __device__ void attn_main_tc(const TcArgs& g, uint8_t* smem_raw, int call) {
 #pragma unroll
           for (int u = 0; u < 4; ++u) mx4[u] = fmaxf(mx4[u], fmaxf(__uint_as_float(s[c + u]), __uint_as_float(s[c + 4 + u])));
         }
-        const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * scale2;     // finite in the first tile: it holds a key the row sees
+        const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * scale2;     // (the first tile holds a key the row sees)
         float alpha = 1.f;
         if (j == 0) m_run = mx;
         else if (mx > m_run + kRescaleAt) { alpha = ex2_approx(m_run - mx); m_run = mx; }
         // p = exp2(s * scale - max): packed FMA for two scores at a time, one ex2.approx each, packed sums. P goes over
         // the first 64 columns of the tile's S buffer: every thread of the row (this one) has read its scores
-        const unsigned long long negm_pair = pack_f32x2(-m_run, -m_run);
+        const float neg_m = fminf(-m_run, 3e38f);      // finite where every key so far scores -inf: their P is 0, not NaN
+        const unsigned long long negm_pair = pack_f32x2(neg_m, neg_m);
         unsigned long long rs[2] = {0ull, 0ull};
 #pragma unroll
         for (int hf = 0; hf < 2; ++hf) {
@@ -588,12 +595,12 @@ __device__ void attn_main_tc(const TcArgs& g, uint8_t* smem_raw, int call) {
   if (warp == 1) ptx::tmem_dealloc(tmem_base, 512);
 }
 
-template <bool kFp16>
+template <bool kFp16, bool kScaleFirst>
 __global__ void __launch_bounds__(kTcThreads, 1) ring_attention_tc_kernel(const __grid_constant__ TcArgs g) {
   extern __shared__ __align__(128) uint8_t smem[];
   const int call = *(volatile int32_t*)&g.a.state[0];
   if ((int)blockIdx.x < g.a.n_comm) comm_main(g.a, smem, kTcSmem, call);
-  else attn_main_tc<kFp16>(g, smem, call);
+  else attn_main_tc<kFp16, kScaleFirst>(g, smem, call);
   finish_call(g.a, call);
 }
 
@@ -646,12 +653,10 @@ int launch_ring_attention_tc(const RingArgs& a, cudaStream_t stream) {
     g.tmKbuf = g.tmKown;
     g.tmVbuf = g.tmVown;
   }
-  static bool attr = false;
-  if (!attr) {
-    if (cudaFuncSetAttribute(ring_attention_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem) != cudaSuccess) return -20;
-    if (cudaFuncSetAttribute(ring_attention_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem) != cudaSuccess) return -20;
-    attr = true;
-  }
+  const bool scale_first = !(a.sm_scale > 0.f);
+  auto* kern = f16 ? (scale_first ? ring_attention_tc_kernel<true, true> : ring_attention_tc_kernel<true, false>)
+                   : (scale_first ? ring_attention_tc_kernel<false, true> : ring_attention_tc_kernel<false, false>);
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem) != cudaSuccess) return -20;
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -664,8 +669,7 @@ int launch_ring_attention_tc(const RingArgs& a, cudaStream_t stream) {
   if (attn > items) attn = items;
   if (attn < 1) return 1;
   const int grid = a.n_comm + attn;
-  if (f16) ring_attention_tc_kernel<true><<<grid, kTcThreads, kTcSmem, stream>>>(g);
-  else ring_attention_tc_kernel<false><<<grid, kTcThreads, kTcSmem, stream>>>(g);
+  kern<<<grid, kTcThreads, kTcSmem, stream>>>(g);
   return cudaGetLastError() == cudaSuccess ? 0 : -21;
 }
 

@@ -249,3 +249,40 @@ def test_quantiser_special_values():
             assert q[0, pos].item() == -448.0 and got.scale[0, 0].item() == got.scale[0, 1].item() == 2.0 ** -8
             assert q[1, 128 + pos].item() == 448.0 and got.scale[1, 1].item() == 2.0 ** 127
             assert (q[2, :128] == 0).all() and (q[2, 128:] == 256).all()
+
+
+@pytest.mark.parametrize("S,layout", [(300, "contiguous"), (384, "contiguous"), (512, "zigzag")])
+@pytest.mark.parametrize("sm_scale", [0.0, -0.05])
+@pytest.mark.parametrize("causal", [False, True])
+def test_attention_scale_that_is_not_positive(ctx, S, layout, sm_scale, causal):
+    """Masked keys stay masked and the maximum stays a maximum: 0 weighs every key that a row sees alike, a negative scale
+    prefers the lowest products. Same bound as above (|v| < 6)."""
+    from iris_b200.models import RingAttention, reference_attention
+
+    g = _gen(S)
+    q, k, v = (torch.randn(S, 4, 128, device="cuda", generator=g).clamp(-6, 6).to(torch.bfloat16) for _ in range(3))
+    mark = ctx.heap_mark()
+    out = RingAttention(ctx, S, 4, 4, sm_scale=sm_scale, layout=layout)(q, k, v, causal=causal)
+    assert (out.float() - reference_attention(q, k, v, causal, sm_scale=sm_scale)).abs().max().item() <= 2 * 2.0 ** -8 * 6
+    ctx.heap_release(mark)
+
+
+@pytest.mark.parametrize("S", [300, 384])
+@pytest.mark.parametrize("tc", [None, False])
+def test_attention_rows_whose_first_keys_score_minus_infinity(ctx, S, tc):
+    """Keys with -inf in a column where every query is 1 score -inf: whole tiles of them in front of the others change
+    nothing, and a row that sees only such keys has weight 0 and a log-sum of -inf."""
+    from iris_b200.models import RingAttention, reference_attention
+
+    g = _gen(S)
+    q, k, v = (torch.randn(S, 4, 128, device="cuda", generator=g).clamp(-6, 6).to(torch.bfloat16) for _ in range(3))
+    q[..., 0], k[..., 0], k[:200, :, 0] = 1.0, 0.0, float("-inf")
+    mark = ctx.heap_mark()
+    layer = RingAttention(ctx, S, 4, 4, use_tcgen05=tc)
+    for causal in (False, True):
+        out, lse = layer(q, k, v, causal=causal, return_lse=True)
+        want = reference_attention(q, k[200:], v[200:], causal, q_offset=-200) if causal else reference_attention(q, k[200:], v[200:])
+        first = 200 if causal else 0
+        assert (out[first:].float() - want[first:]).abs().max().item() <= 2 * 2.0 ** -8 * 6
+        assert (out[:first] == 0).all() and torch.isneginf(lse[:first]).all() and torch.isfinite(lse[first:]).all()
+    ctx.heap_release(mark)
