@@ -8,7 +8,7 @@
 //   warp 1      MMA issuer: per query tile i, S_i = Q_i K^T (tcgen05.mma, M 128, N 128, K 128) and
 //               O_i += P_i V (P from TMEM). Issue order PV_0(j), S_0(j+1), PV_1(j), S_1(j+1): the tensor pipe
 //               works for one query tile while the softmax of the other runs
-//   warps 4..7  softmax of query tile 0, warps 8..11 of tile 1, one thread per query row (208 registers each, the
+//   warps 4..7  softmax of query tile 0, warps 8..11 of tile 1, one thread per query row (216 registers each, the
 //               issuers give theirs up). Per tile: tcgen05.ld of
 //               the 128 scores, row maximum, P = exp2(s - max) (one packed FMA and one packed add per two scores,
 //               one ex2.approx each) written as packed 16-bit pairs over the first 64 columns of the SAME S
@@ -21,12 +21,20 @@
 // 1024 cycles of the MUFU. With one query tile per CTA and two threads per row (the previous split) the softmax of a tile
 // lay open next to its MMAs and the two threads of a row met in shared memory twice: about 3000 cycles per tile
 // (8192 tokens, 32 / 8 heads, causal, bf16: 736 us). Two tiles in turn, one thread per row: 549 us, with the MMAs issued eight
-// to a statement 511; 3000 tokens, full attention, fp16, which the mma.sync kernel took before: 603, 187, 176 us.
+// to a statement 511 (both with their inputs in L2, the second is 554 from HBM), with the loads' waits out of the chain 540 from
+// HBM; 3000 tokens, full attention, fp16, which the mma.sync kernel took before: 603, 187, 178, 174 us.
 // Slower were: 64-key halves with S double-buffered (more MMAs to issue: 746), P released to the MMAs in halves, part of the
 // exponentials as a polynomial on the FMA pipe (the softmax warps are short of issue slots).
 // The two tiles are two query heads of one K/V head group where the group is even (same keys, no work done twice or
 // for padding), else two neighbouring tiles of 128 queries of one head. Items are handed out longest first, in
 // alternating direction, so that a causal mask leaves no CTA with the long items at the end.
+//
+// Few query tiles (kByKeys; at most one per SM, under a causal mask on one rank two): an item is ONE query tile, and its key tiles go
+// in turn to the CTA's two places, each with its own S, O, maximum and sum; at the end each place's warps merge 64 columns of the
+// two O in TMEM. With the softmax of one place only, softmax, P V and S of a tile were a serial chain, slower than the
+// previous split of this kernel (8 heads, causal, us, that / one place / by keys: 512 tokens 14.6 / 15.6 / 11.7, 1024 tokens
+// 19.5 / 22.9 / 16.4, 2304 tokens 34.8 / 41.7 / 27.1). What a short sequence spends outside its tiles counts too: K, V and Q have a
+// producer warp each, the tensor maps are prefetched, and the output goes out by rows through shared memory.
 //
 // Sequences that are not a multiple of 128: the last tile's rows and keys past the end come back as zeros from TMA
 // (the ring buffer is mapped block by block for that), its scores are masked and its rows are not stored.
@@ -36,6 +44,7 @@
 #include "ring_attention_common.cuh"
 
 #include "iris/gemm/sm100_mainloop.cuh"
+#include <type_traits>
 
 using namespace iris;
 using namespace iris_ring;
@@ -51,14 +60,16 @@ constexpr int kTcThreads = 384;          // three warpgroups: issuers (two of fo
 constexpr int kHalf = 128 * 128;         // bytes of a [128 rows][64 columns] 16-bit half tile
 constexpr int kTile = 2 * kHalf;         // 32 KB
 constexpr int kKvStages = 2;
-constexpr int kTcSmem = 1024 + kTile * 2 + kTile * 2 * kKvStages + 256;    // Q tiles, K and V stages, barriers
+constexpr int kStageOut = 32 * 64;       // bytes a softmax warp stages its output rows in, 32 columns at a time (by keys)
+constexpr int kTcSmem = 1024 + kTile * 2 + kTile * 2 * kKvStages + 256;      // Q tiles, K and V stages, barriers
+constexpr int kTcSmemByKeys = kTcSmem + 2 * 128 * 8 + 8 * kStageOut;         // ... (m, l) of both places, output rows
 constexpr float kRescaleAt = 8.f;        // log2 of how far a row's maximum may run ahead of the one P is taken against
 constexpr uint64_t kWaitNs = 4000000000ull;
-static_assert(kTcSmem <= 227 * 1024, "shared memory budget");
+static_assert(kTcSmemByKeys <= 227 * 1024, "shared memory budget");
 
 struct TcArgs {
   RingArgs a;
-  int single;            // 1: items of one query tile (few items: a CTA each, nothing to share the SM with)
+  int by_head;           // 1: an item's two query tiles are two heads of one group, 0: two neighbouring tiles of one head
   CUtensorMap tmQ;       // [S, Hq * D], box 64 x 128
   CUtensorMap tmKown;    // [1][S, Hkv * D], box 64 x 128 x 1
   CUtensorMap tmVown;    // [1][S, Hkv * D], box 64 x 64 x 1
@@ -149,21 +160,21 @@ __device__ __forceinline__ unsigned long long pack_f32x2(float lo, float hi) {
 }
 
 // One item: two query tiles (qt[i], head h[i]) of one K/V head. n_q: how many of them exist (an odd number of
-// query tiles leaves the last item with one).
+// query tiles leaves the last item with one). By keys: one query tile, whose key tiles the two places share, and one item per CTA.
 struct Item {
   int qt[2], h[2], kvh, n_q;
 };
+template <bool kByKeys>
 struct ItemOrder {
   int items, rounds, stride, c, per_q, q_tiles, Hq, group;
-  bool by_head, single;
-  __device__ ItemOrder(const RingArgs& a, int single_) {
-    single = single_ != 0;
+  bool by_head;
+  __device__ ItemOrder(const RingArgs& a, int by_head_) {
     q_tiles = (a.S + kTQ - 1) / kTQ;
     Hq = a.Hq;
     group = a.Hq / a.Hkv;
-    by_head = !single && group % 2 == 0;
+    by_head = !kByKeys && by_head_ != 0;
     per_q = by_head ? Hq / 2 : Hq;
-    items = (by_head || single ? q_tiles : (q_tiles + 1) / 2) * per_q;
+    items = (by_head || kByKeys ? q_tiles : (q_tiles + 1) / 2) * per_q;
     stride = gridDim.x - a.n_comm;
     c = blockIdx.x - a.n_comm;
     rounds = (items + stride - 1) / stride;
@@ -177,10 +188,10 @@ struct ItemOrder {
       it.qt[0] = it.qt[1] = q;
       it.h[0] = 2 * hh; it.h[1] = 2 * hh + 1;
       it.n_q = 2;
-    } else if (single) {
-      it.qt[0] = q; it.qt[1] = q_tiles;
+    } else if (kByKeys) {
+      it.qt[0] = it.qt[1] = q;
       it.h[0] = it.h[1] = hh;
-      it.n_q = 1;
+      it.n_q = 2;
     } else {
       it.qt[0] = 2 * q; it.qt[1] = 2 * q + 1;
       it.h[0] = it.h[1] = hh;
@@ -193,7 +204,8 @@ struct ItemOrder {
 
 // The key tiles of one item, in the order every role walks them: blocks in arrival order (own,
 // r-1, r-2, ...), tiles inside a block in order; causal items skip what lies after their queries. A tile is
-// visited when one of the item's query tiles needs it; needs(i) says which.
+// visited when one of the item's query tiles needs it; needs(i) says which. By keys, place 0 takes the first, third, ... tile of
+// the walk and place 1 the others.
 //
 // Contiguous layout: rank r holds tokens [r*S, (r+1)*S). A causal item of query tile qt takes all
 // tiles of earlier blocks, tiles 0..qt of its own block (the last one masked on the diagonal) and
@@ -202,6 +214,7 @@ struct ItemOrder {
 // 2W-1-r (its block = [chunk r | chunk 2W-1-r]). Under a causal mask a query of chunk r sees
 // chunks 0..r, a query of chunk 2W-1-r sees every first-half chunk and the second-half chunks
 // of origins >= r: every rank does the same amount of work.
+template <bool kByKeys>
 struct TileWalk {
   int W, r, T, causal, zigzag;
   int qt[2], n_q;
@@ -209,6 +222,7 @@ struct TileWalk {
   int b0 = 0;                              // second range of a block starts here (first range ends at or before it)
   int a1[2], b1[2];                        // query tile i takes [0, a1[i]) and [b0, b1[i]) of the current block
   int ua1 = 0, ub1 = 0;                    // their union
+  int n = -1;                              // tiles taken before this one (counted by keys only)
   bool first = false;                      // the current tile is the first one taken from its block
   __device__ TileWalk(const RingArgs& a, const Item& it)
       : W(a.ctx.world), r(a.ctx.rank), T((a.S + kTK - 1) / kTK), causal(a.causal), zigzag(a.zigzag), n_q(it.n_q) {
@@ -246,21 +260,25 @@ struct TileWalk {
       first = t < 0;
       if (t < 0) t = ua1 > 0 ? 0 : b0;
       else if (++t == ua1 && ub1 > b0) t = b0;
-      if (t < ua1 || (t >= b0 && t < ub1)) return true;
+      if (t < ua1 || (t >= b0 && t < ub1)) {
+        if (kByKeys) ++n;
+        return true;
+      }
       ++step;
       open_block();
     }
     return false;
   }
   // (selected, not indexed: an index that is not a constant would put the arrays in local memory)
-  __device__ bool needs(int i) const { return t < (i ? a1[1] : a1[0]) || (t >= b0 && t < (i ? b1[1] : b1[0])); }
+  __device__ bool needs(int i) const { return kByKeys ? (n & 1) == i : t < (i ? a1[1] : a1[0]) || (t >= b0 && t < (i ? b1[1] : b1[0])); }
   __device__ bool diagonal(int i) const { return causal && origin == r && t == (i ? qt[1] : qt[0]); }
 };
 
 // kScaleFirst: a scale that is not positive is applied before the mask and the maximum (0 times a masked -inf is NaN, a negative
 // factor turns maximum and mask round); a positive one changes neither and goes into the exponentials' FMA.
-template <bool kFp16, bool kScaleFirst>
+template <bool kFp16, bool kScaleFirst, bool kByKeys>
 __device__ void attn_main_tc(const TcArgs& g, uint8_t* smem_raw, int call) {
+  using TileWalk = ::TileWalk<kByKeys>;
   const RingArgs& a = g.a;
   const DeviceContext& ctx = a.ctx;
   const int W = ctx.world, r = ctx.rank;
@@ -284,7 +302,10 @@ __device__ void attn_main_tc(const TcArgs& g, uint8_t* smem_raw, int call) {
   uint64_t* o_full = bars + 16;         // [2] the item's O_i is complete
   uint64_t* o_free = bars + 18;         // [2] 4 softmax warps have read the item's O_i
   uint32_t* tmem_slot = (uint32_t*)(bars + 20);
+  float2* ml = (float2*)((uint8_t*)bars + 256);          // [2][128] by keys: a place's maximum and sum per row
 
+  if (kByKeys && warp == 2 && lane < 3)     // the first loads of a short sequence would wait for the maps one by one
+    ptx::prefetch_tmap(lane == 0 ? &g.tmQ : lane == 1 ? &g.tmKown : &g.tmVown);
   if (threadIdx.x == 0) {
     for (int i = 0; i < 2; ++i) {
       ptx::mbar_init(&q_full[i], 1); ptx::mbar_init(&q_free[i], 1);
@@ -306,14 +327,15 @@ __device__ void attn_main_tc(const TcArgs& g, uint8_t* smem_raw, int call) {
   __syncthreads();
   ptx::tc_fence_after();
   const uint32_t tmem_base = *(volatile uint32_t*)tmem_slot;
-  const ItemOrder order(a, g.single);
+  const ItemOrder<kByKeys> order(a, g.by_head);
 
-  // 88 + 208 + 208 = 3 x 168, what the block was launched with (the splits stand at the head of their branches:
-  // the compiler gives each branch its own budget from there)
+  // 72 + 216 + 216 = 3 x 168, what the block was launched with (the splits stand at the head of their branches:
+  // the compiler gives each branch its own budget from there). The compiler still keeps a few words of walk state on the stack.
   if (warp < 4) {
-  asm volatile("setmaxnreg.dec.sync.aligned.u32 88;");
-  if (warp == 0) {
-    // ------------------------------------------------------------------ TMA producer
+  asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
+  if (warp == 0 || (kByKeys && warp != 1)) {
+    // ------------------------------------------------------------------ TMA producer (by keys three: warp 0 K, warp 2 V, warp 3 Q;
+    // K is loaded as soon as its stage is read then, not behind V of the tile before, whose stage is free much later)
     unsigned arrived_mask = 1u << r;
     uint32_t n_tile = 0;                    // K/V tiles issued so far (barrier phases)
     uint32_t n_q[2] = {0, 0};               // Q tiles loaded so far, per place
@@ -321,15 +343,18 @@ __device__ void attn_main_tc(const TcArgs& g, uint8_t* smem_raw, int call) {
     Item item;
     for (int rd = 0; rd < order.rounds && ok; ++rd) {
       if (!order.get(rd, item)) continue;
+      if (!kByKeys || warp == 3) {
 #pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        if (i >= item.n_q || !ok) break;
-        if (!__all_sync(0xffffffffu, ptx::mbar_wait(&q_free[i], (n_q[i] & 1) ^ 1, kWaitNs))) { ctx.fail(kTimeoutPipeline); ok = false; break; }
-        const uint32_t qd = ptx::smem_u32(q_s + i * kTile);
-        ptx::mbar_expect_tx_elect(&q_full[i], kTile);
-        ptx::tma_load_2d_elect(qd, &g.tmQ, &q_full[i], item.h[i] * kD, item.qt[i] * kTQ);
-        ptx::tma_load_2d_elect(qd + kHalf, &g.tmQ, &q_full[i], item.h[i] * kD + 64, item.qt[i] * kTQ);
-        ++n_q[i];
+        for (int i = 0; i < 2; ++i) {
+          if (i >= (kByKeys ? 1 : item.n_q) || !ok) break;          // (by keys both places use Q tile 0)
+          if (!__all_sync(0xffffffffu, ptx::mbar_wait(&q_free[i], (n_q[i] & 1) ^ 1, kWaitNs))) { ctx.fail(kTimeoutPipeline); ok = false; break; }
+          const uint32_t qd = ptx::smem_u32(q_s + i * kTile);
+          ptx::mbar_expect_tx_elect(&q_full[i], kTile);
+          ptx::tma_load_2d_elect(qd, &g.tmQ, &q_full[i], item.h[i] * kD, item.qt[i] * kTQ);
+          ptx::tma_load_2d_elect(qd + kHalf, &g.tmQ, &q_full[i], item.h[i] * kD + 64, item.qt[i] * kTQ);
+          ++n_q[i];
+        }
+        if (kByKeys) continue;
       }
       TileWalk w(a, item);
       while (ok && w.next()) {
@@ -351,17 +376,21 @@ __device__ void attn_main_tc(const TcArgs& g, uint8_t* smem_raw, int call) {
         const int pos0 = w.t * kTK;
         const uint32_t kd = ptx::smem_u32(k_s + st * kTile);
         const uint32_t vd = ptx::smem_u32(v_s + st * kTile);
-        if (!__all_sync(0xffffffffu, ptx::mbar_wait(&k_empty[st], ph, kWaitNs))) { ctx.fail(kTimeoutPipeline); ok = false; break; }
-        ptx::mbar_expect_tx_elect(&k_full[st], kTile);
-        tma_load_3d_elect(kd, mk, &k_full[st], item.kvh * kD, pos0, zk);
-        tma_load_3d_elect(kd + kHalf, mk, &k_full[st], item.kvh * kD + 64, pos0, zk);
-        if (!__all_sync(0xffffffffu, ptx::mbar_wait(&v_empty[st], ph, kWaitNs))) { ctx.fail(kTimeoutPipeline); ok = false; break; }
-        ptx::mbar_expect_tx_elect(&v_full[st], kTile);
+        if (!kByKeys || warp == 0) {
+          if (!__all_sync(0xffffffffu, ptx::mbar_wait(&k_empty[st], ph, kWaitNs))) { ctx.fail(kTimeoutPipeline); ok = false; break; }
+          ptx::mbar_expect_tx_elect(&k_full[st], kTile);
+          tma_load_3d_elect(kd, mk, &k_full[st], item.kvh * kD, pos0, zk);
+          tma_load_3d_elect(kd + kHalf, mk, &k_full[st], item.kvh * kD + 64, pos0, zk);
+        }
+        if (!kByKeys || warp == 2) {
+          if (!__all_sync(0xffffffffu, ptx::mbar_wait(&v_empty[st], ph, kWaitNs))) { ctx.fail(kTimeoutPipeline); ok = false; break; }
+          ptx::mbar_expect_tx_elect(&v_full[st], kTile);
 #pragma unroll
-        for (int kh = 0; kh < 2; ++kh)
+          for (int kh = 0; kh < 2; ++kh)
 #pragma unroll
-          for (int nb = 0; nb < 2; ++nb)
-            tma_load_3d_elect(vd + kh * kHalf + nb * 8192, mv, &v_full[st], item.kvh * kD + nb * 64, pos0 + kh * 64, zv);
+            for (int nb = 0; nb < 2; ++nb)
+              tma_load_3d_elect(vd + kh * kHalf + nb * 8192, mv, &v_full[st], item.kvh * kD + nb * 64, pos0 + kh * 64, zv);
+        }
         ++n_tile;
       }
     }
@@ -383,6 +412,39 @@ __device__ void attn_main_tc(const TcArgs& g, uint8_t* smem_raw, int call) {
     Item item;
     for (int rd = 0; rd < order.rounds && ok; ++rd) {
       if (!order.get(rd, item)) continue;
+      if constexpr (kByKeys) {
+        // S of the walk's tiles j + 1 and j + 2 is issued while the softmax works on tile j
+        int n = 0;
+        for (TileWalk w(a, item); w.next();) ++n;
+        if (!wait(&q_full[0], 0)) break;
+        const uint32_t qb = ptx::smem_u32(q_s);
+        auto wait_k = [&]() { return wait(&k_full[n_k % kKvStages], (n_k / kKvStages) & 1); };
+        auto issue_s = [&](int i) {
+          const int st = n_k % kKvStages;
+          ptx::tc_fence_after();
+          mma_s_elect(tmem_u + i * 128, desc_kmajor(qb), desc_kmajor(ptx::smem_u32(k_s + st * kTile)), idesc_s, 0);
+          ptx::mma_commit_elect(&s_full[i]);
+          ptx::mma_commit_elect(&k_empty[st]);
+          ++n_k;
+        };
+        if (!wait_k()) break;
+        issue_s(0);
+        if (n > 1) {
+          if (!wait_k()) break;
+          issue_s(1);
+        }
+        for (int j = 0; j < n; ++j) {
+          const int i = j & 1, st = j % kKvStages;
+          // (P's wait comes last, see below)
+          if (!wait(&v_full[st], (j / kKvStages) & 1) || (j + 2 < n && !wait_k()) || !wait(&p_full[i], (j >> 1) & 1)) break;
+          ptx::tc_fence_after();
+          mma_pv_elect(tmem_u + 256 + i * 128, tmem_u + i * 128, desc_mnmajor(ptx::smem_u32(v_s + st * kTile)), idesc_o, j >= 2);
+          if (j >= n - 2) ptx::mma_commit_elect(&o_full[i]);
+          ptx::mma_commit_elect(&v_empty[st]);
+          if (j + 2 < n) issue_s(i);
+        }
+        break;
+      }
       int left_s[2] = {0, 0}, left_pv[2];          // S and P V MMAs of the item still to be issued, per query tile
       {
         TileWalk w(a, item);
@@ -424,13 +486,13 @@ __device__ void attn_main_tc(const TcArgs& g, uint8_t* smem_raw, int call) {
       while (ok && has) {
         has_n = nxt.next();
         const int vst = n_v % kKvStages, kst = n_k % kKvStages;
-        bool v_ready = false, k_ready = false;
+        // (the loads' waits stand in front of P's: a wait costs this warp some 200 cycles even when it is over, and what follows P
+        // is the chain that sets the pace. 8192 tokens, 32 / 8 heads, causal, inputs in L2: 485 us with them behind it, now 467.)
+        if (!wait(&v_full[vst], (n_v / kKvStages) & 1) || (has_n && !wait(&k_full[kst], (n_k / kKvStages) & 1))) break;
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
           if (cur.needs(i)) {
             if (!wait(&p_full[i], n_p[i] & 1)) break;
-            if (!v_ready && !wait(&v_full[vst], (n_v / kKvStages) & 1)) break;
-            v_ready = true;
             // the previous item's O must have been read out before this item's first P V overwrites it
             if (left_pv[i] == total[i] && !wait(&o_free[i], (n_qi[i] & 1) ^ 1)) break;
             issue_pv(i, vst);
@@ -438,8 +500,6 @@ __device__ void attn_main_tc(const TcArgs& g, uint8_t* smem_raw, int call) {
           }
           if (cur.needs(i) && (i == 1 || !cur.needs(1))) ptx::mma_commit_elect(&v_empty[vst]);      // the tile's last P V
           if (has_n && nxt.needs(i)) {
-            if (!k_ready && !wait(&k_full[kst], (n_k / kKvStages) & 1)) break;
-            k_ready = true;
             issue_s(i, kst);
           }
         }
@@ -455,7 +515,7 @@ __device__ void attn_main_tc(const TcArgs& g, uint8_t* smem_raw, int call) {
   }
   } else {
     // ------------------------------------------------------------------ softmax / correction / epilogue
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 208;");
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 216;");
     const int quarter = warp & 3;
     const int i = (warp - 4) >> 2;                            // query tile of the item
     const int row = quarter * 32 + lane;                      // query row inside the tile
@@ -552,7 +612,7 @@ __device__ void attn_main_tc(const TcArgs& g, uint8_t* smem_raw, int call) {
         ++n_tile;
         ++j;
       }
-      if (!ok) break;
+      if (!ok && !kByKeys) break;                             // (by keys the other place waits for this one at a barrier)
       // ---- item epilogue: the row sum, the last P V, O / sum -> 16-bit -> global
       float l_all = 0.f;
 #pragma unroll
@@ -560,6 +620,63 @@ __device__ void attn_main_tc(const TcArgs& g, uint8_t* smem_raw, int call) {
         float x0, x1;
         asm("mov.b64 {%0, %1}, %2;" : "=f"(x0), "=f"(x1) : "l"(l_pair[u]));
         l_all += x0 + x1;
+      }
+      if constexpr (kByKeys) {
+        // Both places' warps of a quarter reach the same TMEM lanes, so each merges 64 columns of the two O; only the
+        // rows' maxima and sums go through shared memory. An item of one key tile is place 0's alone.
+        const int n = w.n + 1;
+        const bool both = n > 1, mine = both || i == 0;
+        ml[i * 128 + row] = make_float2(m_run, l_all);
+        for (int k = 0; k < (both ? 2 : 1); ++k)
+          if (ok && !__all_sync(0xffffffffu, ptx::mbar_wait(&o_full[k], 0, kWaitNs))) { ctx.fail(kTimeoutPipeline); ok = false; }
+        ptx::named_barrier(1, 256);
+        ptx::tc_fence_after();
+        if (ok && mine) {
+          float m = m_run, l = l_all, w_own = 1.f, w_other = 0.f;
+          if (both) {
+            const float2 other = ml[(i ^ 1) * 128 + row];
+            m = fmaxf(m_run, other.x);
+            w_own = m_run == -INFINITY ? 0.f : ex2_approx(m_run - m);
+            w_other = other.x == -INFINITY ? 0.f : ex2_approx(other.x - m);
+            l = l_all * w_own + other.y * w_other;
+          }
+          const float inv = l > 0.f ? 1.f / l : 0.f;
+          w_own *= inv; w_other *= inv;
+          const uint32_t other_addr = lane_addr + 256 + (i ^ 1) * 128;
+          // the warp's 32 rows go out through shared memory, 32 columns (64 bytes) of a row by four lanes: with a row per lane every
+          // 16-byte store instruction touched 32 lines
+          uint8_t* stage = (uint8_t*)(ml + 2 * 128) + (warp - 4) * kStageOut;
+          const int c0 = both ? 2 * i : 0, c1 = both ? c0 + 2 : 4;
+#pragma unroll 1
+          for (int c = c0; c < c1; ++c) {
+            uint32_t o[32], o2[32];
+            ptx::tmem_ld_32x32(o_addr + c * 32, o);
+            if (both) ptx::tmem_ld_32x32(other_addr + c * 32, o2);
+            ptx::tmem_ld_wait();
+#pragma unroll
+            for (int e = 0; e < 32; ++e) {
+              float f = __uint_as_float(o[e]) * w_own;
+              if (both) f += __uint_as_float(o2[e]) * w_other;
+              o[e] = __float_as_uint(f);
+            }
+            // 16-byte pieces, XORed by half the row so that eight rows written and two rows read together meet different banks
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+              *(uint4*)(stage + lane * 64 + ((e ^ ((lane >> 1) & 3)) << 4)) =
+                  make_uint4(pack2<kFp16>(__uint_as_float(o[8 * e]), __uint_as_float(o[8 * e + 1])), pack2<kFp16>(__uint_as_float(o[8 * e + 2]), __uint_as_float(o[8 * e + 3])),
+                             pack2<kFp16>(__uint_as_float(o[8 * e + 4]), __uint_as_float(o[8 * e + 5])), pack2<kFp16>(__uint_as_float(o[8 * e + 6]), __uint_as_float(o[8 * e + 7])));
+            __syncwarp();
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+              const int rr = k * 8 + (lane >> 2), e = lane & 3, pos = item.qt[0] * kTQ + quarter * 32 + rr;
+              if (pos < a.S)
+                *(uint4*)(a.out + ((size_t)pos * a.Hq + head) * kD * 2 + c * 64 + e * 16) = *(const uint4*)(stage + rr * 64 + ((e ^ ((rr >> 1) & 3)) << 4));
+            }
+            __syncwarp();
+          }
+          if (a.lse && i == 0 && qpos < a.S) a.lse[(size_t)qpos * a.Hq + head] = l > 0.f ? (m + log2f(l)) / kLog2e : -INFINITY;
+        }
+        break;
       }
       if (!__all_sync(0xffffffffu, ptx::mbar_wait(&o_full[i], n_item & 1, kWaitNs))) { ctx.fail(kTimeoutPipeline); ok = false; break; }
       ptx::tc_fence_after();
@@ -595,12 +712,12 @@ __device__ void attn_main_tc(const TcArgs& g, uint8_t* smem_raw, int call) {
   if (warp == 1) ptx::tmem_dealloc(tmem_base, 512);
 }
 
-template <bool kFp16, bool kScaleFirst>
+template <bool kFp16, bool kScaleFirst, bool kByKeys>
 __global__ void __launch_bounds__(kTcThreads, 1) ring_attention_tc_kernel(const __grid_constant__ TcArgs g) {
   extern __shared__ __align__(128) uint8_t smem[];
   const int call = *(volatile int32_t*)&g.a.state[0];
   if ((int)blockIdx.x < g.a.n_comm) comm_main(g.a, smem, kTcSmem, call);
-  else attn_main_tc<kFp16, kScaleFirst>(g, smem, call);
+  else attn_main_tc<kFp16, kScaleFirst, kByKeys>(g, smem, call);
   finish_call(g.a, call);
 }
 
@@ -633,10 +750,10 @@ namespace iris_ring {
 
 int launch_ring_attention_tc(const RingArgs& a, cudaStream_t stream) {
   if (a.S <= 0) return 1;
-  // The shortest sequences of one rank are a chain of one or two tiles, whose latency counts: the mma.sync CTAs with their
-  // 64 x 64 tiles are through earlier. Measured, us, here / mma.sync: 129 tokens 13.3 / 9.7 (8 heads), 200 tokens 14 / 11
-  // (32 heads), 384 tokens 12.9 / 14.6, 512 tokens 14.5 / 17.8.
-  if (a.ctx.world == 1 && !a.zigzag && a.S <= 256) return 1;
+  // One rank, one key tile: nothing to share or overlap, and the mma.sync CTAs with their 64 x 64 tiles are through earlier. Measured,
+  // us, here / mma.sync, 8 heads, full attention: 32 tokens 7.8 / 6.2, 64 tokens 8.9 / 7.2, 128 tokens 7.9 / 8.4 (32 heads 9.0 / 8.8),
+  // 129 tokens 9.3 / 10.0, 200 tokens 9.5 / 11.5, 256 tokens 9.3 / 11.7.
+  if (a.ctx.world == 1 && !a.zigzag && a.S <= kTK) return 1;
   const int W = a.ctx.world;
   TcArgs g;
   g.a = a;
@@ -653,23 +770,34 @@ int launch_ring_attention_tc(const RingArgs& a, cudaStream_t stream) {
     g.tmKbuf = g.tmKown;
     g.tmVbuf = g.tmVown;
   }
-  const bool scale_first = !(a.sm_scale > 0.f);
-  auto* kern = f16 ? (scale_first ? ring_attention_tc_kernel<true, true> : ring_attention_tc_kernel<true, false>)
-                   : (scale_first ? ring_attention_tc_kernel<false, true> : ring_attention_tc_kernel<false, false>);
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem) != cudaSuccess) return -20;
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const int q_tiles = (a.S + kTQ - 1) / kTQ;
-  int items = (a.Hq / a.Hkv) % 2 == 0 ? q_tiles * (a.Hq / 2) : (q_tiles + 1) / 2 * a.Hq;
-  // one query tile per item while every tile can have an SM of its own (1000 tokens, 8 heads: 26.0 us with two, 22.4 with one)
-  g.single = q_tiles * a.Hq <= sms - a.n_comm ? 1 : 0;
-  if (g.single) items = q_tiles * a.Hq;
-  int attn = sms - a.n_comm;                 // one CTA per SM (194 KB of shared memory), all resident
-  if (attn > items) attn = items;
+  // Key tiles shared by the places while every query tile can have an SM. Under a causal mask also when it takes two turns: the
+  // second ones are the short ones, and of two-tile items there would be fewer than SMs (us, two-tile items / by keys:
+  // 8 heads 2432 tokens 44.7 / 29.2, 4608 tokens 78.5 / 54.1, 32 heads 1024 tokens 26.2 / 26.2, 1280 tokens, 320 tiles 30.9 / 35.4;
+  // full attention, 8 heads 2432 tokens 47.4 / 52.8). The turns need CTAs that wait for nobody: one rank.
+  const int tiles = q_tiles * a.Hq;
+  const bool by_keys = tiles <= sms - a.n_comm || (W == 1 && a.causal && tiles <= 2 * sms);
+  g.by_head = (a.Hq / a.Hkv) % 2 == 0;
+  const int items = by_keys ? tiles : g.by_head ? q_tiles * (a.Hq / 2) : (q_tiles + 1) / 2 * a.Hq;
+  // one CTA per SM (194 KB of shared memory), all resident; by keys a CTA per item, which the SMs take in order (longest first)
+  int attn = sms - a.n_comm;
+  if (by_keys || attn > items) attn = items;
   if (attn < 1) return 1;
   const int grid = a.n_comm + attn;
-  kern<<<grid, kTcThreads, kTcSmem, stream>>>(g);
+  const bool scale_first = !(a.sm_scale > 0.f);
+  auto pick = [&](auto fp16, auto first) -> void (*)(const TcArgs) {
+    return by_keys ? ring_attention_tc_kernel<decltype(fp16)::value, decltype(first)::value, true>
+                   : ring_attention_tc_kernel<decltype(fp16)::value, decltype(first)::value, false>;
+  };
+  using Y = std::true_type;
+  using N = std::false_type;
+  auto* kern = f16 ? (scale_first ? pick(Y{}, Y{}) : pick(Y{}, N{})) : (scale_first ? pick(N{}, Y{}) : pick(N{}, N{}));
+  const int smem = by_keys ? kTcSmemByKeys : kTcSmem;
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -20;
+  kern<<<grid, kTcThreads, smem, stream>>>(g);
   return cudaGetLastError() == cudaSuccess ? 0 : -21;
 }
 

@@ -102,11 +102,16 @@ def test_moe_one_rank_router_sort_gather(ctx, T, E, K):
 
 # ------------------------------------------------------------------------------------ attention on one rank
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
-@pytest.mark.parametrize("S,Hq,Hkv", [(1, 2, 2), (64, 4, 2), (127, 8, 2), (128, 3, 1), (129, 4, 4), (257, 6, 2), (384, 5, 5), (1000, 8, 8), (2500, 16, 2)])
+@pytest.mark.parametrize("S,Hq,Hkv", [(1, 2, 2), (64, 4, 2), (127, 8, 2), (128, 3, 1), (129, 4, 4), (257, 6, 2), (384, 5, 5), (1000, 8, 8), (2500, 16, 2),
+                                      (300, 2, 1), (640, 8, 2), (2304, 4, 2), (4700, 4, 4),
+                                      (2500, 8, 8), (2300, 9, 3), (2400, 9, 3), (2300, 18, 3), (4200, 9, 3), (4300, 9, 3)])
 @pytest.mark.parametrize("causal", [False, True])
 def test_attention_any_length_and_group(ctx, dtype, S, Hq, Hkv, causal):
-    """Lengths on both sides of the 128-row tiles, head groups of odd size (two query tiles of one head per item, the
-    last item of an odd count with one) and of even size (two heads per item), against fp32 attention. P and the
+    """Every form of the dispatch, lengths on both sides of the 128-row tiles, against fp32 attention: the mma.sync CTAs (up to
+    128 tokens); one query tile whose keys two softmax groups share (at most as many query tiles as SMs, 148, under a causal
+    mask twice as many: up to (4700, 4, 4); odd and even numbers of key tiles, one in the first causal tile); two heads of an
+    even group per item ((2500, 16, 2), (2300, 18, 3)); two neighbouring query tiles of one head ((2500, 8, 8), (2300, 9, 3) with
+    full attention, (4300, 9, 3) with either), the last item of an odd count with one tile ((2400, 9, 3), (4200, 9, 3)). P and the
     output are rounded to 16 bits: |error| <= 2 u max|v| with u = 2^-8 (bf16) or 2^-11 (fp16), and max|v| < 6 here.
     The scores are scaled up so that rows move their maximum late (the rescaling of O) as well as early."""
     from iris_b200.models import RingAttention, reference_attention
@@ -249,6 +254,25 @@ def test_quantiser_special_values():
             assert q[0, pos].item() == -448.0 and got.scale[0, 0].item() == got.scale[0, 1].item() == 2.0 ** -8
             assert q[1, 128 + pos].item() == 448.0 and got.scale[1, 1].item() == 2.0 ** 127
             assert (q[2, :128] == 0).all() and (q[2, 128:] == 256).all()
+
+
+@pytest.mark.parametrize("S,Hq,Hkv", [(256, 2, 2), (768, 4, 2), (2560, 16, 2), (2560, 9, 3), (2816, 9, 3), (4352, 9, 3)])
+@pytest.mark.parametrize("causal", [False, True])
+def test_attention_zigzag_forms(ctx, S, Hq, Hkv, causal):
+    """The zigzag walk (on one rank: plain attention) with a query tile's keys shared between the places, with two heads per item
+    ((2560, 16, 2)), with neighbouring tiles of one head, and with a pair of them that lies in both halves of the block
+    ((2816, 9, 3), 11 tiles each, full attention; (4352, 9, 3), 17 tiles each, causal too). Bounds as above."""
+    from iris_b200.models import RingAttention, reference_attention
+
+    g = _gen(S + Hq)
+    mk = lambda h: torch.randn(S, h, 128, device="cuda", generator=g).clamp(-6, 6).to(torch.bfloat16)  # noqa: E731
+    q, k, v = mk(Hq), mk(Hkv), mk(Hkv)
+    mark = ctx.heap_mark()
+    layer = RingAttention(ctx, S, Hq, Hkv, layout="zigzag")
+    out = layer(q, k, v, causal=causal)
+    assert (out.float() - reference_attention(q, k, v, causal)).abs().max().item() <= 2 * 2.0 ** -8 * 6
+    assert torch.equal(out, layer(q, k, v, causal=causal))
+    ctx.heap_release(mark)
 
 
 @pytest.mark.parametrize("S,layout", [(300, "contiguous"), (384, "contiguous"), (512, "zigzag")])
