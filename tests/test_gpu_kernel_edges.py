@@ -275,6 +275,28 @@ def test_attention_zigzag_forms(ctx, S, Hq, Hkv, causal):
     ctx.heap_release(mark)
 
 
+@pytest.mark.parametrize("S,Hq,Hkv", [(384, 8, 8), (2500, 16, 8)])
+def test_attention_largest_weight_is_exact(ctx, S, Hq, Hkv):
+    """A row's largest weight is 1 before it is rounded to 16 bits, also when its key comes after the row's first tile (one
+    of the first eight): key 300 outweighs the others by 2^0.3 to 2^7.3, at points between two bf16 values, and alone has a value, so
+    that the output's own rounding (at most 2^-8 of it: bf16 has 8 significant bits) is all the error there is besides fp32's."""
+    from iris_b200.models import RingAttention
+
+    g = _gen(S)
+    q = torch.ones(S, Hq, 128, device="cuda", dtype=torch.bfloat16)
+    k, v = (torch.zeros(S, Hkv, 128, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    mark = ctx.heap_mark()
+    layer = RingAttention(ctx, S, Hq, Hkv)
+    for lo in (0.02, 0.15, 0.3):
+        c = (lo + 0.15 * torch.rand(Hkv, device="cuda", generator=g)).to(torch.bfloat16)
+        k[300] = c[:, None]
+        v[300] = torch.randn(Hkv, 128, device="cuda", generator=g).to(torch.bfloat16)
+        e = torch.exp(128 * c.double() * 128 ** -0.5)
+        want = ((e / (e + S - 1))[:, None] * v[300].double()).repeat_interleave(Hq // Hkv, dim=0)
+        assert ((layer(q, k, v).double() - want).abs() <= 1.01 * 2.0 ** -8 * want.abs()).all()
+    ctx.heap_release(mark)
+
+
 @pytest.mark.parametrize("S,layout", [(300, "contiguous"), (384, "contiguous"), (512, "zigzag")])
 @pytest.mark.parametrize("sm_scale", [0.0, -0.05])
 @pytest.mark.parametrize("causal", [False, True])
