@@ -38,6 +38,7 @@
 #include "flash_decode_static.h"
 #include <stdio.h>
 #include <mutex>
+#include <type_traits>
 
 using namespace iris;
 
@@ -94,6 +95,11 @@ __device__ __forceinline__ void mma16816(float (&c)[4], const uint32_t (&a)[4], 
 template <bool kFp16> __device__ __forceinline__ uint32_t pack2(float a, float b) {
   if constexpr (kFp16) { __half2 h = __floats2half2_rn(a, b); return *(uint32_t*)&h; }
   else { __nv_bfloat162 h = __floats2bfloat162_rn(a, b); return *(uint32_t*)&h; }
+}
+
+template <bool kFp16> __device__ __forceinline__ float2 unpack2(uint32_t w) {
+  if constexpr (kFp16) return __half22float2(*(const __half2*)&w);
+  else return __bfloat1622float2(*(const __nv_bfloat162*)&w);
 }
 
 // Shared-memory tile of kBlockN positions x 16 chunks of 16 B.
@@ -191,8 +197,15 @@ __device__ __forceinline__ void prefix_tiles(const DecodeArgs& a, int* pre, int 
 
 // Attention state of one of the four computing warps: up to 16 query heads (rows) against the warp's 16 positions of
 // each tile.
-template <bool kFp16, bool kTma>
+// P V is taken with P as two 16-bit numbers, its rounded value and the remainder: rounded once, P's error is as large as the output's
+// own rounding, and more so the longer the runs are (only a run's largest weight is exact; 32 sequences of 8192 to 32768 positions, bf16,
+// 2-norm against 64 bits: 2.21e-3 with the shorter runs of a fixed number of splits, 2.24e-3 with these, 1.65e-3 with the remainder).
+// kRows8 (groups of up to 8 query heads): the remainders are rows 8 to 15 of the same MMA, which are padding otherwise, and the softmax
+// skips those rows (32768 positions, 64 / 8 heads 39.1 -> 38.0 us). Wider groups take a second MMA (64 / 4 heads: 32 sequences by TMA
+// 215 -> 216 us, one 42.6 -> 43.6; 16 sequences by cp.async, 32 / 2 heads, 95 -> 99).
+template <bool kFp16, bool kTma, bool kRows8>
 struct Attend {
+  static constexpr int kE = kRows8 ? 2 : 4, kR = kRows8 ? 1 : 2;       // values per fragment and rows that a lane has
   uint32_t qf[8][4];             // Q fragments (A operand, rows = heads, padded to 16 with zeros)
   float o[16][4], m_run[2], l_run[2];
 
@@ -200,7 +213,7 @@ struct Attend {
     const int r0 = lane >> 2, c0 = (lane & 3) * 2;
     const uint32_t* qrow0 = (const uint32_t*)(a.q + ((size_t)r.b * a.Hq + r.h0 + r0) * kD);
     const uint32_t* qrow1 = (const uint32_t*)(a.q + ((size_t)r.b * a.Hq + r.h0 + r0 + 8) * kD);
-    const bool v0 = r0 < r.heads_here, v1 = r0 + 8 < r.heads_here;
+    const bool v0 = r0 < r.heads_here, v1 = !kRows8 && r0 + 8 < r.heads_here;
 #pragma unroll
     for (int ks = 0; ks < 8; ++ks) {
       const int c = (ks * 16 + c0) >> 1;
@@ -234,7 +247,7 @@ struct Attend {
 #pragma unroll
     for (int nb = 0; nb < 2; ++nb)
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
+      for (int e = 0; e < kE; ++e) {
         float v = s[nb][e] * scale2;
         if (a.soft_cap > 0.f) v = a.soft_cap * kLog2e * tanhf(s[nb][e] * a.sm_scale / a.soft_cap);
         const int pos = pos_base + nb * 8 + (e & 1);
@@ -244,7 +257,7 @@ struct Attend {
       }
     float alpha[2];
 #pragma unroll
-    for (int r = 0; r < 2; ++r) {
+    for (int r = 0; r < kR; ++r) {
       mx[r] = fmaxf(mx[r], __shfl_xor_sync(0xffffffffu, mx[r], 1));
       mx[r] = fmaxf(mx[r], __shfl_xor_sync(0xffffffffu, mx[r], 2));
       const float m_new = fmaxf(m_run[r], mx[r]);
@@ -252,21 +265,25 @@ struct Attend {
       m_run[r] = m_new;
     }
     float rs[2] = {0.f, 0.f};
-    uint32_t pf[4];
+    uint32_t pf[4], pl[4];
 #pragma unroll
     for (int nb = 0; nb < 2; ++nb) {
       float p[4];
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
+      for (int e = 0; e < kE; ++e) {
         const float mr = m_run[e >> 1];
         p[e] = mr == -INFINITY ? 0.f : exp2f(s[nb][e] - mr);
         rs[e >> 1] += p[e];
       }
-      pf[nb * 2 + 0] = pack2<kFp16>(p[0], p[1]);
-      pf[nb * 2 + 1] = pack2<kFp16>(p[2], p[3]);
+#pragma unroll
+      for (int r = 0; r < kR; ++r) {
+        pf[nb * 2 + r] = pack2<kFp16>(p[2 * r], p[2 * r + 1]);
+        const float2 f = unpack2<kFp16>(pf[nb * 2 + r]);
+        (kRows8 ? pf[nb * 2 + 1] : pl[nb * 2 + r]) = pack2<kFp16>(p[2 * r] - f.x, p[2 * r + 1] - f.y);
+      }
     }
 #pragma unroll
-    for (int r = 0; r < 2; ++r) {
+    for (int r = 0; r < kR; ++r) {
       rs[r] += __shfl_xor_sync(0xffffffffu, rs[r], 1);
       rs[r] += __shfl_xor_sync(0xffffffffu, rs[r], 2);
       l_run[r] = l_run[r] * alpha[r] + rs[r];
@@ -274,7 +291,7 @@ struct Attend {
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
       o[i][0] *= alpha[0]; o[i][1] *= alpha[0];
-      o[i][2] *= alpha[1]; o[i][3] *= alpha[1];
+      o[i][2] *= alpha[kR - 1]; o[i][3] *= alpha[kR - 1];
     }
     // ---- O += P V   (A = P: 16 heads x 16 positions, B = V: 16 positions x 128 dims)
 #pragma unroll
@@ -284,6 +301,10 @@ struct Attend {
       ldmatrix_x4_trans(vf, vs + tile_off<kTma>(p0 + (j & 1) * 8 + r, nb2 * 2 + (j >> 1)));
       mma16816<kFp16>(o[nb2 * 2], pf, vf[0], vf[1]);
       mma16816<kFp16>(o[nb2 * 2 + 1], pf, vf[2], vf[3]);
+      if constexpr (!kRows8) {
+        mma16816<kFp16>(o[nb2 * 2], pl, vf[0], vf[1]);
+        mma16816<kFp16>(o[nb2 * 2 + 1], pl, vf[2], vf[3]);
+      }
     }
   }
   // Merges the four warps (each saw a quarter of the positions) and writes the partial of the run. `sm_o` is 32 KB that
@@ -293,12 +314,16 @@ struct Attend {
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
       float* base = sm_o + (warp * 16) * kD + i * 8 + c0;
-      base[r0 * kD] = o[i][0]; base[r0 * kD + 1] = o[i][1];
-      base[(r0 + 8) * kD] = o[i][2]; base[(r0 + 8) * kD + 1] = o[i][3];
+      if constexpr (kRows8) {
+        base[r0 * kD] = o[i][0] + o[i][2]; base[r0 * kD + 1] = o[i][1] + o[i][3];
+      } else {
+        base[r0 * kD] = o[i][0]; base[r0 * kD + 1] = o[i][1];
+        base[(r0 + 8) * kD] = o[i][2]; base[(r0 + 8) * kD + 1] = o[i][3];
+      }
     }
     if ((lane & 3) == 0) {
       sm_ml[(warp * 16 + r0) * 2] = m_run[0]; sm_ml[(warp * 16 + r0) * 2 + 1] = l_run[0];
-      sm_ml[(warp * 16 + r0 + 8) * 2] = m_run[1]; sm_ml[(warp * 16 + r0 + 8) * 2 + 1] = l_run[1];
+      if constexpr (!kRows8) { sm_ml[(warp * 16 + r0 + 8) * 2] = m_run[1]; sm_ml[(warp * 16 + r0 + 8) * 2 + 1] = l_run[1]; }
     }
     ptx::named_barrier(1, kWarps * 32);
     const int tid = warp * 32 + lane;
@@ -334,7 +359,7 @@ struct Attend {
 // issues its load, so the four computing warps never wait for block-table lookups (with them in thread 0 of a computing warp, 16
 // boxes per tile at a page size of 16 took longer than the tile's bytes). The computing warps wait for a tile and hand
 // it back one by one, no barrier of the CTA per tile.
-template <bool kFp16>
+template <bool kFp16, bool kRows8>
 __global__ void __launch_bounds__(kWarps * 32 + 32, 2) decode_splitk_tma_kernel(const __grid_constant__ DecodeArgs a) {
   extern __shared__ __align__(128) uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -378,7 +403,7 @@ __global__ void __launch_bounds__(kWarps * 32 + 32, 2) decode_splitk_tma_kernel(
     }
     return;
   }
-  Attend<kFp16, true> at;
+  Attend<kFp16, true, kRows8> at;
   bool dead = false;                         // a wait ran out (recorded): walk on without data, so that no warp waits at a barrier for this one
   while (list.next(run)) {
     at.begin(a, run, lane);
@@ -413,7 +438,7 @@ __global__ void __launch_bounds__(kWarps * 32 + 32, 2) decode_splitk_tma_kernel(
 }
 
 // cp.async fill by the computing threads themselves: any page size.
-template <bool kFp16>
+template <bool kFp16, bool kRows8>
 __global__ void __launch_bounds__(kWarps * 32, 2) decode_splitk_kernel(const __grid_constant__ DecodeArgs a) {
   extern __shared__ __align__(128) uint8_t smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -425,7 +450,7 @@ __global__ void __launch_bounds__(kWarps * 32, 2) decode_splitk_kernel(const __g
   Run run;
   const uint32_t base = (uint32_t)__cvta_generic_to_shared(smem);
   const size_t pos_stride = (size_t)a.Hkv * kD;   // elements between consecutive positions of a page
-  Attend<kFp16, false> at;
+  Attend<kFp16, false, kRows8> at;
   while (list.next(run)) {
     const int32_t* bt = a.block_table + (size_t)run.b * a.max_blocks;
     auto issue_tile = [&](int t) {
@@ -607,8 +632,13 @@ __global__ void __launch_bounds__(kD) decode_local_finish_kernel(const float* pa
 template <bool kTma>
 int launch_splitk(DecodeArgs a, cudaStream_t s) {
   constexpr int smem = kTma ? kDecodeSmemTma : kDecodeSmem;
-  auto* kern = kTma ? (a.is_fp16 ? decode_splitk_tma_kernel<true> : decode_splitk_tma_kernel<false>)
-                    : (a.is_fp16 ? decode_splitk_kernel<true> : decode_splitk_kernel<false>);
+  auto pick = [&](auto fp16, auto rows8) -> void (*)(const DecodeArgs) {
+    return kTma ? decode_splitk_tma_kernel<decltype(fp16)::value, decltype(rows8)::value>
+                : decode_splitk_kernel<decltype(fp16)::value, decltype(rows8)::value>;
+  };
+  using Y = std::true_type;
+  using N = std::false_type;
+  auto* kern = a.is_fp16 ? (a.group <= 8 ? pick(Y{}, Y{}) : pick(Y{}, N{})) : (a.group <= 8 ? pick(N{}, Y{}) : pick(N{}, N{}));
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -20;
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);

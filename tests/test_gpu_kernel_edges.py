@@ -168,6 +168,36 @@ def test_decode_runs_cut_sequences_anywhere(ctx, tma, B, Hq, Hkv, page, lens):
     ctx.heap_release(mark)
 
 
+@pytest.mark.parametrize("tma", [None, False])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("soft_cap", [0.0, 30.0])
+@pytest.mark.parametrize("Hq,Hkv", [(2, 2), (16, 2), (18, 2), (32, 2)])
+def test_decode_is_exact_to_the_outputs_rounding(ctx, tma, dtype, soft_cap, Hq, Hkv):
+    """Every instantiation (fill, type, groups up to 8 heads and above) against 64 bits. P is held as a rounded value and its
+    remainder, so the output's rounding (u = 2^-8 or 2^-11 of it) is the error, plus 2^-14 of sum p |v| for the remainder's own
+    rounding (2^-16) and fp32 scores and sums: a tile or page that were taken for another would show."""
+    from iris_b200.models import FlashDecodeLayer
+
+    g = _gen(Hq)
+    lens, page = (700, 2500, 5000, 65), 16
+    B, L = len(lens), max(lens)
+    blocks = -(-L // page)
+    r = lambda *sh: torch.randn(*sh, device="cuda", generator=g).to(dtype)  # noqa: E731
+    q, k, v = r(B, Hq, 128), r(B * blocks, page, Hkv, 128), r(B * blocks, page, Hkv, 128)
+    table = torch.randperm(B * blocks, device="cuda", generator=g).to(torch.int32).view(B, blocks)
+    mark = ctx.heap_mark()
+    layer = FlashDecodeLayer(ctx, Hq, Hkv, max_batch=B, soft_cap=soft_cap, dtype=dtype, use_tma=tma)
+    out = layer(q, k, v, torch.tensor([lens], dtype=torch.int32, device="cuda"), table).double()
+    u = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+    for b, n in enumerate(lens):
+        kb, vb = (t[table[b].long()].reshape(-1, Hkv, 128)[:n].repeat_interleave(Hq // Hkv, dim=1).double() for t in (k, v))
+        s = torch.einsum("hd,khd->hk", q[b].double(), kb) * 128 ** -0.5
+        p = torch.softmax(soft_cap * torch.tanh(s / soft_cap) if soft_cap else s, -1)
+        want, size = torch.einsum("hk,khd->hd", p, vb), torch.einsum("hk,khd->hd", p, vb.abs())
+        assert ((out[b] - want).abs() <= 1.01 * u * want.abs() + 2.0 ** -14 * size).all()
+    ctx.heap_release(mark)
+
+
 # ------------------------------------------------------------------------------------ few rows
 @pytest.mark.parametrize("kmajor", [True, False])
 @pytest.mark.parametrize("M,N,K", [(1, 8, 8), (1, 1024, 64), (16, 136, 520), (17, 1032, 2048), (32, 3584, 72), (33, 264, 4096), (64, 2000, 3000),
