@@ -228,8 +228,8 @@ def _one_rank_direct(ctx, out, A, B, bias) -> bool:
     overlaps neither; anything else keeps the staged path, which copies."""
     if ctx.num_ranks != 1 or not (A.is_cuda and B.is_cuda and out.is_cuda) or not (A.dtype == B.dtype == out.dtype) or A.dtype not in _FUSED_DTYPES:
         return False
-    if A.dim() != 2 or out.dim() != 2 or A.stride(1) != 1 or out.stride(1) != 1 or 0 in out.shape or A.shape[1] == 0:
-        return False
+    if A.dim() != 2 or tuple(out.shape) != (A.shape[0], B.shape[1]) or A.stride(1) != 1 or out.stride(1) != 1 or 0 in out.shape or A.shape[1] == 0:
+        return False         # (the staged path's copy broadcasts one row into many)
     if (A.data_ptr() | out.data_ptr()) & 15 or (A.stride(0) | out.stride(0)) & 7 or out.stride(0) < out.shape[1]:
         return False
     lo, hi = _span(out)

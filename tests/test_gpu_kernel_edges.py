@@ -270,6 +270,17 @@ def test_one_rank_ops_take_any_row_count(ctx, T, D, F):
     assert ((x.double() - want).norm() / want.norm()).item() < 4e-3
 
 
+def test_one_rank_op_broadcasts_one_row(ctx):
+    """The result of one token is copied into an output of several rows, as by ``copy_``."""
+    g = _gen(5)
+    x = torch.randn(1, 256, device="cuda", generator=g).to(torch.bfloat16)
+    w = (torch.randn(256, 128, device="cuda", generator=g) * 256 ** -0.5).to(torch.bfloat16)
+    out = torch.zeros(5, 128, device="cuda", dtype=torch.bfloat16)
+    ctx.ops.all_gather_matmul(out, x, w, shard_dim=0)
+    want = (x.double() @ w.double()).expand(5, 128)
+    assert ((out.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-5).all()
+
+
 def test_quantiser_special_values():
     """Infinities saturate, NaN counts as -448 and does not move its block's scale, zeros stay zero, in every position of
     a lane and of a block."""
