@@ -104,8 +104,13 @@ def matmul(A: torch.Tensor, B: torch.Tensor, bias: torch.Tensor | None = None, o
     Bd, kmajor, ldb = b_layout(B)
     bv, bias16 = None, 0
     if bias is not None:         # read as it is when it has the operands' type, else as fp32
-        bias16 = 1 if bias.dtype == A.dtype else 0
-        bv = (bias if bias16 else bias.float()).contiguous()
+        bv = bias.contiguous() if bias.dtype == A.dtype else None
+        # (a bias inside the output, as in x = x_row + product, would be overwritten while other tiles still read it: its fp32 copy then)
+        lo = out.data_ptr()
+        if bv is not None and (bv.data_ptr() + 2 * bv.numel() <= lo or lo + 2 * ((M - 1) * out.stride(0) + N) <= bv.data_ptr()):
+            bias16 = 1
+        else:
+            bv = bias.float().contiguous()
     bp = bv.data_ptr() if bv is not None else 0
     desc, buf = _local_desc()
     _HEAD.pack_into(buf, 0, _lib.GEMM_LOCAL, M, N, K, _lib.DTYPE_CODE[A.dtype], kmajor, bn, 0, 0, 0, 0,

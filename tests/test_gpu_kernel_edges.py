@@ -270,6 +270,22 @@ def test_one_rank_ops_take_any_row_count(ctx, T, D, F):
     assert ((x.double() - want).norm() / want.norm()).item() < 4e-3
 
 
+@pytest.mark.parametrize("M,N,K", [(16, 3584, 512), (256, 4096, 2816), (300, 1000, 256), (2048, 2048, 64)])
+def test_bias_inside_the_output(M, N, K):
+    """A bias that is a row or a column of the output is read before the output is written: same bits as with a copy of it."""
+    from iris_b200.ops import matmul
+
+    g = _gen(M + N)
+    A = torch.randn(M, K, device="cuda", generator=g).to(torch.bfloat16)
+    B = (torch.randn(K, N, device="cuda", generator=g) * K ** -0.5).to(torch.bfloat16)
+    out0 = torch.randn(M, N, device="cuda", generator=g).to(torch.bfloat16)
+    for dim, pick in ((1, lambda t: t[0]), (1, lambda t: t[M - 1]), (0, lambda t: t[:, N - 1]), (0, lambda t: t[:, 0])):
+        for _ in range(3):
+            out = out0.clone()
+            want = matmul(A, B, bias=pick(out).clone(), bias_dim=dim)
+            assert torch.equal(matmul(A, B, bias=pick(out), bias_dim=dim, out=out), want)
+
+
 def test_one_rank_op_broadcasts_one_row(ctx):
     """The result of one token is copied into an output of several rows, as by ``copy_``."""
     g = _gen(5)
