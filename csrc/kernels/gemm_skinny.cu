@@ -218,12 +218,12 @@ int iris_gemm_skinny_split(int M, int N, int K) {
 //             2000 x 3000  22.0 / 17.1    3584 x 4096  18.5 / 17.4    3584 x 8192  32.1 / 23.5
 // It pays while K is long against N (the main loop's few CTAs walk all of it) and its partial tiles, which grow with M,
 // stay small.
-// A tile that the caller of the local GEMM asked for is honoured; a fused op on one rank carries the tile of its
-// workspace's plan, which binds nobody there.
-bool iris_gemm_skinny_takes(const IrisGemmDesc* d) {
-  if (d->op == IRIS_GEMM_LOCAL && (d->bn != 0 || d->two_sm != 0)) return false;
-  if (d->timeline || (d->in_dtype != 0 && d->in_dtype != d->dtype)) return false;
-  if (d->M <= 32) return true;
+// A tile that the caller asked for is honoured; a fused op on one rank otherwise carries the tile of its workspace's
+// plan, which binds nobody there.
+extern "C" int iris_gemm_skinny_takes(const IrisGemmDesc* d) {
+  if (d->op == IRIS_GEMM_LOCAL ? d->bn != 0 || d->two_sm != 0 : d->tile_asked != 0) return 0;
+  if (d->timeline || (d->in_dtype != 0 && d->in_dtype != d->dtype)) return 0;
+  if (d->M <= 32) return 1;
   if (d->M <= 64) return d->K >= 2048 || d->N <= 4096;
   return d->M <= 256 && d->K >= (d->M <= 128 ? 2048 : 2816) && 2ll * d->K >= d->N && (int64_t)d->M * d->N <= (1 << 20);
 }

@@ -87,6 +87,8 @@ typedef struct IrisGemmDesc {
   int32_t overlap;
   // 0: bias_row / bias_col are fp32; 1: they have the output's 16-bit type (IRIS_GEMM_LOCAL)
   int32_t bias16;
+  // 1: bn or two_sm is the caller's own choice, not a plan's (fused ops; IRIS_GEMM_LOCAL carries nothing else there)
+  int32_t tile_asked;
 } IrisGemmDesc;
 
 // Block-scaled fp8 (e4m3) GEMM: C = (A * scale_a) @ (B * scale_b)^T with A [M, K] and B [N, K]

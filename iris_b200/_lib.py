@@ -70,6 +70,7 @@ class IrisGemmDesc(C.Structure):
         ("sf_inbox", C.c_void_p),
         ("overlap", C.c_int32),
         ("bias16", C.c_int32),
+        ("tile_asked", C.c_int32),
     ]
 
 
@@ -111,6 +112,8 @@ def kernels() -> C.CDLL:
             lib.iris_gemm_workspace.restype = C.c_int
             lib.iris_gemm_sf_inbox_bytes.argtypes = [C.POINTER(IrisGemmDesc)]
             lib.iris_gemm_sf_inbox_bytes.restype = C.c_uint64
+            lib.iris_gemm_skinny_takes.argtypes = [C.POINTER(IrisGemmDesc)]
+            lib.iris_gemm_skinny_takes.restype = C.c_int
             _kernels = lib
         return _kernels
 

@@ -93,6 +93,7 @@ def _base_desc(ctx, op, M, N, K, A, B, out, config, bias_row=None, bias_col=None
     d.group_m = config.group_size_m
     d.comm_ctas = config.comm_sms
     d.two_sm = 0 if config.two_sm is None else (2 if config.two_sm else 1)
+    d.tile_asked = 1 if config.tile_n() or config.two_sm is not None else 0
     d.use_mc = 1 if (config.use_multicast and ctx.has_multicast()) else 0
     d.overlap = 1 if config.overlap in ("wg_specialized", "producer_consumer") else 0
     d.ctx = ctx.ctx_struct()
@@ -129,6 +130,7 @@ def _make_workspace(ctx, operation, shape, dtype, variant, d) -> FusedWorkspace 
     ws.extra["comm_ctas"] = d.comm_ctas
     # the staging layout depends on the tile (width, single CTA or CTA pair): pinned with the buffers
     ws.extra["two_sm"] = 2 if pair else 1
+    ws.extra["tile_asked"] = d.tile_asked
     ctx.barrier()
     return ws
 
@@ -207,6 +209,7 @@ def _launch(ctx, d, ws) -> None:
     d.sf_inbox = sfi.data_ptr() if sfi is not None else None
     d.comm_ctas = ws.extra.get("comm_ctas", d.comm_ctas)
     d.two_sm = ws.extra.get("two_sm", d.two_sm)
+    d.tile_asked = ws.extra.get("tile_asked", d.tile_asked)
     tl = ws.extra.get("timeline")
     d.timeline = tl.data_ptr() if tl is not None else None
     if _artifacts.ACTIVE:

@@ -270,6 +270,33 @@ def test_one_rank_ops_take_any_row_count(ctx, T, D, F):
     assert ((x.double() - want).norm() / want.norm()).item() < 4e-3
 
 
+@pytest.mark.parametrize("config", [{}, {"block_size_n": 128}, {"block_size_n": 100}, {"two_sm": False}, {"two_sm": True}])
+def test_one_rank_op_keeps_the_tile_it_is_asked_for(ctx, config):
+    """128 rows go to the few-row kernel unless the config names a tile (100 is none of the kernel's widths: the plan's choice), also when
+    only the workspace was made with it."""
+    import ctypes as C
+
+    from iris_b200 import _lib
+    from iris_b200.ops import FusedConfig, all_gather_matmul_preamble
+
+    cfg = FusedConfig(**config)
+    asked = bool(config) and config.get("block_size_n") != 100
+    g = _gen(9)
+    x = torch.randn(128, 2048, device="cuda", generator=g).to(torch.bfloat16)
+    w = (torch.randn(1024, 2048, device="cuda", generator=g) * 2048 ** -0.5).to(torch.bfloat16).t()
+    want = x.double() @ w.double()
+    mark = ctx.heap_mark()
+    for first, then in ((cfg, cfg), (cfg, None)):
+        out = torch.empty(128, 1024, device="cuda", dtype=torch.bfloat16)
+        ws = all_gather_matmul_preamble(ctx, x, w, first, shard_dim=0)
+        ctx.ops.all_gather_matmul(out, x, w, shard_dim=0, config=first, workspace=ws)
+        ctx.ops.all_gather_matmul(out, x, w, shard_dim=0, config=then, workspace=ws)
+        (d, _), = ws.extra["desc"].values()
+        assert ws.variant == "fused" and bool(_lib.kernels().iris_gemm_skinny_takes(C.byref(d))) == (not asked)
+        assert ((out.double() - want).abs() <= 1.01 * 2.0 ** -8 * want.abs() + 1e-4).all()
+    ctx.heap_release(mark)
+
+
 @pytest.mark.parametrize("M,N,K", [(16, 3584, 512), (256, 4096, 2816), (300, 1000, 256), (2048, 2048, 64)])
 def test_bias_inside_the_output(M, N, K):
     """A bias that is a row or a column of the output is read before the output is written: same bits as with a copy of it."""
