@@ -47,7 +47,7 @@ extra = [int(x) for x in os.environ.get("DIAG_COMM", "").split(",") if x]
 for cc in extra:
     variants += [(cc, True)]
 for comm, mc in variants:
-    cfg = FusedConfig(comm_sms=comm, use_multicast=mc)
+    cfg = FusedConfig(comm_sms=comm, use_multicast=mc, one_rank_fused=True)
     ws = ctx.ops.all_gather_matmul(C, A, B, shard_dim=0, config=cfg)
     ms = timed(lambda: ctx.ops.all_gather_matmul(C, A, B, shard_dim=0, workspace=ws, config=cfg, async_op=True))
     pair = ws.extra.get("two_sm", 1) == 2
@@ -77,7 +77,7 @@ for comm, mc in variants:
 M, Kl, N2 = 8192, 3584, 8192
 A2 = torch.randn(M, Kl, device="cuda", dtype=dtype); B2 = (torch.randn(N2, Kl, device="cuda", dtype=dtype) * 0.02).t()
 C2 = ctx.zeros((M // W, N2), dtype=dtype)
-ws2 = ctx.ops.matmul_reduce_scatter(C2, A2, B2, scatter_rows=True)
+ws2 = ctx.ops.matmul_reduce_scatter(C2, A2, B2, scatter_rows=True, config=FusedConfig(one_rank_fused=True))
 ms = timed(lambda: ctx.ops.matmul_reduce_scatter(C2, A2, B2, scatter_rows=True, workspace=ws2, async_op=True))
 pair = ws2.extra.get("two_sm", 1) == 2
 tiles128 = 64 * (N2 // ws2.bn); order_tiles = tiles128 // 2 if pair else tiles128

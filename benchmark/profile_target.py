@@ -14,7 +14,7 @@
     python benchmark/profile_target.py moe_full  # two passes of the benchmark-size MoE layer (4096 tokens, hidden 7168, 32 experts, top-8):
     python benchmark/profile_target.py moe_fp8_full   # for a launch list (`--metrics gpu__time_duration.sum`, one pass) only, about 6 GB held
 
-The fused ops and collectives run here with ONE rank: the same kernel templates as on several GPUs
+The fused ops (with `one_rank_fused`) and collectives run here with ONE rank: the same kernel templates as on several GPUs
 (policy code, epilogues, flag protocol) with no peer to wait for, which is the form a replaying
 profiler can capture safely.
 """
@@ -79,9 +79,9 @@ def main():
         C = ctx.zeros((4096, 8192), dtype=dt)
         for variant in ("two_shot", "one_shot"):
             for _ in range(2):
-                ctx.ops.matmul_all_reduce(C, A, B, config=FusedConfig(all_reduce_variant=variant), async_op=True)
+                ctx.ops.matmul_all_reduce(C, A, B, config=FusedConfig(all_reduce_variant=variant, one_rank_fused=True), async_op=True)
         for _ in range(2):
-            ctx.ops.matmul_all_gather(C, A, B, async_op=True)
+            ctx.ops.matmul_all_gather(C, A, B, config=FusedConfig(one_rank_fused=True), async_op=True)
     elif what == "ccl":
         x = ctx.zeros((8192, 16384), dtype=dt)            # 256 MB
         y = ctx.zeros((8192, 16384), dtype=dt)
@@ -113,14 +113,17 @@ def main():
         for _ in range(3):
             layer(q, k, v, causal=False)
     elif what == "fused":
+        from iris_b200.ops import FusedConfig
+
+        own = FusedConfig(one_rank_fused=True)
         X = torch.randn(4096, 8192, device="cuda", dtype=dt)
         W1 = torch.randn(8192, 3584, device="cuda", dtype=dt) * 0.02
         W2 = torch.randn(3584, 8192, device="cuda", dtype=dt) * 0.02
         H = torch.empty(4096, 3584, device="cuda", dtype=dt)
         Y = torch.empty(4096, 8192, device="cuda", dtype=dt)
         for _ in range(2):
-            ctx.ops.all_gather_matmul(H, X, W1, shard_dim=0, async_op=True)
-            ctx.ops.matmul_reduce_scatter(Y, H, W2, scatter_rows=True, async_op=True)
+            ctx.ops.all_gather_matmul(H, X, W1, shard_dim=0, config=own, async_op=True)
+            ctx.ops.matmul_reduce_scatter(Y, H, W2, scatter_rows=True, config=own, async_op=True)
     elif what in ("moe", "moe_fp8", "moe_full", "moe_fp8_full"):
         from iris_b200.models import MoELayer
 

@@ -1047,8 +1047,8 @@ extern "C" int iris_gemm_launch(const IrisGemmDesc* d, void* stream_) {
   DeviceContext ctx;
   memcpy(&ctx, &d->ctx, sizeof(ctx));
 
-  // One rank: gathering and reducing over ranks is the identity, and every op is a local GEMM.
-  if (d->op == IRIS_GEMM_LOCAL || ctx.world <= 1) {
+  // One rank: gathering and reducing over ranks is the identity, and every op is a local GEMM unless its own kernel is asked for.
+  if (d->op == IRIS_GEMM_LOCAL || (ctx.world <= 1 && !d->one_rank_fused)) {
     if (iris_gemm_skinny_takes(d)) return iris_gemm_skinny(d, stream);
     LocalGemm pol;
     r = fill_common(pol, d, p.bn, p.pair, p.gemm_ctas, d->A, d->M, d->K, d->lda);

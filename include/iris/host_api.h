@@ -89,6 +89,8 @@ typedef struct IrisGemmDesc {
   int32_t bias16;
   // 1: bn or two_sm is the caller's own choice, not a plan's (fused ops; IRIS_GEMM_LOCAL carries nothing else there)
   int32_t tile_asked;
+  // 1: the op's own kernel with one rank too (else a local GEMM), on a workspace that was made with this set
+  int32_t one_rank_fused;
 } IrisGemmDesc;
 
 // Block-scaled fp8 (e4m3) GEMM: C = (A * scale_a) @ (B * scale_b)^T with A [M, K] and B [N, K]

@@ -71,6 +71,7 @@ class IrisGemmDesc(C.Structure):
         ("overlap", C.c_int32),
         ("bias16", C.c_int32),
         ("tile_asked", C.c_int32),
+        ("one_rank_fused", C.c_int32),
     ]
 
 

@@ -93,6 +93,7 @@ def _base_desc(ctx, op, M, N, K, A, B, out, config, bias_row=None, bias_col=None
     d.group_m = config.group_size_m
     d.comm_ctas = config.comm_sms
     d.two_sm = 0 if config.two_sm is None else (2 if config.two_sm else 1)
+    d.one_rank_fused = 1 if config.one_rank_fused else 0
     d.tile_asked = 1 if config.tile_n() or config.two_sm is not None else 0
     d.use_mc = 1 if (config.use_multicast and ctx.has_multicast()) else 0
     d.overlap = 1 if config.overlap in ("wg_specialized", "producer_consumer") else 0
@@ -114,16 +115,17 @@ def _make_workspace(ctx, operation, shape, dtype, variant, d) -> FusedWorkspace 
         return None
     ws = FusedWorkspace(operation=operation, shape=tuple(shape), dtype=dtype, world_size=ctx.num_ranks, variant=variant, bn=bn)
     ws.sync_block = ctx.zeros(80, dtype=torch.int32)
-    if inbox:
+    own_kernel = ctx.num_ranks > 1 or d.one_rank_fused       # a local GEMM needs no buffers
+    if inbox and own_kernel:
         ws.inbox = ctx.heap.allocate(inbox, torch.uint8)
-    if flags:
+    if flags and own_kernel:
         ws.flags = ctx.zeros(flags // 4, dtype=torch.int32)
         ws.locks = ws.flags
-    if staging:
+    if staging and own_kernel:
         ws.staging = ctx.heap.allocate(staging, torch.uint8)
         ws.aux_buffer = ws.staging
     sf_inbox = int(_lib.kernels().iris_gemm_sf_inbox_bytes(C.byref(d)))
-    if sf_inbox:        # fp8 all-gather: the gathered shards' scale atoms
+    if sf_inbox and own_kernel:        # fp8 all-gather: the gathered shards' scale atoms
         ws.extra["sf_inbox"] = ctx.heap.allocate(sf_inbox, torch.uint8)
     ws.prepared = True
     # arrival counters count communication CTAs: the number used at creation is part of the workspace
@@ -131,6 +133,7 @@ def _make_workspace(ctx, operation, shape, dtype, variant, d) -> FusedWorkspace 
     # the staging layout depends on the tile (width, single CTA or CTA pair): pinned with the buffers
     ws.extra["two_sm"] = 2 if pair else 1
     ws.extra["tile_asked"] = d.tile_asked
+    ws.extra["one_rank_fused"] = d.one_rank_fused
     ctx.barrier()
     return ws
 
@@ -140,7 +143,7 @@ def _auto_workspace(ctx, operation, key, dtype, config, make, extra=None):
     dtype, tile configuration) and kept on the context, so a loop that calls an op without passing
     the returned workspace back does not allocate heap memory (and run a barrier) on every call."""
     cache = ctx.__dict__.setdefault("_ops_workspaces", {})
-    ck = (operation, tuple(key), dtype, config.tile_n(), config.two_sm, config.comm_sms, config.use_multicast, config.overlap, extra)
+    ck = (operation, tuple(key), dtype, config.tile_n(), config.two_sm, config.comm_sms, config.use_multicast, config.overlap, config.one_rank_fused, extra)
     ws = cache.get(ck)
     if ws is None:
         ws = cache[ck] = make()
@@ -210,6 +213,7 @@ def _launch(ctx, d, ws) -> None:
     d.comm_ctas = ws.extra.get("comm_ctas", d.comm_ctas)
     d.two_sm = ws.extra.get("two_sm", d.two_sm)
     d.tile_asked = ws.extra.get("tile_asked", d.tile_asked)
+    d.one_rank_fused = ws.extra.get("one_rank_fused", 0)
     tl = ws.extra.get("timeline")
     d.timeline = tl.data_ptr() if tl is not None else None
     if _artifacts.ACTIVE:

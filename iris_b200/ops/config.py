@@ -32,6 +32,8 @@ class FusedConfig:
     #   "bulk_synchronous"  GEMM kernel, then the all-gather kernel (example 12)
     overlap: str = "fused"
     allow_tf32: bool = True
+    # with one rank an op is a local GEMM; True runs its own kernel there too, communication code included (captures, tests)
+    one_rank_fused: bool = False
 
     def __post_init__(self):
         if self.block_size_m <= 0 or self.block_size_k <= 0 or self.block_size_n < 0:

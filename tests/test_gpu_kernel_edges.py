@@ -270,6 +270,33 @@ def test_one_rank_ops_take_any_row_count(ctx, T, D, F):
     assert ((x.double() - want).norm() / want.norm()).item() < 4e-3
 
 
+@pytest.mark.parametrize("fp8", [False, True])
+@pytest.mark.parametrize("op,kw", [("all_gather_matmul", {"shard_dim": 0}), ("all_gather_matmul", {"shard_dim": 1}), ("matmul_all_gather", {}),
+                                   ("matmul_all_gather", {"scatter_cols": True}), ("matmul_all_reduce", {}), ("matmul_reduce_scatter", {"scatter_rows": True}),
+                                   ("matmul_reduce_scatter", {})])
+def test_fused_kernels_on_one_rank(ctx, op, kw, fp8):
+    """With ``one_rank_fused`` an op's own kernel runs on one rank (its policy, epilogue, flags and double-buffered workspace), else
+    a local GEMM, whose workspace reserves nothing on the heap but the sync block; both round one fp32 sum."""
+    from iris_b200.ops import FusedConfig, quantize_activation, quantize_weight
+
+    g = _gen(11)
+    x = torch.randn(384, 512, device="cuda", generator=g)
+    w = torch.randn(640, 512, device="cuda", generator=g) * 512 ** -0.5
+    a, b = (quantize_activation(x), quantize_weight(w)) if fp8 else (x.to(torch.bfloat16), w.to(torch.bfloat16).t())
+    ref = a.dequantize().double() @ b.dequantize().double() if fp8 else a.double() @ b.double()
+    out = ctx.zeros((384, 640), dtype=torch.bfloat16)
+    for variant in ("two_shot", "one_shot", "atomic") if op == "matmul_all_reduce" else ("auto",):
+        for own in (True, False):
+            ws = None
+            for _ in range(3 if own else 1):
+                out.zero_()
+                ws = getattr(ctx.ops, op)(out, a, b, workspace=ws, config=FusedConfig(one_rank_fused=own, all_reduce_variant=variant), **kw)
+                assert ws.variant == "fused" and bool(ws.extra["one_rank_fused"]) == own
+                assert ((out.double() - ref).abs() <= 1.01 * 2.0 ** -8 * ref.abs() + 1e-4).all()
+            assert own or (ws.inbox is None and ws.flags is None and ws.staging is None)
+    ctx.check()
+
+
 @pytest.mark.parametrize("config", [{}, {"block_size_n": 128}, {"block_size_n": 100}, {"two_sm": False}, {"two_sm": True}])
 def test_one_rank_op_keeps_the_tile_it_is_asked_for(ctx, config):
     """128 rows go to the few-row kernel unless the config names a tile (100 is none of the kernel's widths: the plan's choice), also when
