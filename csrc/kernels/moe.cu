@@ -624,6 +624,9 @@ typedef struct IrisMoeDesc {
   const void* x16;          // one rank, e4m3: the bf16 tokens [T, D], quantised on the way into the inbox (x and x_sf are not read)
 } IrisMoeDesc;
 
+// One rank: up to this many tokens a call is 5 kernels, above it 8.
+int iris_moe_prep_max_tokens(void) { return kPrepMaxTokens; }
+
 int iris_moe_forward(const IrisMoeDesc* d, void* stream_) {
   cudaStream_t s = (cudaStream_t)stream_;
   if (d->K > kMaxTopK || d->E > 1024 || d->E % d->ctx.world || d->D % 64 || d->F % 128 || d->D % 256 || d->K > d->E || d->K < 1) return -3;

@@ -146,8 +146,9 @@ class MoELayer:
         self.inbox_sf.fill_(127)
         self.H = torch.zeros(self.capacity, F, dtype=u8, device=dev)
         self.H_sf = torch.full((self.capacity, self.sf_ld2), 127, dtype=u8, device=dev)
-        self.xq = torch.zeros(self.T, D, dtype=u8, device=dev)                   # the tokens as they are sent (one rank quantises in its gather)
-        self.x_sf = torch.full((self.T, self.sf_ld1), 127, dtype=u8, device=dev)
+        one_rank = ctx.get_num_ranks() == 1                                      # quantises in its gather
+        self.xq = None if one_rank else torch.zeros(self.T, D, dtype=u8, device=dev)      # the tokens as they are sent
+        self.x_sf = None if one_rank else torch.full((self.T, self.sf_ld1), 127, dtype=u8, device=dev)
         del self.w13, self.w2
 
     def _quantise_tokens(self, x) -> None:
@@ -194,9 +195,10 @@ class MoELayer:
                 d.x16 = x.data_ptr()
             else:
                 self._quantise_tokens(x)
+                d.x, d.x_sf = self.xq.data_ptr(), self.x_sf.data_ptr()
             d.fp8, d.sf_ld1, d.sf_ld2 = 1, self.sf_ld1, self.sf_ld2
-            d.x, d.w13, d.w2 = self.xq.data_ptr(), self.w13_q.data_ptr(), self.w2_q.data_ptr()
-            d.x_sf, d.inbox_sf, d.H_sf = self.x_sf.data_ptr(), self.inbox_sf.data_ptr(), self.H_sf.data_ptr()
+            d.w13, d.w2 = self.w13_q.data_ptr(), self.w2_q.data_ptr()
+            d.inbox_sf, d.H_sf = self.inbox_sf.data_ptr(), self.H_sf.data_ptr()
             d.w13_sf, d.w2_sf = self.w13_sf.data_ptr(), self.w2_sf.data_ptr()
         else:
             d.x, d.w13, d.w2 = x.data_ptr(), self.w13.data_ptr(), self.w2.data_ptr()
@@ -208,8 +210,9 @@ class MoELayer:
             setattr(d, name, getattr(self, name).data_ptr())
         d.weights_kmajor = 1
         d.pos_of = self.pos_of.data_ptr() if one_rank else None
-        _lib.check(self._lib().iris_moe_forward(C.byref(d), C.c_void_p(_lib.current_stream_ptr())), "MoE forward launch",
-                   kernels=7 if not one_rank else (5 if T <= 256 else 8))
+        lib = self._lib()
+        _lib.check(lib.iris_moe_forward(C.byref(d), C.c_void_p(_lib.current_stream_ptr())), "MoE forward launch",
+                   kernels=7 if not one_rank else (5 if T <= lib.iris_moe_prep_max_tokens() else 8))
         self._keep = logits
         return out
 

@@ -100,6 +100,28 @@ def test_moe_one_rank_router_sort_gather(ctx, T, E, K):
     ctx.heap_release(mark)
 
 
+@pytest.mark.parametrize("T", [256, 257])
+def test_moe_e4m3_one_rank_preparation(ctx, T):
+    """Both sides of the one-block preparation's limit, the kernels each is counted for, and no buffers for tokens that nobody
+    sends. x, weights and hidden activations in e4m3 (4 significant bits, 2^-4 / sqrt(3) each): in sum below 0.1 of the
+    output's 2-norm."""
+    from iris_b200 import _lib
+    from iris_b200.models import MoELayer, reference_moe
+
+    E, D, F, K = 8, 256, 128, 2
+    wg, wu, wd = _moe_weights(E, D, F, T)
+    mark = ctx.heap_mark()
+    layer = MoELayer(ctx, D, F, E, K, max_tokens=T, w_gate=wg, w_up=wu, w_down=wd, fp8=True)
+    x = torch.randn(T, D, device="cuda", generator=_gen(T)).to(torch.bfloat16)
+    logits = torch.randn(T, E, device="cuda", generator=_gen(T + 1))
+    before = _lib.LAUNCHES.get("MoE forward launch", 0)
+    y = layer(x, logits)
+    assert _lib.LAUNCHES["MoE forward launch"] - before == (5 if T <= _lib.kernels().iris_moe_prep_max_tokens() else 8) == (5 if T == 256 else 8)
+    want = reference_moe(x, logits, wg, wu, wd, K)
+    assert ((y.float() - want).norm() / want.norm()).item() < 0.1 and layer.xq is None and layer.x_sf is None
+    ctx.heap_release(mark)
+
+
 # ------------------------------------------------------------------------------------ attention on one rank
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("S,Hq,Hkv", [(1, 2, 2), (64, 4, 2), (127, 8, 2), (128, 3, 1), (129, 4, 4), (257, 6, 2), (384, 5, 5), (1000, 8, 8), (2500, 16, 2),
