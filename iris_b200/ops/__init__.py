@@ -233,17 +233,23 @@ def _one_rank_direct(ctx, out, A, B, bias) -> bool:
     """One rank, a shape outside the fused kernels' tiles (rows not a multiple of 128): the op is a local GEMM, and it can
     write ``out`` itself when the operands are what the kernel takes as they lie (16-byte aligned rows) and ``out``
     overlaps neither; anything else keeps the staged path, which copies."""
-    if ctx.num_ranks != 1 or not (A.is_cuda and B.is_cuda and out.is_cuda) or not (A.dtype == B.dtype == out.dtype) or A.dtype not in _FUSED_DTYPES:
+    dt = A.dtype
+    if ctx.num_ranks != 1 or dt not in _FUSED_DTYPES or B.dtype != dt or out.dtype != dt or not (A.is_cuda and B.is_cuda and out.is_cuda):
         return False
-    if A.dim() != 2 or tuple(out.shape) != (A.shape[0], B.shape[1]) or A.stride(1) != 1 or out.stride(1) != 1 or 0 in out.shape or A.shape[1] == 0:
-        return False         # (the staged path's copy broadcasts one row into many)
-    if (A.data_ptr() | out.data_ptr()) & 15 or (A.stride(0) | out.stride(0)) & 7 or out.stride(0) < out.shape[1]:
+    M, K = A.shape                                 # (A and B are matrices with one inner dimension: checked by the op)
+    N = B.shape[1]
+    if out.shape != (M, N) or not (M and N and K):
+        return False                               # the staged path's copy broadcasts one row into many
+    (lda, ka), (ldc, nc), (kb, nb) = A.stride(), out.stride(), B.stride()
+    a, b, lo = A.data_ptr(), B.data_ptr(), out.data_ptr()
+    if ka != 1 or nc != 1 or (a | lo) & 15 or (lda | ldc) & 7 or ldc < N:
         return False
-    lo, hi = _span(out)
-    for t in (A, B) if bias is None else (A, B, bias):
-        a, b = _span(t)
-        if a < hi and lo < b:
-            return False
+    hi = lo + 2 * ((M - 1) * ldc + N)
+    if (a < hi and lo < a + 2 * ((M - 1) * lda + K)) or (b < hi and lo < b + 2 * ((K - 1) * kb + (N - 1) * nb + 1)):
+        return False
+    if bias is not None:
+        first, last = _span(bias)
+        return first >= hi or lo >= last
     return True
 
 
