@@ -620,7 +620,7 @@ __global__ void __launch_bounds__(kD) decode_exchange_kernel(const __grid_consta
 __global__ void __launch_bounds__(kD) decode_local_finish_kernel(const float* partial, void* out, float* out_lse, int splits, int is_fp16) {
   const int it = blockIdx.x, d = threadIdx.x;
   __shared__ float s_part[kD];
-  asm volatile("griddepcontrol.wait;" ::: "memory");      // launched early: the partials are complete from here on
+  asm volatile("griddepcontrol.wait;" ::: "memory");      // the partials are complete from here on
   float o, lse;
   combine_splits(partial + (size_t)it * splits * (kD + 1), splits, s_part, o, lse);
   if (is_fp16) ((__half*)out)[(size_t)it * kD + d] = __float2half_rn(o);
@@ -722,7 +722,8 @@ int iris_flash_decode(const IrisDecodeDesc* d, void* stream) {
   if (r) return r;
   if (!d->exchange) return 0;
   if (d->exchange == 2 || d->ctx.world <= 1) {
-    // programmatic launch: the blocks are placed while the split-K kernel drains and wait for it in the kernel
+    // programmatic launch: hides the launch latency (the split-K kernel issues no launch_dependents, so these blocks are placed
+    // when its last one has exited, not while it drains)
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(d->B * d->Hq, 1, 1);
     cfg.blockDim = dim3(kD, 1, 1);

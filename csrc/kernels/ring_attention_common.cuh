@@ -152,7 +152,8 @@ __device__ __forceinline__ void finish_call(const RingArgs& a, int call) {
 }
 
 // Launches the kernel whose attention CTAs use tcgen05 (ring_attention_tc.cu). Returns 1 when the
-// call is not covered (a tensor that is not 16-byte aligned), 0 on success, < 0 on a launch error.
+// call is left to the mma.sync CTAs (a tensor that is not 16-byte aligned; one rank, contiguous layout, at most 128 tokens), 0 on success,
+// < 0 on a launch error.
 int launch_ring_attention_tc(const RingArgs& a, cudaStream_t stream);
 
 }  // namespace iris_ring

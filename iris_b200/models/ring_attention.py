@@ -5,8 +5,8 @@ Every rank holds ``S`` consecutive tokens of the sequence: queries ``[S, Hq, D]`
 output of attention over the WHOLE sequence. One kernel per call: communication CTAs pass the K/V
 blocks round the ring with bulk copies and per-block arrival counters on the heap, attention CTAs
 consume the blocks as they arrive. The attention CTAs run on tcgen05 with TMEM accumulators and
-TMA-fed tiles (``csrc/kernels/ring_attention_tc.cu``), with ``use_tcgen05=False`` on ``mma.sync``
-(``csrc/kernels/ring_attention.cu``). The reference has no
+TMA-fed tiles (``csrc/kernels/ring_attention_tc.cu``); with ``use_tcgen05=False``, for tensors off a 16-byte boundary and for
+up to 128 tokens on one rank (contiguous layout) on ``mma.sync`` (``csrc/kernels/ring_attention.cu``). The reference has no
 counterpart; ``reference_attention`` is the plain fp32 PyTorch statement used by the tests.
 """
 from __future__ import annotations
@@ -71,7 +71,7 @@ class RingAttention:
         self.ctx, self.S, self.Hq, self.Hkv, self.D = ctx, seq_per_rank, num_q_heads, num_kv_heads, head_dim
         self.sm_scale = sm_scale if sm_scale is not None else 1.0 / math.sqrt(head_dim)
         self.comm_sms, self.dtype = comm_sms, dtype
-        # None: the tcgen05 attention CTAs; False: the mma.sync CTAs
+        # None: the tcgen05 attention CTAs where they take the call (see the module's head); False: the mma.sync CTAs
         self.use_tcgen05 = use_tcgen05
         # "contiguous": rank r holds tokens [r*S, (r+1)*S); "zigzag": chunks r and 2W-1-r of 2W chunks
         # (see zigzag_positions), which balances causal attention over the ranks

@@ -496,7 +496,7 @@ def _ring(rank, world):
     Hq, Hkv, D = 8, 2, 128
     dt = torch.bfloat16
     torch.manual_seed(30 + rank)
-    for S in (192, 256):          # 192: mma.sync attention CTAs, 256: tcgen05 attention CTAs
+    for S, tc in ((192, None), (256, None), (192, False)):          # the tcgen05 attention CTAs with and without a ragged tile, the mma.sync ones
         q = torch.randn(S, Hq, D, device="cuda", dtype=dt)
         k = torch.randn(S, Hkv, D, device="cuda", dtype=dt)
         v = torch.randn(S, Hkv, D, device="cuda", dtype=dt)
@@ -504,12 +504,12 @@ def _ring(rank, world):
         vs = torch.empty(world * S, Hkv, D, device="cuda", dtype=dt)
         dist.all_gather_into_tensor(ks, k)
         dist.all_gather_into_tensor(vs, v)
-        layer = RingAttention(ctx, S, Hq, Hkv)
+        layer = RingAttention(ctx, S, Hq, Hkv, use_tcgen05=tc)
         for causal in (False, True):
             for _ in range(3):
                 out = layer(q, k, v, causal=causal)
             ref = reference_attention(q, ks, vs, causal, q_offset=rank * S)
-            assert (out.float() - ref).abs().max().item() < 2e-2, (S, causal)
+            assert (out.float() - ref).abs().max().item() < 2e-2, (S, tc, causal)
         ctx.check()
     ctx.barrier()
 

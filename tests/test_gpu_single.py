@@ -212,7 +212,7 @@ def test_fused_ops_world1(ctx):
                    ("matmul_all_reduce", {}), ("matmul_reduce_scatter", {"scatter_rows": True}), ("matmul_reduce_scatter", {})):
         C = ctx.zeros((384, 640), dtype=dt)
         ws = None
-        for _ in range(3):                       # repeated calls reuse the double-buffered workspace
+        for _ in range(3):                       # repeated calls reuse the workspace (one rank: a local GEMM)
             ws = getattr(ctx.ops, op)(C, A, B, workspace=ws, **kw)
         assert ws.variant == "fused", op
         assert _rel_err(C, ref) < 1e-2, op
@@ -338,7 +338,7 @@ def test_activation_quantiser_kernel(M, K, dtype):
 
 
 def test_fp8_fused_ops_world1(ctx):
-    """The fused ops with block-scaled e4m3 operands (one rank: same kernels, no peers)."""
+    """The fused ops with block-scaled e4m3 operands (one rank: a block-scaled local GEMM)."""
     from iris_b200.ops import quantize_activation, quantize_weight
 
     torch.manual_seed(2)
@@ -482,7 +482,7 @@ def test_router_matches_torch_topk(ctx):
                                                  (128, 2, 2, True, None), (384, 8, 2, True, None), (512, 4, 4, False, None),
                                                  (384, 8, 2, True, False)])
 def test_ring_attention_world1(ctx, S, Hq, Hkv, causal, tc):
-    """Multiples of 128 run the tcgen05 attention CTAs, other lengths (or tc=False) the mma.sync ones."""
+    """More than 128 tokens run the tcgen05 attention CTAs, up to 128 (or tc=False) the mma.sync ones."""
     from iris_b200.models import RingAttention, reference_attention
 
     dt = torch.bfloat16
