@@ -118,6 +118,7 @@ class MoELayer:
         self.counts_local, self.cursor, self.list_off, self.my_off = z(num_experts), z(num_experts), z(num_experts + 1), z(num_experts)
         self.sorted_pairs = z(pairs)
         self.pos_of = z(pairs) if W == 1 else None
+        self._prep_max = None
         self.expert_rows, self.expert_row0, self.tile_prefix, self.expected_cum = z(El), z(El + 1), z(El + 1), z(El)
         ctx.barrier()
 
@@ -211,8 +212,10 @@ class MoELayer:
         d.weights_kmajor = 1
         d.pos_of = self.pos_of.data_ptr() if one_rank else None
         lib = self._lib()
+        if one_rank and self._prep_max is None:
+            self._prep_max = lib.iris_moe_prep_max_tokens()
         _lib.check(lib.iris_moe_forward(C.byref(d), C.c_void_p(_lib.current_stream_ptr())), "MoE forward launch",
-                   kernels=7 if not one_rank else (5 if T <= lib.iris_moe_prep_max_tokens() else 8))
+                   kernels=7 if not one_rank else (5 if T <= self._prep_max else 8))
         self._keep = logits
         return out
 

@@ -102,19 +102,19 @@ def matmul(A: torch.Tensor, B: torch.Tensor, bias: torch.Tensor | None = None, o
     if A.stride(1) != 1 or out.stride(1) != 1:
         raise ValueError("A and the output must be row-major")
     Bd, kmajor, ldb = b_layout(B)
-    bv, bias16 = None, 0
+    op, ldc = out.data_ptr(), out.stride(0)
+    bp, bias16 = 0, 0
     if bias is not None:         # read as it is when it has the operands' type, else as fp32
-        bv = bias.contiguous() if bias.dtype == A.dtype else None
+        if bias.dtype == A.dtype:
+            bv = bias.contiguous()
+            bp, bias16 = bv.data_ptr(), 1
         # (a bias inside the output, as in x = x_row + product, would be overwritten while other tiles still read it: its fp32 copy then)
-        lo = out.data_ptr()
-        if bv is not None and (bv.data_ptr() + 2 * bv.numel() <= lo or lo + 2 * ((M - 1) * out.stride(0) + N) <= bv.data_ptr()):
-            bias16 = 1
-        else:
+        if not bias16 or (bp < op + 2 * ((M - 1) * ldc + N) and op < bp + 2 * (M if bias_dim == 0 else N)):
             bv = bias.float().contiguous()
-    bp = bv.data_ptr() if bv is not None else 0
+            bp, bias16 = bv.data_ptr(), 0
     desc, buf = _local_desc()
     _HEAD.pack_into(buf, 0, _lib.GEMM_LOCAL, M, N, K, _lib.DTYPE_CODE[A.dtype], kmajor, bn, 0, 0, 0, 0,
-                    0 if two_sm is None else (2 if two_sm else 1), A.data_ptr(), A.stride(0), Bd.data_ptr(), ldb, out.data_ptr(), out.stride(0),
+                    0 if two_sm is None else (2 if two_sm else 1), A.data_ptr(), A.stride(0), Bd.data_ptr(), ldb, op, ldc,
                     bp if bias_dim == 0 else 0, bp if bias_dim == 1 else 0)
     desc.bias16 = bias16
     _lib.check(_lib.kernels().iris_gemm_launch(C.byref(desc), _lib.current_stream_ptr()), "gemm launch", kernels=1)
