@@ -27,13 +27,18 @@
 
 #include "gemm_host.cuh"
 #include "quantize_common.cuh"
+#include "moe_experts.cuh"
 
 namespace {
 
 constexpr int kMaxTopK = 16;
+// One rank: token tiles of moe_experts.cuh. An expert has at most T rows, so up to 64 tokens every expert is one tile, and the
+// smaller stages make a deeper ring; e4m3 needs TMEM columns for its scale cells, so its widest tile is 240.
+constexpr int kSmallTokens = 64, kTile16 = 256, kTileFp8 = 240;
 
 struct MoeDims {
   int T, K, E, El, D, F, capacity;
+  int tile_rows;           // most rows of a token tile
 };
 
 // Device-resident metadata of one layer (all int32 unless noted; "heap" = symmetric heap).
@@ -48,7 +53,7 @@ struct MoeMeta {
   int32_t* my_off;         // [E]      first inbox row (on the owner) of my rows for expert e
   int32_t* expert_rows;    // [El]     rows this rank receives per local expert
   int32_t* expert_row0;    // [El + 1] prefix of expert_rows
-  int32_t* tile_prefix;    // [El + 1] prefix of ceil(rows / 128)
+  int32_t* tile_prefix;    // [El + 1] prefix of ceil(rows / tile_rows)
   int32_t* expected_cum;   // [El]     arrivals expected so far (all calls)
   int32_t* arrived;        // heap [El] arrivals so far (all calls)
   long long* inbox_meta;   // heap [capacity]  (source rank << 32) | pair id
@@ -171,7 +176,7 @@ __global__ void __launch_bounds__(1024) moe_meta_kernel(const __grid_constant__ 
       m.tile_prefix[j] = tiles;
       m.expected_cum[j] += r;
       rows += r;
-      tiles += (r + kBM - 1) / kBM;
+      tiles += expert_tiles(r, dm.tile_rows);
     }
     m.expert_row0[El] = rows;
     m.tile_prefix[El] = tiles;
@@ -231,8 +236,8 @@ __global__ void __launch_bounds__(1024) moe_prep_kernel(const float* __restrict_
     }
   }
   __syncthreads();
-  // exclusive prefix sums of rows and 128-row tiles over the experts, one expert per thread
-  const int rows = tid < dm.E ? hist[tid] : 0, tiles = (rows + kBM - 1) / kBM;
+  // exclusive prefix sums of rows and token tiles over the experts, one expert per thread
+  const int rows = tid < dm.E ? hist[tid] : 0, tiles = expert_tiles(rows, dm.tile_rows);
   int pr = rows, pt = tiles;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
@@ -282,14 +287,21 @@ __global__ void __launch_bounds__(256) moe_gather_kernel(const uint8_t* __restri
   }
 }
 
-// The same for e4m3 rows, from the 16-bit tokens: half a warp quantises one 128-column block of a token and stores the
-// values and the scale byte to the token's K rows.
+// The same for e4m3 rows, from the 16-bit tokens: half a warp quantises one 128-column block of a token, stores the values to
+// the token's K rows and the scale byte, four times, to its cell of the scale atoms of each row's tile ([tile][K block][atoms]).
 __global__ void __launch_bounds__(256) moe_gather_quant_kernel(const __nv_bfloat16* __restrict__ x, uint8_t* __restrict__ inbox,
-                                                               uint8_t* __restrict__ inbox_sf, int sf_ld, int D,
-                                                               const int32_t* __restrict__ pos_of, int K, int capacity) {
-  __shared__ int32_t dst[kMaxTopK];
-  const int t = blockIdx.x, half = threadIdx.x >> 4, sub = threadIdx.x & 15;
-  if (threadIdx.x < K) dst[threadIdx.x] = pos_of[(size_t)t * K + threadIdx.x];
+                                                               uint8_t* __restrict__ inbox_sf, int atoms, MoeDims dm, MoeMeta m,
+                                                               const int32_t* __restrict__ pos_of) {
+  __shared__ int32_t dst[kMaxTopK], tile[kMaxTopK], cell[kMaxTopK];
+  const int t = blockIdx.x, half = threadIdx.x >> 4, sub = threadIdx.x & 15, D = dm.D, K = dm.K, kblocks = D / 128;
+  if (threadIdx.x < K) {
+    const int p = t * K + threadIdx.x, e = m.topk_idx[p], pos = pos_of[p], first = m.tile_prefix[e];
+    const int row0 = m.expert_row0[e], per = expert_tile_rows(m.expert_row0[e + 1] - row0, m.tile_prefix[e + 1] - first);
+    const int i = (pos - row0) / per;
+    dst[threadIdx.x] = pos;
+    tile[threadIdx.x] = first + i;
+    cell[threadIdx.x] = sf_cell(pos - row0 - i * per);
+  }
   __syncthreads();
   const int kb = blockIdx.y * 16 + half, c = kb * 128 + sub * 8;       // D is a multiple of 256: whole blocks
   Raw8<__nv_bfloat16> raw;
@@ -298,9 +310,9 @@ __global__ void __launch_bounds__(256) moe_gather_quant_kernel(const __nv_bfloat
   if (c >= D) return;
   const uint2 v = quantised8(raw, e);
   for (int k = 0; k < K; ++k) {
-    if (dst[k] >= capacity) continue;
+    if (dst[k] >= dm.capacity) continue;
     *(uint2*)(inbox + (size_t)dst[k] * D + c) = v;
-    if (sub == 0) inbox_sf[(size_t)dst[k] * sf_ld + kb] = (uint8_t)(e + 127);
+    if (sub == 0) *(uint32_t*)(inbox_sf + ((size_t)tile[k] * kblocks + kb) * (atoms * 512) + cell[k]) = (uint32_t)(e + 127) * 0x01010101u;
   }
 }
 
@@ -621,11 +633,22 @@ typedef struct IrisMoeDesc {
   const void* w13_sf;       // scale atoms of w13: [El][2F / 256][D / 128][2][512]
   const void* w2_sf;        // scale atoms of w2:  [El][ceil(D / 224)][F / 128][2][512]
   int32_t* pos_of;          // [T * K] one rank only: inbox row of each (token, k) pair
-  const void* x16;          // one rank, e4m3: the bf16 tokens [T, D], quantised on the way into the inbox (x and x_sf are not read)
+  // One rank, e4m3: the bf16 tokens [T, D], quantised on the way into the inbox (x and x_sf are not read). inbox_sf and H_sf
+  // are then scale atoms per token tile, iris_moe_sf_bytes(T, K, E, D or F) bytes each; w13_sf is [El][F / 128][D / 128][512], an
+  // atom's first 256 bytes from the gate block's scale and the rest from the up block's; w2_sf is [El][D / 256][F / 128][2][512].
+  const void* x16;
 } IrisMoeDesc;
 
 // One rank: up to this many tokens a call is 5 kernels, above it 8.
 int iris_moe_prep_max_tokens(void) { return kPrepMaxTokens; }
+
+// One rank, e4m3: bytes of the scale atoms of the token tiles of up to T tokens, for rows of `cols` columns.
+long long iris_moe_sf_bytes(int T, int K, int E, int cols) {
+  const long long small = T < kSmallTokens ? T : kSmallTokens;                          // a call may have fewer tokens: E tiles of one atom
+  const long long tiles = (long long)T * K / kTileFp8 + E;
+  const long long big = T > kSmallTokens ? tiles * 2 : 0, few = small > 0 ? E : 0;
+  return (big > few ? big : few) * 512 * ceil_div(cols, 128);
+}
 
 int iris_moe_forward(const IrisMoeDesc* d, void* stream_) {
   cudaStream_t s = (cudaStream_t)stream_;
@@ -633,12 +656,16 @@ int iris_moe_forward(const IrisMoeDesc* d, void* stream_) {
   if (d->T <= 0) return -21;
   DeviceContext ctx;
   memcpy(&ctx, &d->ctx, sizeof(ctx));
-  MoeDims dm{d->T, d->K, d->E, d->El, d->D, d->F, d->capacity};
+  const bool one_rank = ctx.world <= 1, km = d->weights_kmajor != 0;
+  const bool experts = one_rank && km;          // the pair kernel of moe_experts.cuh
+  const bool small = d->T <= kSmallTokens;
+  const int tile_rows = !experts ? kBM : small ? kSmallTokens : d->fp8 ? kTileFp8 : kTile16;
+  MoeDims dm{d->T, d->K, d->E, d->El, d->D, d->F, d->capacity, tile_rows};
   MoeMeta m{d->topk_idx, d->topk_w, d->counts_local, d->counts_all, d->cursor, d->list_off, d->sorted_pairs, d->my_off,
             d->expert_rows, d->expert_row0, d->tile_prefix, d->expected_cum, d->arrived, (long long*)d->inbox_meta};
   const int sms = sm_count();
-  const bool one_rank = ctx.world <= 1;
   int32_t* pos_of = one_rank ? d->pos_of : nullptr;
+  if (d->fp8 && !km) return -3;
   if (one_rank && (!pos_of || ((uintptr_t)d->x & 15) || ((uintptr_t)d->x16 & 15) || (d->fp8 && !d->x16))) return -11;
   if (one_rank && d->T <= kPrepMaxTokens) {
     auto* prep = d->E <= 32 ? moe_prep_kernel<1> : d->E <= 64 ? moe_prep_kernel<2> : d->E <= 128 ? moe_prep_kernel<4>
@@ -657,7 +684,7 @@ int iris_moe_forward(const IrisMoeDesc* d, void* stream_) {
   if (one_rank) {
     if (d->fp8) {
       moe_gather_quant_kernel<<<dim3(d->T, ceil_div(d->D, 2048)), 256, 0, s>>>((const __nv_bfloat16*)d->x16, (uint8_t*)d->inbox, (uint8_t*)d->inbox_sf,
-                                                                             d->sf_ld1, d->D, pos_of, d->K, d->capacity);
+                                                                             small ? 1 : 2, dm, m, pos_of);
     } else {
       const int row16 = d->D * 2 / 16;
       int split = ceil_div(4 * sms, d->T);
@@ -668,7 +695,6 @@ int iris_moe_forward(const IrisMoeDesc* d, void* stream_) {
   if (cudaGetLastError() != cudaSuccess) return -21;
 
   const int comm = one_rank ? 0 : (d->comm_ctas > 0 ? d->comm_ctas : 16);
-  const bool km = d->weights_kmajor != 0;
   auto common = [&](auto& pol, int bn, int N, int Kdim, bool f8) {
     pol.sh = Shape{d->capacity, N, Kdim};
     pol.tiles_m = 0; pol.tiles_n = ceil_div(N, bn); pol.group_m = 1;
@@ -681,7 +707,22 @@ int iris_moe_forward(const IrisMoeDesc* d, void* stream_) {
     pol.a_sf = nullptr; pol.a_sf_ld = 0; pol.x_sf = nullptr; pol.inbox_sf = nullptr; pol.h_sf = nullptr; pol.h_sf_ld = 0;
     pol.sfb_per_expert = pol.tiles_n * pol.kblocks * pol.sfb_atoms;
   };
-  if (d->fp8) {
+  if (experts) {
+    ExpertArgs a;
+    a.row0 = m.expert_row0; a.tiles = m.tile_prefix; a.pairs = m.sorted_pairs;
+    a.status = d->ctx.status; a.El = d->El; a.capacity = d->capacity;
+    const int max_tiles = small ? d->E : d->T * d->K / tile_rows + d->E;
+    const ExpertProblem up{d->w13, d->w13_sf, d->inbox, d->inbox_sf, 2 * d->F, d->D, max_tiles};
+    const ExpertProblem down{d->w2, d->w2_sf, d->H, d->H_sf, d->D, d->F, max_tiles};
+    a.out = (uint8_t*)d->H; a.out_sf = (uint8_t*)d->H_sf; a.ldo = d->F;
+    int r = d->fp8 ? (small ? launch_experts<ExpertCfg<1, true, kSmallTokens>>(a, up, s) : launch_experts<ExpertCfg<1, true, kTileFp8>>(a, up, s))
+                   : (small ? launch_experts<ExpertCfg<1, false, kSmallTokens>>(a, up, s) : launch_experts<ExpertCfg<1, false, kTile16>>(a, up, s));
+    if (r) return r;
+    a.out = (uint8_t*)d->comb; a.out_sf = nullptr; a.ldo = d->D;
+    r = d->fp8 ? (small ? launch_experts<ExpertCfg<2, true, kSmallTokens>>(a, down, s) : launch_experts<ExpertCfg<2, true, kTileFp8>>(a, down, s))
+               : (small ? launch_experts<ExpertCfg<2, false, kSmallTokens>>(a, down, s) : launch_experts<ExpertCfg<2, false, kTile16>>(a, down, s));
+    if (r) return r;
+  } else if (d->fp8) {
     if (!km || d->sf_ld1 % 16 || d->sf_ld2 % 16 || d->sf_ld1 * 128 < d->D || d->sf_ld2 * 128 < d->F || d->D % 128 || d->F % 128) return -3;
     {
       GroupedGemm<1, true> pol;

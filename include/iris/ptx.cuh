@@ -54,6 +54,12 @@ IRIS_D void mbar_arrive_cluster(uint64_t* bar, uint32_t cta) {
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(smem_u32(bar)), "r"(cta));
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(remote) : "memory");
 }
+// Store to the same shared-memory location in CTA `cta` of this cluster.
+IRIS_D void st_cluster_f32(float* p, uint32_t cta, float v) {
+  uint32_t remote;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(smem_u32(p)), "r"(cta));
+  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(remote), "f"(v) : "memory");
+}
 IRIS_D bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(
@@ -312,6 +318,14 @@ IRIS_D void tma_load_2d_pair_elect(uint32_t smem_dst, const CUtensorMap* m, uint
                "@q cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];\n\t}" ::"r"(
                    smem_dst),
                "l"(m), "r"(bar_addr), "r"(x), "r"(y)
+               : "memory");
+}
+IRIS_D void tma_load_3d_pair_elect(uint32_t smem_dst, const CUtensorMap* m, uint64_t* bar, int x, int y, int z) {
+  uint32_t bar_addr = smem_u32(bar) & 0xFEFFFFFFu;
+  asm volatile("{\n\t" IRIS_ELECT
+               "@q cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];\n\t}" ::"r"(
+                   smem_dst),
+               "l"(m), "r"(bar_addr), "r"(x), "r"(y), "r"(z)
                : "memory");
 }
 #undef IRIS_ELECT

@@ -130,24 +130,34 @@ class MoELayer:
         ctx, El, D, F = self.ctx, self.El, self.D, self.F
         if D % 128 or F % 128:
             raise ValueError("the fp8 MoE needs hidden and ffn to be multiples of 128")
+        one_rank = ctx.get_num_ranks() == 1                                      # (the kernels of one rank take other scale layouts, csrc/kernels/moe.cu)
         q13, s13 = quantize_128x128(self.w13.reshape(El * 2 * F, D).float(), pow2=True)
         self.w13_q = q13.view(El, 2 * F, D)
         self.w13_scale = s13                                                     # [El * 2F / 128, D / 128]
         self.w13_sf = pack_scales_b(s13, El * 2 * F, 256)                        # experts start on tile boundaries (2F % 256 == 0)
+        if one_rank:                                                             # rows of gate and up alternate by 16 there: one mixed atom
+            sf = self.w13_sf.view(-1, 2, 512)
+            self.w13_sf = torch.cat([sf[:, 0, :256], sf[:, 1, 256:]], dim=1).contiguous()
         q2, s2 = quantize_128x128(self.w2.reshape(El * D, F).float(), pow2=True)
         self.w2_q = q2.view(El, D, F)
         self.w2_scale = s2                                                       # [El * D / 128, F / 128]
         per = D // 128
-        self.w2_sf = torch.stack([pack_scales_b(s2[j * per:(j + 1) * per], D, 224) for j in range(El)]).contiguous()
+        tile = 256 if one_rank else 224
+        self.w2_sf = torch.stack([pack_scales_b(s2[j * per:(j + 1) * per], D, tile) for j in range(El)]).contiguous()
         self.sf_ld1 = -(-(D // 128) // 16) * 16
         self.sf_ld2 = -(-(F // 128) // 16) * 16
         u8 = torch.uint8
         self.inbox = ctx.heap.allocate(self.capacity * D, u8).view(self.capacity, D)
-        self.inbox_sf = ctx.heap.allocate(self.capacity * self.sf_ld1, u8).view(self.capacity, self.sf_ld1)
-        self.inbox_sf.fill_(127)
         self.H = torch.zeros(self.capacity, F, dtype=u8, device=dev)
-        self.H_sf = torch.full((self.capacity, self.sf_ld2), 127, dtype=u8, device=dev)
-        one_rank = ctx.get_num_ranks() == 1                                      # quantises in its gather
+        if one_rank:                                                             # scale atoms per token tile
+            nbytes = lambda cols: self._lib().iris_moe_sf_bytes(self.T, self.K, self.E, cols)  # noqa: E731
+            self.inbox_sf = torch.full((nbytes(D),), 127, dtype=u8, device=dev)
+            self.H_sf = torch.full((nbytes(F),), 127, dtype=u8, device=dev)
+        else:
+            self.inbox_sf = ctx.heap.allocate(self.capacity * self.sf_ld1, u8).view(self.capacity, self.sf_ld1)
+            self.inbox_sf.fill_(127)
+            self.H_sf = torch.full((self.capacity, self.sf_ld2), 127, dtype=u8, device=dev)
+        # (one rank quantises in its gather)
         self.xq = None if one_rank else torch.zeros(self.T, D, dtype=u8, device=dev)      # the tokens as they are sent
         self.x_sf = None if one_rank else torch.full((self.T, self.sf_ld1), 127, dtype=u8, device=dev)
         del self.w13, self.w2
@@ -168,6 +178,8 @@ class MoELayer:
         if not getattr(lib, "_iris_moe_typed", False):
             lib.iris_moe_forward.argtypes = [C.POINTER(IrisMoeDesc), C.c_void_p]
             lib.iris_moe_forward.restype = C.c_int
+            lib.iris_moe_sf_bytes.argtypes = [C.c_int] * 4
+            lib.iris_moe_sf_bytes.restype = C.c_longlong
             lib._iris_moe_typed = True
         return lib
 

@@ -122,6 +122,37 @@ def test_moe_e4m3_one_rank_preparation(ctx, T):
     ctx.heap_release(mark)
 
 
+@pytest.mark.parametrize("fp8", [False, True])
+@pytest.mark.parametrize("T,E,K,D,F", [(1, 4, 2, 256, 128), (16, 2, 2, 512, 256), (17, 3, 1, 256, 384), (64, 2, 2, 256, 128), (65, 2, 2, 256, 128),
+                                       (240, 2, 2, 512, 128), (241, 2, 2, 256, 256), (256, 3, 3, 256, 128), (257, 2, 2, 512, 128), (513, 5, 2, 256, 128),
+                                       (1000, 40, 1, 256, 128), (1500, 8, 4, 1024, 512)])
+def test_moe_one_rank_token_tiles(ctx, fp8, T, E, K, D, F):
+    """Token tiles of every padded size: experts that take every token (E = K: T rows each, both sides of the tile limits 64, 240 and
+    256), experts without tokens, a layer made for more tokens than the call has. Rows of the buffers behind an expert's last
+    tile hold other experts' rows. Bounds as in the two tests above; the e4m3 layer is compared over its dequantised weights."""
+    from iris_b200.models import MoELayer, reference_moe
+    from iris_b200.ops.gemm_fp8 import dequantize, quantize_128x128
+
+    wg, wu, wd = _moe_weights(E, D, F, T + E)
+    mark = ctx.heap_mark()
+    layer = MoELayer(ctx, D, F, E, K, max_tokens=T + 300, w_gate=wg, w_up=wu, w_down=wd, fp8=fp8)
+    if fp8:
+        deq = lambda w: torch.stack([dequantize(*quantize_128x128(m.t().contiguous().float(), pow2=True), 128).t() for m in w])  # noqa: E731
+        wg, wu, wd = deq(wg), deq(wu), deq(wd)
+    x = torch.randn(T, D, device="cuda", generator=_gen(T)).to(torch.bfloat16)
+    logits = torch.randn(T, E, device="cuda", generator=_gen(T + 1))
+    if K < E:
+        logits[:, E // 2:] -= 1.5 * torch.arange(E - E // 2, device="cuda")        # crowded and empty experts
+    y = layer(x, logits)
+    want = reference_moe(x, logits, wg, wu, wd, K)
+    assert ((y.float() - want).norm() / want.norm()).item() < (0.1 if fp8 else 2e-2)
+    worst = ((y.float() - want).norm(dim=1) / want.norm(dim=1)).max().item()         # no row is another's
+    assert worst < (0.2 if fp8 else 4e-2), worst
+    assert torch.equal(y, layer(x, logits))
+    ctx.check()
+    ctx.heap_release(mark)
+
+
 # ------------------------------------------------------------------------------------ attention on one rank
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("S,Hq,Hkv", [(1, 2, 2), (64, 4, 2), (127, 8, 2), (128, 3, 1), (129, 4, 4), (257, 6, 2), (384, 5, 5), (1000, 8, 8), (2500, 16, 2),
