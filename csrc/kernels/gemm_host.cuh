@@ -176,6 +176,23 @@ int sm_count() {
 
 int ceil_div(int a, int b) { return (a + b - 1) / b; }
 
+// Launch behind the stream's last kernel without waiting for it to finish: the kernel calls ptx::pdl_wait() before it touches
+// anything that an earlier kernel may have written.
+template <class... P, class... A>
+int launch_pdl(void (*kern)(P...), dim3 grid, int block, int smem, cudaStream_t stream, A&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(block, 1, 1);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, static_cast<A&&>(args)...) == cudaSuccess ? 0 : -21;
+}
+
 template <class Cfg, class Policy>
 int launch(const Policy& pol, int grid, cudaStream_t stream) {
   void (*kern)(const Policy);

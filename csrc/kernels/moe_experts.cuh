@@ -8,20 +8,24 @@
 // 74 pairs (6.9 rounds in the time of 7), where 148 single CTAs took the time of 4 for 3.5.
 //   warp 0      TMA producer: weights, tokens and (e4m3) scale atoms into a ring of stages
 //   warp 1      MMA issuer (even CTA of the pair), fp32 accumulators in TMEM, two buffers
-//   warps 2..5  epilogue: TMEM lane = weight row, TMEM column = token; a 16-bit transpose through shared memory
-// Stage 1 (gate|up): the weight rows are stored as blocks of [gate 128 | up 128]. Each CTA loads 64 gate and 64
-// up rows interleaved by 16, so a warp holds the gate and up values of 16 features in lanes l and l + 16,
-// and one shuffle per two values feeds SwiGLU. In e4m3 a 128-feature quantisation block of H spans the pair: the CTAs
-// exchange each token's largest magnitude through distributed shared memory.
+//   warps 2..9  epilogue: TMEM lane = weight row, TMEM column = token; read as mma fragments and transposed by stmatrix
+// Stage 1 (gate|up): the weight rows are stored as blocks of [gate 128 | up 128]. Each CTA loads 64 gate and 64 up rows
+// interleaved by 16, so a warp reads the gate and up values of 16 features into the same threads. In e4m3 a 128-feature
+// quantisation block of H spans the pair: the CTAs exchange each token's largest magnitude by asynchronous stores into each
+// other's shared memory (a release at cluster scope waited for the warp's global stores of the tile before).
 // Stage 2 (down): every output row goes to the (token, k) slot it came from.
-// Whole layer, 32 experts top-8 of 7168 x 2048, before (128-row token tiles) and now: 64 tokens e4m3 336 and 262 us, 4096 tokens bf16
-// 2934 and 2706 us (power cap).
+// Whole layer, before (128-row token tiles on single CTAs) and now: 32 experts top-8 of 7168 x 2048, 64 tokens e4m3 316 and 239 us
+// (its weights' HBM time is 226), bf16 498 and 430; 4096 tokens bf16, the kernels alone, stage 1 1583 and 1320 us, stage 2 780 and 628.
+// 4096 tokens, 32 experts top-8 of 2048 x 1024: stage 1 bf16 218 and 184 us, e4m3 280 and 142 (336 with one shuffle and one 2-byte
+// store per value, four epilogue warps and full-precision divisions), stage 2 117 and 102, 119 and 79.
 #pragma once
 #include "gemm_host.cuh"
 
 namespace {
 
 constexpr int kExpertMax = 1024;         // experts of a layer (the router's limit)
+constexpr int kXEpiWarps = 8;            // epilogue warps: two per quarter of the TMEM lanes, every other 32 tokens each
+constexpr int kXThreads = 64 + 32 * kXEpiWarps;
 
 struct ExpertArgs {
   CUtensorMap tmW;         // weights: stage 1 [2 * blocks][128][D], stage 2 [El * D, F]
@@ -52,7 +56,7 @@ struct ExpertCfg {
   static constexpr int kUsedCols = 2 * kMaxN_ + (kFp8_ ? 2 * kSetCols : 0);
   static constexpr int kTmemCols = kUsedCols <= 128 ? 128 : kUsedCols <= 256 ? 256 : 512;
   // staging: e4m3 stage 1 keeps the tile's H values [token][64 features] and three arrays of magnitudes, else 2 KB per warp
-  static constexpr int kEpiBytes = kQuant ? kMaxN_ * 128 + 3 * kMaxN_ * 4 : kEpiWarps * 2048;
+  static constexpr int kEpiBytes = kQuant ? kMaxN_ * 128 + 3 * kMaxN_ * 4 : kXEpiWarps * 2048;
   static constexpr int kTabBytes = 2 * (kExpertMax + 4) * 4;
   static constexpr int kFree = 227 * 1024 - 1024 - kEpiBytes - kTabBytes - 512;
   static constexpr int kFit = kFree / (kStageBytes + kSfBytes);
@@ -97,7 +101,7 @@ __device__ __forceinline__ ExpertTile expert_unit(const int32_t* s_tiles, const 
 }
 
 template <class Cfg>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) expert_gemm_kernel(const __grid_constant__ ExpertArgs g) {
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kXThreads, 1) expert_gemm_kernel(const __grid_constant__ ExpertArgs g) {
   extern __shared__ uint8_t smem_raw[];
   constexpr int kStages = Cfg::kStages, kStage = Cfg::kStage, kMaxN = Cfg::kMaxN;
   constexpr bool kFp8 = Cfg::kFp8;
@@ -116,12 +120,15 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) expert_
   uint64_t* peer_max = acc_empty + 2;        // [2] e4m3 stage 1: the peer's magnitudes have arrived
   uint32_t* tmem_slot = (uint32_t*)(peer_max + 2);
 
+  // Launched behind the gather (stage 1) or stage 1 (stage 2). What is read before pdl_wait - the weights and the tables of
+  // the preparation - was complete before the kernel in front of this one got past its own pdl_wait or was launched.
+  ptx::pdl_trigger();
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) { ptx::mbar_init(&full[s], 1); ptx::mbar_init(&empty[s], 1); }
     for (int b = 0; b < 2; ++b) {
       ptx::mbar_init(&acc_full[b], 1);
-      ptx::mbar_init(&acc_empty[b], 2 * kEpiWarps);
-      ptx::mbar_init(&peer_max[b], 4 * kEpiWarps);
+      ptx::mbar_init(&acc_empty[b], 2 * kXEpiWarps);
+      ptx::mbar_init(&peer_max[b], 1);
     }
     ptx::fence_mbar_init();
     ptx::fence_proxy_async();
@@ -130,7 +137,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) expert_
     ptx::tmem_alloc_pair(tmem_slot, Cfg::kTmemCols);
     ptx::tmem_relinquish_pair();
   }
-  for (int i = threadIdx.x; i <= g.El; i += kThreads) { s_tiles[i] = g.tiles[i]; s_row0[i] = g.row0[i]; }
+  for (int i = threadIdx.x; i <= g.El; i += kXThreads) { s_tiles[i] = __ldcg(g.tiles + i); s_row0[i] = __ldcg(g.row0 + i); }
   ptx::tc_fence_before();
   __syncthreads();
   ptx::cluster_sync();
@@ -154,23 +161,40 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) expert_
       const uint32_t bytes = 2 * (Cfg::kWBytes + Cfg::kSfBytes + x_bytes);
       const int xrow = u.row + (int)cta * half;
       const int wblk = u.e * g.tiles_w + u.w;
-      for (int kb = 0; kb < g.kblocks; ++kb) {
-        if (!__all_sync(0xffffffffu, ptx::mbar_wait<true>(&empty[s], ph ^ 1, kPipeTimeoutNs))) { fail(); ok = false; break; }
-        const uint32_t sw = stage0 + s * Cfg::kStageBytes, sx = sw + Cfg::kWBytes;
+      auto load_w = [&](int s, int kb) {
+        const uint32_t sw = stage0 + s * Cfg::kStageBytes;
         if (leader) ptx::mbar_expect_tx_elect(&full[s], bytes);
         if constexpr (kStage == 1) {
 #pragma unroll
           for (int i = 0; i < 4; ++i)          // 16 gate rows and their 16 up rows, one warp's lanes of the accumulator
             ptx::tma_load_3d_pair_elect(sw + i * 4096, &g.tmW, &full[s], kb * Cfg::kBKE, (int)cta * 64 + i * 16, 2 * wblk);
-        } else ptx::tma_load_2d_pair_elect(sw, &g.tmW, &full[s], kb * Cfg::kBKE, wblk * 256 + (int)cta * 128);
-        ptx::tma_load_2d_pair_elect(sx, mx, &full[s], kb * Cfg::kBKE, xrow);
-        if constexpr (kFp8) {
-          const uint32_t ss = sf0 + s * Cfg::kSfBytes;
-          // stage 1: both CTAs hold the same interleaved rows' scales, one atom per block; stage 2: one atom per 128 rows
-          const int ws = kStage == 1 ? wblk * g.kblocks + kb : (wblk * g.kblocks + kb) * 2 + (int)cta;
-          ptx::tma_load_2d_pair_elect(ss, &g.tmWS, &full[s], 0, ws);
-          ptx::tma_load_2d_pair_elect(ss + 512, &g.tmXS, &full[s], 0, (u.tile * g.kblocks + kb) * Cfg::kAtoms);
+        } else {
+          ptx::tma_load_2d_pair_elect(sw, &g.tmW, &full[s], kb * Cfg::kBKE, wblk * 256 + (int)cta * 128);
         }
+        // stage 1: both CTAs hold the same interleaved rows' scales, one atom per block; stage 2: one atom per 128 rows
+        if constexpr (kFp8)
+          ptx::tma_load_2d_pair_elect(sf0 + s * Cfg::kSfBytes, &g.tmWS, &full[s], 0,
+                                      kStage == 1 ? wblk * g.kblocks + kb : (wblk * g.kblocks + kb) * 2 + (int)cta);
+      };
+      auto load_x = [&](int s, int kb) {
+        ptx::tma_load_2d_pair_elect(stage0 + s * Cfg::kStageBytes + Cfg::kWBytes, mx, &full[s], kb * Cfg::kBKE, xrow);
+        if constexpr (kFp8)
+          ptx::tma_load_2d_pair_elect(sf0 + s * Cfg::kSfBytes + 512, &g.tmXS, &full[s], 0, (u.tile * g.kblocks + kb) * Cfg::kAtoms);
+      };
+      int kb = 0;
+      if (t == first) {                        // the ring fills with weights while the kernel in front finishes
+        const int pre = min(kStages, g.kblocks);
+        for (int i = 0; i < pre; ++i) load_w(i, i);
+        ptx::pdl_wait();
+        for (int i = 0; i < pre; ++i) load_x(i, i);
+        kb = pre;
+        if (pre == kStages) ph ^= 1;
+        else s = pre;
+      }
+      for (; kb < g.kblocks; ++kb) {
+        if (!__all_sync(0xffffffffu, ptx::mbar_wait<true>(&empty[s], ph ^ 1, kPipeTimeoutNs))) { fail(); ok = false; break; }
+        load_w(s, kb);
+        load_x(s, kb);
         if (++s == kStages) { s = 0; ph ^= 1; }
       }
     }
@@ -214,72 +238,103 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) expert_
       }
     }
   } else {
-    // ------------------------------------------------------------------ epilogue (warps 2..5)
-    const int q = warp & 3;                    // TMEM lanes [32 q, 32 q + 32)
-    uint8_t* stage = epi + (warp - 2) * 2048;
+    // ------------------------------------------------------------------ epilogue (warps 2..9)
+    const int q = warp & 3, w8 = warp - 2;     // TMEM lanes [32 q, 32 q + 32)
+    const int c_first = (w8 >> 2) * 32;        // and of those the 32-token chunks from here, every other one
+    auto release_acc = [&](int buf) {
+      ptx::tc_fence_before();
+      __syncwarp();
+      if (lane == 0) {
+        if (leader) ptx::mbar_arrive(&acc_empty[buf]);
+        else ptx::mbar_arrive_cluster_tmem(&acc_empty[buf], 0);
+      }
+    };
+    uint8_t* stage = epi + w8 * 2048;
     bool live = true;                          // after a wait that ran out the tiles pass without work: barriers stay in step
     int it = 0;
     for (int t = first; t < units; t += step, ++it) {
       const int buf = it & 1;
       const ExpertTile u = expert_unit(s_tiles, s_row0, g.El, g.tiles_w, t);
       const int keep = min(u.cnt, g.capacity - u.row);      // rows to be stored
+      int pr[4];                               // stage 2: the destinations of the chunks' tokens, fetched while the MMAs run
+      if constexpr (kStage == 2) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int tk = c_first + 64 * i + lane;
+          pr[i] = tk < keep ? __ldg(g.pairs + u.row + tk) : -1;
+        }
+      }
       if (live) {
         live = __all_sync(0xffffffffu, ptx::mbar_wait<true>(&acc_full[buf], (it >> 1) & 1, kPipeTimeoutNs));
         if (!live) fail();
       }
       ptx::tc_fence_after();
       const uint32_t t_addr = tmem_base + ((uint32_t)(q * 32) << 16) + buf * kMaxN;
-      for (int c = 0; c < u.n && live; c += 32) {
-        uint32_t r[32];
-        ptx::tmem_ld_32x32(t_addr + c, r);     // (the last load may read allocated columns past the tile)
+      if (live && c_first >= u.n) release_acc(buf);
+      for (int c = c_first; c < u.n && live; c += 64) {
+        // lanes [0, 16) and [16, 32) of the quarter, as fragments: thread l has lanes l / 4 and l / 4 + 8 of each half, and of every
+        // eight tokens the two at 2 (l % 4). (The last load may read allocated columns past the tile.)
+        uint32_t lo[16], hi[16];
+        ptx::tmem_ld_16x256_x4(t_addr + c, lo);
+        ptx::tmem_ld_16x256_x4(t_addr + (16u << 16) + c, hi);
         ptx::tmem_ld_wait();
-        if (c + 32 >= u.n) {
-          ptx::tc_fence_before();
-          __syncwarp();
-          if (lane == 0) {
-            if (leader) ptx::mbar_arrive(&acc_empty[buf]);
-            else ptx::mbar_arrive_cluster(&acc_empty[buf], 0);
-          }
-        }
+        if (c + 64 >= u.n) release_acc(buf);
+        const int mrow = lane & 7, mat = lane >> 3;              // this thread's row of the stored matrices
         if constexpr (kStage == 1) {
-          const bool up = lane >= 16;
+          // gate (lo) and up (hi) of the same features and tokens
+          uint32_t h[8];
 #pragma unroll
-          for (int j = 0; j < 32; j += 2) {
-            // lanes 0..15 finish token c + j, lanes 16..31 token c + j + 1
-            const float mine = __uint_as_float(up ? r[j + 1] : r[j]);
-            const float other = __shfl_xor_sync(0xffffffffu, __uint_as_float(up ? r[j] : r[j + 1]), 16);
-            const float gv = up ? other : mine, uv = up ? mine : other;
-            const __nv_bfloat16 h = __float2bfloat16_rn(gv / (1.f + __expf(-gv)) * uv);
+          for (int i = 0; i < 8; ++i) {
+            float v[2];
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+              const float gv = __uint_as_float(lo[2 * i + e]), uv = __uint_as_float(hi[2 * i + e]);
+              v[e] = __fdividef(gv, 1.f + __expf(-gv)) * uv;
+            }
+            const __nv_bfloat162 p = __floats2bfloat162_rn(v[0], v[1]);
+            h[i] = *(const uint32_t*)&p;
+          }
+#pragma unroll
+          for (int i = 0; i < 2; ++i) {                          // 16 tokens: matrices (token octet mat / 2, feature octet mat % 2)
+            const int tk = 16 * i + 8 * (mat >> 1) + mrow, f = mat & 1;
             if constexpr (Cfg::kQuant) {
-              const int tk = c + j + (lane >> 4);          // 16-byte groups of a token's 128 bytes, odd tokens' pairs swapped
-              const int grp = (q * 2 + ((lane & 15) >> 3)) ^ ((tk & 1) << 1);
-              if (tk < kMaxN) *(__nv_bfloat16*)(epi + tk * 128 + grp * 16 + (lane & 7) * 2) = h;
+              // rows of 128 bytes, their 16-byte groups permuted by the token
+              const int t = c + tk;
+              const uint32_t dst = ptx::smem_u32(epi + t * 128 + (((q * 2 + f) ^ (t & 7)) * 16));
+              if (c + 16 * i < kMaxN) ptx::stmatrix_x4_trans(dst, h[4 * i], h[4 * i + 1], h[4 * i + 2], h[4 * i + 3]);
             } else {
-              *(__nv_bfloat16*)(stage + (j + (lane >> 4)) * 32 + (lane & 15) * 2) = h;
+              ptx::stmatrix_x4_trans(ptx::smem_u32(stage + tk * 32 + ((f ^ ((tk >> 2) & 1)) * 16)), h[4 * i], h[4 * i + 1], h[4 * i + 2], h[4 * i + 3]);
             }
           }
           if constexpr (!Cfg::kQuant) {
             __syncwarp();
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
-              const int tk = i * 16 + (lane >> 1);
-              const uint4 v = *(const uint4*)(stage + tk * 32 + (lane & 1) * 16);
-              if (c + tk < keep)
-                *(uint4*)(g.out + ((size_t)(u.row + c + tk) * g.ldo + u.w * 128 + cta * 64 + q * 16 + (lane & 1) * 8) * 2) = v;
+              const int tk = i * 16 + (lane >> 1), f = lane & 1;
+              const uint4 v = *(const uint4*)(stage + tk * 32 + ((f ^ ((tk >> 2) & 1)) * 16));
+              if (c + tk < keep) *(uint4*)(g.out + ((size_t)(u.row + c + tk) * g.ldo + u.w * 128 + cta * 64 + q * 16 + f * 8) * 2) = v;
             }
             __syncwarp();
           }
         } else {
-          const int pr = c + lane < keep ? g.pairs[u.row + c + lane] : -1;
+          const int pc = c < 64 ? pr[0] : c < 128 ? pr[1] : c < 192 ? pr[2] : pr[3];
+          auto pack = [](uint32_t a, uint32_t b) {
+            const __nv_bfloat162 p = __floats2bfloat162_rn(__uint_as_float(a), __uint_as_float(b));
+            return *(const uint32_t*)&p;
+          };
 #pragma unroll
-          for (int j = 0; j < 32; ++j) *(__nv_bfloat16*)(stage + j * 64 + lane * 2) = __float2bfloat16_rn(__uint_as_float(r[j]));
+          for (int i = 0; i < 4; ++i) {                          // 8 tokens: matrix = feature octet
+            const int tk = 8 * i + mrow;
+            ptx::stmatrix_x4_trans(ptx::smem_u32(stage + tk * 64 + ((mat ^ ((tk >> 1) & 3)) * 16)), pack(lo[4 * i], lo[4 * i + 1]),
+                                   pack(lo[4 * i + 2], lo[4 * i + 3]), pack(hi[4 * i], hi[4 * i + 1]), pack(hi[4 * i + 2], hi[4 * i + 3]));
+          }
           __syncwarp();
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
-            const int tk = i * 8 + (lane >> 2);
-            const int p = __shfl_sync(0xffffffffu, pr, tk);
-            const uint4 v = *(const uint4*)(stage + tk * 64 + (lane & 3) * 16);
-            if (p >= 0) *(uint4*)(g.out + ((size_t)p * g.ldo + u.w * 256 + cta * 128 + q * 32 + (lane & 3) * 8) * 2) = v;
+            const int tk = i * 8 + (lane >> 2), f = lane & 3;
+            const int p = __shfl_sync(0xffffffffu, pc, tk);
+            const uint4 v = *(const uint4*)(stage + tk * 64 + ((f ^ ((tk >> 1) & 3)) * 16));
+            if (p >= 0) *(uint4*)(g.out + ((size_t)p * g.ldo + u.w * 256 + cta * 128 + q * 32 + f * 8) * 2) = v;
           }
           __syncwarp();
         }
@@ -289,11 +344,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) expert_
         // for the other 64, then values and scale. Eight lanes per token.
         float* own = (float*)(epi + kMaxN * 128);
         float* box = own + kMaxN + buf * kMaxN;            // written by the peer
-        ptx::named_barrier(1, kEpiWarps * 32);
+        ptx::named_barrier(1, kXEpiWarps * 32);
         const int sub = lane & 7;
-        auto group_of = [&](int tk) { return (const uint4*)(epi + tk * 128 + ((sub ^ ((tk & 1) << 1)) * 16)); };
+        auto group_of = [&](int tk) { return (const uint4*)(epi + tk * 128 + ((sub ^ (tk & 7)) * 16)); };
         if (live) {
-          for (int tk = q * 4 + (lane >> 3); tk < u.n; tk += 16) {
+          if (w8 == 0 && lane == 0) ptx::mbar_expect_tx(&peer_max[buf], u.n * 4);
+          for (int tk = w8 * 4 + (lane >> 3); tk < u.n; tk += 4 * kXEpiWarps) {
             const uint4 v = *group_of(tk);
             const uint32_t w[4] = {v.x, v.y, v.z, v.w};
             float m = 0.f;
@@ -306,20 +362,20 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) expert_
             for (int o = 4; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
             if (sub == 0) {
               own[tk] = m;
-              ptx::st_cluster_f32(&box[tk], cta ^ 1, m);
+              ptx::st_async_f32(&box[tk], &peer_max[buf], cta ^ 1, m);
             }
           }
-          if (sub == 0) ptx::mbar_arrive_cluster(&peer_max[buf], cta ^ 1);      // (release: each writer lane for its own stores)
           live = __all_sync(0xffffffffu, ptx::mbar_wait<true>(&peer_max[buf], (it >> 1) & 1, kPipeTimeoutNs));
           if (!live) fail();
         }
         if (live) {
           __syncwarp();
-          for (int tk = q * 4 + (lane >> 3); tk < keep; tk += 16) {
+          for (int tk = w8 * 4 + (lane >> 3); tk < keep; tk += 4 * kXEpiWarps) {
             const float m = fmaxf(own[tk], box[tk]);
-            int e8 = (int)ceilf(log2f(fmaxf(m, 1e-12f) * (1.0f / 448.0f)));
-            e8 = max(-127, min(127, e8));
-            const float inv = exp2f((float)-e8);
+            // the smallest power of two >= m / 448, from the bits
+            const uint32_t mb = __float_as_uint(fmaxf(m, 1e-12f) * (1.0f / 448.0f));
+            const int e8 = min(127, (int)(mb >> 23) - 127 + ((mb & 0x7fffffu) ? 1 : 0));
+            const float inv = e8 == 127 ? 0x1p-127f : __uint_as_float((uint32_t)(127 - e8) << 23);
             const uint4 v = *group_of(tk);
             const uint32_t w[4] = {v.x, v.y, v.z, v.w};
             uint32_t o[2];
@@ -334,7 +390,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) expert_
               *(uint32_t*)(g.out_sf + (size_t)(u.tile * g.tiles_w + u.w) * (Cfg::kAtoms * 512) + sf_cell(tk)) = (uint32_t)(e8 + 127) * 0x01010101u;
           }
         }
-        ptx::named_barrier(1, kEpiWarps * 32);             // the values are read before the next tile's overwrite them
+        ptx::named_barrier(1, kXEpiWarps * 32);             // the values are read before the next tile's overwrite them
       }
     }
   }
@@ -386,8 +442,7 @@ int launch_experts(ExpertArgs& a, const ExpertProblem& p, cudaStream_t stream) {
     if (cudaFuncSetAttribute(expert_gemm_kernel<Cfg>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes) != cudaSuccess) return -20;
     attr = true;
   }
-  expert_gemm_kernel<Cfg><<<sm_count() & ~1, kThreads, Cfg::kSmemBytes, stream>>>(a);
-  return cudaGetLastError() == cudaSuccess ? 0 : -21;
+  return launch_pdl(expert_gemm_kernel<Cfg>, dim3(sm_count() & ~1), kXThreads, Cfg::kSmemBytes, stream, a);
 }
 
 }  // namespace

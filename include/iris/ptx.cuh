@@ -54,11 +54,21 @@ IRIS_D void mbar_arrive_cluster(uint64_t* bar, uint32_t cta) {
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(smem_u32(bar)), "r"(cta));
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(remote) : "memory");
 }
-// Store to the same shared-memory location in CTA `cta` of this cluster.
-IRIS_D void st_cluster_f32(float* p, uint32_t cta, float v) {
+// The same with the default scope: no wait for this thread's outstanding global stores. For a barrier that hands over TMEM,
+// whose accesses tcgen05.wait and the tcgen05 fences order, and no memory.
+IRIS_D void mbar_arrive_cluster_tmem(uint64_t* bar, uint32_t cta) {
   uint32_t remote;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(smem_u32(bar)), "r"(cta));
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(remote) : "memory");
+}
+// Asynchronous store to the same shared-memory location in CTA `cta` of this cluster; its four bytes are credited to the
+// barrier at `bar`'s offset there.
+IRIS_D void st_async_f32(float* p, uint64_t* bar, uint32_t cta, float v) {
+  uint32_t remote, rbar;
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(smem_u32(p)), "r"(cta));
-  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(remote), "f"(v) : "memory");
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(rbar) : "r"(smem_u32(bar)), "r"(cta));
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(remote), "r"(__float_as_uint(v)), "r"(rbar)
+               : "memory");
 }
 IRIS_D bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
   uint32_t ok;
@@ -343,7 +353,29 @@ IRIS_D void tmem_ld_32x32(uint32_t taddr, uint32_t (&r)[32]) {
       : "r"(taddr)
       : "memory");
 }
+// TMEM -> registers in the layout of an mma fragment: 16 lanes x 32 fp32 columns. r[4 i + 2 h + e] is lane
+// (thread / 4) + 8 h, column 8 i + 2 (thread % 4) + e.
+IRIS_D void tmem_ld_16x256_x4(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.16x256b.x4.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr)
+      : "memory");
+}
+// Four transposed 8 x 8 matrices of 16-bit elements to shared memory: thread t names the 16-byte row t % 8 of matrix t / 8;
+// a register holds (row t / 4, columns 2 (t % 4) and + 1) of its matrix and lands in memory rows 2 (t % 4) and + 1, column t / 4.
+IRIS_D void stmatrix_x4_trans(uint32_t saddr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(saddr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
 IRIS_D void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+
+// Programmatic dependent launch. pdl_wait: the kernels this one was launched behind have completed and their memory is
+// visible (returns at once in a kernel launched the ordinary way). pdl_trigger: once every CTA of the grid has issued it or has
+// left, CTAs of a kernel launched behind this one with the programmatic attribute may start, up to their pdl_wait.
+IRIS_D void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+IRIS_D void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // Named barrier among `nthreads` threads of the CTA (id 1..15; 0 is __syncthreads).
 IRIS_D void named_barrier(int id, int nthreads) {

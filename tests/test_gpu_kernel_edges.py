@@ -153,6 +153,31 @@ def test_moe_one_rank_token_tiles(ctx, fp8, T, E, K, D, F):
     ctx.heap_release(mark)
 
 
+@pytest.mark.parametrize("T,fp8", [(20, True), (20, False), (300, True)])
+def test_moe_one_rank_in_a_cuda_graph(ctx, T, fp8):
+    """The launches that start behind their predecessors, captured: a replay on new inputs gives the bits of a plain call."""
+    from iris_b200.models import MoELayer
+
+    E, D, F, K = 8, 512, 256, 2
+    mark = ctx.heap_mark()
+    layer = MoELayer(ctx, D, F, E, K, max_tokens=T, **dict(zip(("w_gate", "w_up", "w_down"), _moe_weights(E, D, F, 3))), fp8=fp8)
+    x, logits, out = torch.zeros(T, D, device="cuda", dtype=torch.bfloat16), torch.zeros(T, E, device="cuda"), torch.zeros(T, D, device="cuda", dtype=torch.bfloat16)
+    layer(x, logits, out=out)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        for _ in range(3):                       # the next call's first kernel follows the last call's reduction
+            layer(x, logits, out=out)
+    for seed in (1, 2):
+        x.copy_(torch.randn(T, D, device="cuda", generator=_gen(seed)))
+        logits.copy_(torch.randn(T, E, device="cuda", generator=_gen(seed + 10)))
+        graph.replay()
+        got = out.clone()
+        assert got.abs().max() > 0 and torch.equal(got, layer(x, logits))
+    del graph
+    ctx.heap_release(mark)
+
+
 # ------------------------------------------------------------------------------------ attention on one rank
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("S,Hq,Hkv", [(1, 2, 2), (64, 4, 2), (127, 8, 2), (128, 3, 1), (129, 4, 4), (257, 6, 2), (384, 5, 5), (1000, 8, 8), (2500, 16, 2),
