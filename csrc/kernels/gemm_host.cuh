@@ -13,6 +13,7 @@
 #include "iris/sync.cuh"
 #include "iris/multimem.cuh"
 #include "iris/gemm/sm100_mainloop.cuh"
+#include "launch_pdl.cuh"
 
 using namespace iris;
 using namespace iris::gemm;
@@ -101,6 +102,7 @@ struct Common {
   IRIS_D void store_chunk_local(int width, const uint8_t* smem, int row, int col) const {
     ptx::tma_store_2d(width == 64 ? &tmC : &tmC32, smem, col, row);
   }
+  static constexpr bool kPdl = false;
   static constexpr bool kSfaFromRows = false;
   static constexpr bool kQuantOut = false;
   // defaults of the epilogue hooks a policy may leave out
@@ -176,23 +178,6 @@ int sm_count() {
 
 int ceil_div(int a, int b) { return (a + b - 1) / b; }
 
-// Launch behind the stream's last kernel without waiting for it to finish: the kernel calls ptx::pdl_wait() before it touches
-// anything that an earlier kernel may have written.
-template <class... P, class... A>
-int launch_pdl(void (*kern)(P...), dim3 grid, int block, int smem, cudaStream_t stream, A&&... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = dim3(block, 1, 1);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = stream;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kern, static_cast<A&&>(args)...) == cudaSuccess ? 0 : -21;
-}
-
 template <class Cfg, class Policy>
 int launch(const Policy& pol, int grid, cudaStream_t stream) {
   void (*kern)(const Policy);
@@ -204,6 +189,7 @@ int launch(const Policy& pol, int grid, cudaStream_t stream) {
     if (e != cudaSuccess) return -20;
     attr_set = true;
   }
+  if (Policy::kPdl) return launch_pdl(kern, dim3(grid), kThreads, Cfg::kSmemBytes, stream, pol);
   kern<<<grid, kThreads, Cfg::kSmemBytes, stream>>>(pol);
   return cudaGetLastError() == cudaSuccess ? 0 : -21;
 }

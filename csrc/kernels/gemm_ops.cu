@@ -30,6 +30,7 @@ namespace {
 
 // ------------------------------------------------------------------------------------ local GEMM
 struct LocalGemm : Common {
+  static constexpr bool kPdl = true;
   uint8_t* C;
   int64_t ldc;
   struct State {};

@@ -3,7 +3,7 @@
 //
 // Bound by reading B once (N * K * 2 bytes). The main loop gives every 128- to 256-wide column tile to one CTA, which for few
 // rows means N / 128 CTAs that walk all of K: 16 x 3584 x 8192 ran on 28 of 148 SMs, 32.8 us against 8.9 us of
-// HBM time, now 16.4. Here
+// HBM time, now 14.2 (16.4 before it started behind the kernel in front of it, launch_pdl.cuh). Here
 //   * the tile is turned round: 128 columns of B are the M side of tcgen05.mma and the tokens, padded to 16,
 //     the N side, so a stage holds 16 KB of weights and 128 bytes per token instead of 128 rows of padding;
 //   * K is split over the CTAs of a cluster (up to 8). Each CTA keeps its partial tile in its own shared memory as fp32
@@ -70,6 +70,8 @@ __global__ void __launch_bounds__(kSkinnyThreads) skinny_gemm_kernel(const __gri
   __syncthreads();
   ptx::tc_fence_after();
   const uint32_t tmem_base = *(volatile uint32_t*)tmem_slot;
+  ptx::pdl_trigger();
+  ptx::pdl_wait();
   const int kb0 = (int)((int64_t)g.kblocks * rank / S), kb1 = (int)((int64_t)g.kblocks * (rank + 1) / S);
   auto fail = [&]() { if (g.status) atomicCAS(g.status, 0, (int)kTimeoutPipeline); };
 
@@ -264,9 +266,11 @@ int iris_gemm_skinny(const IrisGemmDesc* d, cudaStream_t stream) {
   cfg.blockDim = dim3(kSkinnyThreads, 1, 1);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeClusterDimension;
   at[0].val.clusterDim.x = S; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
-  cfg.attrs = at; cfg.numAttrs = 1;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;      // see launch_pdl.cuh
+  at[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at; cfg.numAttrs = 2;
   return cudaLaunchKernelEx(&cfg, kern, g) == cudaSuccess && cudaGetLastError() == cudaSuccess ? 0 : -21;
 }

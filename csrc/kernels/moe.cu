@@ -212,6 +212,7 @@ __global__ void __launch_bounds__(256) moe_sort_kernel(MoeDims dm, MoeMeta m, in
   }
 }
 __global__ void moe_clear_kernel(MoeDims dm, MoeMeta m) {
+  ptx::pdl_wait();
   ptx::pdl_trigger();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < dm.E) m.counts_local[i] = 0;
@@ -224,6 +225,7 @@ constexpr int kPrepMaxTokens = 256;
 template <int kPer>
 __global__ void __launch_bounds__(1024) moe_prep_kernel(const float* __restrict__ logits, const __grid_constant__ DeviceContext ctx, MoeDims dm,
                                                         MoeMeta m, int32_t* pos_of) {
+  ptx::pdl_wait();
   ptx::pdl_trigger();
   __shared__ int32_t hist[1024], off[1024], w_rows[32], w_tiles[32];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -580,6 +582,7 @@ struct GroupedGemm : Common {
 __global__ void __launch_bounds__(128) moe_reduce_kernel(const __nv_bfloat16* __restrict__ comb, const float* __restrict__ w, __nv_bfloat16* out,
                                                          int T, int K, int D) {
   ptx::pdl_wait();
+  ptx::pdl_trigger();
   __shared__ float s_w[kMaxTopK];
   const int t = blockIdx.x;
   if (threadIdx.x < K) s_w[threadIdx.x] = w[(size_t)t * K + threadIdx.x];
@@ -677,9 +680,8 @@ int iris_moe_forward(const IrisMoeDesc* d, void* stream_) {
   int32_t* pos_of = one_rank ? d->pos_of : nullptr;
   if (d->fp8 && !km) return -3;
   if (one_rank && (!pos_of || ((uintptr_t)d->x & 15) || ((uintptr_t)d->x16 & 15) || (d->fp8 && !d->x16))) return -11;
-  // On one rank every kernel but the first is launched behind its predecessor without waiting for it to finish (64 tokens,
-  // 32 experts, e4m3: 243 us in all, 262 when each waited). The first waits for the stream as usual, so buffers that a pdl_wait does
-  // not cover are never those of an earlier call still running.
+  // On one rank every kernel is launched behind its predecessor without waiting for it to finish (64 tokens, 32 experts,
+  // e4m3: 243 us in all, 262 when each waited).
   auto go = [&](auto kern, dim3 grid, int block, auto... args) {
     if (experts) return launch_pdl(kern, grid, block, 0, s, args...);
     kern<<<grid, block, 0, s>>>(args...);
@@ -688,9 +690,9 @@ int iris_moe_forward(const IrisMoeDesc* d, void* stream_) {
   if (one_rank && d->T <= kPrepMaxTokens) {
     auto* prep = d->E <= 32 ? moe_prep_kernel<1> : d->E <= 64 ? moe_prep_kernel<2> : d->E <= 128 ? moe_prep_kernel<4>
                  : d->E <= 256 ? moe_prep_kernel<8> : moe_prep_kernel<32>;
-    prep<<<1, 1024, 0, s>>>(d->logits, ctx, dm, m, pos_of);
+    if (const int r = go(prep, dim3(1), 1024, d->logits, ctx, dm, m, pos_of)) return r;
   } else {
-    moe_clear_kernel<<<(d->E + 255) / 256, 256, 0, s>>>(dm, m);
+    if (const int r = go(moe_clear_kernel, dim3((d->E + 255) / 256), 256, dm, m)) return r;
     const int warps = d->T > 16 * sms ? 16 : 4;      // warps per block: few tokens spread over more SMs
     const int blocks = ceil_div(d->T, warps) < sms ? ceil_div(d->T, warps) : sms;
     auto* router = d->E <= 32 ? router_topk_kernel<1> : d->E <= 64 ? router_topk_kernel<2> : d->E <= 128 ? router_topk_kernel<4>

@@ -120,9 +120,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kXThreads, 1) expert
   uint64_t* peer_max = acc_empty + 2;        // [2] e4m3 stage 1: the peer's magnitudes have arrived
   uint32_t* tmem_slot = (uint32_t*)(peer_max + 2);
 
-  // Launched behind the gather (stage 1) or stage 1 (stage 2). What is read before pdl_wait - the weights and the tables of
-  // the preparation - was complete before the kernel in front of this one got past its own pdl_wait or was launched.
-  ptx::pdl_trigger();
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) { ptx::mbar_init(&full[s], 1); ptx::mbar_init(&empty[s], 1); }
     for (int b = 0; b < 2; ++b) {
@@ -143,6 +140,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kXThreads, 1) expert
   ptx::cluster_sync();
   ptx::tc_fence_after();
   const uint32_t tmem_base = *(volatile uint32_t*)tmem_slot;
+  // Launched behind the gather (stage 1) or stage 1 (stage 2). What is read before pdl_wait - the weights and the tables of
+  // the preparation - was complete before the kernel in front of this one got past its own pdl_wait or was launched.
+  ptx::pdl_trigger();
   const int units = s_tiles[g.El] * g.tiles_w, first = blockIdx.x >> 1, step = gridDim.x >> 1;
   auto fail = [&]() { if (g.status) atomicCAS(g.status, 0, (int)kTimeoutPipeline); };
 
@@ -250,6 +250,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kXThreads, 1) expert
       }
     };
     uint8_t* stage = epi + w8 * 2048;
+    ptx::pdl_wait();
     bool live = true;                          // after a wait that ran out the tiles pass without work: barriers stay in step
     int it = 0;
     for (int t = first; t < units; t += step, ++it) {

@@ -182,6 +182,7 @@ struct Pipeline {
 //   void comm_main(uint8_t* smem, int smem_bytes) const;    (CTAs with blockIdx.x >= gemm_ctas())
 //   void post_main() const;                                 (GEMM CTAs, all threads, after their tiles)
 //   void fail(int code) const;
+//   static constexpr bool kPdl;                            (launched behind the stream's last kernel: waits for it after the set-up)
 //   void stamp(int tile_seq, int what) const;              (optional per-tile timestamps: 0 tile
 //        start, 1 first A tile available, 2 tile stored; reference examples collect the same with
 //        COLLECT_TIMESTAMPS, examples/07_gemm_all_scatter/gemm_all_scatter.py:64-66)
@@ -243,6 +244,10 @@ IRIS_D void gemm_cta_main(const Policy& pol, uint8_t* smem_raw) {
   if constexpr (kPair) ptx::cluster_sync();   // both CTAs' barriers exist before anyone signals remotely
   ptx::tc_fence_after();
   const uint32_t tmem_base = *(volatile uint32_t*)tmem_slot;
+  if constexpr (Policy::kPdl) {     // the set-up above runs while the kernel in front finishes
+    ptx::pdl_trigger();
+    ptx::pdl_wait();
+  }
 
   const int num_tiles = pol.num_tiles();
   const int k_blocks = (sh.K + Cfg::kBKElems - 1) / Cfg::kBKElems;

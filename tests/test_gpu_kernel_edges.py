@@ -68,6 +68,60 @@ def test_activation_passes_match_fp64(dtype, name, shape):
         assert ((got.double() - want).abs() <= ulp * want.abs() + 4e-6 * (1 + dh.double().abs()) + tiny).all()
 
 
+# ------------------------------------------------------------------------------------ kernels that start behind their predecessor
+@pytest.mark.parametrize("rows", [16, 300, 2000])
+def test_chains_of_early_started_kernels(ctx, rows):
+    """Every kernel that is launched before its predecessor has finished, in chains where each reads what the one in front wrote and
+    buffers are written again at once, among ordinary kernels, with a second stream joined in, plain and as a CUDA graph: the bits
+    of the same calls with the device idle in between."""
+    from iris_b200.models import FlashDecodeLayer, RingAttention
+    from iris_b200.ops import matmul, quantize_activation, quantize_weight
+
+    g = _gen(rows)
+    r = lambda *sh: torch.randn(*sh, device="cuda", generator=g) * sh[-1] ** -0.5  # noqa: E731
+    D = 1024
+    w1, w2, wq = r(D, D).bfloat16().t(), r(D, D).bfloat16(), quantize_weight(r(D, D))
+    cache = [torch.randn(64, 16, 2, 128, device="cuda", generator=g).bfloat16() for _ in range(2)]
+    table, lens = torch.randperm(64, device="cuda", generator=g).int().view(2, 32), torch.tensor([[511, 77]], device="cuda", dtype=torch.int32)
+    mark = ctx.heap_mark()
+    dec, att = FlashDecodeLayer(ctx, 8, 2, 128, max_batch=2), RingAttention(ctx, rows, 8, 2)
+    x0 = torch.randn(rows, D, device="cuda", generator=g).bfloat16()
+    x, h, y = x0.clone(), torch.empty_like(x0), torch.empty_like(x0)
+    side = torch.cuda.Stream()
+
+    def chain(sync):
+        gap = torch.cuda.synchronize if sync else (lambda: None)
+        x.copy_(x0)
+        for _ in range(3):
+            gap(); matmul(x, w1, out=h)
+            gap(); matmul(h, w2, out=x)
+            gap(); a = quantize_activation(x)
+            gap(); matmul(a, wq, out=y)
+            side.wait_stream(torch.cuda.current_stream())
+            with torch.cuda.stream(side):
+                gap(); matmul(y, w2, out=h)
+            torch.cuda.current_stream().wait_stream(side)
+            gap(); o = att(h.view(rows, 8, 128), x.view(rows, 8, 128)[:, :2].contiguous(), y.view(rows, 8, 128)[:, 2:4].contiguous(), causal=True)
+            gap(); d = dec(o[:2], *cache, lens, table)
+            gap(); x[:2] = d.view(2, D)
+            gap(); x.mul_(4.0)
+        return x.clone(), y.clone()
+
+    want = chain(True)
+    assert all(torch.isfinite(t.float()).all() and t.float().abs().max() > 0 for t in want)
+    for _ in range(5):
+        assert all(torch.equal(a, b) for a, b in zip(chain(False), want))
+    graph = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph):
+        got = chain(False)
+    for _ in range(3):
+        graph.replay()
+        assert all(torch.equal(a, b) for a, b in zip(got, want))
+    del graph, got
+    ctx.heap_release(mark)
+
+
 # ------------------------------------------------------------------------------------ MoE on one rank
 def _moe_weights(E, D, F, seed):
     g = _gen(seed)
