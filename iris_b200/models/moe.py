@@ -119,6 +119,7 @@ class MoELayer:
         self.sorted_pairs = z(pairs)
         self.pos_of = z(pairs) if W == 1 else None
         self._prep_max = None
+        self._proto = None                       # descriptor fields that no call changes
         self.expert_rows, self.expert_row0, self.tile_prefix, self.expected_cum = z(El), z(El + 1), z(El + 1), z(El)
         ctx.barrier()
 
@@ -150,7 +151,9 @@ class MoELayer:
         self.inbox = ctx.heap.allocate(self.capacity * D, u8).view(self.capacity, D)
         self.H = torch.zeros(self.capacity, F, dtype=u8, device=dev)
         if one_rank:                                                             # scale atoms per token tile
-            nbytes = lambda cols: self._lib().iris_moe_sf_bytes(self.T, self.K, self.E, cols)  # noqa: E731
+            lib = self._lib()
+            lib.iris_moe_sf_bytes.argtypes, lib.iris_moe_sf_bytes.restype = [C.c_int] * 4, C.c_longlong
+            nbytes = lambda cols: lib.iris_moe_sf_bytes(self.T, self.K, self.E, cols)  # noqa: E731
             self.inbox_sf = torch.full((nbytes(D),), 127, dtype=u8, device=dev)
             self.H_sf = torch.full((nbytes(F),), 127, dtype=u8, device=dev)
         else:
@@ -178,10 +181,25 @@ class MoELayer:
         if not getattr(lib, "_iris_moe_typed", False):
             lib.iris_moe_forward.argtypes = [C.POINTER(IrisMoeDesc), C.c_void_p]
             lib.iris_moe_forward.restype = C.c_int
-            lib.iris_moe_sf_bytes.argtypes = [C.c_int] * 4
-            lib.iris_moe_sf_bytes.restype = C.c_longlong
             lib._iris_moe_typed = True
         return lib
+
+    def _fixed_fields(self, one_rank: bool) -> bytes:
+        """The descriptor without what a call brings or a program may exchange (the weights): the layer's sizes and its
+        own buffers. Set field by field on every call they took as long as the launches."""
+        d = IrisMoeDesc()
+        d.K, d.E, d.El, d.D, d.F, d.capacity, d.comm_ctas = self.K, self.E, self.El, self.D, self.F, self.capacity, self.comm_sms
+        if self.fp8:
+            d.fp8, d.sf_ld1, d.sf_ld2 = 1, self.sf_ld1, self.sf_ld2
+            d.inbox_sf, d.H_sf = self.inbox_sf.data_ptr(), self.H_sf.data_ptr()
+        d.inbox, d.H, d.comb = self.inbox.data_ptr(), self.H.data_ptr(), self.comb.data_ptr()
+        d.sync_meta, d.sync_gemm2 = self.sync_meta.data_ptr(), self.sync_gemm2.data_ptr()
+        for name in ("topk_idx", "topk_w", "counts_local", "counts_all", "cursor", "list_off", "sorted_pairs", "my_off",
+                     "expert_rows", "expert_row0", "tile_prefix", "expected_cum", "arrived", "inbox_meta"):
+            setattr(d, name, getattr(self, name).data_ptr())
+        d.weights_kmajor = 1
+        d.pos_of = self.pos_of.data_ptr() if one_rank else None
+        return bytes(d)
 
     def forward(self, x: torch.Tensor, router_logits: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
         ctx = self.ctx
@@ -200,29 +218,23 @@ class MoELayer:
         one_rank = self.pos_of is not None
         if one_rank and x.data_ptr() % 16:       # the gather reads 16 bytes at a time
             x = x.clone()
-        d = IrisMoeDesc()
+        proto = self._proto
+        if proto is None:
+            proto = self._proto = self._fixed_fields(one_rank)
+        d = IrisMoeDesc.from_buffer_copy(proto)
         d.ctx = ctx.ctx_struct()
-        d.T, d.K, d.E, d.El, d.D, d.F, d.capacity, d.comm_ctas = T, self.K, self.E, self.El, self.D, self.F, self.capacity, self.comm_sms
+        d.T = T
         if self.fp8:
             if one_rank:                         # quantised by the gather
                 d.x16 = x.data_ptr()
             else:
                 self._quantise_tokens(x)
                 d.x, d.x_sf = self.xq.data_ptr(), self.x_sf.data_ptr()
-            d.fp8, d.sf_ld1, d.sf_ld2 = 1, self.sf_ld1, self.sf_ld2
             d.w13, d.w2 = self.w13_q.data_ptr(), self.w2_q.data_ptr()
-            d.inbox_sf, d.H_sf = self.inbox_sf.data_ptr(), self.H_sf.data_ptr()
             d.w13_sf, d.w2_sf = self.w13_sf.data_ptr(), self.w2_sf.data_ptr()
         else:
             d.x, d.w13, d.w2 = x.data_ptr(), self.w13.data_ptr(), self.w2.data_ptr()
         d.logits, d.out = logits.data_ptr(), out.data_ptr()
-        d.inbox, d.H, d.comb = self.inbox.data_ptr(), self.H.data_ptr(), self.comb.data_ptr()
-        d.sync_meta, d.sync_gemm2 = self.sync_meta.data_ptr(), self.sync_gemm2.data_ptr()
-        for name in ("topk_idx", "topk_w", "counts_local", "counts_all", "cursor", "list_off", "sorted_pairs", "my_off",
-                     "expert_rows", "expert_row0", "tile_prefix", "expected_cum", "arrived", "inbox_meta"):
-            setattr(d, name, getattr(self, name).data_ptr())
-        d.weights_kmajor = 1
-        d.pos_of = self.pos_of.data_ptr() if one_rank else None
         lib = self._lib()
         if one_rank and self._prep_max is None:
             self._prep_max = lib.iris_moe_prep_max_tokens()
