@@ -3,7 +3,7 @@
 //
 // Bound by reading B once (N * K * 2 bytes). The main loop gives every 128- to 256-wide column tile to one CTA, which for few
 // rows means N / 128 CTAs that walk all of K: 16 x 3584 x 8192 ran on 28 of 148 SMs, 32.8 us against 8.9 us of
-// HBM time, now 14.2 (16.4 before it started behind the kernel in front of it, launch_pdl.cuh). Here
+// HBM time, now 13.3 (16.4 before it started behind the kernel in front of it, launch_pdl.cuh). Here
 //   * the tile is turned round: 128 columns of B are the M side of tcgen05.mma and the tokens, padded to 16,
 //     the N side, so a stage holds 16 KB of weights and 128 bytes per token instead of 128 rows of padding;
 //   * K is split over the CTAs of a cluster (up to 8). Each CTA keeps its partial tile in its own shared memory as fp32
@@ -71,8 +71,22 @@ __global__ void __launch_bounds__(kSkinnyThreads) skinny_gemm_kernel(const __gri
   ptx::tc_fence_after();
   const uint32_t tmem_base = *(volatile uint32_t*)tmem_slot;
   ptx::pdl_trigger();
-  ptx::pdl_wait();
   const int kb0 = (int)((int64_t)g.kblocks * rank / S), kb1 = (int)((int64_t)g.kblocks * (rank + 1) / S);
+  // The first ring's weights on their way into L2 while the kernel in front drains (its writes, if it wrote them, are in L2 as well):
+  // 16 x 3584 x 8192 13.7 -> 13.3 us back to back, 48-token MLP 29.6 -> 28.9. More than the ring holds was slower (14.0, 30.1), and so
+  // were smaller rings that leave room for a third CTA, whose prefetches met the running kernel's own loads (15.2, 33.2).
+  if (warp == 0) {
+    for (int kb = kb0 + lane; kb < min(kb1, kb0 + g.stages); kb += 32) {
+      if constexpr (kKMajor) {
+        ptx::tma_prefetch_2d(&g.tmW, kb * kBK, n0);
+      } else {
+        ptx::tma_prefetch_2d(&g.tmW, n0, kb * kBK);
+        ptx::tma_prefetch_2d(&g.tmW, n0 + 64, kb * kBK);
+      }
+    }
+    __syncwarp();
+  }
+  ptx::pdl_wait();
   auto fail = [&]() { if (g.status) atomicCAS(g.status, 0, (int)kTimeoutPipeline); };
 
   bool live = true;

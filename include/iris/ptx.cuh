@@ -132,6 +132,10 @@ IRIS_D void tma_load_2d_pair(void* smem_dst, const CUtensorMap* m, uint64_t* bar
       ::"r"(smem_u32(smem_dst)), "l"(m), "r"(bar_addr), "r"(x), "r"(y)
       : "memory");
 }
+// Bring a tile into L2. Where it is written by a kernel still running, a later load sees what was written: L2 is where all SMs meet.
+IRIS_D void tma_prefetch_2d(const CUtensorMap* m, int x, int y) {
+  asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global [%0, {%1, %2}];" ::"l"(m), "r"(x), "r"(y) : "memory");
+}
 // 2-D tiled store shared -> global (bulk async group).
 IRIS_D void tma_store_2d(const CUtensorMap* m, const void* smem_src, int x, int y) {
   asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];" ::"l"(m),
