@@ -23,7 +23,11 @@
 // (8192 tokens, 32 / 8 heads, causal, bf16: 736 us). Two tiles in turn, one thread per row: 549 us, with the MMAs issued eight
 // to a statement 511 (both with their inputs in L2, the second is 554 from HBM), with the loads' waits out of the chain 540 from
 // HBM; 3000 tokens, full attention, fp16, which the mma.sync kernel took before: 603, 187, 178, 174 us.
-// Slower were: 64-key halves with S double-buffered (more MMAs to issue: 746), P released to the MMAs in halves, part of the
+// An item's start and end cost about 9000 cycles each time, next to 3500 a pair of tiles: with its tiles counted in closed form instead of by walking
+// and the output stored by rows 554 -> 541 us, 3000 tokens 180 -> 176 (both under the power cap); three-operand maxima: by keys, 2304
+// tokens, 8 heads, causal 31.1 -> 29.2. A pair of tiles now (cycles, one tile's chain): load 150, maximum 410, exponentials 1350, P 190,
+// to the issuing warp 100, P V and S until the next softmax sees it 1290.
+// Slower were: 64-key halves with S double-buffered (more MMAs to issue: 746), P released to the MMAs in halves (541 -> 572 under the power cap), part of the
 // exponentials as a polynomial on the FMA pipe (the softmax warps are short of issue slots).
 // The two tiles are two query heads of one K/V head group where the group is even (same keys, no work done twice or
 // for padding), else two neighbouring tiles of 128 queries of one head. Items are handed out longest first, in
@@ -40,7 +44,7 @@
 // (the ring buffer is mapped block by block for that), its scores are masked and its rows are not stored.
 //
 // TMEM: S0 / P0 columns [0, 128), S1 / P1 [128, 256), O0 [256, 384), O1 [384, 512). Shared memory: Q 2 x 32 KB,
-// K 2 x 32 KB, V 2 x 32 KB. Every wait (mbarriers, arrival counters) is bounded.
+// K 2 x 32 KB, V 2 x 32 KB, output rows 16 KB. Every wait (mbarriers, arrival counters) is bounded.
 #include "ring_attention_common.cuh"
 
 #include "iris/gemm/sm100_mainloop.cuh"
@@ -61,9 +65,9 @@ constexpr int kTcThreads = 384;          // three warpgroups: issuers (two of fo
 constexpr int kHalf = 128 * 128;         // bytes of a [128 rows][64 columns] 16-bit half tile
 constexpr int kTile = 2 * kHalf;         // 32 KB
 constexpr int kKvStages = 2;
-constexpr int kStageOut = 32 * 64;       // bytes a softmax warp stages its output rows in, 32 columns at a time (by keys)
-constexpr int kTcSmem = 1024 + kTile * 2 + kTile * 2 * kKvStages + 256;      // Q tiles, K and V stages, barriers
-constexpr int kTcSmemByKeys = kTcSmem + 2 * 128 * 8 + 8 * kStageOut;         // ... (m, l) of both places, output rows
+constexpr int kStageOut = 32 * 64;       // bytes a softmax warp stages its output rows in, 32 columns at a time
+// Q tiles, K and V stages, barriers, (m, l) of both places (by keys), output rows
+constexpr int kTcSmem = 1024 + kTile * 2 + kTile * 2 * kKvStages + 256 + 2 * 128 * 8 + 8 * kStageOut;
 constexpr float kRescaleAt = 8.f;        // log2 of how far a row's maximum may run ahead of the one P is taken against
 // ... while the tile's number among its row's is below this it may not: a row's largest weight is exactly 1 then and loses nothing when P
 // is rounded, which counts most where few keys share the weight. Error against 64 bits (2-norm) of 8192 tokens, causal, bf16: 2.13e-3
@@ -71,7 +75,7 @@ constexpr float kRescaleAt = 8.f;        // log2 of how far a row's maximum may 
 // time with inputs in L2 467, 484, 530 us. By keys (short rows) always: 512 tokens 2.25e-3 -> 2.18e-3, within 3 % of the time.
 constexpr int kExactTiles = 8;
 constexpr uint64_t kWaitNs = 4000000000ull;
-static_assert(kTcSmemByKeys <= 227 * 1024, "shared memory budget");
+static_assert(kTcSmem <= 227 * 1024, "shared memory budget");
 
 struct TcArgs {
   RingArgs a;
@@ -144,6 +148,11 @@ __device__ __forceinline__ void mma_pv_elect(uint32_t tmem_d, uint32_t tmem_a, u
       "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [a], b, %3, t;\n\t"
       "}" ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float d;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
 }
 __device__ __forceinline__ float ex2_approx(float x) {
   float y;
@@ -240,7 +249,7 @@ struct TileWalk {
     b0 = causal && zigzag ? Th : T;
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
-      a1[i] = T; b1[i] = b0;
+      a1[i] = T; b1[i] = b0;                 // (b1[i] >= b0 always)
       if (i >= n_q) { a1[i] = 0; continue; }
       if (!causal) continue;
       if (!zigzag) a1[i] = origin > r ? 0 : origin == r ? qt[i] + 1 : T;
@@ -258,6 +267,17 @@ struct TileWalk {
       if (origin < 0) origin += W;
       ranges();
       if (ua1 > 0 || ub1 > b0) { t = -1; return; }
+    }
+  }
+  // tiles of the whole walk: query tile 0's, query tile 1's, and all. (Counted by walking, at 93 cycles a tile, they held back the
+  // first product of an item of 63 tiles by 6000 cycles.)
+  __device__ void count(int& n0, int& n1, int& all) {
+    n0 = n1 = all = 0;
+    for (step = 0; step < W; ++step) {
+      origin = r - step;
+      if (origin < 0) origin += W;
+      ranges();
+      n0 += a1[0] + b1[0] - b0; n1 += a1[1] + b1[1] - b0; all += ua1 + ub1 - b0;
     }
   }
   // advances to the next tile; false when the item is finished
@@ -421,8 +441,8 @@ __device__ void attn_main_tc(const TcArgs& g, uint8_t* smem_raw, int call) {
       if (!order.get(rd, item)) continue;
       if constexpr (kByKeys) {
         // S of the walk's tiles j + 1 and j + 2 is issued while the softmax works on tile j
-        int n = 0;
-        for (TileWalk w(a, item); w.next();) ++n;
+        int n, n0, n1;
+        TileWalk(a, item).count(n0, n1, n);
         if (!wait(&q_full[0], 0)) break;
         const uint32_t qb = ptx::smem_u32(q_s);
         auto wait_k = [&]() { return wait(&k_full[n_k % kKvStages], (n_k / kKvStages) & 1); };
@@ -452,15 +472,9 @@ __device__ void attn_main_tc(const TcArgs& g, uint8_t* smem_raw, int call) {
         }
         break;
       }
-      int left_s[2] = {0, 0}, left_pv[2];          // S and P V MMAs of the item still to be issued, per query tile
-      {
-        TileWalk w(a, item);
-        while (w.next()) {
-          if (w.needs(0)) ++left_s[0];
-          if (w.needs(1)) ++left_s[1];
-        }
-        left_pv[0] = left_s[0]; left_pv[1] = left_s[1];
-      }
+      int left_s[2], left_pv[2], all;               // S and P V MMAs of the item still to be issued, per query tile
+      TileWalk(a, item).count(left_s[0], left_s[1], all);
+      left_pv[0] = left_s[0]; left_pv[1] = left_s[1];
       const int total[2] = {left_s[0], left_s[1]};
 #pragma unroll
       for (int i = 0; i < 2; ++i)
@@ -533,6 +547,25 @@ __device__ void attn_main_tc(const TcArgs& g, uint8_t* smem_raw, int call) {
     uint32_t n_item = 0, n_tile = 0;
     bool ok = true;
     Item item;
+    // The warp's 32 rows go out through shared memory, 32 columns (64 bytes) of a row by four lanes: with a row per lane every
+    // 16-byte store instruction touched 32 lines, and an item's output took 3700 cycles. 16-byte pieces, XORed by half the
+    // row so that eight rows written and two rows read together meet different banks.
+    uint8_t* stage = (uint8_t*)(ml + 2 * 128) + (warp - 4) * kStageOut;
+    auto put_rows = [&](const uint32_t (&o)[32], int c, int q_tile, int h) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        *(uint4*)(stage + lane * 64 + ((e ^ ((lane >> 1) & 3)) << 4)) =
+            make_uint4(pack2<kFp16>(__uint_as_float(o[8 * e]), __uint_as_float(o[8 * e + 1])), pack2<kFp16>(__uint_as_float(o[8 * e + 2]), __uint_as_float(o[8 * e + 3])),
+                       pack2<kFp16>(__uint_as_float(o[8 * e + 4]), __uint_as_float(o[8 * e + 5])), pack2<kFp16>(__uint_as_float(o[8 * e + 6]), __uint_as_float(o[8 * e + 7])));
+      __syncwarp();
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const int rr = k * 8 + (lane >> 2), e = lane & 3, pos = q_tile * kTQ + quarter * 32 + rr;
+        if (pos < a.S)
+          *(uint4*)(a.out + ((size_t)pos * a.Hq + h) * kD * 2 + c * 64 + e * 16) = *(const uint4*)(stage + rr * 64 + ((e ^ ((rr >> 1) & 3)) << 4));
+      }
+      __syncwarp();
+    };
     for (int rd = 0; rd < order.rounds && ok; ++rd) {
       if (!order.get(rd, item)) continue;
       if (i >= item.n_q) continue;
@@ -562,16 +595,36 @@ __device__ void attn_main_tc(const TcArgs& g, uint8_t* smem_raw, int call) {
           for (int c = 0; c < 128; ++c)
             if (c > lim) s[c] = 0xff800000u;     // -inf
         }
-        float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};      // four chains: the maximum is latency bound otherwise
+        float mx4[4];             // four chains: the maximum is latency bound otherwise
 #pragma unroll
-        for (int c = 0; c < 128; c += 8) {
+        for (int u = 0; u < 4; ++u) mx4[u] = max3(__uint_as_float(s[u]), __uint_as_float(s[4 + u]), __uint_as_float(s[8 + u]));
 #pragma unroll
-          for (int u = 0; u < 4; ++u) mx4[u] = fmaxf(mx4[u], fmaxf(__uint_as_float(s[c + u]), __uint_as_float(s[c + 4 + u])));
+        for (int c = 12; c + 7 < 128; c += 8) {
+#pragma unroll
+          for (int u = 0; u < 4; ++u) mx4[u] = max3(mx4[u], __uint_as_float(s[c + u]), __uint_as_float(s[c + 4 + u]));
         }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) mx4[u] = fmaxf(mx4[u], __uint_as_float(s[124 + u]));
         const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * scale2;     // (the first tile holds a key the row sees)
         float alpha = 1.f;
         if (j == 0) m_run = mx;
         else if (mx > m_run + (kByKeys || j < kExactTiles ? 0.f : kRescaleAt)) { alpha = ex2_approx(m_run - mx); m_run = mx; }
+        // rescale O when some row of this warp moved its maximum (this tile's S was issued after the previous tile's
+        // P V, and its barrier covers both: O holds every earlier tile)
+        if (__any_sync(0xffffffffu, alpha != 1.f)) {
+          const unsigned long long al = pack_f32x2(alpha, alpha);
+#pragma unroll
+          for (int u = 0; u < 2; ++u) asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(l_pair[u]) : "l"(al));
+#pragma unroll 1
+          for (int c = 0; c < 4; ++c) {
+            uint32_t o[32];
+            ptx::tmem_ld_32x32(o_addr + c * 32, o);
+            ptx::tmem_ld_wait();
+#pragma unroll
+            for (int e = 0; e < 32; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * alpha);
+            tmem_st_32x32(o_addr + c * 32, o);
+          }
+        }
         // p = exp2(s * scale - max): packed FMA for two scores at a time, one ex2.approx each, packed sums. P goes over
         // the first 64 columns of the tile's S buffer: every thread of the row (this one) has read its scores
         const float neg_m = fminf(-m_run, 3e38f);      // finite where every key so far scores -inf: their P is 0, not NaN
@@ -593,22 +646,6 @@ __device__ void attn_main_tc(const TcArgs& g, uint8_t* smem_raw, int call) {
             pw[e] = pack2<kFp16>(p0, p1);
           }
           tmem_st_32x32(s_addr + hf * 32, pw);
-        }
-        // rescale O when some row of this warp moved its maximum (this tile's S was issued after the previous tile's
-        // P V, and its barrier covers both: O holds every earlier tile)
-        if (__any_sync(0xffffffffu, alpha != 1.f)) {
-          const unsigned long long al = pack_f32x2(alpha, alpha);
-#pragma unroll
-          for (int u = 0; u < 2; ++u) asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(l_pair[u]) : "l"(al));
-#pragma unroll 1
-          for (int c = 0; c < 4; ++c) {
-            uint32_t o[32];
-            ptx::tmem_ld_32x32(o_addr + c * 32, o);
-            ptx::tmem_ld_wait();
-#pragma unroll
-            for (int e = 0; e < 32; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * alpha);
-            tmem_st_32x32(o_addr + c * 32, o);
-          }
         }
         tmem_st_wait();                         // P (and a rescaled O) are in TMEM before the MMA is told
         ptx::tc_fence_before();
@@ -650,9 +687,6 @@ __device__ void attn_main_tc(const TcArgs& g, uint8_t* smem_raw, int call) {
           const float inv = l > 0.f ? 1.f / l : 0.f;
           w_own *= inv; w_other *= inv;
           const uint32_t other_addr = lane_addr + 256 + (i ^ 1) * 128;
-          // the warp's 32 rows go out through shared memory, 32 columns (64 bytes) of a row by four lanes: with a row per lane every
-          // 16-byte store instruction touched 32 lines
-          uint8_t* stage = (uint8_t*)(ml + 2 * 128) + (warp - 4) * kStageOut;
           const int c0 = both ? 2 * i : 0, c1 = both ? c0 + 2 : 4;
 #pragma unroll 1
           for (int c = c0; c < c1; ++c) {
@@ -666,20 +700,7 @@ __device__ void attn_main_tc(const TcArgs& g, uint8_t* smem_raw, int call) {
               if (both) f += __uint_as_float(o2[e]) * w_other;
               o[e] = __float_as_uint(f);
             }
-            // 16-byte pieces, XORed by half the row so that eight rows written and two rows read together meet different banks
-#pragma unroll
-            for (int e = 0; e < 4; ++e)
-              *(uint4*)(stage + lane * 64 + ((e ^ ((lane >> 1) & 3)) << 4)) =
-                  make_uint4(pack2<kFp16>(__uint_as_float(o[8 * e]), __uint_as_float(o[8 * e + 1])), pack2<kFp16>(__uint_as_float(o[8 * e + 2]), __uint_as_float(o[8 * e + 3])),
-                             pack2<kFp16>(__uint_as_float(o[8 * e + 4]), __uint_as_float(o[8 * e + 5])), pack2<kFp16>(__uint_as_float(o[8 * e + 6]), __uint_as_float(o[8 * e + 7])));
-            __syncwarp();
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-              const int rr = k * 8 + (lane >> 2), e = lane & 3, pos = item.qt[0] * kTQ + quarter * 32 + rr;
-              if (pos < a.S)
-                *(uint4*)(a.out + ((size_t)pos * a.Hq + head) * kD * 2 + c * 64 + e * 16) = *(const uint4*)(stage + rr * 64 + ((e ^ ((rr >> 1) & 3)) << 4));
-            }
-            __syncwarp();
+            put_rows(o, c, item.qt[0], head);
           }
           if (a.lse && i == 0 && qpos < a.S) a.lse[(size_t)qpos * a.Hq + head] = l > 0.f ? (m + log2f(l)) / kLog2e : -INFINITY;
         }
@@ -688,27 +709,20 @@ __device__ void attn_main_tc(const TcArgs& g, uint8_t* smem_raw, int call) {
       if (!__all_sync(0xffffffffu, ptx::mbar_wait(&o_full[i], n_item & 1, kWaitNs))) { ctx.fail(kTimeoutPipeline); ok = false; break; }
       ptx::tc_fence_after();
       const float inv = l_all > 0.f ? 1.f / l_all : 0.f;
-      uint8_t* orow = a.out + ((size_t)qpos * a.Hq + head) * kD * 2;
 #pragma unroll 1
       for (int c = 0; c < 4; ++c) {
         uint32_t o[32];
         ptx::tmem_ld_32x32(o_addr + c * 32, o);
         ptx::tmem_ld_wait();
-        if (qpos < a.S) {
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            uint4 v;
-            v.x = pack2<kFp16>(__uint_as_float(o[8 * e]) * inv, __uint_as_float(o[8 * e + 1]) * inv);
-            v.y = pack2<kFp16>(__uint_as_float(o[8 * e + 2]) * inv, __uint_as_float(o[8 * e + 3]) * inv);
-            v.z = pack2<kFp16>(__uint_as_float(o[8 * e + 4]) * inv, __uint_as_float(o[8 * e + 5]) * inv);
-            v.w = pack2<kFp16>(__uint_as_float(o[8 * e + 6]) * inv, __uint_as_float(o[8 * e + 7]) * inv);
-            *(uint4*)(orow + c * 64 + e * 16) = v;
-          }
+        if (c == 3) {                           // O is in registers: the next item's first P V may overwrite it
+          ptx::tc_fence_before();
+          __syncwarp();
+          if (lane == 0) ptx::mbar_arrive(&o_free[i]);
         }
+#pragma unroll
+        for (int e = 0; e < 32; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * inv);
+        put_rows(o, c, i ? item.qt[1] : item.qt[0], head);
       }
-      ptx::tc_fence_before();
-      __syncwarp();
-      if (lane == 0) ptx::mbar_arrive(&o_free[i]);
       if (a.lse && qpos < a.S) a.lse[(size_t)qpos * a.Hq + head] = l_all > 0.f ? (m_run + log2f(l_all)) / kLog2e : -INFINITY;
       ++n_item;
     }
@@ -790,7 +804,7 @@ int launch_ring_attention_tc(const RingArgs& a, cudaStream_t stream) {
   const bool by_keys = tiles <= sms - a.n_comm || (W == 1 && a.causal && tiles <= 2 * sms);
   g.by_head = (a.Hq / a.Hkv) % 2 == 0;
   const int items = by_keys ? tiles : g.by_head ? q_tiles * (a.Hq / 2) : (q_tiles + 1) / 2 * a.Hq;
-  // one CTA per SM (194 KB of shared memory), all resident; by keys a CTA per item, which the SMs take in order (longest first)
+  // one CTA per SM (212 KB of shared memory), all resident; by keys a CTA per item, which the SMs take in order (longest first)
   int attn = sms - a.n_comm;
   if (by_keys || attn > items) attn = items;
   if (attn < 1) return 1;
@@ -803,7 +817,7 @@ int launch_ring_attention_tc(const RingArgs& a, cudaStream_t stream) {
   using Y = std::true_type;
   using N = std::false_type;
   auto* kern = f16 ? (scale_first ? pick(Y{}, Y{}) : pick(Y{}, N{})) : (scale_first ? pick(N{}, Y{}) : pick(N{}, N{}));
-  const int smem = by_keys ? kTcSmemByKeys : kTcSmem;
+  const int smem = kTcSmem;
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -20;
   // Short calls start behind the stream's last kernel (512 tokens, 8 heads, causal 16.4 -> 15.6 us); the long ones have nothing to gain
   // (8192 tokens, 32 / 8 heads, causal 551 -> 558).
