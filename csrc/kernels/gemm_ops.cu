@@ -972,9 +972,17 @@ int make_plan(const IrisGemmDesc* d, Plan& p) {
   }
   if (is_fp8(d)) {
     // block-scaled e4m3 tiles are 224 (or 128) wide: two accumulator buffers plus the scale cells fill TMEM.
-    // CTA pairs only on request.
+    // CTA pairs on request, and for a local GEMM whose main loop is long enough for the 1.2 us that a cluster costs at its ends: long K,
+    // with weights of 28 M elements or 4e10 products. Single tiles / pairs, us, each back to back at first and then for a while (power cap):
+    //   K = 8192   16 x 3584  35.2 / 33.8    200 x 8192  28.6 / 25.4    4096 x 3584  113.8 / 108.4    8192 x 8192  504 / 456
+    //              512 x 1024  22.1 / 24.9   4096 x 1024  61.9 / 62.9   8192 x 1024  90.0 / 79.7
+    //   K = 4096   1024 x 3584  16.3 / 16.6  1024 x 8192  33.6 / 33.4   3000 x 3584  45.1 / 43.4     8192 x 8192  247 / 237
+    //   K = 1024   4096 x 8192  34.3 / 36.2  8192 x 8192  77.9 / 78.6
     if (d->bn != 0 && d->bn != 224 && d->bn != 128) return -5;
-    choose_tile(d->M, d->N, p.gemm_ctas, d->bn == 128 ? 128 : 224, d->two_sm == 2 ? 2 : 1, pair_ok && d->bn != 128, p.bn, p.pair);
+    const double weights = (double)d->N * d->K;
+    const bool long_loop = d->op == IRIS_GEMM_LOCAL && d->K >= 4096 && (weights >= 28e6 || weights * d->M >= 4e10);
+    const bool pairs = d->two_sm == 2 || (d->two_sm == 0 && long_loop);
+    choose_tile(d->M, d->N, p.gemm_ctas, d->bn == 128 ? 128 : 224, pairs ? 2 : 1, pair_ok && d->bn != 128, p.bn, p.pair);
   } else {
     choose_tile(d->M, d->N, p.gemm_ctas, d->bn, d->two_sm, pair_ok, p.bn, p.pair);
   }
