@@ -37,6 +37,60 @@ namespace {
 constexpr unsigned kBehindMax = 1024;
 constexpr int kUnroll = 4;      // pairs of blocks a warp has in flight (the reduction below is written for four)
 
+// The four blocks' maxima by halving: each exchange leaves a lane with half of its blocks, until four lanes share one
+// block; they work its exponent out once, and everybody fetches the four exponents. Returns that of block sub / 4.
+template <typename T>
+__device__ __forceinline__ int shared_exponent(const Raw8<T> (&raw)[kUnroll], int sub) {
+  float amax[kUnroll];
+#pragma unroll
+  for (int i = 0; i < kUnroll; ++i) amax[i] = block_amax_lane(raw[i]);
+  const bool hi8 = sub & 8, hi4 = sub & 4;
+  float m0 = hi8 ? amax[2] : amax[0], m1 = hi8 ? amax[3] : amax[1];
+  m0 = fmaxf(m0, __shfl_xor_sync(0xffffffffu, hi8 ? amax[0] : amax[2], 8));
+  m1 = fmaxf(m1, __shfl_xor_sync(0xffffffffu, hi8 ? amax[1] : amax[3], 8));
+  float mine = fmaxf(hi4 ? m1 : m0, __shfl_xor_sync(0xffffffffu, hi4 ? m0 : m1, 4));
+  mine = fmaxf(mine, __shfl_xor_sync(0xffffffffu, mine, 2));
+  mine = fmaxf(mine, __shfl_xor_sync(0xffffffffu, mine, 1));
+  return scale_exponent(mine);
+}
+
+// Rows of whole blocks on 16-byte boundaries: a warp takes eight blocks of ONE row, so its addresses are one base and constants.
+// The general kernel below spends half of its instructions on rows and columns that change from block to block, and it is
+// bound by issue slots (4096 x 8192 bf16: 24.0 us at 0.78 instructions per cycle and scheduler; this one NNN).
+template <typename T>
+__global__ void __launch_bounds__(128) quantize_rows_kernel(const T* __restrict__ x, int64_t ldx, uint8_t* __restrict__ q, int64_t ldq,
+                                                             float* __restrict__ scale, uint8_t* __restrict__ atoms, uint8_t* __restrict__ rows,
+                                                             int64_t ld_rows, int M, int M_pad, int KB, int groups) {
+  if (gridDim.x <= kBehindMax) iris::ptx::pdl_trigger();
+  iris::ptx::pdl_wait();
+  const unsigned unit = blockIdx.x * 4 + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31, sub = lane & 15;
+  const int row = (int)(unit / (unsigned)groups), kb0 = (int)(unit % (unsigned)groups) * (2 * kUnroll) + (lane >> 4);
+  if (row >= M_pad) return;
+  Raw8<T> raw[kUnroll];
+  const T* src = x + (int64_t)row * ldx + kb0 * 128 + sub * 8;
+#pragma unroll
+  for (int i = 0; i < kUnroll; ++i) raw[i].load(src + i * 256, row < M && kb0 + 2 * i < KB ? 8 : 0, 2);
+  const int e_mine = shared_exponent(raw, sub);       // of block sub / 4
+  const int kb_mine = kb0 + 2 * (sub >> 2);
+  if ((sub & 3) == 0 && kb_mine < KB) {               // whose scale one of the four lanes writes
+    if (row < M) {
+      if (scale) scale[(int64_t)row * KB + kb_mine] = exp2f((float)e_mine);
+      if (rows) rows[(int64_t)row * ld_rows + kb_mine] = (uint8_t)(e_mine + 127);
+    }
+    if (atoms) {
+      const uint32_t byte = row < M ? (uint32_t)(e_mine + 127) : 127u;      // rows past M: scale 1
+      *(uint32_t*)(atoms + ((int64_t)(row >> 7) * KB + kb_mine) * 512 + (row & 31) * 16 + ((row >> 5) & 3) * 4) = byte * 0x01010101u;
+    }
+  }
+  uint8_t* dst = q + (int64_t)row * ldq + kb0 * 128 + sub * 8;
+#pragma unroll
+  for (int i = 0; i < kUnroll; ++i) {
+    const int e = __shfl_sync(0xffffffffu, e_mine, (lane & 16) + i * 4);
+    if (row < M && kb0 + 2 * i < KB) *(uint2*)(dst + i * 256) = quantised8(raw[i], e);
+  }
+}
+
 template <typename T>
 __global__ void __launch_bounds__(128) quantize_1x128_pow2_kernel(const T* __restrict__ x, int64_t ldx, uint8_t* __restrict__ q, int64_t ldq,
                                                                    float* __restrict__ scale, uint8_t* __restrict__ atoms,
@@ -62,19 +116,8 @@ __global__ void __launch_bounds__(128) quantize_1x128_pow2_kernel(const T* __res
     raw[i].load(x + (int64_t)row * ldx + k0, n_valid, x_aligned);
     for (kb += 2; kb >= KB; kb -= KB) ++row;
   }
-  // The four blocks' maxima by halving: each exchange leaves a lane with half of its blocks, until four lanes share one
-  // block; they work its exponent out once, and everybody fetches the four exponents.
-  float amax[kUnroll];
-#pragma unroll
-  for (int i = 0; i < kUnroll; ++i) amax[i] = block_amax_lane(raw[i]);
   const bool hi8 = sub & 8, hi4 = sub & 4;
-  float m0 = hi8 ? amax[2] : amax[0], m1 = hi8 ? amax[3] : amax[1];
-  m0 = fmaxf(m0, __shfl_xor_sync(0xffffffffu, hi8 ? amax[0] : amax[2], 8));
-  m1 = fmaxf(m1, __shfl_xor_sync(0xffffffffu, hi8 ? amax[1] : amax[3], 8));
-  float mine = fmaxf(hi4 ? m1 : m0, __shfl_xor_sync(0xffffffffu, hi4 ? m0 : m1, 4));
-  mine = fmaxf(mine, __shfl_xor_sync(0xffffffffu, mine, 2));
-  mine = fmaxf(mine, __shfl_xor_sync(0xffffffffu, mine, 1));
-  const int e_mine = scale_exponent(mine);           // of block sub / 4
+  const int e_mine = shared_exponent(raw, sub);       // of block sub / 4
   if ((sub & 3) == 0) {                               // whose scale one of the four lanes writes
     const int r = hi8 ? (hi4 ? rows_u[3] : rows_u[2]) : (hi4 ? rows_u[1] : rows_u[0]);
     const int b = hi8 ? (hi4 ? kbs_u[3] : kbs_u[2]) : (hi4 ? kbs_u[1] : kbs_u[0]);
@@ -126,10 +169,20 @@ static int quantize_launch(const void* x, int64_t ldx, int32_t dtype, void* q, i
     return bits % big == 0 ? 2 : (bits % small == 0 ? 1 : 0);
   };
   const int xa = level(x, ldx * esz, 16, 8), qa = level(q, ldq, 8, 4);
+  // by rows while at most a fifth of a warp's eight blocks fall behind the row's end
+  const int groups = (KB + 2 * kUnroll - 1) / (2 * kUnroll);
+  const bool by_rows = xa == 2 && qa == 2 && K % 128 == 0 && 5 * KB >= 4 * groups * 2 * kUnroll && (int64_t)M_pad * groups < (1ll << 31);
   int r = 0;
   auto run = [&](auto* typed) {
     using T = std::remove_cv_t<std::remove_pointer_t<decltype(typed)>>;
-    if (blocks <= kBehindMax)
+    if (by_rows) {
+      const unsigned n = (unsigned)(((int64_t)M_pad * groups + 3) / 4);
+      if (n <= kBehindMax)
+        r = launch_pdl(quantize_rows_kernel<T>, dim3(n), 128, 0, s, (const T*)typed, ldx, (uint8_t*)q, ldq, scale, (uint8_t*)atoms, (uint8_t*)rows, ld_rows,
+                       M, M_pad, KB, groups);
+      else
+        quantize_rows_kernel<T><<<n, 128, 0, s>>>(typed, ldx, (uint8_t*)q, ldq, scale, (uint8_t*)atoms, (uint8_t*)rows, ld_rows, M, M_pad, KB, groups);
+    } else if (blocks <= kBehindMax)
       r = launch_pdl(quantize_1x128_pow2_kernel<T>, dim3((unsigned)blocks), 128, 0, s, (const T*)typed, ldx, (uint8_t*)q, ldq, scale, (uint8_t*)atoms,
                      (uint8_t*)rows, ld_rows, M, M_pad, K, KB, xa, qa);
     else

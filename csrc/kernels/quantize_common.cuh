@@ -6,6 +6,7 @@
 #include <cuda_fp16.h>
 #include <cuda_fp8.h>
 #include <stdint.h>
+#include <type_traits>
 
 namespace {
 
@@ -72,18 +73,39 @@ __device__ __forceinline__ int block_exponent(const Raw8<T>& raw) {
   for (int o = 8; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
   return scale_exponent(amax);
 }
+// NaN counts as the format's lowest value. 16-bit types: -inf in its place, two elements at a time; fp32 is left alone.
+template <typename T>
+__device__ __forceinline__ Raw8<T> nan_lowest(const Raw8<T>& raw) {
+  if constexpr (sizeof(T) == 4) return raw;
+  else {
+    using T2 = std::conditional_t<std::is_same<T, __half>::value, __half2, __nv_bfloat162>;
+    const uint32_t inf = std::is_same<T, __half>::value ? 0xfc00fc00u : 0xff80ff80u;
+    Raw8<T> out;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) ((T2*)out.w)[i] = __hmax2(((const T2*)raw.w)[i], *(const T2*)&inf);
+    return out;
+  }
+}
+// Four values as e4m3, the first in the lowest byte (saturating at 448).
+__device__ __forceinline__ uint32_t e4m3x4(float a, float b, float c, float d) {
+  uint32_t r;
+  asm("{\n\t.reg .b16 lo, hi;\n\tcvt.rn.satfinite.e4m3x2.f32 lo, %2, %1;\n\tcvt.rn.satfinite.e4m3x2.f32 hi, %4, %3;\n\tmov.b32 %0, {lo, hi};\n\t}"
+      : "=r"(r) : "f"(a), "f"(b), "f"(c), "f"(d));
+  return r;
+}
 // The lane's eight values divided by 2^e, as e4m3.
 template <typename T>
 __device__ __forceinline__ uint2 quantised8(const Raw8<T>& raw, int e) {
   const float inv = e == 127 ? 0x1p-127f : __int_as_float((127 - e) << 23);      // 2^-e
-  uint32_t packed[2] = {0u, 0u};
+  const Raw8<T> clean = nan_lowest(raw);
+  float v[8];
 #pragma unroll
-  for (int j = 0; j < 8; j += 2) {
-    // (the conversion saturates at 448; the maximum is for the lower end's sake of NaN, which counts as -448)
-    const float2 v = make_float2(fmaxf(raw.get(j) * inv, -448.f), fmaxf(raw.get(j + 1) * inv, -448.f));
-    packed[j >> 2] |= (uint32_t)__nv_cvt_float2_to_fp8x2(v, __NV_SATFINITE, __NV_E4M3) << (8 * (j & 3));
+  for (int j = 0; j < 8; ++j) v[j] = clean.get(j) * inv;
+  if constexpr (sizeof(T) == 4) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v[j] = fmaxf(v[j], -448.f);      // (NaN becomes -448)
   }
-  return make_uint2(packed[0], packed[1]);
+  return make_uint2(e4m3x4(v[0], v[1], v[2], v[3]), e4m3x4(v[4], v[5], v[6], v[7]));
 }
 
 }  // namespace

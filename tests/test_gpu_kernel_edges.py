@@ -68,6 +68,28 @@ def test_activation_passes_match_fp64(dtype, name, shape):
         assert ((got.double() - want).abs() <= ulp * want.abs() + 4e-6 * (1 + dh.double().abs()) + tiny).all()
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("M,KB", [(1, 8), (3, 7), (127, 16), (129, 13), (130, 9), (300, 24), (257, 40), (2050, 8)])
+def test_quantiser_by_rows_equals_the_general_one(dtype, M, KB):
+    """Aligned rows of whole blocks go eight blocks of a row to a warp (7, 8, 13, 16 ... blocks; 9 do not); the same values a few elements off the
+    boundary take the general kernel: every value, scale and scale atom has to be the same, with NaN, infinities and zeros among them."""
+    from iris_b200.ops import quantize_activation
+
+    K = KB * 128
+    base = torch.zeros(M * (K + 8) + 8, device="cuda", dtype=dtype)
+    x = torch.randn(M, K, device="cuda", generator=_gen(M + KB)) * torch.logspace(-6, 4, M, device="cuda")[:, None]
+    x[0, :128] = 0
+    x[M // 2, 5], x[M - 1, K - 1], x[M // 3, K // 2] = float("nan"), float("inf"), -float("inf")
+    x = x.to(dtype)
+    off = base[4:4 + M * K].view(M, K)                # 8 or 16 bytes off a 16-byte boundary's multiple: rows take 8-byte loads at most
+    if dtype == torch.float32:
+        off = base[2:2 + M * K].view(M, K)
+    off.copy_(x)
+    assert x.data_ptr() % 16 == 0 and off.data_ptr() % 16 == 8
+    a, b = quantize_activation(x), quantize_activation(off)
+    assert torch.equal(a.q.view(torch.uint8), b.q.view(torch.uint8)) and torch.equal(a.scale, b.scale) and torch.equal(a.sf(), b.sf())
+
+
 # ------------------------------------------------------------------------------------ kernels that start behind their predecessor
 @pytest.mark.parametrize("rows", [16, 300, 2000])
 def test_chains_of_early_started_kernels(ctx, rows):
