@@ -7,8 +7,8 @@
 //      partial output and its log-sum-exp per run. The tiles of all (sequence, KV head) pairs form one list that
 //      is cut into equal pieces, one per CTA, on the device, from the lengths: a CTA may end one pair and begin the next, a pair
 //      may be spread over many CTAs. (With the same number of splits for every sequence, the CTAs of the longest
-//      one finished last: 32 sequences of 8192 to 32768 positions, 640 us where the bytes take 404; now 450. One
-//      sequence of 32768: 512 CTAs on 296 places; 53 us, now 39.)
+//      one finished last: 32 sequences of 8192 to 32768 positions, 640 us where the bytes take 404; now 423. One
+//      sequence of 32768: 512 CTAs on 296 places; 53 us, now 32.)
 //      K/V stream through a ring of swizzled shared-memory tiles; QK^T and PV run on tensor
 //      cores with the query heads of the group as the M dimension (each K/V byte is read from HBM
 //      exactly once; the kernel is bound by HBM bandwidth). Two ways of filling the ring: a
@@ -308,18 +308,21 @@ struct Attend {
       }
     }
   }
-  // Merges the four warps (each saw a quarter of the positions) and writes the partial of the run. `sm_o` is 32 KB that
+  // Merges the four warps (each saw a quarter of the positions) and writes the partial of the run (3 us at the end of every run while rows
+  // stored met in one bank and every thread worked the weights out per value; with this and the fold below a sequence of 32768
+  // positions 39.0 -> 32.1 us). `sm_o` is 32 KB that
   // nobody else uses, `sm_ml` 512 bytes; the computing warps' threads call it together (named barrier 1).
   __device__ __forceinline__ void finish(const DecodeArgs& a, const Run& run, float* sm_o, float* sm_ml, int warp, int lane) {
+    // rows of 128 floats, the column XORed by the row times 8: eight rows stored and one row read meet different banks
     const int r0 = lane >> 2, c0 = (lane & 3) * 2;
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
-      float* base = sm_o + (warp * 16) * kD + i * 8 + c0;
+      float* base = sm_o + (warp * 16) * kD + ((i * 8 + c0) ^ (r0 << 3));
       if constexpr (kRows8) {
-        base[r0 * kD] = o[i][0] + o[i][2]; base[r0 * kD + 1] = o[i][1] + o[i][3];
+        *(float2*)(base + r0 * kD) = make_float2(o[i][0] + o[i][2], o[i][1] + o[i][3]);
       } else {
-        base[r0 * kD] = o[i][0]; base[r0 * kD + 1] = o[i][1];
-        base[(r0 + 8) * kD] = o[i][2]; base[(r0 + 8) * kD + 1] = o[i][3];
+        *(float2*)(base + r0 * kD) = make_float2(o[i][0], o[i][1]);
+        *(float2*)(base + (r0 + 8) * kD) = make_float2(o[i][2], o[i][3]);
       }
     }
     if ((lane & 3) == 0) {
@@ -328,22 +331,25 @@ struct Attend {
     }
     ptx::named_barrier(1, kWarps * 32);
     const int tid = warp * 32 + lane;
-    for (int idx = tid; idx < run.heads_here * kD; idx += kWarps * 32) {
-      const int h = idx / kD, d = idx - h * kD;
+    // a warp per head, four columns 32 apart per lane
+#pragma unroll 2
+    for (int h = warp; h < run.heads_here; h += kWarps) {
+      float2 ml[kWarps];
       float m = -INFINITY;
 #pragma unroll
-      for (int w = 0; w < kWarps; ++w) m = fmaxf(m, sm_ml[(w * 16 + h) * 2]);
-      float l = 0.f, acc = 0.f;
+      for (int w = 0; w < kWarps; ++w) { ml[w] = *(const float2*)(sm_ml + (w * 16 + h) * 2); m = fmaxf(m, ml[w].x); }
+      float l = 0.f, acc[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
       for (int w = 0; w < kWarps; ++w) {
-        const float mw = sm_ml[(w * 16 + h) * 2];
-        const float sc = mw == -INFINITY ? 0.f : exp2f(mw - m);
-        l += sm_ml[(w * 16 + h) * 2 + 1] * sc;
-        acc += sm_o[(w * 16 + h) * kD + d] * sc;
+        const float sc = ml[w].x == -INFINITY ? 0.f : exp2f(ml[w].x - m);
+        l += ml[w].y * sc;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[j] += sm_o[(w * 16 + h) * kD + ((j * 32 + lane) ^ ((h & 7) << 3))] * sc;
       }
       float* dst = a.partial + (((size_t)run.b * a.Hq + run.h0 + h) * a.splits + run.slot) * (kD + 1);
-      dst[d] = l > 0.f ? acc / l : 0.f;
-      if (d == 0) dst[kD] = l > 0.f ? m + log2f(l) : -INFINITY;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) dst[j * 32 + lane] = l > 0.f ? acc[j] / l : 0.f;
+      if (lane == 0) dst[kD] = l > 0.f ? m + log2f(l) : -INFINITY;
     }
     // the run that begins a pair marks the places no run fills
     const int spare = a.splits - run.n_slots;
@@ -623,15 +629,59 @@ __global__ void __launch_bounds__(kD) decode_exchange_kernel(const __grid_consta
 // exchange == 2 it is what a decode over a KV shard returns when the cross-rank merge is done elsewhere, e.g. by an
 // all-gather of the partial results as in the reference's RCCL baseline
 // (examples/benchmark/reference/flash_decode_rccl/flash_decode_layer_rccl.py:100-130).
-__global__ void __launch_bounds__(kD) decode_local_finish_kernel(const float* partial, void* out, float* out_lse, int splits, int is_fp16) {
-  const int it = blockIdx.x, d = threadIdx.x;
-  __shared__ float s_part[kD];
+// A block per (sequence, head); kGroups threads per column share its places, and a thread's loads are all in flight together: first the
+// places' weights, then the values that have one. Few heads with many places wait for latency only (one sequence of 32768 positions, 64
+// heads with 37 places each: 3.8 us with one thread per column and eight loads in flight); with many heads one
+// thread per column reads what there is to read.
+template <int kGroups, int kAhead>
+__global__ void __launch_bounds__(kD * kGroups) decode_local_finish_kernel(const float* partial, void* out, float* out_lse, int splits, int is_fp16) {
+  const int it = blockIdx.x, d = threadIdx.x % kD, g = threadIdx.x / kD;
+  __shared__ float s_o[kGroups][kD];
+  __shared__ float2 s_ml[kGroups];
   ptx::pdl_wait();                                         // the partials are complete from here on
-  float o, lse;
-  combine_splits(partial + (size_t)it * splits * (kD + 1), splits, s_part, o, lse);
+  const float* p = partial + (size_t)it * splits * (kD + 1);
+  float m = -INFINITY, l = 0.f, acc = 0.f;
+  for (int s0 = g; s0 < splits; s0 += kGroups * kAhead) {
+    float w[kAhead], v[kAhead], top = m;
+#pragma unroll
+    for (int k = 0; k < kAhead; ++k) {
+      const int s = s0 + k * kGroups;
+      w[k] = s < splits ? __ldcg(p + (size_t)s * (kD + 1) + kD) : -INFINITY;
+    }
+#pragma unroll
+    for (int k = 0; k < kAhead; ++k) {                     // (a place that no run filled holds no numbers)
+      v[k] = w[k] != -INFINITY ? __ldcg(p + (size_t)(s0 + k * kGroups) * (kD + 1) + d) : 0.f;
+      top = fmaxf(top, w[k]);
+    }
+    if (top == -INFINITY) continue;
+    const float keep = exp2f(m - top);
+    m = top; l *= keep; acc *= keep;
+#pragma unroll
+    for (int k = 0; k < kAhead; ++k) {
+      const float e = exp2f(w[k] - m);
+      l += e; acc += e * v[k];
+    }
+  }
+  if constexpr (kGroups > 1) {
+    s_o[g][d] = acc;
+    if (d == 0) s_ml[g] = make_float2(m, l);
+    __syncthreads();
+    if (g) return;
+    float top = -INFINITY;
+#pragma unroll
+    for (int k = 0; k < kGroups; ++k) top = fmaxf(top, s_ml[k].x);
+    l = acc = 0.f;
+#pragma unroll
+    for (int k = 0; k < kGroups; ++k) {
+      const float e = s_ml[k].x == -INFINITY ? 0.f : exp2f(s_ml[k].x - top);
+      l += s_ml[k].y * e; acc += s_o[k][d] * e;
+    }
+    m = top;
+  }
+  const float o = l > 0.f ? acc / l : 0.f;
   if (is_fp16) ((__half*)out)[(size_t)it * kD + d] = __float2half_rn(o);
   else ((__nv_bfloat16*)out)[(size_t)it * kD + d] = __float2bfloat16_rn(o);
-  if (out_lse && d == 0) out_lse[it] = lse == -INFINITY ? -INFINITY : lse / kLog2e;
+  if (out_lse && d == 0) out_lse[it] = l > 0.f ? (m + log2f(l)) / kLog2e : -INFINITY;
 }
 
 // Split-K pass over `a.B` sequences, in launches of up to kMaxSeqs, on two CTAs per SM.
@@ -728,7 +778,10 @@ int iris_flash_decode(const IrisDecodeDesc* d, void* stream) {
   if (r) return r;
   if (!d->exchange) return 0;
   if (d->exchange == 2 || d->ctx.world <= 1) {
-    return launch_pdl(decode_local_finish_kernel, dim3(d->B * d->Hq), kD, 0, s, (const float*)d->partial, d->out, d->out_lse, (int)d->splits, a.is_fp16);
+    const int items = d->B * d->Hq;
+    if (items <= 296 && d->splits > 8)
+      return launch_pdl(decode_local_finish_kernel<4, 10>, dim3(items), 4 * kD, 0, s, (const float*)d->partial, d->out, d->out_lse, (int)d->splits, a.is_fp16);
+    return launch_pdl(decode_local_finish_kernel<1, 8>, dim3(items), kD, 0, s, (const float*)d->partial, d->out, d->out_lse, (int)d->splits, a.is_fp16);
   }
   ExchangeArgs x;
   memcpy(&x.ctx, &d->ctx, sizeof(DeviceContext));
