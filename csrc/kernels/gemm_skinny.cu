@@ -203,7 +203,9 @@ __global__ void __launch_bounds__(kSkinnyThreads) skinny_gemm_kernel(const __gri
           for (int e = 0; e < 4; ++e) dst[e] = h[e];
       }
     }
-    ptx::cluster_sync();                     // a CTA's shared memory stays until every CTA has read it
+    // a CTA's shared memory stays until every CTA has read it (with a release here, the CTA stayed until its output was written: 1.5 us)
+    __syncwarp();
+    ptx::cluster_sync_relaxed();
   } else {
     __syncthreads();
   }

@@ -392,6 +392,11 @@ IRIS_D uint32_t cluster_ctarank() {
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
   return r;
 }
+// The same without memory ordering: no wait for this thread's outstanding stores. Enough where a CTA's shared memory only has to
+// stay until the others' loads from it have returned (a value that was used has).
+IRIS_D void cluster_sync_relaxed() {
+  asm volatile("barrier.cluster.arrive.relaxed.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
+}
 IRIS_D void cluster_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
