@@ -15,7 +15,8 @@
 //                loop) wait for an expert's arrivals, then multiply its rows by the expert's fused
 //                gate|up weight and write silu(gate) * up
 //                (the fusion the reference leaves as NotImplementedError, moe.py:285-286).
-//                One rank: a gather kernel copies the rows into expert order first, and all CTAs are GEMM CTAs
+//                One rank: a gather kernel copies the rows into expert order first, and both grouped GEMMs are those
+//                of moe_experts.cuh
 //   5 grouped GEMM 2 + combine, ONE kernel: down projection whose epilogue stores every output row
 //                straight into the (token, k) slot of the token's home rank; cross-rank round at exit
 //   6 reduce     out[t] = sum_k weight[t, k] * slot[t, k]   (the reference's sum is unweighted)
@@ -277,20 +278,24 @@ __global__ void __launch_bounds__(1024) moe_prep_kernel(const float* __restrict_
 // With one rank every pair's row stays here, so nothing is sent: the token rows are copied into expert order by a
 // kernel of their own and the grouped GEMM runs on every SM. The communication CTAs of the multi-rank form cost the
 // GEMM 16 of 148 SMs for its whole run, and with few tokens their chain of one release per expert was what it waited
-// for (64 tokens, 32 experts, e4m3: stage 1 306 us, now 199; 4096 tokens bf16: 1808 us, now 1538 plus 89 for
+// for (64 tokens, 32 experts, e4m3: stage 1 306 us with them and 199 without; 4096 tokens bf16: 1808 us and 1538, plus 89 for
 // this copy, which is bound by the 470 MB it writes). A block reads a piece of one token's row once and stores it to the
 // token's K rows.
 __global__ void __launch_bounds__(256) moe_gather_kernel(const uint8_t* __restrict__ x, uint8_t* __restrict__ inbox, int row16,
                                                          const int32_t* __restrict__ pos_of, int K, int capacity) {
-  ptx::pdl_wait();
-  ptx::pdl_trigger();
   __shared__ int32_t dst[kMaxTopK];
   const int t = blockIdx.x;
+  // the tokens were complete before the kernel in front got past its own pdl_wait: the first piece is read while it runs (16 tokens,
+  // 16 experts of 2048 x 1024: 45.0 -> 43.9 us a pass; quantising e4m3 rows that early was slower, 30.6 -> 31.5)
+  const uint4* src = (const uint4*)x + (size_t)t * row16;
+  const int c0 = blockIdx.y * blockDim.x + threadIdx.x;
+  uint4 v = c0 < row16 ? __ldcg(src + c0) : make_uint4(0, 0, 0, 0);
+  ptx::pdl_wait();
+  ptx::pdl_trigger();
   if (threadIdx.x < K) dst[threadIdx.x] = pos_of[(size_t)t * K + threadIdx.x];
   __syncthreads();
-  const uint4* src = (const uint4*)x + (size_t)t * row16;
-  for (int c = blockIdx.y * blockDim.x + threadIdx.x; c < row16; c += gridDim.y * blockDim.x) {
-    const uint4 v = __ldg(src + c);
+  for (int c = c0; c < row16; c += gridDim.y * blockDim.x) {
+    if (c != c0) v = __ldcg(src + c);
     for (int k = 0; k < K; ++k)
       if (dst[k] < capacity) ((uint4*)inbox)[(size_t)dst[k] * row16 + c] = v;
   }
