@@ -9,7 +9,7 @@
 //   * K is split over the CTAs of a cluster (up to 8). Each CTA keeps its partial tile in its own shared memory as fp32
 //     and after one cluster barrier every CTA adds up a share of the tokens over distributed shared memory, in rank order:
 //     no workspace, no atomics, the same bits on every run, one launch;
-//   * the stage ring takes about 100 KB, so two CTAs fit an SM and clusters pack into any GPC.
+//   * the stage ring takes about 100 KB, so two CTAs fit an SM and clusters pack into any GPC (wider token tiles: see skinny_one_per_sm).
 // The reference has no counterpart (its GEMMs go through tritonblas, iris/ops/matmul_all_reduce.py:95-105).
 #include "gemm_host.cuh"
 #include "gemm_skinny.h"
@@ -215,16 +215,28 @@ __global__ void __launch_bounds__(kSkinnyThreads) skinny_gemm_kernel(const __gri
 
 }  // namespace
 
-// Up to 128 tokens the ring is kept to about 100 KB and two CTAs share an SM; wider token tiles take an SM each, and then
+// Up to 64 tokens, and mostly up to 128, the ring is kept to about 100 KB and two CTAs share an SM; wider token tiles take an SM each, and then
 // clusters of 8 leave SMs of a GPC unused (256 x 2000 x 3000: 16 clusters of 8 did not fit at once, 26 us), so 4 is
 // the limit unless there are few of them.
-int iris_gemm_skinny_split(int M, int N, int K) {
-  const int tiles = ceil_div(N, 128), kb = ceil_div(K, kBK), tn = ceil_div(M, 16) * 16;
-  const int slots = sm_count() * (tn <= 128 ? 2 : 1);
-  const int most = tn <= 128 || tiles <= 12 ? 8 : 4;
+static int split_for(int tiles, int kb, int slots, int most) {
   int s = 1;
   while (s < most && tiles * (s * 2) <= slots && kb >= 4 * (s * 2)) s *= 2;
   return s;
+}
+// 65 to 128 tokens fill 100 KB with three stages. Where CTAs that take an SM each, with six, still cover most of the chip, or a handful of
+// tiles is split by 8 either way, those are the faster ones (us, two CTAs per SM / one): 100 x 4096 x 2048 10.7 / 8.2, 128 x 3584 x 8192
+// 18.9 / 16.7, 100 x 4096 x 4096 13.7 / 12.6, 128 x 1024 x 8192 11.8 / 9.6, but 100 x 8192 x 8192 (64 tiles, split by 2 then) 27.4 / 28.8
+// and 100 x 2048 x 4096 (16 clusters of 8 do not fit at once) 10.2 / 14.4.
+static bool skinny_one_per_sm(int tn, int tiles, int kb) {
+  if (tn <= 64) return false;
+  if (tn > 128) return true;
+  const int s = split_for(tiles, kb, sm_count(), tiles <= 12 ? 8 : 4);
+  return tiles <= 12 || (s == 4 && tiles * s >= 96);
+}
+int iris_gemm_skinny_split(int M, int N, int K) {
+  const int tiles = ceil_div(N, 128), kb = ceil_div(K, kBK), tn = ceil_div(M, 16) * 16;
+  if (!skinny_one_per_sm(tn, tiles, kb)) return split_for(tiles, kb, 2 * sm_count(), 8);
+  return split_for(tiles, kb, sm_count(), tiles <= 12 ? 8 : 4);
 }
 
 // Where the split-K kernel is the faster one, both measured in us with weights that are not in L2 (main loop / this):
@@ -264,7 +276,7 @@ int iris_gemm_skinny(const IrisGemmDesc* d, cudaStream_t stream) {
   g.vec8 = ((uintptr_t)d->C & 7) == 0 && d->ldc % 4 == 0;
   const int S = iris_gemm_skinny_split(d->M, d->N, d->K);
   const int stage = kWTile + g.tn * (kBK * 2);
-  const int budget = g.tn <= 128 ? 104 * 1024 : 208 * 1024;
+  const int budget = skinny_one_per_sm(g.tn, ceil_div(g.N, 128), g.kblocks) ? 208 * 1024 : 104 * 1024;
   g.stages = budget / stage;
   if (g.stages > kMaxStages) g.stages = kMaxStages;
   const int ring = S > 1 && g.tn * 512 > g.stages * stage ? g.tn * 512 : g.stages * stage;

@@ -90,6 +90,23 @@ def test_quantiser_by_rows_equals_the_general_one(dtype, M, KB):
     assert torch.equal(a.q.view(torch.uint8), b.q.view(torch.uint8)) and torch.equal(a.scale, b.scale) and torch.equal(a.sf(), b.sf())
 
 
+@pytest.mark.parametrize("M", [64, 65, 100, 128, 129])
+@pytest.mark.parametrize("N,K", [(1000, 2048), (1544, 3000), (2048, 4096), (3072, 2112), (4096, 2048), (4744, 4096)])
+@pytest.mark.parametrize("linear", [False, True])
+def test_few_rows_on_both_ring_depths(M, N, K, linear):
+    """Both sides of the rules that give a CTA an SM of its own (64 / 65 and 128 / 129 rows; up to 12 column tiles, 24 to 37, others), ragged
+    tiles and K blocks. One rounding to bf16 (2^-8 of the value); fp32 sums of K products whose magnitudes add up to S, in any order: K 2^-24 S."""
+    from iris_b200.ops import matmul
+
+    g = _gen(M + N + K)
+    a = torch.randn(M, K, device="cuda", generator=g).bfloat16()
+    w = (torch.randn(N, K, device="cuda", generator=g) * K ** -0.5).bfloat16()
+    b = w.t() if linear else w.t().contiguous()
+    got, want = matmul(a, b).double(), a.double() @ w.double().t()
+    sums = a.double().abs() @ w.double().abs().t()
+    assert ((got - want).abs() <= 2.0 ** -8 * want.abs() + K * 2.0 ** -24 * sums).all()
+
+
 # ------------------------------------------------------------------------------------ kernels that start behind their predecessor
 @pytest.mark.parametrize("rows", [16, 300, 2000])
 def test_chains_of_early_started_kernels(ctx, rows):
