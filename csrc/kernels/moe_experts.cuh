@@ -290,7 +290,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kXThreads, 1) expert
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
               const float gv = __uint_as_float(lo[2 * i + e]), uv = __uint_as_float(hi[2 * i + e]);
-              v[e] = __fdividef(gv, 1.f + __expf(-gv)) * uv;
+              v[e] = gv / (1.f + __expf(-gv)) * uv;
             }
             const __nv_bfloat162 p = __floats2bfloat162_rn(v[0], v[1]);
             h[i] = *(const uint32_t*)&p;

@@ -271,6 +271,29 @@ def test_moe_one_rank_in_a_cuda_graph(ctx, T, fp8):
     ctx.heap_release(mark)
 
 
+@pytest.mark.parametrize("fp8", [False, True])
+@pytest.mark.parametrize("T", [3, 70])
+def test_moe_one_rank_swiglu_divides_exactly(ctx, fp8, T):
+    """Gates around -88, where 1 + exp(-gate) lies above 2^126 and a fast division returns zero, against up values of 2^120. Products and sums are exact
+    here; __expf is within 105 ulp (1.3e-5) there; bf16 rounds the hidden value and the output (2^-9 each), e4m3 the hidden value (2^-4)."""
+    from iris_b200.models import MoELayer
+
+    D, F = 256, 128
+    gate = torch.full((F,), -88.0, device="cuda") if fp8 else -80.0 - 0.5 * (torch.arange(F, device="cuda") % 18)
+    w_gate, w_up, w_down = torch.zeros(1, D, F, device="cuda"), torch.zeros(1, D, F, device="cuda"), torch.zeros(1, F, D, device="cuda")
+    w_gate[0, 0], w_up[0, 0] = gate, 2.0 ** 120
+    w_down[0, :, :F] = torch.eye(F, device="cuda")
+    x = torch.zeros(T, D, device="cuda", dtype=torch.bfloat16)
+    x[:, 0] = 1
+    mark = ctx.heap_mark()
+    layer = MoELayer(ctx, D, F, 1, 1, max_tokens=T, w_gate=w_gate.bfloat16(), w_up=w_up.bfloat16(), w_down=w_down.bfloat16(), fp8=fp8)
+    got = layer(x, torch.zeros(T, 1, device="cuda"))[:, :F].double()
+    g = gate.double()
+    want = g / (1 + torch.exp(-g)) * 2.0 ** 120
+    assert ((got - want).abs() <= ((2.0 ** -4 if fp8 else 0.0) + 2.0 ** -8 + 2e-5) * want.abs()).all()
+    ctx.heap_release(mark)
+
+
 # ------------------------------------------------------------------------------------ attention on one rank
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("S,Hq,Hkv", [(1, 2, 2), (64, 4, 2), (127, 8, 2), (128, 3, 1), (129, 4, 4), (257, 6, 2), (384, 5, 5), (1000, 8, 8), (2500, 16, 2),
