@@ -362,6 +362,32 @@ def test_decode_runs_cut_sequences_anywhere(ctx, tma, B, Hq, Hkv, page, lens):
     ctx.heap_release(mark)
 
 
+@pytest.mark.parametrize("B,L,low", [(1, 32768, 4096), (40, 512, 256)])
+@pytest.mark.parametrize("at", [5, 200])
+def test_decode_fold_ignores_places_of_no_weight(ctx, B, L, low, at):
+    """The first `low` positions score 524 powers of two below the others and one of them has an infinite value: the runs they lie in (at most 640 of the
+    4096 positions, 256 of 256) have weight zero and do not touch the result, in both forms of the fold. The others' values are equal: the
+    output is that value, rounded (P and the output to 2^-8 each)."""
+    from iris_b200.models import FlashDecodeLayer
+
+    Hq, page = 8, 64
+    blocks = L // page
+    q = torch.zeros(B, Hq, 128, device="cuda", dtype=torch.bfloat16)
+    k, v = torch.zeros(B, L, 128, device="cuda", dtype=torch.bfloat16), torch.zeros(B, L, 128, device="cuda", dtype=torch.bfloat16)
+    q[..., 0], k[:, :low, 0] = 64, -64
+    want = (1 + torch.arange(128, device="cuda") / 128).to(torch.bfloat16)
+    v[:, low:] = want
+    v[:, at] = float("inf")
+    table = torch.arange(B * blocks, device="cuda", dtype=torch.int32).view(B, blocks)
+    mark = ctx.heap_mark()
+    layer = FlashDecodeLayer(ctx, Hq, 1, max_batch=B)
+    out, lse = layer(q, k.view(B * blocks, page, 1, 128), v.view(B * blocks, page, 1, 128), torch.full((1, B), L, device="cuda", dtype=torch.int32), table,
+                     return_lse=True)
+    assert ((out.float() - want.float()).abs() <= 2 * 2.0 ** -8 * want.float()).all()
+    assert (lse - torch.tensor(float(L - low)).log().item()).abs().max().item() < 1e-3
+    ctx.heap_release(mark)
+
+
 @pytest.mark.parametrize("tma", [None, False])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("soft_cap", [0.0, 30.0])
