@@ -656,11 +656,11 @@ __global__ void __launch_bounds__(kD * kGroups) decode_local_finish_kernel(const
     if (top == -INFINITY) continue;
     // (a place whose weight vanishes counts nothing, whatever it holds: no zero is multiplied by an infinity)
     const float keep = exp2f(m - top);
-    m = top; l *= keep; acc = keep != 0.f ? acc * keep : 0.f;
+    m = top; l *= keep; acc = keep * (keep != 0.f ? acc : 0.f);
 #pragma unroll
     for (int k = 0; k < kAhead; ++k) {
       const float e = exp2f(w[k] - m);
-      l += e; acc += e != 0.f ? e * v[k] : 0.f;
+      l += e; acc += e * (e != 0.f ? v[k] : 0.f);
     }
   }
   if constexpr (kGroups > 1) {
@@ -675,7 +675,7 @@ __global__ void __launch_bounds__(kD * kGroups) decode_local_finish_kernel(const
 #pragma unroll
     for (int k = 0; k < kGroups; ++k) {
       const float e = s_ml[k].x == -INFINITY ? 0.f : exp2f(s_ml[k].x - top);
-      l += s_ml[k].y * e; acc += e != 0.f ? s_o[k][d] * e : 0.f;
+      l += s_ml[k].y * e; acc += (e != 0.f ? s_o[k][d] : 0.f) * e;
     }
     m = top;
   }

@@ -362,11 +362,11 @@ def test_decode_runs_cut_sequences_anywhere(ctx, tma, B, Hq, Hkv, page, lens):
     ctx.heap_release(mark)
 
 
-@pytest.mark.parametrize("B,L,low", [(1, 32768, 4096), (40, 512, 256)])
+@pytest.mark.parametrize("B,L,low", [(1, 32768, 4096), (40, 2048, 1024)])
 @pytest.mark.parametrize("at", [5, 200])
 def test_decode_fold_ignores_places_of_no_weight(ctx, B, L, low, at):
     """The first `low` positions score 524 powers of two below the others and one of them has an infinite value: the runs they lie in (at most 640 of the
-    4096 positions, 256 of 256) have weight zero and do not touch the result, in both forms of the fold. The others' values are equal: the
+    4096 positions, 320 of the 1024) have weight zero and do not touch the result, in both forms of the fold. The others' values are equal: the
     output is that value, rounded (P and the output to 2^-8 each)."""
     from iris_b200.models import FlashDecodeLayer
 
