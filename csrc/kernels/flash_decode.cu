@@ -402,7 +402,7 @@ __global__ void __launch_bounds__(kWarps * 32 + 32, 2) decode_splitk_tma_kernel(
         const int nbox = (rows + a.box_rows - 1) / a.box_rows;
         const int pos = pos0 + j * a.box_rows;
         int y = 0;
-        if (j < nbox) y = __ldg(bt + pos / a.page) * a.page + pos % a.page;      // looked up before the stage is waited for
+        if (j < nbox) y = bt[pos / a.page] * a.page + pos % a.page;      // looked up before the stage is waited for
         if (!__all_sync(0xffffffffu, ptx::mbar_wait(&empty[stage], ((it / kStages) & 1) ^ 1, kTmaWaitNs))) { fail(); return; }
         if (lane == 0) ptx::mbar_expect_tx(&full[stage], (uint32_t)(nbox * a.box_rows * 128 * 4));
         __syncwarp();

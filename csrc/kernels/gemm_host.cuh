@@ -77,10 +77,10 @@ struct Common {
 #pragma unroll
         for (int i = 0; i < 8; ++i) v[g + i] += bias_at(bias_col, col + g + i);
       } else if (!bias16) {
-        const float4 a = __ldg((const float4*)(bias_col + col + g)), b = __ldg((const float4*)(bias_col + col + g) + 1);
+        const float4 a = *(const float4*)(bias_col + col + g), b = *((const float4*)(bias_col + col + g) + 1);
         v[g] += a.x; v[g + 1] += a.y; v[g + 2] += a.z; v[g + 3] += a.w; v[g + 4] += b.x; v[g + 5] += b.y; v[g + 6] += b.z; v[g + 7] += b.w;
       } else {
-        const uint4 u = __ldg((const uint4*)((const uint16_t*)bias_col + col + g));
+        const uint4 u = *(const uint4*)((const uint16_t*)bias_col + col + g);
         const uint32_t w[4] = {u.x, u.y, u.z, u.w};
 #pragma unroll
         for (int i = 0; i < 4; ++i) {

@@ -67,7 +67,7 @@ struct MoeMeta {
 // of the same order (0 = no candidate, below -inf's), so a round is two warp reductions, the largest key and the lowest index
 // that has it; ten dependent shuffles took 300 cycles a round.
 template <int kPer>
-__device__ __forceinline__ void route_token(const float* __restrict__ row, int E, int K, int lane, int& my_i, float& my_w) {
+__device__ __forceinline__ void route_token(const float* row, int E, int K, int lane, int& my_i, float& my_w) {
   uint32_t key[kPer];
 #pragma unroll
   for (int i = 0; i < kPer; ++i) {
@@ -102,7 +102,7 @@ __device__ __forceinline__ void route_token(const float* __restrict__ row, int E
 // once per expert. With one global atomic per (token, k) the counters were the bottleneck: 4096 tokens, 32 experts,
 // top-8: 36 us, now 11.
 template <int kPer>
-__global__ void __launch_bounds__(512) router_topk_kernel(const float* __restrict__ logits, MoeDims dm, MoeMeta m) {
+__global__ void __launch_bounds__(512) router_topk_kernel(const float* logits, MoeDims dm, MoeMeta m) {
   ptx::pdl_wait();
   ptx::pdl_trigger();
   __shared__ int32_t hist[1024];
@@ -224,7 +224,7 @@ __global__ void moe_clear_kernel(MoeDims dm, MoeMeta m) {
 // (64 tokens, 32 experts: 18 us in four kernels, now 12). With more tokens the work of a single block would be the longer.
 constexpr int kPrepMaxTokens = 256;
 template <int kPer>
-__global__ void __launch_bounds__(1024) moe_prep_kernel(const float* __restrict__ logits, const __grid_constant__ DeviceContext ctx, MoeDims dm,
+__global__ void __launch_bounds__(1024) moe_prep_kernel(const float* logits, const __grid_constant__ DeviceContext ctx, MoeDims dm,
                                                         MoeMeta m, int32_t* pos_of) {
   ptx::pdl_wait();
   ptx::pdl_trigger();
@@ -281,8 +281,8 @@ __global__ void __launch_bounds__(1024) moe_prep_kernel(const float* __restrict_
 // for (64 tokens, 32 experts, e4m3: stage 1 306 us with them and 199 without; 4096 tokens bf16: 1808 us and 1538, plus 89 for
 // this copy, which is bound by the 470 MB it writes). A block reads a piece of one token's row once and stores it to the
 // token's K rows.
-__global__ void __launch_bounds__(256) moe_gather_kernel(const uint8_t* __restrict__ x, uint8_t* __restrict__ inbox, int row16,
-                                                         const int32_t* __restrict__ pos_of, int K, int capacity) {
+__global__ void __launch_bounds__(256) moe_gather_kernel(const uint8_t* x, uint8_t* inbox, int row16,
+                                                         const int32_t* pos_of, int K, int capacity) {
   __shared__ int32_t dst[kMaxTopK];
   const int t = blockIdx.x;
   // the tokens were complete before the kernel in front got past its own pdl_wait: the first piece is read while it runs (16 tokens,
@@ -303,9 +303,8 @@ __global__ void __launch_bounds__(256) moe_gather_kernel(const uint8_t* __restri
 
 // The same for e4m3 rows, from the 16-bit tokens: half a warp quantises one 128-column block of a token, stores the values to
 // the token's K rows and the scale byte, four times, to its cell of the scale atoms of each row's tile ([tile][K block][atoms]).
-__global__ void __launch_bounds__(256) moe_gather_quant_kernel(const __nv_bfloat16* __restrict__ x, uint8_t* __restrict__ inbox,
-                                                               uint8_t* __restrict__ inbox_sf, int atoms, MoeDims dm, MoeMeta m,
-                                                               const int32_t* __restrict__ pos_of) {
+__global__ void __launch_bounds__(256) moe_gather_quant_kernel(const __nv_bfloat16* x, uint8_t* inbox, uint8_t* inbox_sf, int atoms, MoeDims dm, MoeMeta m,
+                                                               const int32_t* pos_of) {
   ptx::pdl_wait();
   ptx::pdl_trigger();
   __shared__ int32_t dst[kMaxTopK], tile[kMaxTopK], cell[kMaxTopK];
@@ -584,7 +583,7 @@ struct GroupedGemm : Common {
 // Bound by the K rows it reads per token. One thread per eight columns of a token, the loads of all K rows issued
 // before the first is used (64 tokens of 7168, top-8: 12 us with one block per token, now 5; 4096 tokens: 80 us, the time
 // its 530 MB take).
-__global__ void __launch_bounds__(128) moe_reduce_kernel(const __nv_bfloat16* __restrict__ comb, const float* __restrict__ w, __nv_bfloat16* out,
+__global__ void __launch_bounds__(128) moe_reduce_kernel(const __nv_bfloat16* comb, const float* w, __nv_bfloat16* out,
                                                          int T, int K, int D) {
   ptx::pdl_wait();
   ptx::pdl_trigger();

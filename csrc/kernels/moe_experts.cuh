@@ -262,7 +262,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kXThreads, 1) expert
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           const int tk = c_first + 64 * i + lane;
-          pr[i] = tk < keep ? __ldg(g.pairs + u.row + tk) : -1;
+          pr[i] = tk < keep ? __ldcg(g.pairs + u.row + tk) : -1;
         }
       }
       if (live) {

@@ -59,8 +59,7 @@ __device__ __forceinline__ int shared_exponent(const Raw8<T> (&raw)[kUnroll], in
 // bound by issue slots (4096 x 8192 bf16: 24.0 us, 152 instructions per warp and 256 values; this one 18.1 us and 98, with NaN
 // replaced two values at a time and four conversions to a word).
 template <typename T>
-__global__ void __launch_bounds__(128) quantize_rows_kernel(const T* __restrict__ x, int64_t ldx, uint8_t* __restrict__ q, int64_t ldq,
-                                                             float* __restrict__ scale, uint8_t* __restrict__ atoms, uint8_t* __restrict__ rows,
+__global__ void __launch_bounds__(128) quantize_rows_kernel(const T* x, int64_t ldx, uint8_t* q, int64_t ldq, float* scale, uint8_t* atoms, uint8_t* rows,
                                                              int64_t ld_rows, int M, int M_pad, int KB, int groups) {
   if (gridDim.x <= kBehindMax) iris::ptx::pdl_trigger();
   iris::ptx::pdl_wait();
@@ -93,9 +92,8 @@ __global__ void __launch_bounds__(128) quantize_rows_kernel(const T* __restrict_
 }
 
 template <typename T>
-__global__ void __launch_bounds__(128) quantize_1x128_pow2_kernel(const T* __restrict__ x, int64_t ldx, uint8_t* __restrict__ q, int64_t ldq,
-                                                                   float* __restrict__ scale, uint8_t* __restrict__ atoms,
-                                                                   uint8_t* __restrict__ rows, int64_t ld_rows, int M, int M_pad, int K, int KB,
+__global__ void __launch_bounds__(128) quantize_1x128_pow2_kernel(const T* x, int64_t ldx, uint8_t* q, int64_t ldq, float* scale, uint8_t* atoms,
+                                                                   uint8_t* rows, int64_t ld_rows, int M, int M_pad, int K, int KB,
                                                                    int x_aligned, int q_aligned) {
   if (gridDim.x <= kBehindMax) iris::ptx::pdl_trigger();
   iris::ptx::pdl_wait();
