@@ -62,15 +62,7 @@ __global__ void __launch_bounds__(kSkinnyThreads) skinny_gemm_kernel(const __gri
     ptx::fence_mbar_init();
     ptx::fence_proxy_async();
   }
-  if (warp == 1) {
-    ptx::tmem_alloc(tmem_slot, cols);
-    ptx::tmem_relinquish();
-  }
-  ptx::tc_fence_before();
   __syncthreads();
-  ptx::tc_fence_after();
-  const uint32_t tmem_base = *(volatile uint32_t*)tmem_slot;
-  ptx::pdl_trigger();
   const int kb0 = (int)((int64_t)g.kblocks * rank / S), kb1 = (int)((int64_t)g.kblocks * (rank + 1) / S);
   // The first ring's weights on their way into L2 while the kernel in front drains (its writes, if it wrote them, are in L2 as well):
   // 16 x 3584 x 8192 13.7 -> 13.3 us back to back, 48-token MLP 29.6 -> 28.9. More than the ring holds was slower (14.0, 30.1), and so
@@ -87,6 +79,19 @@ __global__ void __launch_bounds__(kSkinnyThreads) skinny_gemm_kernel(const __gri
     __syncwarp();
   }
   ptx::pdl_wait();
+  // only now the columns (launch_pdl.cuh), while warp 0 already loads
+  uint32_t tmem_base = 0;
+  if (warp == 1) {
+    ptx::tmem_alloc(tmem_slot, cols);
+    ptx::tmem_relinquish();
+    ptx::tc_fence_before();
+    ptx::pdl_trigger();
+  }
+  if (warp != 0) {
+    ptx::named_barrier(1, kSkinnyThreads - 32);
+    ptx::tc_fence_after();
+    tmem_base = *(volatile uint32_t*)tmem_slot;
+  }
   auto fail = [&]() { if (g.status) atomicCAS(g.status, 0, (int)kTimeoutPipeline); };
 
   bool live = true;

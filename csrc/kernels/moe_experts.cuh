@@ -130,6 +130,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kXThreads, 1) expert
     ptx::fence_mbar_init();
     ptx::fence_proxy_async();
   }
+  // (in front of pdl_wait: the kernel in front is the gather, which has no tensor memory and triggered when all kernels before it had completed,
+  // or stage 1, which triggered when it had its columns. Behind it: 64 tokens, 32 experts, e4m3 236 -> 240 us)
   if (warp == 1) {
     ptx::tmem_alloc_pair(tmem_slot, Cfg::kTmemCols);
     ptx::tmem_relinquish_pair();

@@ -182,7 +182,7 @@ struct Pipeline {
 //   void comm_main(uint8_t* smem, int smem_bytes) const;    (CTAs with blockIdx.x >= gemm_ctas())
 //   void post_main() const;                                 (GEMM CTAs, all threads, after their tiles)
 //   void fail(int code) const;
-//   static constexpr bool kPdl;                            (launched behind the stream's last kernel: waits for it after the set-up)
+//   static constexpr bool kPdl;                            (launched behind the stream's last kernel: waits for it after the barriers' set-up)
 //   void stamp(int tile_seq, int what) const;              (optional per-tile timestamps: 0 tile
 //        start, 1 first A tile available, 2 tile stored; reference examples collect the same with
 //        COLLECT_TIMESTAMPS, examples/07_gemm_all_scatter/gemm_all_scatter.py:64-66)
@@ -230,6 +230,7 @@ IRIS_D void gemm_cta_main(const Policy& pol, uint8_t* smem_raw) {
     ptx::fence_mbar_init();
     ptx::fence_proxy_async();
   }
+  if constexpr (Policy::kPdl) ptx::pdl_wait();     // in front of the allocation: a CTA that waits holds no tensor memory
   if (warp == 1) {
     if constexpr (kPair) {
       ptx::tmem_alloc_pair(tmem_slot, Cfg::kTmemCols);   // one warp of each CTA of the pair
@@ -244,10 +245,7 @@ IRIS_D void gemm_cta_main(const Policy& pol, uint8_t* smem_raw) {
   if constexpr (kPair) ptx::cluster_sync();   // both CTAs' barriers exist before anyone signals remotely
   ptx::tc_fence_after();
   const uint32_t tmem_base = *(volatile uint32_t*)tmem_slot;
-  if constexpr (Policy::kPdl) {     // the set-up above runs while the kernel in front finishes
-    ptx::pdl_trigger();
-    ptx::pdl_wait();
-  }
+  if constexpr (Policy::kPdl) ptx::pdl_trigger();
 
   const int num_tiles = pol.num_tiles();
   const int k_blocks = (sh.K + Cfg::kBKElems - 1) / Cfg::kBKElems;
