@@ -16,6 +16,7 @@ combine and the output stay bf16. ``reference_moe`` is the unsharded fp32 PyTorc
 from __future__ import annotations
 
 import ctypes as C
+import struct
 
 import torch
 
@@ -41,6 +42,10 @@ class IrisMoeDesc(C.Structure):
         ("pos_of", C.c_void_p),
         ("x16", C.c_void_p),
     ]
+
+
+# The descriptor's fields behind `ctx`, in the C compiler's layout.
+_DESC_TAIL = struct.Struct("@" + "".join("i" if t is C.c_int32 else "P" for _, t in IrisMoeDesc._fields_[1:]))
 
 
 def route(logits: torch.Tensor, top_k: int):
@@ -119,7 +124,6 @@ class MoELayer:
         self.sorted_pairs = z(pairs)
         self.pos_of = z(pairs) if W == 1 else None
         self._prep_max = None
-        self._proto = None                       # descriptor fields that no call changes
         self.expert_rows, self.expert_row0, self.tile_prefix, self.expected_cum = z(El), z(El + 1), z(El + 1), z(El)
         ctx.barrier()
 
@@ -184,22 +188,23 @@ class MoELayer:
             lib._iris_moe_typed = True
         return lib
 
-    def _fixed_fields(self, one_rank: bool) -> bytes:
-        """The descriptor without what a call brings or a program may exchange (the weights): the layer's sizes and its
-        own buffers. Set field by field on every call they took as long as the launches."""
+    def _descriptor(self, x, logits, out) -> IrisMoeDesc:
+        """The call's descriptor, every field read from the layer as it is now (a program may exchange buffers and weights, or change
+        ``comm_sms``, between calls). One pack instead of a store per field: 3.2 against 4.6 us on the host."""
+        fp8, one_rank, p = self.fp8, self.pos_of is not None, torch.Tensor.data_ptr
         d = IrisMoeDesc()
-        d.K, d.E, d.El, d.D, d.F, d.capacity, d.comm_ctas = self.K, self.E, self.El, self.D, self.F, self.capacity, self.comm_sms
-        if self.fp8:
-            d.fp8, d.sf_ld1, d.sf_ld2 = 1, self.sf_ld1, self.sf_ld2
-            d.inbox_sf, d.H_sf = self.inbox_sf.data_ptr(), self.H_sf.data_ptr()
-        d.inbox, d.H, d.comb = self.inbox.data_ptr(), self.H.data_ptr(), self.comb.data_ptr()
-        d.sync_meta, d.sync_gemm2 = self.sync_meta.data_ptr(), self.sync_gemm2.data_ptr()
-        for name in ("topk_idx", "topk_w", "counts_local", "counts_all", "cursor", "list_off", "sorted_pairs", "my_off",
-                     "expert_rows", "expert_row0", "tile_prefix", "expected_cum", "arrived", "inbox_meta"):
-            setattr(d, name, getattr(self, name).data_ptr())
-        d.weights_kmajor = 1
-        d.pos_of = self.pos_of.data_ptr() if one_rank else None
-        return bytes(d)
+        d.ctx = self.ctx.ctx_struct()
+        w13, w2 = (self.w13_q, self.w2_q) if fp8 else (self.w13, self.w2)
+        send = fp8 and not one_rank              # e4m3 tokens travel; one rank quantises them in its gather, from x16
+        _DESC_TAIL.pack_into(
+            d, IrisMoeDesc.T.offset, x.shape[0], self.K, self.E, self.El, self.D, self.F, self.capacity, self.comm_sms,
+            p(self.xq) if send else 0 if fp8 else p(x), p(logits), p(w13), p(w2), p(out), p(self.inbox), p(self.H), p(self.comb),
+            p(self.sync_meta), p(self.sync_gemm2), p(self.topk_idx), p(self.topk_w), p(self.counts_local), p(self.counts_all), p(self.cursor), p(self.list_off),
+            p(self.sorted_pairs), p(self.my_off), p(self.expert_rows), p(self.expert_row0), p(self.tile_prefix), p(self.expected_cum), p(self.arrived),
+            p(self.inbox_meta), 1, int(fp8), self.sf_ld1 if fp8 else 0, self.sf_ld2 if fp8 else 0, p(self.x_sf) if send else 0,
+            p(self.inbox_sf) if fp8 else 0, p(self.H_sf) if fp8 else 0, p(self.w13_sf) if fp8 else 0, p(self.w2_sf) if fp8 else 0,
+            p(self.pos_of) if one_rank else 0, p(x) if fp8 and one_rank else 0)
+        return d
 
     def forward(self, x: torch.Tensor, router_logits: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
         ctx = self.ctx
@@ -218,23 +223,9 @@ class MoELayer:
         one_rank = self.pos_of is not None
         if one_rank and x.data_ptr() % 16:       # the gather reads 16 bytes at a time
             x = x.clone()
-        proto = self._proto
-        if proto is None:
-            proto = self._proto = self._fixed_fields(one_rank)
-        d = IrisMoeDesc.from_buffer_copy(proto)
-        d.ctx = ctx.ctx_struct()
-        d.T = T
-        if self.fp8:
-            if one_rank:                         # quantised by the gather
-                d.x16 = x.data_ptr()
-            else:
-                self._quantise_tokens(x)
-                d.x, d.x_sf = self.xq.data_ptr(), self.x_sf.data_ptr()
-            d.w13, d.w2 = self.w13_q.data_ptr(), self.w2_q.data_ptr()
-            d.w13_sf, d.w2_sf = self.w13_sf.data_ptr(), self.w2_sf.data_ptr()
-        else:
-            d.x, d.w13, d.w2 = x.data_ptr(), self.w13.data_ptr(), self.w2.data_ptr()
-        d.logits, d.out = logits.data_ptr(), out.data_ptr()
+        if self.fp8 and not one_rank:
+            self._quantise_tokens(x)
+        d = self._descriptor(x, logits, out)
         lib = self._lib()
         if one_rank and self._prep_max is None:
             self._prep_max = lib.iris_moe_prep_max_tokens()

@@ -389,3 +389,41 @@ def _models_dry_run(rank, world):
 
 def test_gpu_paths_of_the_model_layers_world2():
     run_ranks(_models_dry_run, 2)
+
+
+def _moe_descriptor(rank, world):
+    import iris_b200 as iris
+    from iris_b200.models import MoELayer
+    from iris_b200.models.moe import _DESC_TAIL, IrisMoeDesc
+
+    assert IrisMoeDesc.T.offset + _DESC_TAIL.size == IrisMoeDesc.x16.offset + 8
+    ctx = iris.iris(1 << 28)
+    rec = _pretend_gpu(ctx)
+    rec.iris_moe_prep_max_tokens = lambda: 256
+    dt, (D, F, E, K, T) = torch.bfloat16, (256, 128, 2 * world, 2, 64)
+    El = E // world
+    moe = MoELayer(ctx, D, F, E, K, T, w_gate=torch.zeros(El, D, F, dtype=dt), w_up=torch.zeros(El, D, F, dtype=dt), w_down=torch.zeros(El, F, D, dtype=dt))
+    buffers = ("inbox", "H", "comb", "sync_meta", "sync_gemm2", "topk_idx", "topk_w", "counts_local", "counts_all", "cursor", "list_off", "sorted_pairs",
+               "my_off", "expert_rows", "expert_row0", "tile_prefix", "expected_cum", "arrived", "inbox_meta", "w13", "w2") + (("pos_of",) if world == 1 else ())
+    x, logits = torch.zeros(T, D, dtype=dt), torch.zeros(T, E)
+    for turn in range(2):
+        y = moe(x, logits)
+        d = rec.models[-1][1]
+        assert (d.T, d.K, d.E, d.El, d.D, d.F, d.capacity, d.comm_ctas) == (T, K, E, El, D, F, moe.capacity, moe.comm_sms)
+        assert (d.x, d.logits, d.out) == (x.data_ptr(), logits.data_ptr(), y.data_ptr()) and (d.weights_kmajor, d.fp8, d.sf_ld1, d.sf_ld2) == (1, 0, 0, 0)
+        for name in buffers:
+            assert getattr(d, name) == getattr(moe, name).data_ptr(), (turn, name)
+        assert all(getattr(d, name) is None for name in ("x_sf", "inbox_sf", "H_sf", "w13_sf", "w2_sf", "x16")) and (d.pos_of is None) == (world > 1)
+        # a program exchanges what it likes between calls
+        moe.comm_sms = 5
+        for name in buffers:
+            setattr(moe, name, getattr(moe, name).clone())
+
+
+def test_moe_descriptor_follows_the_layer():
+    """Every call launches with the layer's attributes as they are then, not as they were at the first call."""
+    run_ranks(_moe_descriptor, 2)
+
+
+def test_moe_descriptor_follows_the_layer_world1():
+    run_ranks(_moe_descriptor, 1)
