@@ -9,8 +9,9 @@
 //   * tensor memory is allocated behind pdl_wait(). A CTA that held columns while it waits could share an SM with a CTA of the kernel in
 //     front that still asks for its own (a library's kernel may trigger before it has them), and each would wait for the other;
 //   * pdl_trigger() stands behind the allocation, for the same reason the other way round: a kernel behind this one may allocate first.
-// So nothing is expected of kernels from elsewhere, in front or behind. (Allocating behind the wait instead of in front of it: 16 x 3584 x 8192
-// 13.2 us both ways, two few-row products 28.6, e4m3 4096 x 3584 x 8192 128.7 and 128.2.) expert_gemm_kernel allocates in front of its
+// So nothing is expected of kernels from elsewhere, in front or behind. (Allocating behind the wait instead of in front of it costs nothing where the
+// loading warp goes ahead meanwhile: 16 x 3584 x 8192 13.2 us both ways, two products of 2048 x 2048 x 2048 33.5 and 33.1, but 34.7 when
+// the loads waited for the allocation too; e4m3 4096 x 3584 x 8192 128.7 and 128.2.) expert_gemm_kernel allocates in front of its
 // wait: it is launched behind the MoE layer's own kernels only, and everything that was in front of those has completed by then.
 // A kernel behind one of these that is launched the ordinary way waits for it to finish, as always.
 #pragma once

@@ -216,7 +216,8 @@ IRIS_D void gemm_cta_main(const Policy& pol, uint8_t* smem_raw) {
   uint8_t* sf_base = scratch_base + kEpiWarps * 256;               // fp8: per stage one scale atom of A, then B's
   uint64_t* bars = (uint64_t*)(sf_base + Cfg::kStages * Cfg::kSfBytes);
   Pipeline pipe{bars, bars + Cfg::kStages, bars + 2 * Cfg::kStages, bars + 2 * Cfg::kStages + 2};
-  uint32_t* tmem_slot = (uint32_t*)(bars + 2 * Cfg::kStages + 4);
+  uint64_t* tmem_ready = bars + 2 * Cfg::kStages + 4;     // in the even CTA of a pair: both have their columns
+  uint32_t* tmem_slot = (uint32_t*)(tmem_ready + 1);
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < Cfg::kStages; ++s) {
@@ -227,10 +228,15 @@ IRIS_D void gemm_cta_main(const Policy& pol, uint8_t* smem_raw) {
       ptx::mbar_init(&pipe.tmem_full[b], 1);
       ptx::mbar_init(&pipe.tmem_empty[b], kEpiWarps * (kPair ? 2 : 1));
     }
+    if constexpr (kPair) ptx::mbar_init(tmem_ready, 2);
     ptx::fence_mbar_init();
     ptx::fence_proxy_async();
   }
-  if constexpr (Policy::kPdl) ptx::pdl_wait();     // in front of the allocation: a CTA that waits holds no tensor memory
+  __syncthreads();
+  if constexpr (kPair) ptx::cluster_sync();   // both CTAs' barriers exist before anyone signals remotely
+  if constexpr (Policy::kPdl) ptx::pdl_wait();
+  // Only now the columns, and only with them the trigger (a CTA that waits holds no tensor memory), while warp 0 already loads.
+  uint32_t tmem_base = 0;
   if (warp == 1) {
     if constexpr (kPair) {
       ptx::tmem_alloc_pair(tmem_slot, Cfg::kTmemCols);   // one warp of each CTA of the pair
@@ -239,13 +245,16 @@ IRIS_D void gemm_cta_main(const Policy& pol, uint8_t* smem_raw) {
       ptx::tmem_alloc(tmem_slot, Cfg::kTmemCols);
       ptx::tmem_relinquish();
     }
+    ptx::tc_fence_before();
+    if constexpr (Policy::kPdl) ptx::pdl_trigger();
+    if constexpr (kPair)
+      if (lane == 0) ptx::mbar_arrive_cluster(tmem_ready, 0);
   }
-  ptx::tc_fence_before();
-  __syncthreads();
-  if constexpr (kPair) ptx::cluster_sync();   // both CTAs' barriers exist before anyone signals remotely
-  ptx::tc_fence_after();
-  const uint32_t tmem_base = *(volatile uint32_t*)tmem_slot;
-  if constexpr (Policy::kPdl) ptx::pdl_trigger();
+  if (warp != 0) {
+    ptx::named_barrier(2, kThreads - 32);
+    ptx::tc_fence_after();
+    tmem_base = *(volatile uint32_t*)tmem_slot;
+  }
 
   const int num_tiles = pol.num_tiles();
   const int k_blocks = (sh.K + Cfg::kBKElems - 1) / Cfg::kBKElems;
@@ -341,6 +350,10 @@ IRIS_D void gemm_cta_main(const Policy& pol, uint8_t* smem_raw) {
     uint32_t ph = 0;
     int it = 0;
     bool ok = leader;      // the even CTA of a pair issues for both
+    if constexpr (kPair) {
+      if (ok && !__all_sync(0xffffffffu, ptx::mbar_wait<true>(tmem_ready, 0, kPipeTimeoutNs))) { pol.fail(kTimeoutPipeline); ok = false; }
+      ptx::tc_fence_after();
+    }
     for (int t = first; t < num_tiles && ok; t += step, ++it) {
       const int buf = Cfg::kAccBufs == 2 ? (it & 1) : 0;
       const uint32_t acc_ph = Cfg::kAccBufs == 2 ? ((it >> 1) & 1) : (it & 1);
