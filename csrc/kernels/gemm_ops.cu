@@ -972,15 +972,19 @@ int make_plan(const IrisGemmDesc* d, Plan& p) {
   }
   if (is_fp8(d)) {
     // block-scaled e4m3 tiles are 224 (or 128) wide: two accumulator buffers plus the scale cells fill TMEM.
-    // CTA pairs on request, and for a local GEMM whose main loop is long enough for the 1.2 us that a cluster costs at its ends: long K,
-    // with weights of 28 M elements or 4e10 products. Single tiles / pairs, us, each back to back at first and then for a while (power cap):
-    //   K = 8192   16 x 3584  35.2 / 33.8    200 x 8192  28.6 / 25.4    4096 x 3584  113.8 / 108.4    8192 x 8192  504 / 456
-    //              512 x 1024  22.1 / 24.9   4096 x 1024  61.9 / 62.9   8192 x 1024  90.0 / 79.7
-    //   K = 4096   1024 x 3584  16.3 / 16.6  1024 x 8192  33.6 / 33.4   3000 x 3584  45.1 / 43.4     8192 x 8192  247 / 237
-    //   K = 1024   4096 x 8192  34.3 / 36.2  8192 x 8192  77.9 / 78.6
+    // CTA pairs on request, and for a local GEMM whose main loop is long enough for what a cluster costs at its ends: K of 4096 or more, where either
+    // few rows leave every tile to itself (the pair's ring is six stages deep, four otherwise) or the products are many (4e10).
+    // Single tiles / pairs, us back to back with weights that are not in L2, M x N:
+    //   K = 8192   16 x 1024  25.7 / 22.9    16 x 3584  26.3 / 23.1    1024 x 2048  26.9 / 25.1    2048 x 2048  42.2 / 42.3    4096 x 3584  110.8 / 108.7
+    //   K = 6144   16 x 3072  21.4 / 19.0    512 x 4096  21.1 / 19.5    1024 x 4096  33.1 / 33.0    3000 x 3072  56.8 / 57.2    4096 x 4096  97.4 / 94.0
+    //   K = 4096   16 x 1024  14.9 / 14.2    1024 x 2048  15.6 / 15.5    1536 x 3584  29.1 / 30.4    3000 x 1024  14.7 / 15.4    8192 x 5120  158 / 152
+    //   K = 2048   16 x 4096  11.9 / 12.4    512 x 8192  10.7 / 11.0    4096 x 4096  31.0 / 30.1
+    // At the lines: 1024 rows 0.99 to 1.10 times as fast with pairs, 1536 to 3000 rows below 4e10 products 0.96 to 1.03, 4e10 to 5e10 0.98 to 1.01.
+    // A single row with more than 24 column tiles loses up to 15 % (4096 x 8192: 16.0 / 18.6; 5120 columns 15.4 / 14.4): the reason is not known.
     if (d->bn != 0 && d->bn != 224 && d->bn != 128) return -5;
     const double weights = (double)d->N * d->K;
-    const bool long_loop = d->op == IRIS_GEMM_LOCAL && d->K >= 4096 && (weights >= 28e6 || weights * d->M >= 4e10);
+    const bool lone_row = d->M == 1 && ceil_div(d->N, 224) > 24;
+    const bool long_loop = d->op == IRIS_GEMM_LOCAL && d->K >= 4096 && !lone_row && (d->M <= 1024 || weights * d->M >= 4e10);
     const bool pairs = d->two_sm == 2 || (d->two_sm == 0 && long_loop);
     choose_tile(d->M, d->N, p.gemm_ctas, d->bn == 128 ? 128 : 224, pairs ? 2 : 1, pair_ok && d->bn != 128, p.bn, p.pair);
   } else {

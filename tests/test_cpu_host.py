@@ -504,6 +504,32 @@ def test_gemm_plan_tile_choice():
     assert plan(_lib.GEMM_RS_TILES, 8192, 8192, 3584, W=8)[2] == 0                   # tile-granular scatter keeps single CTAs
 
 
+def test_gemm_plan_e4m3_pairs():
+    """Both sides of the rule that gives a block-scaled local GEMM CTA pairs: K of 4096, 1024 rows, 4e10 products, a single row with more than 24
+    column tiles; asked for and forbidden, narrow tiles, and never for the fused ops unless asked for."""
+    import ctypes as C
+
+    from iris_b200 import _lib
+
+    def pair(M, N, K, op=_lib.GEMM_LOCAL, two_sm=0, bn=224):
+        import torch
+
+        d = _lib.IrisGemmDesc()
+        d.op, d.M, d.N, d.K, d.dtype, d.two_sm, d.bn, d.b_kmajor = op, M, N, K, 1, two_sm, bn, 1
+        d.in_dtype, d.ctx.world, d.M_local = _lib.DTYPE_CODE[torch.float8_e4m3fn], 1, M
+        out = [C.c_uint64(), C.c_uint64(), C.c_uint64(), C.c_int32(), C.c_int32()]
+        assert _lib.kernels().iris_gemm_workspace(C.byref(d), *[C.byref(o) for o in out]) == 0
+        return out[4].value
+
+    assert pair(16, 1024, 4096) == 1 and pair(16, 1024, 4080) == 0
+    assert pair(1024, 2048, 4096) == 1 and pair(1025, 2048, 4096) == 0
+    assert pair(4769, 2048, 4096) == 1 and pair(4768, 2048, 4096) == 0               # 4e10 / (2048 x 4096) = 4768.4
+    assert pair(1, 5376, 4096) == 1 and pair(1, 5377, 4096) == 0 and pair(2, 5377, 4096) == 1
+    assert pair(16, 223, 8192) == 0 and pair(16, 224, 8192) == 1                     # a pair's tile is 224 wide
+    assert pair(16, 3584, 8192, two_sm=1) == 0 and pair(16, 3584, 1024, two_sm=2) == 1 and pair(16, 3584, 8192, bn=128) == 0
+    assert pair(256, 3584, 8192, op=_lib.GEMM_AG_M) == 0 and pair(256, 3584, 8192, op=_lib.GEMM_AG_M, two_sm=2) == 1
+
+
 def test_zigzag_positions_cover_the_sequence_and_balance_causal_work():
     from iris_b200.models import reference_attention, zigzag_positions
 

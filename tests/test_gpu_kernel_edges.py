@@ -107,6 +107,50 @@ def test_few_rows_on_both_ring_depths(M, N, K, linear):
     assert ((got - want).abs() <= 2.0 ** -8 * want.abs() + K * 2.0 ** -24 * sums).all()
 
 
+def _e4m3_operands(M, N, K, seed):
+    """Values and power-of-two scales that differ from block to block: a scale atom or a tile taken for another shows."""
+    from iris_b200.ops.gemm_fp8 import quantize_1x128, quantize_128x128
+
+    g = _gen(seed)
+    spread = lambda *sh: torch.exp2(torch.randint(-3, 4, sh, device="cuda", generator=g).float())  # noqa: E731
+    kb = -(-K // 128)
+    x = torch.randn(M, K, device="cuda", generator=g) * spread(M, kb).repeat_interleave(128, 1)[:, :K]
+    w = torch.randn(N, K, device="cuda", generator=g) * spread(-(-N // 128), kb).repeat_interleave(128, 0)[:N].repeat_interleave(128, 1)[:, :K]
+    return quantize_1x128(x, pow2=True), quantize_128x128(w, pow2=True)
+
+
+def _e4m3_pairs(M, N, K):
+    """Whether the plan takes CTA pairs when nothing is asked for."""
+    import ctypes as C
+
+    from iris_b200 import _lib
+
+    d = _lib.IrisGemmDesc()
+    d.op, d.M, d.N, d.K, d.dtype, d.in_dtype, d.b_kmajor = _lib.GEMM_LOCAL, M, N, K, _lib.DTYPE_CODE[torch.bfloat16], _lib.DTYPE_CODE[torch.float8_e4m3fn], 1
+    d.ctx.world = 1
+    out = [C.c_uint64(), C.c_uint64(), C.c_uint64(), C.c_int32(), C.c_int32()]
+    assert _lib.kernels().iris_gemm_workspace(C.byref(d), *[C.byref(o) for o in out]) == 0
+    return bool(out[4].value)
+
+
+@pytest.mark.parametrize("M", [1, 16, 129, 300, 385])
+@pytest.mark.parametrize("N,K,by_rule", [(3656, 8192, True), (8200, 4224, True), (456, 4096, True), (1000, 1168, False), (224, 128, False)])
+def test_e4m3_pairs_with_ragged_tiles(M, N, K, by_rule):
+    """CTA pairs with rows for one of the two CTAs only, odd counts of 128-row tiles, ragged last columns and K blocks: where the rule chooses them,
+    where they are asked for, and against single tiles. fp32 sums of K exact products in K order in both: the same values; against 64 bits one
+    rounding to bf16 (2^-8 of it) and the sums' own, K 2^-24 of the magnitudes added up."""
+    from iris_b200.ops.gemm_fp8 import dequantize, matmul_fp8_blockscaled, pack_scales_a, pack_scales_b
+
+    (aq, asc), (bq, bsc) = _e4m3_operands(M, N, K, M + N)
+    run = lambda two_sm: matmul_fp8_blockscaled(aq, pack_scales_a(asc), bq, pack_scales_b(bsc, N, 224), two_sm=two_sm)  # noqa: E731
+    assert _e4m3_pairs(M, N, K) == (by_rule and not (M == 1 and N == 8200))
+    pairs, single, chosen = run(True), run(False), run(None)
+    a, b = dequantize(aq, asc, 1).double(), dequantize(bq, bsc, 128).double()
+    want, sums = a @ b.t(), a.abs() @ b.abs().t()
+    assert ((pairs.double() - want).abs() <= 2.0 ** -8 * want.abs() + K * 2.0 ** -24 * sums).all()
+    assert torch.equal(pairs, single) and torch.equal(chosen, pairs)
+
+
 # ------------------------------------------------------------------------------------ kernels that start behind their predecessor
 @pytest.mark.parametrize("rows", [16, 300, 2000])
 def test_chains_of_early_started_kernels(ctx, rows):
