@@ -685,6 +685,13 @@ __global__ void __launch_bounds__(kD * kGroups) decode_local_finish_kernel(const
   if (out_lse && d == 0) out_lse[it] = l > 0.f ? (m + log2f(l)) / kLog2e : -INFINITY;
 }
 
+int decode_sms() {
+  int dev = 0, sms = 148;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return sms;
+}
+
 // Split-K pass over `a.B` sequences, in launches of up to kMaxSeqs, on two CTAs per SM.
 template <bool kTma>
 int launch_splitk(DecodeArgs a, cudaStream_t s) {
@@ -697,9 +704,7 @@ int launch_splitk(DecodeArgs a, cudaStream_t s) {
   using N = std::false_type;
   auto* kern = a.is_fp16 ? (a.group <= 8 ? pick(Y{}, Y{}) : pick(Y{}, N{})) : (a.group <= 8 ? pick(N{}, Y{}) : pick(N{}, N{}));
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -20;
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int sms = decode_sms();
   const int total = a.B;
   for (int b0 = 0; b0 < total; b0 += kMaxSeqs) {
     DecodeArgs p = a;
@@ -780,7 +785,7 @@ int iris_flash_decode(const IrisDecodeDesc* d, void* stream) {
   if (!d->exchange) return 0;
   if (d->exchange == 2 || d->ctx.world <= 1) {
     const int items = d->B * d->Hq;
-    if (items <= 296 && d->splits > 8)
+    if (items <= 2 * decode_sms() && d->splits > 8)      // (few heads: see the kernel)
       return launch_pdl(decode_local_finish_kernel<4, 10>, dim3(items), 4 * kD, 0, s, (const float*)d->partial, d->out, d->out_lse, (int)d->splits, a.is_fp16);
     return launch_pdl(decode_local_finish_kernel<1, 8>, dim3(items), kD, 0, s, (const float*)d->partial, d->out, d->out_lse, (int)d->splits, a.is_fp16);
   }
@@ -791,7 +796,8 @@ int iris_flash_decode(const IrisDecodeDesc* d, void* stream) {
   x.out = d->out; x.out_lse = d->out_lse; x.B = d->B; x.Bmax = d->Bmax; x.Hq = d->Hq; x.splits = d->splits;
   x.is_fp16 = a.is_fp16;
   int items = d->B * d->Hq;
-  int grid2 = items < 148 * 8 ? items : 148 * 8;   // every CTA resident: pushes precede all waits anyway
+  const int most = 8 * decode_sms();
+  int grid2 = items < most ? items : most;         // every CTA resident: pushes precede all waits anyway
   decode_exchange_kernel<<<grid2, kD, 0, s>>>(x);
   return cudaGetLastError() == cudaSuccess ? 0 : -21;
 }

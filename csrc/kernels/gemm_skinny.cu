@@ -236,7 +236,7 @@ static bool skinny_one_per_sm(int tn, int tiles, int kb) {
   if (tn <= 64) return false;
   if (tn > 128) return true;
   const int s = split_for(tiles, kb, sm_count(), tiles <= 12 ? 8 : 4);
-  return tiles <= 12 || (s == 4 && tiles * s >= 96);
+  return tiles <= 12 || (s == 4 && 8 * tiles * s >= 5 * sm_count());      // (24 tiles and more of 148 SMs)
 }
 int iris_gemm_skinny_split(int M, int N, int K) {
   const int tiles = ceil_div(N, 128), kb = ceil_div(K, kBK), tn = ceil_div(M, 16) * 16;
