@@ -3,7 +3,11 @@
 // A kernel launched this way may start while the stream's last kernel still runs: when all of its CTAs have issued
 // ptx::pdl_trigger(), or have left. So the launch latency, the set-up (barriers, descriptors) and the last wave of the
 // kernel in front overlap; back to back that was 2 to 4 us of every pass. Rules for the kernels:
-//   * ptx::pdl_wait() by every thread before it touches memory that an earlier kernel may have written or may still read;
+//   * ptx::pdl_wait() by every thread before it touches memory that an earlier kernel may have written or may still read. Before it a kernel may
+//     read only what was complete when the kernel in front of it triggered, and so only behind one that triggers behind its own wait: everything
+//     in front of that one has completed by then. The MoE layer on one rank does so: the gather of 16-bit tokens reads them behind the preparation or the
+//     sort, stage 1 of the grouped GEMMs reads weights and the preparation's tables behind the gather, stage 2 the same behind stage 1 (which
+//     starts when the gather has triggered). Their triggers must not move in front of their waits. An L2 prefetch is no read;
 //   * and by no read-only promise about such memory: a `const T* __restrict__` parameter, __ldg or ld.global.nc lets a load move in front
 //     of the wait, or return what lay there before;
 //   * tensor memory is allocated behind pdl_wait(). A CTA that held columns while it waits could share an SM with a CTA of the kernel in

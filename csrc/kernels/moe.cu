@@ -192,7 +192,7 @@ __global__ void __launch_bounds__(1024) moe_meta_kernel(const __grid_constant__ 
 // With one rank the bucket position is also the pair's inbox row: it is kept in `pos_of` for the gather.
 __global__ void __launch_bounds__(256) moe_sort_kernel(MoeDims dm, MoeMeta m, int32_t* pos_of) {
   ptx::pdl_wait();
-  ptx::pdl_trigger();
+  ptx::pdl_trigger();      // not earlier: the gather reads the tokens before its own wait: see launch_pdl.cuh
   __shared__ int32_t cnt[1024], base[1024];
   for (int e = threadIdx.x; e < dm.E; e += blockDim.x) cnt[e] = 0;
   __syncthreads();
@@ -227,7 +227,7 @@ template <int kPer>
 __global__ void __launch_bounds__(1024) moe_prep_kernel(const float* logits, const __grid_constant__ DeviceContext ctx, MoeDims dm,
                                                         MoeMeta m, int32_t* pos_of) {
   ptx::pdl_wait();
-  ptx::pdl_trigger();
+  ptx::pdl_trigger();      // not earlier: the gather reads the tokens before its own wait: see launch_pdl.cuh
   __shared__ int32_t hist[1024], off[1024], w_rows[32], w_tiles[32];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   hist[tid] = 0;
@@ -291,7 +291,7 @@ __global__ void __launch_bounds__(256) moe_gather_kernel(const uint8_t* x, uint8
   const int c0 = blockIdx.y * blockDim.x + threadIdx.x;
   uint4 v = c0 < row16 ? __ldcg(src + c0) : make_uint4(0, 0, 0, 0);
   ptx::pdl_wait();
-  ptx::pdl_trigger();
+  ptx::pdl_trigger();      // not earlier: stage 1 reads weights and tables before its own wait: see launch_pdl.cuh
   if (threadIdx.x < K) dst[threadIdx.x] = pos_of[(size_t)t * K + threadIdx.x];
   __syncthreads();
   for (int c = c0; c < row16; c += gridDim.y * blockDim.x) {
@@ -306,7 +306,7 @@ __global__ void __launch_bounds__(256) moe_gather_kernel(const uint8_t* x, uint8
 __global__ void __launch_bounds__(256) moe_gather_quant_kernel(const __nv_bfloat16* x, uint8_t* inbox, uint8_t* inbox_sf, int atoms, MoeDims dm, MoeMeta m,
                                                                const int32_t* pos_of) {
   ptx::pdl_wait();
-  ptx::pdl_trigger();
+  ptx::pdl_trigger();      // not earlier: stage 1 reads weights and tables before its own wait: see launch_pdl.cuh
   __shared__ int32_t dst[kMaxTopK], tile[kMaxTopK], cell[kMaxTopK];
   const int t = blockIdx.x, half = threadIdx.x >> 4, sub = threadIdx.x & 15, D = dm.D, K = dm.K, kblocks = D / 128;
   if (threadIdx.x < K) {

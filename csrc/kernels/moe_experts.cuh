@@ -143,7 +143,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kXThreads, 1) expert
   ptx::tc_fence_after();
   const uint32_t tmem_base = *(volatile uint32_t*)tmem_slot;
   // Launched behind the gather (stage 1) or stage 1 (stage 2). What is read before pdl_wait - the weights and the tables of
-  // the preparation - was complete before the kernel in front of this one got past its own pdl_wait or was launched.
+  // the preparation - was complete when the gather triggered, without which neither stage starts (launch_pdl.cuh).
   ptx::pdl_trigger();
   const int units = s_tiles[g.El] * g.tiles_w, first = blockIdx.x >> 1, step = gridDim.x >> 1;
   auto fail = [&]() { if (g.status) atomicCAS(g.status, 0, (int)kTimeoutPipeline); };

@@ -66,6 +66,14 @@ def test_tensor_memory_is_allocated_between_wait_and_trigger(path, function):
     assert wait < alloc < trigger, path
 
 
+@pytest.mark.parametrize("name", ["router_topk_kernel", "moe_meta_kernel", "moe_sort_kernel", "moe_clear_kernel", "moe_prep_kernel", "moe_gather_kernel",
+                                  "moe_gather_quant_kernel", "moe_reduce_kernel"])
+def test_moe_kernels_trigger_behind_their_wait(name):
+    """The kernel behind one of them reads tokens, weights or tables before its own wait: they are complete because this one has waited."""
+    body = _body(EARLY["moe.cu"], " " + name + "(")
+    assert body.index("pdl_wait()") < body.index("pdl_trigger()")
+
+
 def test_attention_waits_before_anything_else():
     """The attention kernel's CTA body allocates and triggers; the kernel waits in front of it."""
     text = EARLY["ring_attention_tc.cu"]
