@@ -338,6 +338,117 @@ def test_moe_one_rank_swiglu_divides_exactly(ctx, fp8, T):
     ctx.heap_release(mark)
 
 
+@pytest.mark.parametrize("T,fp8", [(48, True), (48, False), (700, True), (700, False)])
+def test_moe_one_rank_many_units_per_pair(ctx, T, fp8):
+    """Four or more units per CTA pair in both grouped GEMMs, and K blocks (22 and 11 in e4m3, 44 and 22 in bf16) that pass every ring (9, 10, 5 and 6 stages)
+    more than once without being a multiple: accumulator buffers, barrier phases and the exchanged magnitudes are used again and again. Other inputs
+    in between. Bounds as in test_moe_one_rank_token_tiles."""
+    from iris_b200.models import MoELayer, reference_moe
+    from iris_b200.ops.gemm_fp8 import dequantize, quantize_128x128
+
+    E, K, D, F = 32, 8, 2816, 1408
+    wg, wu, wd = _moe_weights(E, D, F, T)
+    mark = ctx.heap_mark()
+    layer = MoELayer(ctx, D, F, E, K, max_tokens=T, w_gate=wg, w_up=wu, w_down=wd, fp8=fp8)
+    if fp8:
+        deq = lambda w: torch.stack([dequantize(*quantize_128x128(m.t().contiguous().float(), pow2=True), 128).t() for m in w])  # noqa: E731
+        wg, wu, wd = deq(wg), deq(wu), deq(wd)
+    calls = [(torch.randn(T, D, device="cuda", generator=_gen(i)).to(torch.bfloat16), torch.randn(T, E, device="cuda", generator=_gen(i + 50))) for i in range(3)]
+    first = []
+    for x, logits in calls:
+        y, want = layer(x, logits), reference_moe(x, logits, wg, wu, wd, K)
+        # 32 x 11 weight tiles of 256 rows each (down: the same number), times the token tiles of the experts in use, on 74 pairs
+        assert layer.tile_prefix[E].item() * 11 >= 4 * 74
+        assert ((y.float() - want).norm() / want.norm()).item() < (0.1 if fp8 else 2e-2)
+        assert ((y.float() - want).norm(dim=1) / want.norm(dim=1)).max().item() < (0.2 if fp8 else 4e-2)
+        first.append(y)
+    for _ in range(3):
+        outs = [layer(x, logits) for x, logits in calls]
+        assert all(torch.equal(a, b) for a, b in zip(outs, first))
+    ctx.check()
+    ctx.heap_release(mark)
+
+
+@pytest.mark.parametrize("T", [40, 300])
+def test_moe_one_rank_weights_that_are_not_k_major(ctx, T):
+    """What only a C caller asks for (weights_kmajor 0: w13 [El, D, 2F], w2 [El, F, D]): the grouped GEMM of several ranks, on one. Sums in the same order as with
+    K-major weights up to the tile's shape, so both are within the bf16 bounds above of the reference."""
+    import ctypes as C
+
+    from iris_b200 import _lib
+    from iris_b200.models import MoELayer, reference_moe
+    from iris_b200.models.moe import fuse_gate_up
+
+    E, K, D, F = 6, 2, 512, 256
+    wg, wu, wd = _moe_weights(E, D, F, T)
+    mark = ctx.heap_mark()
+    layer = MoELayer(ctx, D, F, E, K, max_tokens=T, w_gate=wg, w_up=wu, w_down=wd)
+    x, logits = torch.randn(T, D, device="cuda", generator=_gen(T)).to(torch.bfloat16), torch.randn(T, E, device="cuda", generator=_gen(1))
+    out, w13, w2 = torch.empty_like(x), fuse_gate_up(wg, wu), wd.contiguous()
+    d = layer._descriptor(x, logits, out)
+    d.weights_kmajor, d.w13, d.w2 = 0, w13.data_ptr(), w2.data_ptr()
+    for _ in range(2):
+        assert layer._lib().iris_moe_forward(C.byref(d), C.c_void_p(_lib.current_stream_ptr())) == 0
+        want = reference_moe(x, logits, wg, wu, wd, K)
+        assert ((out.float() - want).norm() / want.norm()).item() < 2e-2
+        assert ((out.float() - want).norm(dim=1) / want.norm(dim=1)).max().item() < 4e-2
+        y = layer(x, logits)                       # and the layer's own form between the two
+        assert ((y.float() - want).norm() / want.norm()).item() < 2e-2
+        out.zero_()
+    ctx.check()
+    ctx.heap_release(mark)
+
+
+@pytest.mark.parametrize("T,fp8", [(24, True), (24, False), (300, True), (300, False)])
+def test_moe_among_other_early_started_kernels(ctx, T, fp8):
+    """The MoE layer between GEMMs, the quantiser, decode and elementwise kernels, each reading what the one in front wrote, plain and as a CUDA graph: the bits of
+    the same calls with the device idle in between."""
+    from iris_b200.models import FlashDecodeLayer, MoELayer
+    from iris_b200.ops import matmul, quantize_activation, quantize_weight
+
+    g, D, E = _gen(T), 1024, 8
+    r = lambda *sh: torch.randn(*sh, device="cuda", generator=g) * sh[-1] ** -0.5  # noqa: E731
+    w1, w2, wr, wq = r(D, D).bfloat16().t(), r(D, D).bfloat16(), r(E, D).bfloat16().t(), quantize_weight(r(D, D))
+    cache = [torch.randn(64, 16, 2, 128, device="cuda", generator=g).bfloat16() for _ in range(2)]
+    table, lens = torch.randperm(64, device="cuda", generator=g).int().view(2, 32), torch.tensor([[511, 77]], device="cuda", dtype=torch.int32)
+    mark = ctx.heap_mark()
+    dec = FlashDecodeLayer(ctx, 8, 2, 128, max_batch=2)
+    moe = MoELayer(ctx, D, 512, E, 2, max_tokens=T, **dict(zip(("w_gate", "w_up", "w_down"), _moe_weights(E, D, 512, 5))), fp8=fp8)
+    x0 = torch.randn(T, D, device="cuda", generator=g).bfloat16()
+    x, h, y, logits = x0.clone(), torch.empty_like(x0), torch.empty_like(x0), torch.empty(T, E, device="cuda", dtype=torch.bfloat16)
+
+    def chain(sync):
+        gap = torch.cuda.synchronize if sync else (lambda: None)
+        x.copy_(x0)
+        for _ in range(3):
+            gap(); matmul(x, w1, out=h)
+            gap(); matmul(h, wr, out=logits)
+            gap(); moe(h, logits, out=y)                       # tokens straight from a GEMM
+            gap(); matmul(y, w2, out=x)                        # and its sum straight into one
+            gap(); a = quantize_activation(x)
+            gap(); matmul(a, wq, out=h)
+            gap(); moe(h, logits, out=y)
+            gap(); moe(y, logits, out=x)                       # back to back, tokens from the reduction in front
+            gap(); d = dec(x[:2].view(2, 8, 128), *cache, lens, table)
+            gap(); x[:2] = d.view(2, D)
+            gap(); x.mul_(8.0)
+        return x.clone(), y.clone()
+
+    want = chain(True)
+    assert all(torch.isfinite(t.float()).all() and t.float().abs().max() > 0 for t in want)
+    for _ in range(5):
+        assert all(torch.equal(a, b) for a, b in zip(chain(False), want))
+    graph = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph):
+        got = chain(False)
+    for _ in range(3):
+        graph.replay()
+        assert all(torch.equal(a, b) for a, b in zip(got, want))
+    del graph, got
+    ctx.heap_release(mark)
+
+
 # ------------------------------------------------------------------------------------ attention on one rank
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("S,Hq,Hkv", [(1, 2, 2), (64, 4, 2), (127, 8, 2), (128, 3, 1), (129, 4, 4), (257, 6, 2), (384, 5, 5), (1000, 8, 8), (2500, 16, 2),
@@ -403,6 +514,29 @@ def test_decode_runs_cut_sequences_anywhere(ctx, tma, B, Hq, Hkv, page, lens):
         seen = kv[0] > 0
         assert (lse[seen] - want_lse[seen]).abs().max().item() < 1e-3 if bool(seen.any()) else True
         assert torch.isneginf(lse[~seen]).all() and (out[~seen] == 0).all()
+    ctx.heap_release(mark)
+
+
+@pytest.mark.parametrize("B,Hq,Hkv,L,places", [(1, 8, 1, 32768, 41), (2, 16, 1, 20000, 41), (3, 128, 1, 4096, 9), (5, 64, 1, 9000, 9)])
+def test_decode_fold_with_many_places(ctx, B, Hq, Hkv, L, places):
+    """More places than a pass of the fold takes: above 40 where four threads share a column (few heads), above 8 where one does (more heads than two per SM).
+    Bound as in the test above."""
+    from iris_b200.models import FlashDecodeLayer, reference_decode
+
+    g, page = _gen(B + L), 16
+    blocks = -(-L // page)
+    r = lambda *sh: torch.randn(*sh, device="cuda", generator=g).clamp(-6, 6).to(torch.bfloat16)  # noqa: E731
+    q, k, v = r(B, Hq, 128), r(B * blocks, page, Hkv, 128), r(B * blocks, page, Hkv, 128)
+    table = torch.randperm(B * blocks, device="cuda", generator=g).to(torch.int32).view(B, blocks)
+    kv = torch.full((1, B), L, dtype=torch.int32, device="cuda")
+    mark = ctx.heap_mark()
+    layer = FlashDecodeLayer(ctx, Hq, Hkv, max_batch=B)
+    out, lse = layer(q, k, v, kv, table, return_lse=True)
+    splits = layer.num_splits(B, blocks * page)
+    filled = ~torch.isneginf(layer.partial.view(-1)[:B * Hq * splits * 129].view(B * Hq, splits, 129)[:, :, 128])
+    assert filled.sum(dim=1).max().item() >= places and (B * Hq > 2 * ctx.get_cu_count()) == (places == 9)
+    want, want_lse = reference_decode(q, k, v, kv[0], table)
+    assert (out.float() - want).abs().max().item() <= 2 * 2.0 ** -8 * 6 and (lse - want_lse).abs().max().item() < 1e-3
     ctx.heap_release(mark)
 
 
