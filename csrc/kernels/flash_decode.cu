@@ -7,7 +7,7 @@
 //      partial output and its log-sum-exp per run. The tiles of all (sequence, KV head) pairs form one list that
 //      is cut into equal pieces, one per CTA, on the device, from the lengths: a CTA may end one pair and begin the next, a pair
 //      may be spread over many CTAs. (With the same number of splits for every sequence, the CTAs of the longest
-//      one finished last: 32 sequences of 8192 to 32768 positions, 640 us where the bytes take 404; now 423. One
+//      one finished last: 32 sequences of 8192 to 32768 positions, 640 us where the bytes take 404; now 427. One
 //      sequence of 32768: 512 CTAs on 296 places; 53 us, now 32.)
 //      K/V stream through a ring of swizzled shared-memory tiles; QK^T and PV run on tensor
 //      cores with the query heads of the group as the M dimension (each K/V byte is read from HBM
@@ -504,7 +504,8 @@ __global__ void __launch_bounds__(kWarps * 32, 2) decode_splitk_kernel(const __g
   }
 }
 
-// Folds the partial results of one (sequence, head) into (o, lse), thread d taking dimension d. All of the block's
+// Folds the partial results of one (sequence, head) into (o, lse), thread d taking dimension d, for the exchange across ranks and the entry
+// point that allocates nothing (one rank: decode_local_finish_kernel). All of the block's
 // threads call it; `s_w` is kD floats of shared memory. The weights are taken once, by a thread per place, and the loads
 // of eight places are in flight together (two serial passes over 64 places took most of 24 us).
 __device__ __forceinline__ void combine_splits(const float* p, int splits, float* s_w, float& o, float& lse) {

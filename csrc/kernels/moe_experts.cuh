@@ -14,7 +14,9 @@
 // quantisation block of H spans the pair: the CTAs exchange each token's largest magnitude by asynchronous stores into each
 // other's shared memory (a release at cluster scope waited for the warp's global stores of the tile before).
 // Stage 2 (down): every output row goes to the (token, k) slot it came from.
-// Whole layer, before (128-row token tiles on single CTAs) and now: 32 experts top-8 of 7168 x 2048, 64 tokens e4m3 316 and 239 us
+// Gate and up stay fp32 up to SwiGLU (the kernel of several ranks rounds e4m3's to bf16 first, and is the further one from 64 bits: 1.81e-2 and 1.64e-2 with
+// hidden values rounded once). The division is exact; a fast one, which returns 0 for denominators above 2^126, saves 1 to 4 % of a pass.
+// Whole layer, before (128-row token tiles on single CTAs) and now: 32 experts top-8 of 7168 x 2048, 64 tokens e4m3 316 and 241 us
 // (its weights' HBM time is 226), bf16 498 and 430; 4096 tokens bf16, the kernels alone, stage 1 1583 and 1320 us, stage 2 780 and 628.
 // 4096 tokens, 32 experts top-8 of 2048 x 1024: stage 1 bf16 218 and 184 us, e4m3 280 and 142 (336 with one shuffle and one 2-byte
 // store per value, four epilogue warps and full-precision divisions), stage 2 117 and 102, 119 and 79.

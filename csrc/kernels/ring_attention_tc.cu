@@ -26,7 +26,8 @@
 // An item's start and end cost about 9000 cycles each time, next to 3500 a pair of tiles: with its tiles counted in closed form instead of by walking
 // and the output stored by rows 554 -> 541 us, 3000 tokens 180 -> 176 (both under the power cap); three-operand maxima: by keys, 2304
 // tokens, 8 heads, causal 31.1 -> 29.2. A pair of tiles now (cycles, one tile's chain): load 150, maximum 410, exponentials 1350, P 190,
-// to the issuing warp 100, P V and S until the next softmax sees it 1290.
+// to the issuing warp 100, P V and S until the next softmax sees it 1290. Outside this chain remain about 20 k cycles an item (of 928 k cycles an SM 8192 tokens
+// spend 785 k in it, of 316 k 3000 tokens 251 k): the softmax warps rescale O early on, read it, scale and store it, and only then take the next item's scores.
 // Slower were: 64-key halves with S double-buffered (more MMAs to issue: 746), P released to the MMAs in halves (541 -> 572 under the power cap), part of the
 // exponentials as a polynomial on the FMA pipe (the softmax warps are short of issue slots).
 // The two tiles are two query heads of one K/V head group where the group is even (same keys, no work done twice or
