@@ -973,18 +973,21 @@ int make_plan(const IrisGemmDesc* d, Plan& p) {
   if (is_fp8(d)) {
     // block-scaled e4m3 tiles are 224 (or 128) wide: two accumulator buffers plus the scale cells fill TMEM.
     // CTA pairs on request, and for a local GEMM whose main loop is long enough for what a cluster costs at its ends: K of 4096 or more, where either
-    // few rows leave every tile to itself (the pair's ring is six stages deep, four otherwise) or the products are many (4e10).
-    // Single tiles / pairs, us back to back with weights that are not in L2, M x N:
-    //   K = 8192   16 x 1024  25.7 / 22.9    16 x 3584  26.3 / 23.1    1024 x 2048  26.9 / 25.1    2048 x 2048  42.2 / 42.3    4096 x 3584  110.8 / 108.7
-    //   K = 6144   16 x 3072  21.4 / 19.0    512 x 4096  21.1 / 19.5    1024 x 4096  33.1 / 33.0    3000 x 3072  56.8 / 57.2    4096 x 4096  97.4 / 94.0
-    //   K = 4096   16 x 1024  14.9 / 14.2    1024 x 2048  15.6 / 15.5    1536 x 3584  29.1 / 30.4    3000 x 1024  14.7 / 15.4    8192 x 5120  158 / 152
-    //   K = 2048   16 x 4096  11.9 / 12.4    512 x 8192  10.7 / 11.0    4096 x 4096  31.0 / 30.1
-    // At the lines: 1024 rows 0.99 to 1.10 times as fast with pairs, 1536 to 3000 rows below 4e10 products 0.96 to 1.03, 4e10 to 5e10 0.98 to 1.01.
-    // A single row with more than 24 column tiles loses up to 15 % (4096 x 8192: 16.0 / 18.6; 5120 columns 15.4 / 14.4): the reason is not known.
+    // few rows leave every tile to itself (the pair's ring is six stages deep, four otherwise) or the products are many (3e10), and where pairs need
+    // no more rounds of tiles than single CTAs (an odd number of 128-row tiles leaves half a pair idle: 1040 x 3584 is 144 tiles or 80 pairs,
+    // one round or two). Single tiles / pairs, us back to back with weights that are not in L2, M x N:
+    //   K = 8192   16 x 1024  25.7 / 22.9    16 x 3584  26.3 / 23.1    1024 x 3584  27.8 / 26.0    1040 x 3584  28.3 / 43.4    4096 x 3584  110.8 / 108.7
+    //   K = 6144   16 x 3072  21.4 / 19.0    512 x 4096  21.1 / 19.5   1024 x 4096  33.1 / 33.0    1200 x 5120  38.0 / 35.5    4096 x 4096  97.4 / 94.0
+    //   K = 4096   16 x 1024  14.9 / 14.2    1024 x 2048  15.6 / 15.5  1100 x 7168  29.3 / 37.3    3000 x 1024  14.7 / 15.4    8192 x 5120  158 / 152
+    //   K = 2048   16 x 4096  11.9 / 12.4    512 x 8192  10.7 / 11.0   4096 x 4096  31.0 / 30.1
+    // At the lines, with equal rounds: 1024 rows 0.99 to 1.10 times as fast with pairs, 1536 to 3000 rows below 3e10 products 0.96 to 1.02, 3e10 to 4e10
+    // 0.97 to 1.07. A single row with more than 24 column tiles loses up to 15 % (4096 x 8192: 16.0 / 18.6; 5120 columns 15.4 / 14.4): the reason is not known.
     if (d->bn != 0 && d->bn != 224 && d->bn != 128) return -5;
     const double weights = (double)d->N * d->K;
-    const bool lone_row = d->M == 1 && ceil_div(d->N, 224) > 24;
-    const bool long_loop = d->op == IRIS_GEMM_LOCAL && d->K >= 4096 && !lone_row && (d->M <= 1024 || weights * d->M >= 4e10);
+    const int cols = ceil_div(d->N, 224), slots = p.gemm_ctas;
+    const bool more_rounds = slots < 2 || ceil_div(ceil_div(tiles_m, 2) * cols, slots / 2) > ceil_div(tiles_m * cols, slots);
+    const bool lone_row = d->M == 1 && cols > 24;
+    const bool long_loop = d->op == IRIS_GEMM_LOCAL && d->K >= 4096 && !lone_row && !more_rounds && (d->M <= 1024 || weights * d->M >= 3e10);
     const bool pairs = d->two_sm == 2 || (d->two_sm == 0 && long_loop);
     choose_tile(d->M, d->N, p.gemm_ctas, d->bn == 128 ? 128 : 224, pairs ? 2 : 1, pair_ok && d->bn != 128, p.bn, p.pair);
   } else {

@@ -505,8 +505,8 @@ def test_gemm_plan_tile_choice():
 
 
 def test_gemm_plan_e4m3_pairs():
-    """Both sides of the rule that gives a block-scaled local GEMM CTA pairs: K of 4096, 1024 rows, 4e10 products, a single row with more than 24
-    column tiles; asked for and forbidden, narrow tiles, and never for the fused ops unless asked for."""
+    """Both sides of the rule that gives a block-scaled local GEMM CTA pairs: K of 4096, 1024 rows, 3e10 products, a single row with more than 24
+    column tiles, rounds of tiles; asked for and forbidden, narrow tiles, and never for the fused ops unless asked for."""
     import ctypes as C
 
     from iris_b200 import _lib
@@ -523,8 +523,13 @@ def test_gemm_plan_e4m3_pairs():
 
     assert pair(16, 1024, 4096) == 1 and pair(16, 1024, 4080) == 0
     assert pair(1024, 2048, 4096) == 1 and pair(1025, 2048, 4096) == 0
-    assert pair(4769, 2048, 4096) == 1 and pair(4768, 2048, 4096) == 0               # 4e10 / (2048 x 4096) = 4768.4
+    assert pair(3577, 2048, 4096) == 1 and pair(3576, 2048, 4096) == 0               # 3e10 / (2048 x 4096) = 3576.3
     assert pair(1, 5376, 4096) == 1 and pair(1, 5377, 4096) == 0 and pair(2, 5377, 4096) == 1
+    # never more rounds of tiles than single CTAs (148 of them or 74 pairs): 8 x 16 tiles are one round either way, 9 x 16 one or two, 10 x 16 two and two;
+    # 7 x 18 and 7 x 19, 5 x 24 and 5 x 25
+    assert pair(1024, 3584, 8192) == 1 and pair(1025, 3584, 8192) == 0 and pair(1152, 3584, 8192) == 0 and pair(1153, 3584, 8192) == 1
+    assert pair(896, 4032, 8192) == 1 and pair(896, 4033, 8192) == 0 and pair(897, 4033, 8192) == 1
+    assert pair(640, 5376, 4096) == 1 and pair(640, 5377, 4096) == 0 and pair(512, 5377, 4096) == 1
     assert pair(16, 223, 8192) == 0 and pair(16, 224, 8192) == 1                     # a pair's tile is 224 wide
     assert pair(16, 3584, 8192, two_sm=1) == 0 and pair(16, 3584, 1024, two_sm=2) == 1 and pair(16, 3584, 8192, bn=128) == 0
     assert pair(256, 3584, 8192, op=_lib.GEMM_AG_M) == 0 and pair(256, 3584, 8192, op=_lib.GEMM_AG_M, two_sm=2) == 1
